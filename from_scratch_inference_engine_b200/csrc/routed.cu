@@ -23,6 +23,7 @@
 namespace fsie {
 
 constexpr int MOE_TILE = 64;          // rows (and output columns) per tile of the tiled products
+constexpr int MOE_FEW_TILE = 16;      // rows per tile of the products that stream the experts' matrices
 
 // what a router's logits become: sigmoid, softmax over all experts, softmax over the chosen ones
 enum { SCORES_SIGMOID = 0, SCORES_SOFTMAX = 1, SCORES_CHOSEN_SOFTMAX = 2 };
@@ -440,6 +441,303 @@ __global__ void __launch_bounds__(128) moe_product_mma_kernel(
     }
 }
 
+// ------------------------------------------------ few rows per expert: the matrices streamed once
+// A decode step gives an expert one to a few rows, so the product is the time its matrices take to come
+// in.  The tiled kernel above waits for every 64 k-elements with one chunk asked for ahead and keeps 18 KB
+// per block on the way.  Here blocks stay (two of 256 threads per SM) and walk items of (tile of up to 16
+// rows, 32 rows of w - GATED: 16 of the gate and the same 16 of the up projection); the 8 warps of a block
+// take turns along k in chunks of 32, each lane asks for its own 16 bytes of four rows with cp.async into a
+// ring of its own (no barrier guards it), and the ring runs on into the next item while the current one is
+// summed up: 64 KB per block are on the way at any time.  What the next item needs besides - its expert, its
+// rows of x, their first values - is asked for before the current item's sums meet in shared memory (double-
+// buffered, one barrier per item).  The rows of x are the N side of mma.sync m16n8k16.
+constexpr int FEW_WARPS = 8, FEW_CHUNK = 32, FEW_AHEAD = 4, FEW_ROWS = 32;
+constexpr int FEW_SLOT = FEW_ROWS * FEW_CHUNK * 2;                           // bytes a warp asks for at once
+constexpr int FEW_RING = FEW_WARPS * FEW_AHEAD * FEW_SLOT;
+constexpr int FEW_PITCH = FEW_ROWS + 4;                                      // the sums' rows start in other banks
+constexpr int FEW_RED = FEW_WARPS * MOE_FEW_TILE * FEW_PITCH;                // floats per buffer
+constexpr size_t FEW_SMEM = FEW_RING + 2 * FEW_RED * sizeof(float);
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * FEW_WARPS, 2) moe_product_few_kernel(
+        const bf16* __restrict__ x, long long x_ld, const bf16* __restrict__ w, bf16* __restrict__ out,
+        long long out_ld, const int* __restrict__ offsets, const int* __restrict__ sorted,
+        const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ meta,
+        int top, int n, int k, int gate_kind) {
+    constexpr bool GATED = MODE == 1, FIRST = MODE != 0;
+    constexpr int COLS = GATED ? 16 : 32;                    // outputs per row and item
+    extern __shared__ __align__(16) unsigned char few_smem[];
+    float* const red = reinterpret_cast<float*>(few_smem + FEW_RING);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    grid_dependency_wait();
+    grid_dependents_go();
+    const int tiles = meta[0];
+    // neighbouring items are the tiles of the same columns: an expert's further tiles find its rows in L2
+    const int items = tiles * ((n + COLS - 1) / COLS);
+    if ((int)blockIdx.x >= items) return;
+    const int chunks = k / FEW_CHUNK, per = (chunks + FEW_WARPS - 1) / FEW_WARPS;      // a warp's slots per item
+    const int step_tile = gridDim.x % tiles, step_n0 = (gridDim.x / tiles) * COLS;
+    auto advance = [&](int& tile, int& n0) {                 // the block's next item
+        tile += step_tile;
+        n0 += step_n0;
+        if (tile >= tiles) { tile -= tiles; n0 += COLS; }
+    };
+    unsigned char* const mine = few_smem + (size_t)warp * FEW_AHEAD * FEW_SLOT + lane * 16;
+
+    int ask_tile = blockIdx.x % tiles, ask_n0 = (blockIdx.x / tiles) * COLS, ask_j = 0, ask_slot = 0;
+    const bf16* wr[4];
+    auto point = [&]() {                                     // this lane's four rows of w of the item asked for
+        if (ask_n0 >= n) return;
+        const bf16* we = w + (size_t)tile_expert[ask_tile] * (GATED ? 2 : 1) * n * k + 8 * t;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = GATED ? (i >> 1) * n + min(ask_n0 + g + 8 * (i & 1), n - 1) : min(ask_n0 + g + 8 * i, n - 1);
+            wr[i] = we + (size_t)row * k;
+        }
+    };
+    auto ask = [&]() {
+        const int c = warp + ask_j * FEW_WARPS;
+        if (ask_n0 < n && c < chunks) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mm_cp16(mine + ask_slot * FEW_SLOT + i * 512, wr[i] + c * FEW_CHUNK, true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");            // one group per slot, also when empty
+        ask_slot = ask_slot + 1 == FEW_AHEAD ? 0 : ask_slot + 1;
+        if (++ask_j == per) {
+            ask_j = 0;
+            advance(ask_tile, ask_n0);
+            point();
+        }
+    };
+    point();
+#pragma unroll
+    for (int j = 0; j < FEW_AHEAD; ++j) ask();
+
+    int tile = blockIdx.x % tiles, n0 = (blockIdx.x / tiles) * COLS, r0 = 0, rows = 0, slot = 0, buffer = 0;
+    const bf16* xr[2];
+    auto open = [&](int of) {                                // the tile's rows of x
+        r0 = tile_row0[of];
+        rows = min(MOE_FEW_TILE, offsets[tile_expert[of] + 1] - r0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = g + 8 * h;
+            xr[h] = r < rows ? x + (size_t)(FIRST ? sorted[r0 + r] / top : r0 + r) * x_ld + 8 * t : nullptr;
+        }
+    };
+    uint4 b[4][2];
+    auto load_x = [&](int j0) {                              // the rows' values of four chunks are asked for together
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = warp + (j0 + u) * FEW_WARPS;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                b[u][h] = (c < chunks && xr[h]) ? *reinterpret_cast<const uint4*>(xr[h] + c * FEW_CHUNK) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    open(tile);
+    load_x(0);
+    for (;;) {
+        float acc[2][2][4];                                  // [rows of w 0-15, 16-31][rows of x 0-7, 8-15]
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[i >> 1][i & 1][v] = 0.f;
+        for (int j0 = 0; j0 < per; j0 += 4) {
+            if (j0) load_x(j0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (j0 + u >= per) break;
+                asm volatile("cp.async.wait_group %0;" ::"n"(FEW_AHEAD - 1) : "memory");      // the oldest slot has landed
+                if (warp + (j0 + u) * FEW_WARPS < chunks) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const uint4 lo = *reinterpret_cast<const uint4*>(mine + slot * FEW_SLOT + i * 1024);
+                        const uint4 hi = *reinterpret_cast<const uint4*>(mine + slot * FEW_SLOT + i * 1024 + 512);
+                        const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+                        mm_mma(acc[i][0], a0, b[u][0].x, b[u][0].y);
+                        mm_mma(acc[i][0], a1, b[u][0].z, b[u][0].w);
+                        if (rows > 8) {
+                            mm_mma(acc[i][1], a0, b[u][1].x, b[u][1].y);
+                            mm_mma(acc[i][1], a1, b[u][1].z, b[u][1].w);
+                        }
+                    }
+                }
+                slot = slot + 1 == FEW_AHEAD ? 0 : slot + 1;
+                ask();
+            }
+        }
+        // acc[i][h]: rows g (0, 1) and g + 8 (2, 3) of w, rows 8 h + 2 t and 8 h + 2 t + 1 of x
+        float* const sums = red + buffer * FEW_RED;          // [warp][row of x][32 rows of w]
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (8 * h >= rows) break;
+            float* at = sums + ((size_t)warp * MOE_FEW_TILE + 8 * h + 2 * t) * FEW_PITCH + g;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                at[16 * i] = acc[i][h][0];
+                at[16 * i + FEW_PITCH] = acc[i][h][1];
+                at[16 * i + 8] = acc[i][h][2];
+                at[16 * i + 8 + FEW_PITCH] = acc[i][h][3];
+            }
+        }
+        const int done_n0 = n0, done_r0 = r0, done_rows = rows;
+        advance(tile, n0);
+        if (n0 < n) {
+            open(tile);
+            load_x(0);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < done_rows * COLS; e += 32 * FEW_WARPS) {
+            const int r = e / COLS, c = e - r * COLS;        // consecutive threads: consecutive columns of a row
+            float lo = 0.f, hi = 0.f;
+#pragma unroll
+            for (int v = 0; v < FEW_WARPS; ++v) {
+                lo += sums[(v * MOE_FEW_TILE + r) * FEW_PITCH + c];
+                if (GATED) hi += sums[(v * MOE_FEW_TILE + r) * FEW_PITCH + c + 16];
+            }
+            if (done_n0 + c >= n) continue;
+            lo = __bfloat162float(__float2bfloat16_rn(lo));  // as a product that stored it in between would have
+            if (GATED) lo = gate_fn(lo, gate_kind) * __bfloat162float(__float2bfloat16_rn(hi));
+            else if (MODE == 2) lo = gate_fn(lo, gate_kind);
+            const int to = FIRST ? done_r0 + r : sorted[done_r0 + r];
+            out[(size_t)to * out_ld + done_n0 + c] = __float2bfloat16_rn(lo);
+        }
+        if (n0 >= n) break;
+        buffer ^= 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// The same in 32 bits: a warp owns two rows of w (GATED: a gate row and its up row), its lanes lie side by side
+// along k, the rows of w of the next three passes of 128 elements are on their way into registers, and
+// the tile's rows of x wait in shared memory, where every value read serves both rows of w.  8 tokens x 6 of 64
+// experts of 1,408 x 2,048: 164 + 92 us (floor 124 + 62; the tiled kernel 1,220 + 596: its blocks multiply 64 rows
+// whatever the tile holds).
+constexpr int FEW32_WARPS = 8, FEW32_XC = 512, FEW32_DEPTH = 4;
+constexpr size_t FEW32_SMEM = 2 * MOE_FEW_TILE * FEW32_XC * sizeof(float);
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * FEW32_WARPS, 2) moe_product_few_f32_kernel(
+        const float* __restrict__ x, long long x_ld, const float* __restrict__ w, float* __restrict__ out,
+        long long out_ld, const int* __restrict__ offsets, const int* __restrict__ sorted,
+        const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ meta,
+        int top, int n, int k, int gate_kind) {
+    constexpr bool GATED = MODE == 1, FIRST = MODE != 0;
+    constexpr int PER_CHUNK = FEW32_XC / 128, D = FEW32_DEPTH;
+    extern __shared__ __align__(16) float few32_smem[];
+    float (*xs)[MOE_FEW_TILE][FEW32_XC] = reinterpret_cast<float (*)[MOE_FEW_TILE][FEW32_XC]>(few32_smem);
+    __shared__ int src[MOE_FEW_TILE], dst[MOE_FEW_TILE];
+    grid_dependency_wait();
+    grid_dependents_go();
+    const int tile = blockIdx.x;
+    if (tile >= meta[0]) return;
+    const int e = tile_expert[tile], r0 = tile_row0[tile], rows = min(MOE_FEW_TILE, offsets[e + 1] - r0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < rows) {
+        const int pair = sorted[r0 + tid];
+        src[tid] = FIRST ? pair / top : r0 + tid;
+        dst[tid] = FIRST ? r0 + tid : pair;
+    }
+    const int c0 = (blockIdx.y * FEW32_WARPS + warp) * (GATED ? 1 : 2);
+    const float* we = w + (size_t)e * (GATED ? 2 : 1) * n * k + lane * 4;
+    const int row0 = min(c0, n - 1);
+    const float* wrow[2] = {we + (size_t)row0 * k, we + (size_t)(GATED ? n + row0 : min(c0 + 1, n - 1)) * k};
+    const int passes = (k + 127) / 128;
+    float4 ring[D][2];
+    auto load_w = [&](int pass, float4 (&to)[2]) {
+        const bool in_range = pass < passes && pass * 128 + lane * 4 < k;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            to[r] = in_range ? __ldg(reinterpret_cast<const float4*>(wrow[r] + pass * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+#pragma unroll
+    for (int d = 0; d < D - 1; ++d) load_w(d, ring[d]);
+    __syncthreads();
+    auto stage_x = [&](int chunk) {
+        const int k0 = chunk * FEW32_XC;
+        for (int i = tid; i < rows * (FEW32_XC / 4); i += 32 * FEW32_WARPS) {
+            const int m = i / (FEW32_XC / 4), c = (i - m * (FEW32_XC / 4)) * 4;
+            const bool in = k0 + c < k;
+            mm_cp16(&xs[chunk & 1][m][c], x + (in ? (size_t)src[m] * x_ld + k0 + c : 0), in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage_x(0);
+    float acc[2][MOE_FEW_TILE];
+#pragma unroll
+    for (int m = 0; m < MOE_FEW_TILE; ++m) acc[0][m] = acc[1][m] = 0.f;
+    for (int base = 0; base < passes; base += D) {
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+            const int pass = base + u;
+            load_w(pass + D - 1, ring[(u + D - 1) % D]);
+            if (pass >= passes) continue;
+            const int chunk = pass / PER_CHUNK, within = pass - chunk * PER_CHUNK;
+            if (within == 0) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncthreads();              // this chunk's x has landed, the other half is no longer read
+                if ((chunk + 1) * FEW32_XC < k) stage_x(chunk + 1);
+            }
+            const float* xrow = &xs[chunk & 1][0][within * 128 + lane * 4];
+#pragma unroll
+            for (int m = 0; m < MOE_FEW_TILE; ++m) {
+                if (m >= rows) break;
+                const float4 xv = *reinterpret_cast<const float4*>(xrow + m * FEW32_XC);
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+                    acc[r][m] = fmaf(xv.w, ring[u][r].w, fmaf(xv.z, ring[u][r].z,
+                                fmaf(xv.y, ring[u][r].y, fmaf(xv.x, ring[u][r].x, acc[r][m]))));
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MOE_FEW_TILE; ++m) {
+        if (m >= rows) break;
+        const float lo = warp_sum(acc[0][m]), hi = warp_sum(acc[1][m]);
+        float* o = out + (size_t)dst[m] * out_ld + c0;
+        if (lane != 0 || c0 >= n) continue;
+        if (GATED) {
+            o[0] = gate_fn(lo, gate_kind) * hi;
+        } else {
+            o[0] = MODE == 2 ? gate_fn(lo, gate_kind) : lo;
+            if (c0 + 1 < n) o[1] = MODE == 2 ? gate_fn(hi, gate_kind) : hi;
+        }
+    }
+}
+
+template <typename F>
+static int allow_smem(F* kernel, size_t bytes, bool& done) {
+    if (done) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done = true;
+    return (int)e;
+}
+
+template <int MODE>
+static int launch_few(const void* x, long long x_ld, const void* w, void* out, long long out_ld, const int* offsets,
+                      const int* sorted, const int* tile_expert, const int* tile_row0, const int* meta, int tiles,
+                      int top, int n, int k, int gate_kind, int dtype, cudaStream_t stream) {
+    static bool allowed[2] = {false, false};
+    if (dtype == DTYPE_F32) {
+        if (int e = allow_smem(moe_product_few_f32_kernel<MODE>, FEW32_SMEM, allowed[0])) return e;
+        const int cols = FEW32_WARPS * (MODE == 1 ? 1 : 2);
+        const dim3 grid(tiles, (n + cols - 1) / cols);
+        if (grid.y > 65535) return ERR_UNSUPPORTED;
+        return launch_dependent(moe_product_few_f32_kernel<MODE>, grid, dim3(32 * FEW32_WARPS), FEW32_SMEM, stream,
+                                (const float*)x, x_ld, (const float*)w, (float*)out, out_ld, offsets, sorted,
+                                tile_expert, tile_row0, meta, top, n, k, gate_kind);
+    }
+    if (int e = allow_smem(moe_product_few_kernel<MODE>, FEW_SMEM, allowed[1])) return e;
+    int device = 0, sms = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int cols = MODE == 1 ? FEW_ROWS / 2 : FEW_ROWS;
+    const long long most = (long long)tiles * ((n + cols - 1) / cols);
+    return launch_dependent(moe_product_few_kernel<MODE>, dim3((unsigned)(most < 2 * sms ? most : 2 * sms)),
+                            dim3(32 * FEW_WARPS), FEW_SMEM, stream, (const bf16*)x, x_ld, (const bf16*)w, (bf16*)out,
+                            out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind);
+}
+
 // -------------------------------------------------------------------------------- combine
 template <typename T, bool VEC>
 __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float* __restrict__ weights,
@@ -495,6 +793,7 @@ using namespace fsie;
 extern "C" {
 
 int fsie_moe_tile_rows() { return MOE_TILE; }
+int fsie_moe_few_tile_rows() { return MOE_FEW_TILE; }
 
 // y [tokens, y_ld] of the storage type; w_router float32 [experts, width]; bias and correction float32
 // [experts] or null; ids int32 / weights float32 [tokens, top].
@@ -530,7 +829,7 @@ int fsie_moe_route(const void* y, int y_ld, const float* w_router, const float* 
 int fsie_moe_align(const int* ids, int pairs, int experts, int tile, int padded, int* offsets, int* sorted,
                    int* tile_expert, int* tile_row0, int* meta, int* place, cudaStream_t stream) {
     if (pairs <= 0) return 0;
-    if (experts <= 0 || tile <= 0 || (!padded && tile != MOE_TILE)) return ERR_BAD_ARGUMENT;
+    if (experts <= 0 || tile <= 0 || (!padded && tile != MOE_TILE && tile != MOE_FEW_TILE)) return ERR_BAD_ARGUMENT;
     const size_t smem = (3 * (size_t)experts + 2) * sizeof(int);
     if (smem > 40 * 1024) return ERR_UNSUPPORTED;
     const int threads = pairs >= 4096 ? 1024 : (pairs >= 512 ? 256 : 64);
@@ -551,13 +850,25 @@ int fsie_moe_gather(const void* x, long long x_ld, const int* sorted, const int*
 // gated = 1: x [tokens, x_ld] read at pair / top, w [experts, 2 n, k] (gate rows, then up rows), out
 // [pairs, out_ld] in sorted order.  gated = 2: the same rows in and out, w [experts, n, k], out = f(x w^T)
 // (an expert without a gate: gate_kind names f).  gated = 0: x [pairs, x_ld] in sorted order, w [experts, n, k], out
-// written at the pair's own row.
+// written at the pair's own row.  `tile`: the rows per tile that the lists were made with; MOE_FEW_TILE takes
+// the kernels that stream the matrices (k a multiple of 32 in bfloat16 and of 4 in float32, rows on 16 bytes).
 int fsie_moe_product(const void* x, long long x_ld, const void* w, void* out, long long out_ld,
                      const int* offsets, const int* sorted, const int* tile_expert, const int* tile_row0,
                      const int* meta, int pairs, int experts, int top, int n, int k, int gated, int gate_kind,
-                     int dtype, cudaStream_t stream) {
+                     int dtype, int tile, cudaStream_t stream) {
     if (pairs <= 0 || n <= 0) return 0;
     if (k <= 0 || experts <= 0 || top <= 0 || gated < 0 || gated > 2) return ERR_BAD_ARGUMENT;
+    if (tile == MOE_FEW_TILE) {
+        const int step = dtype == DTYPE_F32 ? 4 : 8;                 // elements in 16 bytes
+        if (k % (dtype == DTYPE_F32 ? 4 : FEW_CHUNK) || x_ld % step || ((((size_t)x) | ((size_t)w)) & 15))
+            return ERR_BAD_ARGUMENT;
+#define FSIE_MOE_FEW(M)                                                                                           \
+        launch_few<M>(x, x_ld, w, out, out_ld, offsets, sorted, tile_expert, tile_row0, meta, pairs / tile + experts, \
+                      top, n, k, gate_kind, dtype, stream)
+        return gated == 1 ? FSIE_MOE_FEW(1) : (gated == 2 ? FSIE_MOE_FEW(2) : FSIE_MOE_FEW(0));
+#undef FSIE_MOE_FEW
+    }
+    if (tile != MOE_TILE) return ERR_BAD_ARGUMENT;
     const int cols = gated == 1 ? MOE_TILE / 2 : MOE_TILE;
     const dim3 grid(pairs / MOE_TILE + experts, (n + cols - 1) / cols);
     if (grid.y > 65535) return ERR_UNSUPPORTED;

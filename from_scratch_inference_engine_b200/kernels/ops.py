@@ -1780,13 +1780,14 @@ def routed():
         lib = build.load_library("routed")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_moe_tile_rows.argtypes = []
+        lib.fsie_moe_few_tile_rows.argtypes = []
         lib.fsie_moe_route.argtypes = [p, i, p, p, p, p, p, p, i, i, i, i, i, i, f, i, i, i, i, p]
         lib.fsie_moe_align.argtypes = [p, i, i, i, i, p, p, p, p, p, p, p]
         lib.fsie_moe_gather.argtypes = [p, ll, p, p, i, i, p, i, i, p]
-        lib.fsie_moe_product.argtypes = [p, ll, p, p, ll, p, p, p, p, p, i, i, i, i, i, i, i, i, p]
+        lib.fsie_moe_product.argtypes = [p, ll, p, p, ll, p, p, p, p, p, i, i, i, i, i, i, i, i, i, p]
         lib.fsie_moe_combine.argtypes = [p, p, p, p, p, i, i, i, p, i, p, ll, i, p]
-        for name in ("fsie_moe_tile_rows", "fsie_moe_route", "fsie_moe_align", "fsie_moe_gather", "fsie_moe_product",
-                     "fsie_moe_combine"):
+        for name in ("fsie_moe_tile_rows", "fsie_moe_few_tile_rows", "fsie_moe_route", "fsie_moe_align",
+                     "fsie_moe_gather", "fsie_moe_product", "fsie_moe_combine"):
             getattr(lib, name).restype = i
         _routed = lib
     return _routed
@@ -1882,6 +1883,18 @@ def moe_tile_rows() -> int:
     return routed().fsie_moe_tile_rows()
 
 
+def moe_few_tile_rows() -> int:
+    """Rows per tile of lists for the products that stream the experts' matrices."""
+    return routed().fsie_moe_few_tile_rows()
+
+
+def moe_few_fits(x: torch.Tensor, hidden: int, inner: int) -> bool:
+    """Whether those products take rows like x's and experts of these sizes (any row on 16 bytes, in
+    bfloat16 whole chunks of 32 elements along k)."""
+    step, chunk = (4, 4) if x.dtype is torch.float32 else (8, 32)
+    return hidden % chunk == 0 and inner % chunk == 0 and x.stride(0) % step == 0 and x.data_ptr() % 16 == 0
+
+
 def moe_route(y: Optional[torch.Tensor], w_router: Optional[torch.Tensor], correction: Optional[torch.Tensor],
               ids: torch.Tensor, weights: torch.Tensor, top: int, groups: int, keep: int, scale: float,
               scores: str = "sigmoid", normalise: bool = True, logits: Optional[torch.Tensor] = None,
@@ -1970,8 +1983,8 @@ def moe_gather(x: torch.Tensor, lists, tile: int, top: int, out: torch.Tensor) -
 
 
 def moe_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, lists, pairs: int, top: int,
-                gated: bool, activation: str = "silu", first: Optional[bool] = None) -> torch.Tensor:
-    """The experts' products over the sorted pairs.  gated: weight [experts, 2 n, k] (gate rows, then up
+                gated: bool, activation: str = "silu", first: Optional[bool] = None, tile: int = 0) -> torch.Tensor:
+    """The experts' products over the sorted pairs (`tile`: what the lists were made with).  gated: weight [experts, 2 n, k] (gate rows, then up
     rows), x [tokens, k] read at pair // top, out [pairs, n] = f(gate) * up in sorted order.  Not gated:
     weight [experts, n, k], x [pairs, k] in sorted order, out [pairs, n] at each pair's own row - or,
     `first` (an expert without a gate: its first product), x [tokens, k] read at pair // top and
@@ -1989,7 +2002,8 @@ def moe_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, lists,
     _check(routed().fsie_moe_product(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), out.stride(0),
                                      _ptr(offsets), _ptr(order), _ptr(tile_expert), _ptr(tile_row0),
                                      _ptr(meta), pairs, experts, int(top), n, k, mode,
-                                     GATE_KINDS[activation], _tag(x.dtype), _stream()), "moe_product")
+                                     GATE_KINDS[activation], _tag(x.dtype), int(tile) or moe_tile_rows(),
+                                     _stream()), "moe_product")
     return out
 
 

@@ -33,14 +33,20 @@ class RoutedExperts(Part):
     All experts' matrices are stacked at bind ([experts, 2 ff, width] gate rows then up rows;
     [experts, width, ff]).  The router's logits are a product with a 32-bit result.  A step sorts
     its (token, choice) pairs by expert on the device and runs the two products over tiles of rows
-    that share an expert, so it launches the same kernels whatever the router says: tiles of 64
-    rows through the mma.sync / FFMA kernels, or - bfloat16 steps with at least `GROUPED_MIN_ROWS`
+    that share an expert, so it launches the same kernels whatever the router says: tiles of 16
+    rows through kernels that stream the experts' matrices while an expert meets few rows on average
+    (`FEW_MAX_ROWS`), tiles of 64 through the mma.sync / FFMA kernels beyond that, or - bfloat16 steps with at least `GROUPED_MIN_ROWS`
     rows per expert on average - the tokens' rows gathered into a layout in which every expert's
     rows start on a multiple of 256, and the grouped form of the tiled tcgen05 product (SwiGLU in
     its epilogue) over it.  `names` gives the tensor names below the prefix ("expert" takes the
     expert's index).
     """
 
+    # Average rows per expert up to which the products that stream the matrices are taken.  Measured on 64
+    # experts of 1,408 x 2,048 (both products, us, streaming / tiled): bfloat16 at 6 rows 236 / 314, at 16 297 /
+    # 342, at 24 376 / 369; float32 at 6 rows 631 / 2,964, at 24 1,757 / 2,968 - there the streaming kernel's
+    # time grows by about 65 us a row and meets the tiled one's at about 40.
+    FEW_MAX_ROWS = {torch.bfloat16: 20, torch.float32: 32}
     GROUPED_MIN_ROWS = 32       # average rows per expert from which the tcgen05 form is taken
 
     NAMES = {"expert": "e{index}.", "gate": "gate", "up": "up", "down": "down", "router": "router",
@@ -165,11 +171,15 @@ class RoutedExperts(Part):
             expert_out = rt.buffer("routed.expert_out", rows, self.hidden_size, y.dtype)
             ops.gemm_tiles_grouped(down, act, expert_out, lists[2], lists[4], ctx.error, rt.sm_count)
             return ops.moe_combine(expert_out, weights, shared, out, top, place=lists[5], **identity)
+        few = (pairs <= self.FEW_MAX_ROWS[y.dtype] * self.experts
+               and ops.moe_few_fits(y, self.hidden_size, self.intermediate_size))
+        tile = ops.moe_few_tile_rows() if few else ops.moe_tile_rows()
         lists = ops.moe_align(ids, pairs, self.experts,
-                              rt.buffer("routed.lists", 1, ops.moe_lists_size(pairs, self.experts),
-                                        torch.int32).view(-1))
+                              rt.buffer("routed.lists", 1, ops.moe_lists_size(pairs, self.experts, tile),
+                                        torch.int32).view(-1), tile)
         act = rt.buffer("routed.act", pairs, self.intermediate_size, y.dtype)
-        ops.moe_product(y, self.w_gate_up, act, lists, pairs, top, self.gated, self.activation, first=True)
+        ops.moe_product(y, self.w_gate_up, act, lists, pairs, top, self.gated, self.activation, first=True,
+                        tile=tile)
         expert_out = rt.buffer("routed.expert_out", pairs, self.hidden_size, y.dtype)
-        ops.moe_product(act, self.w_down, expert_out, lists, pairs, top, False)
+        ops.moe_product(act, self.w_down, expert_out, lists, pairs, top, False, tile=tile)
         return ops.moe_combine(expert_out, weights, shared, out, top, **identity)
