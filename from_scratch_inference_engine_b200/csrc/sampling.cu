@@ -6,8 +6,8 @@
 // softmax(logit / temperature), cut to the shortest prefix whose mass reaches top_p
 // (>= 1 = all), and the token is found by walking that prefix until the running mass
 // reaches u * (mass of the prefix).  The reference sorts the whole vocabulary on the
-// host; here nothing is sorted.  "The running mass over tokens in descending order
-// reaches a target" is answered by a search over the 32 bits of an order-preserving
+// host; here at most a short list is: the kept tokens of a small top_k.  Otherwise "the running mass over
+// tokens in descending order reaches a target" is answered by a search over the 32 bits of an order-preserving
 // integer key of the logit: each of the 32 rounds measures the mass (or the count) of
 // all tokens whose key is at least a candidate, with a block reduction in a fixed
 // order.  Tokens with equal logits are ordered by ascending index.  The uniform number
@@ -295,6 +295,154 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     if (threadIdx.x == 0) out[rix] = choice < 0 ? 0 : choice;
 }
 
+namespace cg = cooperative_groups;
+constexpr int CLUSTER = 8;                // blocks that share a row
+
+// ------------------------------------------------------------------ a short top-k
+// With a top_k of at most SHORT_TOP_K the kept tokens are so few that they can be sorted.  A cluster of
+// CLUSTER blocks holds the row in registers.  Every block finds a key that at least k (and few more) of its
+// threads' largest keys reach: its k largest tokens are at or above it, so the tokens that reach it go to
+// block 0, which sorts them by (key, index) and walks the sorted weights.  One pass over the row and two
+// cluster barriers, where the searches below take a barrier for each of up to 48 rounds: 151,936 logits,
+// top_k 40 and top_p 0.95 took 259 us for one row and 333 us for 24 with the searches alone, 21 us here.
+// Rows it does not settle get -2 and are left to the kernel that follows: top_k outside 1 .. SHORT_TOP_K,
+// more than SHORT_CANDIDATES tokens (many equal logits), infinite or NaN weights.
+constexpr int SHORT_TOP_K = 104, SHORT_CANDIDATES = 1024, SHORT_PER_THREAD = 25;
+
+__device__ __forceinline__ float key_value(unsigned key) {
+    return __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key);
+}
+
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS)
+sample_short_kernel(const float* __restrict__ logits, int vocab, int slice, const float* __restrict__ temperature,
+                    const int* __restrict__ top_k, const float* __restrict__ top_p,
+                    const float* __restrict__ uniform, int* __restrict__ out) {
+    __shared__ unsigned long long tokens[SHORT_CANDIDATES];    // in block 0: the candidates, (key, ~index)
+    __shared__ unsigned filled;                                // in block 0: how many the blocks have brought
+    __shared__ unsigned here, base;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), rix = blockIdx.y;
+    grid_dependency_wait();
+    grid_dependents_go();
+    const float temp = temperature[rix];
+    const int k = top_k[rix];
+    if (!(temp > 0.f) || k <= 0 || k > SHORT_TOP_K || k >= vocab) {      // uniform over the cluster
+        if (rank == 0 && threadIdx.x == 0) out[rix] = temp > 0.f ? -2 : -1;
+        return;
+    }
+    const int first = rank * slice, count = max(0, min(slice, vocab - first));
+    const float* row = logits + (size_t)rix * vocab + first;
+    unsigned keys[SHORT_PER_THREAD], largest = 0;
+#pragma unroll
+    for (int j = 0; j < SHORT_PER_THREAD; ++j) {
+        const int i = j * SAMPLE_THREADS + threadIdx.x;
+        keys[j] = i < count ? order_key(row[i]) : 0u;
+        largest = max(largest, keys[j]);
+    }
+    if (threadIdx.x == 0) { filled = 0; here = 0; }
+    unsigned floor_key = 0;
+    for (int bit = 31; bit >= 0; --bit) {
+        const unsigned candidate = floor_key | (1u << bit);
+        const int reached = __syncthreads_count(largest >= candidate);
+        if (reached >= k) {
+            floor_key = candidate;
+            if (reached <= k + k / 8) break;
+        }
+    }
+    cluster.sync();                                            // block 0's counter is set
+    auto reaches = [&](int j) { return j * SAMPLE_THREADS + (int)threadIdx.x < count && keys[j] >= floor_key; };
+    unsigned mine = 0, at = 0;
+#pragma unroll
+    for (int j = 0; j < SHORT_PER_THREAD; ++j) mine += reaches(j);
+    if (mine) at = atomicAdd(&here, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) base = atomicAdd(cluster.map_shared_rank(&filled, 0), here);
+    __syncthreads();
+    if (mine && base + at + mine <= SHORT_CANDIDATES) {        // places differ from run to run, the sorted list does not
+        unsigned long long* to = cluster.map_shared_rank(tokens, 0) + base + at;
+#pragma unroll
+        for (int j = 0; j < SHORT_PER_THREAD; ++j)
+            if (reaches(j))
+                *to++ = ((unsigned long long)keys[j] << 32) | ~(unsigned)(first + j * SAMPLE_THREADS + threadIdx.x);
+    }
+    cluster.sync();
+    if (rank != 0) return;
+    const int n = (int)filled, t = threadIdx.x;
+    if (n > SHORT_CANDIDATES) {
+        if (t == 0) out[rix] = -2;
+        return;
+    }
+    // ---- bitonic sort, largest first: equal logits by rising index
+    int size_all = 32;
+    while (size_all < n) size_all *= 2;
+    unsigned long long v = t < n ? tokens[t] : 0ull;
+    for (int size = 2; size <= size_all; size *= 2)
+        for (int stride = size / 2; stride > 0; stride /= 2) {
+            unsigned long long other;
+            if (stride >= 32) {
+                __syncthreads();
+                tokens[t] = v;
+                __syncthreads();
+                other = tokens[t ^ stride];
+            } else {
+                other = __shfl_xor_sync(0xffffffffu, v, stride);
+            }
+            const bool keep_larger = ((t & size) == 0) == ((t & stride) == 0);
+            v = keep_larger == (other > v) ? other : v;
+        }
+    __syncthreads();
+    tokens[t] = v;
+    __syncthreads();
+    if (t >= 32) return;
+    // ---- running weights of the k first: four per lane
+    constexpr int EACH = (SHORT_TOP_K + 31) / 32;
+    const unsigned top_key = (unsigned)(tokens[0] >> 32), last_key = (unsigned)(tokens[k - 1] >> 32);
+    const float maxl = key_value(top_key), inv_temp = 1.0f / temp;
+    float running[EACH], sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < EACH; ++e) {
+        const int i = t * EACH + e;
+        if (i < k) sum += expf((key_value((unsigned)(tokens[i] >> 32)) - maxl) * inv_temp);
+        running[e] = sum;
+    }
+    float upto = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+        const float up = __shfl_up_sync(0xffffffffu, upto, o);
+        if (t >= o) upto += up;
+    }
+    const float below = __shfl_up_sync(0xffffffffu, upto, 1);
+#pragma unroll
+    for (int e = 0; e < EACH; ++e) running[e] = t == 0 ? running[e] : below + running[e];
+    const float total = __shfl_sync(0xffffffffu, running[EACH - 1], 31);     // of all k: the others add nothing
+    // the first token whose running weight reaches a target (-1: none), and that weight
+    auto locate_sorted = [&](float target, float& weight) {
+        int found = 0x7fffffff;
+        float w = 0.f;
+#pragma unroll
+        for (int e = EACH - 1; e >= 0; --e)
+            if (t * EACH + e < k && running[e] >= target) { found = t * EACH + e; w = running[e]; }
+        const unsigned lanes = __ballot_sync(0xffffffffu, found != 0x7fffffff);
+        if (!lanes) return -1;
+        const int lane = __ffs(lanes) - 1;
+        weight = __shfl_sync(0xffffffffu, w, lane);
+        return __shfl_sync(0xffffffffu, found, lane);
+    };
+    // +-inf at the top, NaN (key 0) among the kept or a temperature whose inverse overflows: the general search
+    const bool finite = top_key < 0xff800000u && top_key > 0x007fffffu && last_key != 0u && inv_temp < INFINITY;
+    float nucleus = total;
+    int choice = 0;
+    if (finite) {
+        const float pp = top_p[rix];
+        if (pp < 1.0f && locate_sorted(pp * total, nucleus) < 0) choice = -1;
+        if (choice >= 0) {
+            float unused;
+            choice = locate_sorted(uniform[rix] * nucleus, unused);
+        }
+    }
+    if (t == 0) out[rix] = finite && choice >= 0 ? (int)~(unsigned)tokens[choice] : -2;
+}
+
 // ------------------------------------------------------------------ cluster version
 // The same choice with a cluster of CLUSTER blocks per row (thread-block clusters,
 // distributed shared memory).  Each block keeps its slice of the row in shared memory as
@@ -302,8 +450,6 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
 // memory only; the blocks' partial sums meet through distributed shared memory, summed in
 // rank order (the same bits on every run).  Rows then take microseconds per round instead
 // of a pass over global memory by a single block.
-namespace cg = cooperative_groups;
-constexpr int CLUSTER = 8;
 
 struct ClusterRow {
     const unsigned* keys; const float* w; int count;    // this block's slice
@@ -420,6 +566,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int vocab, int slice,
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int rix = blockIdx.y;
+    grid_dependency_wait();
+    if (out[rix] != -2) return;                  // settled; uniform over the cluster: nothing is written before a sync
     const float temp = temperature[rix];
     if (!(temp > 0.f)) {                         // uniform over the cluster: no sync is skipped
         if (rank == 0 && threadIdx.x == 0) out[rix] = -1;
@@ -557,7 +705,8 @@ int fsie_sample(const float* logits, int rows, int vocab, const float* temperatu
                 cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0) return fsie::ERR_BAD_ARGUMENT;
-    // a cluster of 8 blocks per row while a slice of the row fits in shared memory
+    // a cluster of 8 blocks per row while a slice of the row fits in shared memory (and in registers)
+    static_assert(200 * 1024 / 8 <= fsie::SHORT_PER_THREAD * fsie::SAMPLE_THREADS, "a slice in registers");
     const int slice = ((vocab + fsie::CLUSTER - 1) / fsie::CLUSTER + 3) / 4 * 4;
     const size_t smem = (size_t)slice * 8;
     if (vocab >= 4096 && smem <= 200 * 1024 && rows <= 65535) {
@@ -568,9 +717,13 @@ int fsie_sample(const float* logits, int rows, int vocab, const float* temperatu
             if (e != cudaSuccess) return (int)e;
             configured = true;
         }
-        fsie::sample_cluster_kernel<<<dim3(fsie::CLUSTER, rows), fsie::SAMPLE_THREADS, smem, stream>>>(
-            logits, vocab, slice, temperature, top_k, top_p, uniform, out);
-        return FSIE_LAUNCH_CHECK();
+        const int rc = fsie::launch_dependent(fsie::sample_short_kernel, dim3(fsie::CLUSTER, rows),
+                                              dim3(fsie::SAMPLE_THREADS), 0, stream, logits, vocab, slice, temperature,
+                                              top_k, top_p, uniform, out);
+        if (rc != 0) return rc;
+        return fsie::launch_dependent(fsie::sample_cluster_kernel, dim3(fsie::CLUSTER, rows),
+                                      dim3(fsie::SAMPLE_THREADS), smem, stream, logits, vocab, slice, temperature,
+                                      top_k, top_p, uniform, out);
     }
     fsie::sample_kernel<<<rows, fsie::SAMPLE_THREADS, 0, stream>>>(logits, vocab, temperature, top_k,
                                                                   top_p, uniform, out);
