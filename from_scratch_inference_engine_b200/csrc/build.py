@@ -40,6 +40,8 @@ LIBRARIES: Dict[str, Sequence[str]] = {
     "gemm_decode": ("gemm_decode_tcgen05.cu",),
     # tcgen05 / TMA matrix product for steps of many tokens, with fused bias or SwiGLU
     "gemm_tiles": ("gemm_tiles_tcgen05.cu",),
+    # tcgen05 / TMA float32 product for steps of many tokens, operands split into three bfloat16 parts
+    "gemm_f32_split": ("gemm_f32_tcgen05.cu",),
     # mma.sync product without set-up for steps of few tokens against small matrices
     "gemm_skinny": ("gemm_skinny.cu",),
     # parts of hybrid decoders: layer norm on a sublayer's output, and windowed attention with mixed

@@ -1,6 +1,7 @@
 // True 32-bit matrix products for the float32 path: y[M,N] = x[M,K] * w[N,K]^T (+ bias[N]).
-// Plain FFMA on CUDA cores, no tensor-core mode of any precision (the reference instead asks
-// its library for strict fp32, src/cuda/device.cu:322-357).  Three kernels:
+// Plain FFMA on CUDA cores (the reference instead asks its library for strict fp32,
+// src/cuda/device.cu:322-357); steps of many tokens take the product that splits its operands into three
+// bfloat16 parts, which loses nothing of the 32 bits (gemm_f32_tcgen05.cu).  Three kernels:
 //
 //  * gemm_f32_rows_kernel - steps of few tokens (M <= 48, in tiles of up to 16 rows).  The
 //    product is bound by reading w once from HBM, so a warp owns R rows of w and streams them
@@ -8,7 +9,7 @@
 //    memory and every x value read from there is used for R rows of w.  A lane's partial sums
 //    run over k in ascending order and the 32 lanes are then added in a fixed tree, so an
 //    output does not depend on how many other rows share the launch.
-//  * gemm_f32_tiles_kernel - prompts: tiles of 128 x 128 outputs, k in steps of 16 through
+//  * gemm_f32_tiles_kernel - more rows than that, by name: tiles of 128 x 128 outputs, k in steps of 16 through
 //    shared memory, 8 x 8 outputs per thread in registers.  Each output is one thread's sum over
 //    k in ascending order.
 //  * gemm_f32_plain_kernel - any sizes and alignments (k no multiple of 4, unaligned rows).
@@ -16,6 +17,7 @@
 // An output of the rows kernel and the same output of the tiles kernel differ in the order of
 // their sums, that is by rounding; within one kernel a row's result does not depend on the batch.
 #include "common.cuh"
+#include "gemm_f32_tile.cuh"
 
 namespace fsie {
 
@@ -157,96 +159,11 @@ static int launch_rows(const float* x, const float* w, const float* bias, float*
 }
 
 // ---------------------------------------------------------------------------- tiles
-constexpr int TM = 128, TN = 128, TK = 16;      // block tile; 256 threads, 8 x 8 outputs each
-
 __global__ void __launch_bounds__(256, 2)
 gemm_f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w,
                       const float* __restrict__ bias, float* __restrict__ y,
                       int M, int N, int K, int ldx, int ldy) {
-    // k-major in shared memory, so that a thread's 8 rows (columns) are two 16-byte reads
-    __shared__ __align__(16) float xs[2][TK][TM + 4];      // + 4: the four k of a thread's load fall into other banks
-    __shared__ __align__(16) float ws[2][TK][TN + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;           // tx -> columns (N), ty -> rows (M)
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    // loads: 128 rows x 16 k per operand = 512 float4; thread t takes rows t / 4 and t / 4 + 64,
-    // k offset (t % 4) * 4
-    const int lrow = tid >> 2, lk = (tid & 3) * 4;
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-    float4 xr[2], wr[2];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int m = m0 + lrow + h * 64, n = n0 + lrow + h * 64, k = k0 + lk;
-            xr[h] = (m < M && k < K) ? *reinterpret_cast<const float4*>(x + (size_t)m * ldx + k)
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-            wr[h] = (n < N && k < K) ? __ldg(reinterpret_cast<const float4*>(w + (size_t)n * K + k))
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    auto stash = [&](int buf) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = lrow + h * 64;
-            xs[buf][lk + 0][r] = xr[h].x; xs[buf][lk + 1][r] = xr[h].y;
-            xs[buf][lk + 2][r] = xr[h].z; xs[buf][lk + 3][r] = xr[h].w;
-            ws[buf][lk + 0][r] = wr[h].x; ws[buf][lk + 1][r] = wr[h].y;
-            ws[buf][lk + 2][r] = wr[h].z; ws[buf][lk + 3][r] = wr[h].w;
-        }
-    };
-    fetch(0);
-    stash(0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        const bool more = k0 + TK < K;
-        if (more) fetch(k0 + TK);                 // the next step's operands travel while this one computes
-#pragma unroll
-        for (int c = 0; c < TK; ++c) {
-            // rows ty*4 .. +3 and 64 + ty*4 .. +3, columns tx*4 .. +3 and 64 + tx*4 .. +3:
-            // consecutive threads read consecutive 16 bytes, no bank conflicts
-            const float4 a0 = *reinterpret_cast<const float4*>(&xs[buf][c][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&xs[buf][c][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&ws[buf][c][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&ws[buf][c][64 + tx * 4]);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        if (more) {
-            stash(buf ^ 1);
-            __syncthreads();
-            buf ^= 1;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-        if (m >= M) continue;
-#pragma unroll
-        for (int jh = 0; jh < 2; ++jh) {
-            const int n = n0 + jh * 64 + tx * 4;
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = acc[i][jh * 4 + j] + ((bias && n + j < N) ? bias[n + j] : 0.f);
-            float* out = y + (size_t)m * ldy + n;
-            if (n + 3 < N && (((size_t)out) & 15) == 0) {
-                *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (n + j < N) out[j] = v[j];
-            }
-        }
-    }
+    f32_tile(x, w, bias, y, M, N, K, ldx, ldy, blockIdx.y * TM, blockIdx.x * TN);
 }
 
 // ---------------------------------------------------------------------------- plain

@@ -343,5 +343,8 @@ class ModelRunner:
                     37: "tcgen05 decode attention: scores or outputs never completed",
                     38: "tcgen05 decode attention: shared memory does not start on a 1,024-byte "
                         "boundary",
+                    41: "tiled float32 product: the copy engine's stage never became free",
+                    42: "tiled float32 product: a stage never arrived",
+                    43: "tiled float32 product: a stage was never multiplied",
                     3: "attention: a visible key lies in a page that was given back"}
             raise DeviceFault(what.get(code, f"device error flag {code}"))

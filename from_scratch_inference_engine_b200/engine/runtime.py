@@ -195,12 +195,33 @@ class Runtime:
         splits = ops.gemm_decode_splits(tiles, prepared.k, self.sm_count)
         return ops.gemm_decode(prepared, x, out, bias, self.error, splits)
 
+    def _product_f32(self, x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor],
+                     tag: Optional[str]) -> torch.Tensor:
+        """The float32 product: on the tensor cores in three bfloat16 parts per operand for steps of many
+        tokens, else FFMA."""
+        rows, (n, k) = x.shape[0], weight.shape
+        out = self.buffer(tag, rows, n, torch.float32)
+        # Beyond the rows of the FFMA kernel for few rows the tensor cores won at every size measured (us, split /
+        # FFMA tiles: 49 rows of 192 x 192 16 / 27, of 1,536 x 8,960 245 / 1,045, of 37,888 x 3,584 229 / 844; 1,668
+        # rows of 1,536 x 8,960 304 / 1,856, of 37,888 x 3,584 1,715 / 11,329).  Below, a tile of 256 columns takes as
+        # long whatever its rows (2 us per 64 k-elements), so it takes columns for half of the pairs of SMs: 17 and
+        # 48 rows of 17,920 x 1,536 57 / 119 and 57 / 179, of 4,096 x 4,096 119 / 64 and 119 / 94; up to 16 rows the
+        # FFMA kernel reads w once and is level (16 rows of 17,920 x 1,536 58 / 66) or ahead.
+        least = 17 if 2 * -(-n // ops.GEMM_F32_SPLIT_COLUMNS) >= self.sm_count // 2 else ops.gemm_f32_rows_limit() + 1
+        if rows < least or not ops.gemm_f32_split_takes(x, weight):
+            return ops.gemm_f32(x, weight, bias, out)
+        planes, notes = ops.gemm_f32_split_room(rows, n, k)
+        return ops.gemm_f32_split(x, weight, bias, out,
+                                  self.buffer("gemm_f32.planes", 1, planes, torch.bfloat16).view(-1),
+                                  self.buffer("gemm_f32.notes", 1, notes, torch.int32).view(-1),
+                                  self.error, self.sm_count)
+
     def linear(self, x: torch.Tensor, weight: torch.Tensor,
                bias: Optional[torch.Tensor], tag: Optional[str] = None) -> torch.Tensor:
         """x @ weight.T (+ bias) in the compute dtype.  `tag`: see `buffer` (the result may then
         live where the last result under that tag lived)."""
         if self.dtype is torch.float32:
-            return ops.gemm_f32(x, weight, bias, self.buffer(tag, x.shape[0], weight.shape[0], torch.float32))
+            return self._product_f32(x, weight, bias, tag)
         prepared = self._few_tokens(x, weight)
         if prepared is not None and not prepared.swiglu:
             return self._few_token_product(prepared, x, bias, torch.bfloat16, tag)
@@ -293,7 +314,7 @@ class Runtime:
                        tag: Optional[str] = None) -> torch.Tensor:
         """x @ weight.T with a float32 result (the logits)."""
         if self.dtype is torch.float32:
-            return ops.gemm_f32(x, weight, None, self.buffer(tag, x.shape[0], weight.shape[0], torch.float32))
+            return self._product_f32(x, weight, None, tag)
         prepared = self._few_tokens(x, weight)
         if prepared is not None and not prepared.swiglu:
             return self._few_token_product(prepared, x, None, torch.float32, tag)

@@ -229,7 +229,7 @@ def gemm_f32_rows_limit() -> int:
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor],
              out: Optional[torch.Tensor] = None, kind: str = "auto",
              rows_per_warp: int = 0) -> torch.Tensor:
-    """out = x @ weight.T (+ bias), all float32, plain FFMA (no tensor-core mode).  `kind`
+    """out = x @ weight.T (+ bias), all float32, plain FFMA.  `kind`
     names one of the three kernels (few rows, tiles, plain) instead of the choice by size;
     `rows_per_warp` (1, 2, 4) fixes how many rows of the weight a warp of the few-rows kernel
     owns instead of the choice by size."""
@@ -252,6 +252,66 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]
                                 x.stride(0), out.stride(0), GEMM_F32_KINDS[kind], int(rows_per_warp),
                                 _stream()),
            "gemm_f32")
+    return out
+
+
+GEMM_F32_SPLIT_COLUMNS = 256      # columns of a tile of `gemm_f32_split`
+_gemm_f32_split = None
+
+
+def gemm_f32_split_lib():
+    global _gemm_f32_split
+    if _gemm_f32_split is None:
+        lib = build.load_library("gemm_f32_split")
+        i, ll, p = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p
+        lib.fsie_gemm_f32_split.argtypes = [p, ll, p, p, p, ll, i, i, i, p, ll, p, i, i, p, p]
+        lib.fsie_gemm_f32_split_room.argtypes = [i, i, i, ctypes.POINTER(ll), ctypes.POINTER(i)]
+        lib.fsie_gemm_f32_split_pairs.argtypes = []
+        for name in ("fsie_gemm_f32_split", "fsie_gemm_f32_split_room", "fsie_gemm_f32_split_pairs"):
+            getattr(lib, name).restype = i
+        pairs = lib.fsie_gemm_f32_split_pairs()       # also sets the kernel up, outside any capture
+        if pairs <= 0:
+            raise KernelError(f"gemm_f32_split: pairs of blocks cannot be launched here (code {pairs})")
+        _gemm_f32_split = lib
+    return _gemm_f32_split
+
+
+def gemm_f32_split_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether `gemm_f32_split` can take these operands (rows on 16 bytes)."""
+    return (weight.shape[1] % 4 == 0 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
+            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def gemm_f32_split_room(rows: int, n: int, k: int) -> Tuple[int, int]:
+    """(bfloat16 elements of planes, ints of notes) that `gemm_f32_split` works in."""
+    planes, notes = ctypes.c_longlong(0), ctypes.c_int(0)
+    _check(gemm_f32_split_lib().fsie_gemm_f32_split_room(rows, n, k, ctypes.byref(planes), ctypes.byref(notes)),
+           "gemm_f32_split room")
+    return int(planes.value), int(notes.value)
+
+
+def gemm_f32_split(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
+                   planes: torch.Tensor, notes: torch.Tensor, error: torch.Tensor, blocks: int) -> torch.Tensor:
+    """out = x @ weight.T (+ bias), all float32, on the tensor cores: operands as exact sums of three
+    bfloat16 numbers, 64 k-elements at a time summed up in float32 registers (results that are not finite
+    come from the FFMA kernel).  planes and notes of the sizes `gemm_f32_split_room` names; `blocks`:
+    size of the persistent grid."""
+    _need(x, torch.float32, "x", contiguous=False)
+    _need(weight, torch.float32, "weight")
+    _need(out, torch.float32, "out", contiguous=False)
+    _need(planes, torch.bfloat16, "planes")
+    _need(notes, torch.int32, "notes")
+    rows, k = x.shape
+    n = weight.shape[0]
+    if weight.shape[1] != k or x.stride(1) != 1 or not gemm_f32_split_takes(x, weight):
+        raise KernelError("gemm_f32_split: operands do not fit (rows must start on 16 bytes)")
+    if out.shape != (rows, n) or out.stride(1) != 1:
+        raise KernelError("gemm_f32_split: out must be [rows of x, rows of weight] with unit inner stride")
+    if bias is not None:
+        _need(bias, torch.float32, "bias")
+    _check(gemm_f32_split_lib().fsie_gemm_f32_split(
+        _ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(out), out.stride(0), rows, n, k, _ptr(planes),
+        planes.numel(), _ptr(notes), notes.numel(), blocks, _ptr(error), _stream()), "gemm_f32_split")
     return out
 
 

@@ -1,0 +1,110 @@
+"""The float32 product on the tensor cores (operands in three bfloat16 parts) against 64-bit products: no
+further off than the FFMA kernel, at the edges of tiles, stages and rounds of tiles, and with numbers that
+the parts cannot hold."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BLOCKS = 148
+
+
+def product(x, w, bias=None, out=None, blocks=BLOCKS):
+    from from_scratch_inference_engine_b200.kernels import ops
+    rows, n, k = x.shape[0], w.shape[0], w.shape[1]
+    planes, notes = ops.gemm_f32_split_room(rows, n, k)
+    out = torch.full((rows, n), float("nan"), device="cuda") if out is None else out
+    error = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ops.gemm_f32_split(x, w, bias, out, torch.empty(planes, dtype=torch.bfloat16, device="cuda"),
+                             torch.full((notes,), 7, dtype=torch.int32, device="cuda"), error, blocks)
+    assert error.item() == 0
+    return got
+
+
+def ffma(x, w, bias=None):
+    from from_scratch_inference_engine_b200.kernels import ops
+    return ops.gemm_f32(x, w, bias, kind="tiles")
+
+
+def distance(got, want):
+    return ((got.double() - want).norm() / want.norm().clamp_min(1e-300)).item()
+
+
+# rows, n, k: single elements, edges of a tile (256) and of a stage (64), one stage per tile, several rounds
+# of tiles on few pairs, k where the FFMA sums drift furthest, tiles for all pairs and more
+SIZES = [(1, 1, 4), (5, 7, 8), (127, 129, 60), (128, 128, 64), (129, 255, 68), (256, 256, 128), (257, 513, 132),
+         (300, 3000, 64), (49, 2048, 1536), (700, 1300, 2052), (64, 300, 18944), (1668, 17920, 1536)]
+
+
+@pytest.mark.parametrize("rows,n,k", SIZES)
+@pytest.mark.parametrize("held", ["any", "positive", "bfloat16", "mixed"])
+def test_split_product(rows, n, k, held):
+    torch.manual_seed(rows + n + k)
+    x, w, bias = torch.randn(rows, k, device="cuda"), torch.randn(n, k, device="cuda"), torch.randn(n, device="cuda")
+    if held == "positive":
+        x, w = x.abs(), w.abs()
+    elif held == "bfloat16":                 # the parts of w beyond the first are zero
+        w = w.bfloat16().float()
+    elif held == "mixed":                    # in some stages and rows only
+        w[: n // 2] = w[: n // 2].bfloat16().float()
+        w[:, : k // 8 * 4] = w[:, : k // 8 * 4].bfloat16().float()
+        x *= torch.exp(4 * torch.randn(rows, 1, device="cuda"))
+    want = x.double() @ w.double().T
+    got = product(x, w)
+    # Errors are measured against the sums of |x w|: where a sum cancels, what is left of it says nothing.  Never
+    # further off than FFMA; where k is one stage or less and FFMA has next to no error, the four truncated steps
+    # of a stage may show: 4 x 2^-23 at most, half of that on average.
+    size = x.abs().double() @ w.abs().double().T
+
+    def off(got, want, size):
+        return ((got.double() - want).norm() / size.norm()).item()
+    assert off(got, want, size) <= max(off(ffma(x, w), want, size), 2.0 ** -22)
+    # no single output is far off either
+    assert ((got.double() - want).abs() / size).max().item() < 2e-6
+    size = size + bias.double().abs()
+    biased = product(x, w, bias, blocks=6 if rows < 1000 else BLOCKS)   # three pairs: several tiles each
+    want += bias.double()
+    assert off(biased, want, size) <= max(off(ffma(x, w, bias), want, size), 2.0 ** -22)
+    alone = product(x[rows // 2:rows // 2 + 1].contiguous(), w)
+    assert torch.equal(alone[0], got[rows // 2])
+
+
+@pytest.mark.parametrize("offset", [1, 4])
+def test_split_product_of_views(offset):
+    """x as columns of a wider matrix, the result into one whose rows do (4) or do not (1) start on 16 bytes."""
+    torch.manual_seed(offset)
+    wide, w = torch.randn(200, 140, device="cuda"), torch.randn(131, 132, device="cuda")
+    room = torch.full((200, 140 + offset), float("nan"), device="cuda")
+    x = wide[:, 4:136]
+    product(x, w, None, room[:, offset:offset + 131])
+    want = x.double() @ w.double().T
+    assert distance(room[:, offset:offset + 131], want) < 2e-7
+    assert torch.isnan(room[:, :offset]).all() and torch.isnan(room[:, offset + 131:]).all()
+
+
+def test_split_product_of_infinities():
+    """Infinite, NaN, overflowing and largest inputs give what the FFMA kernel gives."""
+    torch.manual_seed(2)
+    x, w = torch.randn(300, 200, device="cuda"), torch.randn(600, 200, device="cuda")
+    x[3, 5], x[40, 7], x[200, 9] = float("inf"), float("nan"), -float("inf")
+    x[260, 11], w[17, 11] = 3.4e38, 0.5          # finite, but rounds to infinity as bfloat16
+    x[261], w[300] = 1e30, 1e30                  # overflows in the sum
+    got, want = product(x, w), ffma(x, w)
+    same = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(got[~same & ~torch.isnan(want)], want[~same & ~torch.isnan(want)])
+    quiet = torch.ones(300, dtype=torch.bool, device="cuda")
+    quiet[[3, 40, 200, 260, 261]] = False
+    exact = x[quiet].double() @ w.double().T
+    keep = torch.ones(600, dtype=torch.bool, device="cuda")
+    keep[300] = False
+    assert distance(got[quiet][:, keep], exact[:, keep]) < 4e-7
+
+
+def test_split_product_refuses():
+    from from_scratch_inference_engine_b200.kernels.ops import KernelError
+    with pytest.raises(KernelError):
+        product(torch.randn(64, 6, device="cuda"), torch.randn(8, 6, device="cuda"))
+    with pytest.raises(KernelError):
+        product(torch.randn(64, 13, device="cuda")[:, 1:9], torch.randn(8, 8, device="cuda"))
