@@ -445,166 +445,131 @@ __global__ void __launch_bounds__(128) moe_product_mma_kernel(
 // A decode step gives an expert one to a few rows, so the product is the time its matrices take to come
 // in.  The tiled kernel above waits for every 64 k-elements with one chunk asked for ahead and keeps 18 KB
 // per block on the way.  Here blocks stay (two of 256 threads per SM) and walk items of (tile of up to 16
-// rows, 32 rows of w - GATED: 16 of the gate and the same 16 of the up projection); the 8 warps of a block
-// take turns along k in chunks of 32, each lane asks for its own 16 bytes of four rows with cp.async into a
-// ring of its own (no barrier guards it), and the ring runs on into the next item while the current one is
-// summed up: 64 KB per block are on the way at any time.  What the next item needs besides - its expert, its
-// rows of x, their first values - is asked for before the current item's sums meet in shared memory (double-
-// buffered, one barrier per item).  The rows of x are the N side of mma.sync m16n8k16.
-constexpr int FEW_WARPS = 8, FEW_CHUNK = 32, FEW_AHEAD = 4, FEW_ROWS = 32;
-constexpr int FEW_SLOT = FEW_ROWS * FEW_CHUNK * 2;                           // bytes a warp asks for at once
-constexpr int FEW_RING = FEW_WARPS * FEW_AHEAD * FEW_SLOT;
-constexpr int FEW_PITCH = FEW_ROWS + 4;                                      // the sums' rows start in other banks
-constexpr int FEW_RED = FEW_WARPS * MOE_FEW_TILE * FEW_PITCH;                // floats per buffer
-constexpr size_t FEW_SMEM = FEW_RING + 2 * FEW_RED * sizeof(float);
+// rows, 32 rows of w - GATED: 16 of the gate and the same 16 of the up projection) in slots of 128 k-elements:
+// all threads ask for a slot's 8 KB of w and its rows of x with cp.async, seven slots ahead (56 KB of w per
+// block on the way), and the slots run on into the next items.  One barrier per slot.  Up to four warps
+// multiply, 16 rows of w by 8 rows of x (the N side of mma.sync m16n8k16) each; GATED: 8 gate rows and their 8
+// up rows, so that a lane ends with both.  A warp's sum runs over k in steps of 16 in ascending order, as
+// in the tiled kernel: the results are the same to the bit.
+constexpr int FEW_THREADS = 256, FEW_K = 128, FEW_SLOTS = 8, FEW_ROWS = 32;
+constexpr int FEW_CHUNK = 32;                                                // k comes in these: two steps of 16
+constexpr int FEW_PIECES = FEW_K / 8;                                        // 16-byte pieces of a slot's row
+constexpr int FEW_SLOT = (FEW_ROWS + MOE_FEW_TILE) * FEW_K * 2;              // rows of w, rows of x
+constexpr size_t FEW_SMEM = (size_t)FEW_SLOTS * FEW_SLOT;
+
+// a piece's place in its slot: moved by the row, so that eight rows' pieces lie in different banks
+__device__ __forceinline__ int few_place(int row, int piece) { return row * (FEW_K * 2) + ((piece ^ (row & 7)) << 4); }
 
 template <int MODE>
-__global__ void __launch_bounds__(32 * FEW_WARPS, 2) moe_product_few_kernel(
+__global__ void __launch_bounds__(FEW_THREADS, 2) moe_product_few_kernel(
         const bf16* __restrict__ x, long long x_ld, const bf16* __restrict__ w, bf16* __restrict__ out,
         long long out_ld, const int* __restrict__ offsets, const int* __restrict__ sorted,
         const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ meta,
         int top, int n, int k, int gate_kind) {
     constexpr bool GATED = MODE == 1, FIRST = MODE != 0;
     constexpr int COLS = GATED ? 16 : 32;                    // outputs per row and item
-    extern __shared__ __align__(16) unsigned char few_smem[];
-    float* const red = reinterpret_cast<float*>(few_smem + FEW_RING);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
+    extern __shared__ __align__(128) unsigned char few_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     grid_dependency_wait();
     grid_dependents_go();
     const int tiles = meta[0];
     // neighbouring items are the tiles of the same columns: an expert's further tiles find its rows in L2
     const int items = tiles * ((n + COLS - 1) / COLS);
     if ((int)blockIdx.x >= items) return;
-    const int chunks = k / FEW_CHUNK, per = (chunks + FEW_WARPS - 1) / FEW_WARPS;      // a warp's slots per item
+    const int per = (k + FEW_K - 1) / FEW_K;                 // slots per item
     const int step_tile = gridDim.x % tiles, step_n0 = (gridDim.x / tiles) * COLS;
     auto advance = [&](int& tile, int& n0) {                 // the block's next item
         tile += step_tile;
         n0 += step_n0;
         if (tile >= tiles) { tile -= tiles; n0 += COLS; }
     };
-    unsigned char* const mine = few_smem + (size_t)warp * FEW_AHEAD * FEW_SLOT + lane * 16;
 
+    // ---- asking: a thread's two pieces of w (rows `row` and row + 16 of the slot) and its piece of x (row `row`)
+    const int row = tid / FEW_PIECES, piece = tid % FEW_PIECES;
     int ask_tile = blockIdx.x % tiles, ask_n0 = (blockIdx.x / tiles) * COLS, ask_j = 0, ask_slot = 0;
-    const bf16* wr[4];
-    auto point = [&]() {                                     // this lane's four rows of w of the item asked for
+    const bf16 *wr[2], *xr = nullptr;
+    auto point = [&]() {
         if (ask_n0 >= n) return;
-        const bf16* we = w + (size_t)tile_expert[ask_tile] * (GATED ? 2 : 1) * n * k + 8 * t;
+        const int e = tile_expert[ask_tile], r0 = tile_row0[ask_tile];
+        const bf16* we = w + (size_t)e * (GATED ? 2 : 1) * n * k + piece * 8;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = GATED ? (i >> 1) * n + min(ask_n0 + g + 8 * (i & 1), n - 1) : min(ask_n0 + g + 8 * i, n - 1);
-            wr[i] = we + (size_t)row * k;
+        for (int i = 0; i < 2; ++i) {
+            // GATED: rows 0-7 of every 16 are gate rows, rows 8-15 the up rows of the same outputs
+            const int at = GATED ? ((row & 8) ? n : 0) + min(ask_n0 + 8 * i + (row & 7), n - 1) : min(ask_n0 + 16 * i + row, n - 1);
+            wr[i] = we + (size_t)at * k;
         }
+        const bool met = row < min(MOE_FEW_TILE, offsets[e + 1] - r0);
+        xr = met ? x + (size_t)(FIRST ? sorted[r0 + row] / top : r0 + row) * x_ld + piece * 8 : nullptr;
     };
     auto ask = [&]() {
-        const int c = warp + ask_j * FEW_WARPS;
-        if (ask_n0 < n && c < chunks) {
+        const int k0 = ask_j * FEW_K;
+        if (ask_n0 < n && k0 + piece * 8 < k) {
+            unsigned char* slot = few_smem + ask_slot * FEW_SLOT;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) mm_cp16(mine + ask_slot * FEW_SLOT + i * 512, wr[i] + c * FEW_CHUNK, true);
+            for (int i = 0; i < 2; ++i) mm_cp16(slot + few_place(16 * i + row, piece), wr[i] + k0, true);
+            if (xr) mm_cp16(slot + few_place(FEW_ROWS + row, piece), xr + k0, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");            // one group per slot, also when empty
-        ask_slot = ask_slot + 1 == FEW_AHEAD ? 0 : ask_slot + 1;
+        ask_slot = ask_slot + 1 == FEW_SLOTS ? 0 : ask_slot + 1;
         if (++ask_j == per) {
             ask_j = 0;
             advance(ask_tile, ask_n0);
             point();
         }
     };
+    static_assert(FEW_THREADS == MOE_FEW_TILE * FEW_PIECES && FEW_ROWS == 2 * MOE_FEW_TILE, "a thread's pieces");
     point();
 #pragma unroll
-    for (int j = 0; j < FEW_AHEAD; ++j) ask();
+    for (int j = 0; j < FEW_SLOTS - 1; ++j) ask();
 
-    int tile = blockIdx.x % tiles, n0 = (blockIdx.x / tiles) * COLS, r0 = 0, rows = 0, slot = 0, buffer = 0;
-    const bf16* xr[2];
-    auto open = [&](int of) {                                // the tile's rows of x
-        r0 = tile_row0[of];
-        rows = min(MOE_FEW_TILE, offsets[tile_expert[of] + 1] - r0);
+    // ---- multiplying: warp = (16 rows of w, 8 rows of x)
+    const int half = warp & 1, eight = warp >> 1;
+    const int a_row = half * 16 + (lane & 15), a_piece = lane >> 4;
+    const int b_row = FEW_ROWS + eight * 8 + (lane & 7), b_piece = lane >> 3;          // two steps of 16 at a time
+    int slot = 0;
+    for (int tile = blockIdx.x % tiles, n0 = (blockIdx.x / tiles) * COLS; n0 < n; advance(tile, n0)) {
+        const int r0 = tile_row0[tile], rows = min(MOE_FEW_TILE, offsets[tile_expert[tile] + 1] - r0);
+        const bool mine = eight * 8 < rows;                  // (warps 4 to 7 never)
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int j = 0; j < per; ++j) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(FEW_SLOTS - 2) : "memory");   // the oldest slot has landed
+            __syncthreads();                                 // for all threads; and the slot before it is no longer read
+            ask();
+            if (mine) {
+                const unsigned char* at = few_smem + slot * FEW_SLOT;
+                const int end = min(FEW_K, k - j * FEW_K) / 8;       // pieces, a multiple of 4
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = g + 8 * h;
-            xr[h] = r < rows ? x + (size_t)(FIRST ? sorted[r0 + r] / top : r0 + r) * x_ld + 8 * t : nullptr;
-        }
-    };
-    uint4 b[4][2];
-    auto load_x = [&](int j0) {                              // the rows' values of four chunks are asked for together
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int c = warp + (j0 + u) * FEW_WARPS;
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                b[u][h] = (c < chunks && xr[h]) ? *reinterpret_cast<const uint4*>(xr[h] + c * FEW_CHUNK) : make_uint4(0, 0, 0, 0);
-        }
-    };
-    open(tile);
-    load_x(0);
-    for (;;) {
-        float acc[2][2][4];                                  // [rows of w 0-15, 16-31][rows of x 0-7, 8-15]
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) acc[i >> 1][i & 1][v] = 0.f;
-        for (int j0 = 0; j0 < per; j0 += 4) {
-            if (j0) load_x(j0);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (j0 + u >= per) break;
-                asm volatile("cp.async.wait_group %0;" ::"n"(FEW_AHEAD - 1) : "memory");      // the oldest slot has landed
-                if (warp + (j0 + u) * FEW_WARPS < chunks) {
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const uint4 lo = *reinterpret_cast<const uint4*>(mine + slot * FEW_SLOT + i * 1024);
-                        const uint4 hi = *reinterpret_cast<const uint4*>(mine + slot * FEW_SLOT + i * 1024 + 512);
-                        const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
-                        mm_mma(acc[i][0], a0, b[u][0].x, b[u][0].y);
-                        mm_mma(acc[i][0], a1, b[u][0].z, b[u][0].w);
-                        if (rows > 8) {
-                            mm_mma(acc[i][1], a0, b[u][1].x, b[u][1].y);
-                            mm_mma(acc[i][1], a1, b[u][1].z, b[u][1].w);
-                        }
-                    }
+                for (int q = 0; q < FEW_PIECES; q += 4) {
+                    if (q >= end) break;
+                    uint32_t a0[4], a1[4], b[4];
+                    mm_ldsm_x4(a0, at + few_place(a_row, q + a_piece));
+                    mm_ldsm_x4(a1, at + few_place(a_row, q + 2 + a_piece));
+                    mm_ldsm_x4(b, at + few_place(b_row, q + b_piece));
+                    mm_mma(acc, a0, b[0], b[1]);
+                    mm_mma(acc, a1, b[2], b[3]);
                 }
-                slot = slot + 1 == FEW_AHEAD ? 0 : slot + 1;
-                ask();
+            }
+            slot = slot + 1 == FEW_SLOTS ? 0 : slot + 1;
+        }
+        if (!mine) continue;
+        // acc: rows g (0, 1) and g + 8 (2, 3) of the 16 of w, rows 2 t and 2 t + 1 of the 8 of x
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const int r = eight * 8 + 2 * t + v;
+            if (r >= rows) continue;
+            bf16* o = out + (size_t)(FIRST ? r0 + r : sorted[r0 + r]) * out_ld;
+            // rounded as a product that stored its result in between would have
+            const float lo = __bfloat162float(__float2bfloat16_rn(acc[v])), hi = __bfloat162float(__float2bfloat16_rn(acc[2 + v]));
+            if (GATED) {
+                const int c = n0 + half * 8 + g;
+                if (c < n) o[c] = __float2bfloat16_rn(gate_fn(lo, gate_kind) * hi);
+            } else {
+                const int c = n0 + half * 16 + g;
+                if (c < n) o[c] = __float2bfloat16_rn(MODE == 2 ? gate_fn(lo, gate_kind) : lo);
+                if (c + 8 < n) o[c + 8] = __float2bfloat16_rn(MODE == 2 ? gate_fn(hi, gate_kind) : hi);
             }
         }
-        // acc[i][h]: rows g (0, 1) and g + 8 (2, 3) of w, rows 8 h + 2 t and 8 h + 2 t + 1 of x
-        float* const sums = red + buffer * FEW_RED;          // [warp][row of x][32 rows of w]
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (8 * h >= rows) break;
-            float* at = sums + ((size_t)warp * MOE_FEW_TILE + 8 * h + 2 * t) * FEW_PITCH + g;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                at[16 * i] = acc[i][h][0];
-                at[16 * i + FEW_PITCH] = acc[i][h][1];
-                at[16 * i + 8] = acc[i][h][2];
-                at[16 * i + 8 + FEW_PITCH] = acc[i][h][3];
-            }
-        }
-        const int done_n0 = n0, done_r0 = r0, done_rows = rows;
-        advance(tile, n0);
-        if (n0 < n) {
-            open(tile);
-            load_x(0);
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < done_rows * COLS; e += 32 * FEW_WARPS) {
-            const int r = e / COLS, c = e - r * COLS;        // consecutive threads: consecutive columns of a row
-            float lo = 0.f, hi = 0.f;
-#pragma unroll
-            for (int v = 0; v < FEW_WARPS; ++v) {
-                lo += sums[(v * MOE_FEW_TILE + r) * FEW_PITCH + c];
-                if (GATED) hi += sums[(v * MOE_FEW_TILE + r) * FEW_PITCH + c + 16];
-            }
-            if (done_n0 + c >= n) continue;
-            lo = __bfloat162float(__float2bfloat16_rn(lo));  // as a product that stored it in between would have
-            if (GATED) lo = gate_fn(lo, gate_kind) * __bfloat162float(__float2bfloat16_rn(hi));
-            else if (MODE == 2) lo = gate_fn(lo, gate_kind);
-            const int to = FIRST ? done_r0 + r : sorted[done_r0 + r];
-            out[(size_t)to * out_ld + done_n0 + c] = __float2bfloat16_rn(lo);
-        }
-        if (n0 >= n) break;
-        buffer ^= 1;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
@@ -734,7 +699,7 @@ static int launch_few(const void* x, long long x_ld, const void* w, void* out, l
     const int cols = MODE == 1 ? FEW_ROWS / 2 : FEW_ROWS;
     const long long most = (long long)tiles * ((n + cols - 1) / cols);
     return launch_dependent(moe_product_few_kernel<MODE>, dim3((unsigned)(most < 2 * sms ? most : 2 * sms)),
-                            dim3(32 * FEW_WARPS), FEW_SMEM, stream, (const bf16*)x, x_ld, (const bf16*)w, (bf16*)out,
+                            dim3(FEW_THREADS), FEW_SMEM, stream, (const bf16*)x, x_ld, (const bf16*)w, (bf16*)out,
                             out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind);
 }
 

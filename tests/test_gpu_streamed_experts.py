@@ -1,5 +1,5 @@
 """The products that stream the matrices of experts with few rows (lists of tiles of 16 rows) against plain
-64-bit products, at the edges of tiles, items, chunks and warps' turns along k."""
+64-bit products, at the edges of tiles, items and slots along k; in bfloat16 they give the tiled products' bits."""
 
 import pytest
 import torch
@@ -9,9 +9,9 @@ pytestmark = pytest.mark.gpu
 
 # experts, top, tokens, hidden, inner, experts that are met (None: any)
 SIZES = [
-    (5, 1, 1, 32, 32, None),          # a single row, a single chunk: seven of eight warps have nothing
+    (5, 1, 1, 32, 32, None),          # a single row, a quarter of a slot
     (4, 2, 3, 64, 96, None),          # items of 32 and 16 columns that end inside
-    (7, 3, 16, 288, 40 * 4, None),    # nine chunks: one warp takes a second turn
+    (7, 3, 16, 288, 40 * 4, None),    # two whole slots and a quarter, one and a quarter
     (3, 1, 17, 1056, 96, [1]),        # one expert meets 17 rows: a full tile and a tile of one row
     (2, 1, 40, 512, 2080, [0]),       # three tiles of one expert, many items per block
     (64, 6, 8, 2048, 1408, None),     # a routed layer of a decode step
@@ -39,6 +39,14 @@ def test_streamed_expert_products(experts, top, tokens, hidden, inner, met, mode
     out = torch.full((pairs, hidden), float("nan"), device="cuda", dtype=dtype)
     ops.moe_product(x, w1, act, lists, pairs, top, gated, "silu" if gated else "relu2", first=True, tile=tile)
     ops.moe_product(act, w2, out, lists, pairs, top, False, tile=tile)
+
+    if dtype is torch.bfloat16:
+        wide = ops.moe_align(ids, pairs, experts, torch.zeros(ops.moe_lists_size(pairs, experts), dtype=torch.int32,
+                                                              device="cuda"))
+        tiled_act, tiled = torch.empty_like(act), torch.empty_like(out)
+        ops.moe_product(x, w1, tiled_act, wide, pairs, top, gated, "silu" if gated else "relu2", first=True)
+        ops.moe_product(act, w2, tiled, wide, pairs, top, False)
+        assert torch.equal(act, tiled_act) and torch.equal(out, tiled)
 
     order = lists[1].long()
     expert = ids.view(-1).long()[order]
