@@ -444,14 +444,16 @@ __global__ void __launch_bounds__(128) moe_product_mma_kernel(
 // ------------------------------------------------ few rows per expert: the matrices streamed once
 // A decode step gives an expert one to a few rows, so the product is the time its matrices take to come
 // in.  The tiled kernel above waits for every 64 k-elements with one chunk asked for ahead and keeps 18 KB
-// per block on the way.  Here blocks stay (two of 256 threads per SM) and walk items of (tile of up to 16
+// per block on the way.  Here blocks stay (three of 256 threads per SM) and walk items of (tile of up to 16
 // rows, 32 rows of w - GATED: 16 of the gate and the same 16 of the up projection) in slots of 128 k-elements:
-// all threads ask for a slot's 8 KB of w and its rows of x with cp.async, seven slots ahead (56 KB of w per
-// block on the way), and the slots run on into the next items.  One barrier per slot.  Up to four warps
+// all threads ask for a slot's 8 KB of w and its rows of x with cp.async, five slots ahead (40 KB of w per
+// block on the way), and the slots run on into the next items.  One barrier per slot: three blocks with 6
+// slots hide it from each other (64 experts of 1,408 x 2,048, 8 tokens x 6, 36 experts met, us for gate-up + down:
+// 69 + 38, floor 64 + 32; two blocks with 8 slots 81 + 44; the tiled kernel 124 + 85).  Up to four warps
 // multiply, 16 rows of w by 8 rows of x (the N side of mma.sync m16n8k16) each; GATED: 8 gate rows and their 8
 // up rows, so that a lane ends with both.  A warp's sum runs over k in steps of 16 in ascending order, as
 // in the tiled kernel: the results are the same to the bit.
-constexpr int FEW_THREADS = 256, FEW_K = 128, FEW_SLOTS = 8, FEW_ROWS = 32;
+constexpr int FEW_THREADS = 256, FEW_K = 128, FEW_SLOTS = 6, FEW_ROWS = 32;
 constexpr int FEW_CHUNK = 32;                                                // k comes in these: two steps of 16
 constexpr int FEW_PIECES = FEW_K / 8;                                        // 16-byte pieces of a slot's row
 constexpr int FEW_SLOT = (FEW_ROWS + MOE_FEW_TILE) * FEW_K * 2;              // rows of w, rows of x
@@ -461,7 +463,7 @@ constexpr size_t FEW_SMEM = (size_t)FEW_SLOTS * FEW_SLOT;
 __device__ __forceinline__ int few_place(int row, int piece) { return row * (FEW_K * 2) + ((piece ^ (row & 7)) << 4); }
 
 template <int MODE>
-__global__ void __launch_bounds__(FEW_THREADS, 2) moe_product_few_kernel(
+__global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
         const bf16* __restrict__ x, long long x_ld, const bf16* __restrict__ w, bf16* __restrict__ out,
         long long out_ld, const int* __restrict__ offsets, const int* __restrict__ sorted,
         const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ meta,
@@ -538,15 +540,16 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) moe_product_few_kernel(
             if (mine) {
                 const unsigned char* at = few_smem + slot * FEW_SLOT;
                 const int end = min(FEW_K, k - j * FEW_K) / 8;       // pieces, a multiple of 4
+                uint32_t a[FEW_PIECES / 2][4], b[FEW_PIECES / 4][4];
+#pragma unroll
+                for (int q = 0; q < FEW_PIECES; q += 2) mm_ldsm_x4(a[q / 2], at + few_place(a_row, q + a_piece));
+#pragma unroll
+                for (int q = 0; q < FEW_PIECES; q += 4) mm_ldsm_x4(b[q / 4], at + few_place(b_row, q + b_piece));
 #pragma unroll
                 for (int q = 0; q < FEW_PIECES; q += 4) {
                     if (q >= end) break;
-                    uint32_t a0[4], a1[4], b[4];
-                    mm_ldsm_x4(a0, at + few_place(a_row, q + a_piece));
-                    mm_ldsm_x4(a1, at + few_place(a_row, q + 2 + a_piece));
-                    mm_ldsm_x4(b, at + few_place(b_row, q + b_piece));
-                    mm_mma(acc, a0, b[0], b[1]);
-                    mm_mma(acc, a1, b[2], b[3]);
+                    mm_mma(acc, a[q / 2], b[q / 4][0], b[q / 4][1]);
+                    mm_mma(acc, a[q / 2 + 1], b[q / 4][2], b[q / 4][3]);
                 }
             }
             slot = slot + 1 == FEW_SLOTS ? 0 : slot + 1;
@@ -698,7 +701,7 @@ static int launch_few(const void* x, long long x_ld, const void* w, void* out, l
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int cols = MODE == 1 ? FEW_ROWS / 2 : FEW_ROWS;
     const long long most = (long long)tiles * ((n + cols - 1) / cols);
-    return launch_dependent(moe_product_few_kernel<MODE>, dim3((unsigned)(most < 2 * sms ? most : 2 * sms)),
+    return launch_dependent(moe_product_few_kernel<MODE>, dim3((unsigned)(most < 3 * sms ? most : 3 * sms)),
                             dim3(FEW_THREADS), FEW_SMEM, stream, (const bf16*)x, x_ld, (const bf16*)w, (bf16*)out,
                             out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind);
 }

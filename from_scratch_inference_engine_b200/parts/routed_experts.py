@@ -43,9 +43,9 @@ class RoutedExperts(Part):
     """
 
     # Average rows per expert up to which the products that stream the matrices are taken.  Measured on 64
-    # experts of 1,408 x 2,048 (both products, us, streaming / tiled): bfloat16 at 6 rows 236 / 314, at 16 297 /
-    # 342, at 24 376 / 369; float32 at 6 rows 631 / 2,964, at 24 1,757 / 2,968 - there the streaming kernel's
-    # time grows by about 65 us a row and meets the tiled one's at about 40.
+    # experts of 1,408 x 2,048 (both products, us, streaming / tiled): bfloat16 at 4 rows 185 / 314 (6 rows), at 16 287 /
+    # 342 - 17 rows are two tiles of 16; float32 at 6 rows 631 / 2,964, at 24 1,757 / 2,968 - there the streaming
+    # kernel's time grows by about 65 us a row and meets the tiled one's at about 40.
     FEW_MAX_ROWS = {torch.bfloat16: 20, torch.float32: 32}
     GROUPED_MIN_ROWS = 32       # average rows per expert from which the tcgen05 form is taken
 
