@@ -39,17 +39,21 @@ def _ptr(tensor: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
     """The current CUDA stream's handle.  Asked for at every launch (streams change under
-    graph capture), so by the cheapest route torch offers."""
-    if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+    graph capture), so by the cheapest route torch offers; the launch's tensors live on the GPU, so
+    CUDA is set up."""
+    if _raw_stream is not None and _raw_device is not None:
+        return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
 
 
 def _need(tensor: torch.Tensor, dtype, name: str, contiguous: bool = True) -> None:
+    if tensor.is_cuda and (dtype is None or tensor.dtype is dtype) and (not contiguous or tensor.is_contiguous()):
+        return
     if not tensor.is_cuda:
         raise KernelError(f"{name} must live on the GPU (the engine has no CPU path)")
     if dtype is not None and tensor.dtype is not dtype:
