@@ -309,6 +309,11 @@ class Runtime:
         tiled = self._tiled(x, gate_up) if self.dtype is torch.bfloat16 else None
         if tiled is not None and tiled.swiglu:
             return self._tiled_product(tiled, x, None, torch.bfloat16, tag)
+        if (self.dtype is torch.bfloat16 and prepared is None and activation == "silu"
+                and gate_up.shape[0] % 2 == 0 and self._skinny(x, gate_up)):
+            # the product that `linear` would take, with the activation in its epilogue
+            return ops.gemm_skinny_swiglu(gate_up, x, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2,
+                                                                  torch.bfloat16))
         wide = None if tag is None else tag + ".gate_up"
         both = self.linear(x, gate_up, None, wide) if prepared is None else F.linear(x, gate_up)
         act = self.buffer(tag, x.shape[0], gate_up.shape[0] // 2, both.dtype)

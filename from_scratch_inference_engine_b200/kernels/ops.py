@@ -710,6 +710,8 @@ def gemm_skinny_lib():
         i, ll, p = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_gemm_skinny.argtypes = [p, p, ll, p, ll, p, i, i, i, i, i, p]
         lib.fsie_gemm_skinny.restype = i
+        lib.fsie_gemm_skinny_swiglu.argtypes = [p, p, ll, p, ll, i, i, i, p]
+        lib.fsie_gemm_skinny_swiglu.restype = i
         lib.fsie_gemm_skinny_qkv_rope.argtypes = [p, p, ll, p, ll, p, i, i, p, p, i, p, p, p, ll, i,
                                                   i, i, i, p, p]
         lib.fsie_gemm_skinny_qkv_rope.restype = i
@@ -778,6 +780,24 @@ def gemm_skinny(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
                                          _ptr(bias), tokens, n, k, int(out.dtype is torch.float32),
                                          int(_epilogue("gemm_skinny", False, "silu", plain_activation) == 3),
                                          _stream()), "gemm_skinny")
+    return out
+
+
+def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out[T, N] = silu(x @ gate.T) * (x @ up.T) for T <= 16 and weight = [gate rows (N); up rows (N)]: the bits of
+    `gemm_skinny` and `swiglu` one after the other, in one launch."""
+    gemm_skinny_lib()
+    _need(weight, torch.bfloat16, "weight")
+    _need(x, torch.bfloat16, "x", contiguous=False)
+    _need(out, torch.bfloat16, "out", contiguous=False)
+    tokens, k = x.shape
+    n = weight.shape[0] // 2
+    if weight.shape[0] % 2 or weight.shape[1] != k or x.stride(1) != 1 or not gemm_skinny_fits(tokens, k):
+        raise KernelError("gemm_skinny_swiglu: x does not fit the weight, or the sizes are beyond the kernel")
+    if out.shape[0] != tokens or out.shape[1] != n or out.stride(1) != 1:
+        raise KernelError("gemm_skinny_swiglu: out does not fit")
+    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(_ptr(weight), _ptr(x), x.stride(0), _ptr(out), out.stride(0), tokens, n,
+                                                k, _stream()), "gemm_skinny_swiglu")
     return out
 
 
