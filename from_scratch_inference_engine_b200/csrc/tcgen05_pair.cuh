@@ -24,9 +24,16 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(smem_addr(dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_addr(bar) & FIRST_BLOCK_MASK) : "memory");
 }
-// Arrival on the barrier at this offset in the first block of the pair.
+// Arrival on the barrier at this offset in the first block of the pair.  It says that something was done (tensor
+// memory was read out); it does not publish shared memory to the other block.
 __device__ __forceinline__ void mbar_arrive_first_block(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(smem_addr(bar) & FIRST_BLOCK_MASK) : "memory");
+}
+// The arrival that does: this block's shared memory, as the arriving thread knows it, for whoever waits with
+// mbar_wait_cluster.  The fence is restricted to shared memory: it waits for nothing in global memory.
+__device__ __forceinline__ void mbar_release_first_block(uint64_t* bar) {
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_addr(bar) & FIRST_BLOCK_MASK) : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzle: rows of 128

@@ -70,6 +70,23 @@ def test_split_product(rows, n, k, held):
     assert torch.equal(alone[0], got[rows // 2])
 
 
+@pytest.mark.parametrize("parts", [2, 3])
+def test_whole_numbers_are_exact(parts):
+    """Whole numbers whose sums stay below 2^24 come out exactly: a plane of w that either block's tensor core reads
+    before its warps have filled it, in any stage, tile or launch, changes a result.  w is another one at every launch and
+    needs `parts` planes; three pairs of blocks have several tiles each."""
+    torch.manual_seed(parts)
+    rows, n, k = 300, 2000, 1536
+    x = torch.randint(-3, 4, (rows, k), device="cuda").float()
+    if parts == 3:                               # 20 bits of w: room for few terms
+        x = torch.where(torch.rand(rows, k, device="cuda") < 4 / k, x.clamp(-1, 1), torch.zeros_like(x))
+        assert x.abs().sum(1).max() < 16
+    for launch in range(30):
+        w = torch.randint(-2 ** (11 if parts == 2 else 20), 2 ** (11 if parts == 2 else 20), (n, k), device="cuda").float()
+        got = product(x, w, blocks=(6, BLOCKS)[launch % 2])
+        assert torch.equal(got.double(), x.double() @ w.double().T)
+
+
 @pytest.mark.parametrize("offset", [1, 4])
 def test_split_product_of_views(offset):
     """x as columns of a wider matrix, the result into one whose rows do (4) or do not (1) start on 16 bytes."""
