@@ -1,9 +1,11 @@
 // 32-bit matrix products for steps of many tokens on the 5th-generation tensor cores, without giving
 // up precision: y[M, N] = x[M, K] * w[N, K]^T (+ bias[N]), everything float32.
 //
-// A float32 number is exactly the sum of three bfloat16 numbers (8 bits of the significand each, rounded
-// to nearest, what is left goes to the next): x = x0 + x1 + x2, w = w0 + w1 + w2.  Products of bfloat16
-// numbers are exact in the tensor cores, so
+// A float32 number times 2^40 is exactly the sum of three bfloat16 numbers (8 bits of the significand each, rounded
+// to nearest, what is left goes to the next): x = x0 + x1 + x2, w = w0 + w1 + w2.  Without the factor the third
+// part of a number below 2^-109 would fall under bfloat16's smallest step; with it the last bit of the smallest
+// float32 number is 2^-109, and numbers from 2^88 and sums from 2^48 on, which overflow, go the way of infinities (below).
+// Sums are multiplied by 2^-80 when their tile is complete.  Products of bfloat16 numbers are exact in the tensor cores, so
 //     x w = x0 w0 + (x0 w1 + x1 w0) + (x1 w1 + x0 w2 + x2 w0) + ...
 // and what the six products leave out is below 2^-24 of |x w|.  The tensor cores round their running sums
 // towards zero at every step, which over a long k would cost more than float32 does: the accumulator is
@@ -56,6 +58,7 @@ constexpr int F3_THREADS = 128 + 32 * F3_WORKERS;    // and a warp for the plane
 constexpr uint32_t F3_OUT_BOX = 32 * 128;            // a warp's 4 KB: 16 rows of w (64 k-elements), or 32 rows x 32 outputs on their way out
 constexpr uint32_t F3_SMEM = 1024 + F3_STAGES * F3_STAGE + F3_WORKERS * F3_OUT_BOX;
 constexpr uint32_t F3_TMEM = 512;                    // an accumulator of 256 columns per stage
+constexpr float F3_UP = 0x1p40f, F3_DOWN = 0x1p-80f; // of the operands, of their products
 constexpr int F3_RASTER = 8;                         // tiles of rows that run side by side (they share w in L2)
 
 enum { ERR_F3_TMA_WAIT = 41, ERR_F3_MMA_WAIT = 42, ERR_F3_WORKER_WAIT = 43 };
@@ -77,6 +80,9 @@ __device__ __forceinline__ void f3_place(int tile, int m_tiles, int n_tiles, int
     n = in_band / height;
 }
 
+// four floats as they are split: exact, and so are the three parts then
+__device__ __forceinline__ void scale_up(float4& v) { v.x *= F3_UP; v.y *= F3_UP; v.z *= F3_UP; v.w *= F3_UP; }
+
 // the three bfloat16 parts of four floats, as 8 bytes per plane
 __device__ __forceinline__ void split3(const float4& v, uint2 (&plane)[3]) {
     float a[4] = {v.x, v.y, v.z, v.w};
@@ -92,7 +98,7 @@ __device__ __forceinline__ void split3(const float4& v, uint2 (&plane)[3]) {
     }
 }
 
-// planes[p][m][0 .. K) = part p of x[m]; also clears the notes of the tiles to come
+// planes[p][m][0 .. K) = part p of x[m] * F3_UP; also clears the notes of the tiles to come
 __global__ void __launch_bounds__(256)
 gemm_f32_split_rows_kernel(const float* __restrict__ x, long long ldx, bf16* __restrict__ planes, int M, int K,
                            int plane_ld, int* __restrict__ odd, int tiles) {
@@ -104,7 +110,9 @@ gemm_f32_split_rows_kernel(const float* __restrict__ x, long long ldx, bf16* __r
     for (long long q = first; q < quads; q += step) {
         const int m = (int)(q / (K / 4)), k = (int)(q - (long long)m * (K / 4)) * 4;
         uint2 plane[3];
-        split3(*reinterpret_cast<const float4*>(x + m * ldx + k), plane);
+        float4 v = *reinterpret_cast<const float4*>(x + m * ldx + k);
+        scale_up(v);
+        split3(v, plane);
 #pragma unroll
         for (int p = 0; p < 3; ++p)
             *reinterpret_cast<uint2*>(planes + ((size_t)p * M + m) * plane_ld + k) = plane[p];
@@ -229,7 +237,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const float4& v = f[i >> 1][i & 1];
+                    float4& v = f[i >> 1][i & 1];
+                    scale_up(v);
                     bits |= __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w);
                 }
                 // A number whose lower half is zero is a bfloat16 number.  The vote needs every lane's numbers, so
@@ -267,7 +276,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     if (n < p.N) {
                         float* v = sum + q * 32;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) finite = finite && fabsf(v[j]) <= 3.402823466e38f;
+                        for (int j = 0; j < 32; ++j) {
+                            finite = finite && fabsf(v[j]) <= 3.402823466e38f;
+                            v[j] *= F3_DOWN;
+                        }
                         if (p.bias) {
 #pragma unroll
                             for (int j = 0; j < 32; ++j) if (n + j < p.N) v[j] += p.bias[n + j];

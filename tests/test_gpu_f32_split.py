@@ -119,6 +119,24 @@ def test_split_product_of_infinities():
     assert distance(got[quiet][:, keep], exact[:, keep]) < 4e-7
 
 
+@pytest.mark.parametrize("x_power,w_power", [(-115, 0), (0, -118), (-117, -20), (-75, -75), (-140, 40), (60, -130), (70, -70),
+                                             (40, 0), (63, 63), (90, -90), (-120, 100), (127, -127)])
+def test_split_product_of_small_and_large_numbers(x_power, w_power):
+    """Operands of any size, subnormal numbers and results among them: no further off than FFMA, which rounds at every
+    k (a unit of the smallest result beside it); sums that overflow are infinite in both."""
+    torch.manual_seed(x_power + w_power)
+    rows, n, k = 130, 270, 192
+    x = ((torch.rand(rows, k, device="cuda").double() + 1) * 2.0 ** x_power).float()
+    w = (torch.randn(n, k, device="cuda").double() * 2.0 ** w_power).float()
+    assert torch.isfinite(x).all() and torch.isfinite(w).all()
+    got, plain, want = product(x, w), ffma(x, w), x.double() @ w.double().T
+    finite = torch.isfinite(plain)
+    assert torch.equal(torch.isfinite(got), finite)
+    torch.testing.assert_close(got[~finite], plain[~finite], rtol=0, atol=0, equal_nan=True)
+    off = [(v.double() - want)[finite].norm().item() for v in (got, plain)]
+    assert off[0] <= off[1] + 2.0 ** -150 * got.numel() ** 0.5
+
+
 def test_split_product_refuses():
     from from_scratch_inference_engine_b200.kernels.ops import KernelError
     with pytest.raises(KernelError):
