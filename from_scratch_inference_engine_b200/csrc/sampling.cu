@@ -307,6 +307,8 @@ constexpr int CLUSTER = 8;                // blocks that share a row
 // top_k 40 and top_p 0.95 took 259 us for one row and 333 us for 24 with the searches alone, 21 us here.
 // Rows it does not settle get -2 and are left to the kernel that follows: top_k outside 1 .. SHORT_TOP_K,
 // more than SHORT_CANDIDATES tokens (many equal logits), infinite or NaN weights.
+// The limit on k: up to k + k / 8 threads of each of the 8 blocks bring at least a token, 936 of 1,024 places at 104,
+// and some threads bring more than one.
 constexpr int SHORT_TOP_K = 104, SHORT_CANDIDATES = 1024, SHORT_PER_THREAD = 25;
 
 __device__ __forceinline__ float key_value(unsigned key) {
@@ -554,7 +556,7 @@ __device__ __forceinline__ unsigned cluster_ties_needed(const Found& at, float t
 }
 
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS)
-sample_cluster_kernel(const float* __restrict__ logits, int vocab, int slice,
+sample_cluster_kernel(const float* __restrict__ logits, int vocab, int slice, int behind_short,
                       const float* __restrict__ temperature, const int* __restrict__ top_k,
                       const float* __restrict__ top_p, const float* __restrict__ uniform,
                       int* __restrict__ out) {
@@ -567,7 +569,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int vocab, int slice,
     const int rank = (int)cluster.block_rank();
     const int rix = blockIdx.y;
     grid_dependency_wait();
-    if (out[rix] != -2) return;                  // settled; uniform over the cluster: nothing is written before a sync
+    if (behind_short && out[rix] != -2) return;  // settled; uniform over the cluster: nothing is written before a sync
     const float temp = temperature[rix];
     if (!(temp > 0.f)) {                         // uniform over the cluster: no sync is skipped
         if (rank == 0 && threadIdx.x == 0) out[rix] = -1;
@@ -699,10 +701,14 @@ int fsie_argmax_staged(const float* logits, int rows, int vocab, int* out, void*
     return FSIE_LAUNCH_CHECK();
 }
 
-// Rows with temperature <= 0 get -1 (use fsie_argmax for them).
+// The largest top_k whose kept tokens are gathered and sorted.
+int fsie_sample_short_top_k() { return fsie::SHORT_TOP_K; }
+
+// Rows with temperature <= 0 get -1 (use fsie_argmax for them).  short_lists = 0 leaves out the kernel for a
+// short top_k (with no such row it would only say so row by row); the tokens are the same either way.
 int fsie_sample(const float* logits, int rows, int vocab, const float* temperature,
                 const int* top_k, const float* top_p, const float* uniform, int* out,
-                cudaStream_t stream) {
+                int short_lists, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0) return fsie::ERR_BAD_ARGUMENT;
     // a cluster of 8 blocks per row while a slice of the row fits in shared memory (and in registers)
@@ -717,13 +723,15 @@ int fsie_sample(const float* logits, int rows, int vocab, const float* temperatu
             if (e != cudaSuccess) return (int)e;
             configured = true;
         }
-        const int rc = fsie::launch_dependent(fsie::sample_short_kernel, dim3(fsie::CLUSTER, rows),
-                                              dim3(fsie::SAMPLE_THREADS), 0, stream, logits, vocab, slice, temperature,
-                                              top_k, top_p, uniform, out);
-        if (rc != 0) return rc;
+        if (short_lists) {
+            const int rc = fsie::launch_dependent(fsie::sample_short_kernel, dim3(fsie::CLUSTER, rows),
+                                                  dim3(fsie::SAMPLE_THREADS), 0, stream, logits, vocab, slice,
+                                                  temperature, top_k, top_p, uniform, out);
+            if (rc != 0) return rc;
+        }
         return fsie::launch_dependent(fsie::sample_cluster_kernel, dim3(fsie::CLUSTER, rows),
-                                      dim3(fsie::SAMPLE_THREADS), smem, stream, logits, vocab, slice, temperature,
-                                      top_k, top_p, uniform, out);
+                                      dim3(fsie::SAMPLE_THREADS), smem, stream, logits, vocab, slice,
+                                      short_lists ? 1 : 0, temperature, top_k, top_p, uniform, out);
     }
     fsie::sample_kernel<<<rows, fsie::SAMPLE_THREADS, 0, stream>>>(logits, vocab, temperature, top_k,
                                                                   top_p, uniform, out);

@@ -106,10 +106,11 @@ def core():
         lib.fsie_attn_rows16_takes.restype = i
         lib.fsie_argmax.argtypes = [p, i, i, p, p]
         lib.fsie_argmax_staged.argtypes = [p, i, i, p, p, i, p]
-        lib.fsie_sample.argtypes = [p, i, i, p, p, p, p, p, p]
+        lib.fsie_sample.argtypes = [p, i, i, p, p, p, p, p, i, p]
+        lib.fsie_sample_short_top_k.argtypes = []
         for name in ("fsie_embed_gather", "fsie_add_rmsnorm", "fsie_rope_kv_write", "fsie_swiglu",
                      "fsie_gemm_f32", "fsie_attn_generic", "fsie_attn_generic_rows",
-                     "fsie_argmax", "fsie_argmax_staged", "fsie_sample"):
+                     "fsie_argmax", "fsie_argmax_staged", "fsie_sample", "fsie_sample_short_top_k"):
             getattr(lib, name).restype = ctypes.c_int
         _core = lib
     return _core
@@ -982,8 +983,15 @@ def argmax(logits: torch.Tensor, out: torch.Tensor,
     return out
 
 
+def sample_short_top_k() -> int:
+    """The largest top_k whose kept tokens are gathered and sorted instead of searched for."""
+    return int(core().fsie_sample_short_top_k())
+
+
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
-           top_p: torch.Tensor, uniform: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+           top_p: torch.Tensor, uniform: torch.Tensor, out: torch.Tensor, short_lists: bool = True) -> torch.Tensor:
+    """One token per row (-1 where the temperature is not above 0).  `short_lists`: False when the caller knows
+    that no row has a top_k of 1 .. `sample_short_top_k()`: the kernel for those is not launched then."""
     _need(logits, torch.float32, "logits")
     _need(temperature, torch.float32, "temperature")
     _need(top_k, torch.int32, "top_k")
@@ -992,7 +1000,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     _need(out, torch.int32, "out")
     rows, vocab = logits.shape
     _check(core().fsie_sample(_ptr(logits), rows, vocab, _ptr(temperature), _ptr(top_k),
-                              _ptr(top_p), _ptr(uniform), _ptr(out), _stream()), "sample")
+                              _ptr(top_p), _ptr(uniform), _ptr(out), int(short_lists), _stream()), "sample")
     return out
 
 

@@ -51,6 +51,11 @@ def request_seed(engine_seed: int, request_id: int) -> int:
     return _splitmix((engine_seed & _MASK) ^ _splitmix(request_id + 0x51ED270B))
 
 
+def any_short_list(params: Sequence[SamplingParams], longest: int) -> bool:
+    """Whether some row draws from a top_k of at most `longest`, the rows that the sampler's first kernel is for."""
+    return any(not p.greedy and 0 < p.top_k <= longest for p in params)
+
+
 class Picked:
     """The tokens one sampling call chose: on the device at once (`device`, int32 [rows]), on
     the host after `result()`, which waits for the copy that was started with the call."""
@@ -134,7 +139,9 @@ class Sampler:
             staged = self._ring.stage(host.reshape(-1).view(np.int32), self.device).view(5, rows)
             dev = staged.view(torch.float32)
             self.bytes_to_device += host.nbytes
-            ops.sample(logits, dev[0], staged[3], dev[1], dev[2], picks[1])
+            # the first of the sampler's two kernels would find no row to work on (2 to 3 us a step)
+            ops.sample(logits, dev[0], staged[3], dev[1], dev[2], picks[1],
+                       short_lists=any_short_list(params, ops.sample_short_top_k()))
             chosen = torch.where(dev[4] > 0, picks[0], picks[1]) if any_greedy else picks[1]
         else:
             chosen = picks[0]
