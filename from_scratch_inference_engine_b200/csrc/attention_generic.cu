@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "attention_params.cuh"
 #include <math.h>
+#include <type_traits>
 
 namespace fsie {
 
@@ -441,10 +442,13 @@ attn_rows16_kernel(const AttnParams p) {
 // HD / 16 columns (values) in registers, so 8 and 12 16-byte reads serve 64 and 128 fmaf; 16 lanes share
 // four rows from the scores to the result, so a row's maximum and weights never leave their half warp.  What
 // bounds it then is FFMA.  The next keys are copied (cp.async) while the values are summed up, the next values
-// while the scores are; two blocks share an SM.  28 layers of prompts of 167, 500 and 1,000 tokens, 12 heads of
+// while the scores are; two blocks share an SM.  A key that a row does not see adds nothing to it, whatever its value
+// holds (0 times an infinity would be NaN): steps at the edge of what the tile's rows see have a sum of their own that
+// leaves such keys out.  28 layers of prompts of 167, 500 and 1,000 tokens, 12 heads of
 // 128: 850 us a layer before, 182 now (21 TFLOP/s).  Same arguments, key ranges, splits and outputs.
 constexpr int TKEYS = 64;         // keys per step
 constexpr int TTHREADS = 128;
+constexpr int UNSEEN = (int)0x80000000;      // the weight of a key that the row does not see: -0, which expf never gives
 
 template <int HD> constexpr size_t f32_tile_smem() {
     return sizeof(float) * ((size_t)ROWS * HD + (size_t)TKEYS * (HD + 4) + (size_t)TKEYS * HD + (size_t)ROWS * (TKEYS + 4));
@@ -572,7 +576,7 @@ attn_f32_tile_kernel(const AttnParams p) {
             float sum = 0.f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float w = seen[j] && m_new > -INFINITY ? expf(s[i][j] - m_new) : 0.f;
+                const float w = seen[j] && m_new > -INFINITY ? expf(s[i][j] - m_new) : __int_as_float(UNSEEN);
                 ps[(r0 + i) * pld + tx + 16 * j] = w;
                 sum += w;
             }
@@ -585,27 +589,40 @@ attn_f32_tile_kernel(const AttnParams p) {
         fetch(c + 1, kp, ks, kld);
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();                                    // the step's values have landed
+        auto add_values = [&](auto edge) {                  // edge: some row does not see some key
 #pragma unroll 4
-        for (int j = 0; j < TKEYS; j += 4) {
-            float4 w[4];
+            for (int j = 0; j < TKEYS; j += 4) {
+                float4 w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (r0 + i) * pld + j);
+                for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (r0 + i) * pld + j);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-#pragma unroll
-                for (int n = 0; n < NC; ++n) {
-                    const float4 v = *reinterpret_cast<const float4*>(vs + (j + u) * HD + n * 64 + tx * 4);
+                for (int u = 0; u < 4; ++u) {
+                    bool sees[4];
+                    float wi[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float wi = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
-                        acc[i][4 * n] = fmaf(wi, v.x, acc[i][4 * n]);
-                        acc[i][4 * n + 1] = fmaf(wi, v.y, acc[i][4 * n + 1]);
-                        acc[i][4 * n + 2] = fmaf(wi, v.z, acc[i][4 * n + 2]);
-                        acc[i][4 * n + 3] = fmaf(wi, v.w, acc[i][4 * n + 3]);
+                        wi[i] = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+                        sees[i] = !decltype(edge)::value || __float_as_int(wi[i]) != UNSEEN;
+                    }
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) {
+                        const float4 v = *reinterpret_cast<const float4*>(vs + (j + u) * HD + n * 64 + tx * 4);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (!sees[i]) continue;
+                            acc[i][4 * n] = fmaf(wi[i], v.x, acc[i][4 * n]);
+                            acc[i][4 * n + 1] = fmaf(wi[i], v.y, acc[i][4 * n + 1]);
+                            acc[i][4 * n + 2] = fmaf(wi[i], v.z, acc[i][4 * n + 2]);
+                            acc[i][4 * n + 3] = fmaf(wi[i], v.w, acc[i][4 * n + 3]);
+                        }
                     }
                 }
             }
-        }
+        };
+        if (k0 + TKEYS - 1 <= pos_first && k0 + TKEYS <= kend && (p.window <= 0 || k0 > pos_last - p.window))
+            add_values(std::false_type());
+        else
+            add_values(std::true_type());
         __syncthreads();                                    // the values are used up
         fetch(c + 1, vp, vs, HD);
     }

@@ -14,3 +14,18 @@ def test_tiles(ops, hd, heads, kv_heads, window, nsplit):  # noqa: F811
     items = [(0, 63), (0, 64), (0, 65), (63, 2), (127, 33), (64, 1), (190, 31)]
     case = PagedCase(torch.float32, heads, kv_heads, hd, 8, items, window=window, seed=hd + window)
     assert_rows_close(case.run(ops, nsplit), case.want, case, torch.float32)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("heads,kv_heads,window,nsplit", [(2, 2, 0, 1), (6, 1, 0, 1), (12, 2, 40, 1), (7, 1, 0, 2)])
+def test_values_that_a_row_does_not_see(ops, hd, heads, kv_heads, window, nsplit):  # noqa: F811
+    """An infinite value and a NaN key of the last token reach none of the rows before it."""
+    new = 140
+    case = PagedCase(torch.float32, heads, kv_heads, hd, 8, [(0, new)], window=window, seed=hd)
+    want = case.run(ops, nsplit)
+    page, offset = int(case.tables[0, (new - 1) // 8]), (new - 1) % 8
+    case.pages[page, 0, 0, :, offset] = float("nan")
+    case.pages[page, 0, 1, :, offset] = float("inf")
+    got = case.run(ops, nsplit)
+    assert torch.equal(got[:-1], want[:-1])
+    assert not torch.isfinite(got[-1]).any()
