@@ -37,10 +37,11 @@
 // a single one per block and stage by a warp of its own 420 us instead of 380 (1,668 rows of 17,920 x 1,536).
 //
 // A sum with an infinite or NaN input, or one that overflows, would come out as NaN where FFMA gives an
-// infinity (0 * inf among the planes): tiles with such a result are noted and computed again by the FFMA
-// kernel behind this one, which is a launch of one block per SM that finds nothing to do otherwise.
+// infinity (0 * inf among the planes): tiles with such a result are noted, and a launch of one block per SM behind this
+// one, which finds nothing to do otherwise, computes them by FFMA and replaces the results that are not finite.
 //
-// An output does not depend on the other rows of the launch.  Every wait on an mbarrier is bounded.
+// An output does not depend on the other rows of the launch: which of the two kernels it comes from is decided by
+// itself.  Every wait on an mbarrier is bounded.
 #include "common.cuh"
 #include "gemm_f32_tile.cuh"
 #include "tcgen05_pair.cuh"
@@ -276,14 +277,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     if (n < p.N) {
                         float* v = sum + q * 32;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            finite = finite && fabsf(v[j]) <= 3.402823466e38f;
-                            v[j] *= F3_DOWN;
-                        }
+                        for (int j = 0; j < 32; ++j) v[j] *= F3_DOWN;
                         if (p.bias) {
 #pragma unroll
                             for (int j = 0; j < 32; ++j) if (n + j < p.N) v[j] += p.bias[n + j];
                         }
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) finite = finite && fabsf(v[j]) <= 3.402823466e38f;
                         if (p.tma_store) {
                             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                             __syncwarp();
@@ -392,7 +392,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
 }
 
-// The tiles whose results were not finite, computed by FFMA.
+// In tiles with results that are not finite those results, computed by FFMA.
 __global__ void __launch_bounds__(256, 2)
 gemm_f32_odd_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                           float* __restrict__ y, int M, int N, int K, int ldx, int ldy, int m_tiles, int n_tiles,
@@ -407,7 +407,7 @@ gemm_f32_odd_tiles_kernel(const float* __restrict__ x, const float* __restrict__
         const int m0 = mt * F3_TILE + (t & 1) * TM, n0 = nt * F3_TILE + ((t >> 1) & 1) * TN;
         if (m0 >= M || n0 >= N) continue;
         __syncthreads();
-        f32_tile(x, w, bias, y, M, N, K, ldx, ldy, m0, n0);
+        f32_tile<true>(x, w, bias, y, M, N, K, ldx, ldy, m0, n0);
     }
 }
 

@@ -9,7 +9,9 @@ namespace fsie {
 
 constexpr int TM = 128, TN = 128, TK = 16;      // block tile; 256 threads, 8 x 8 outputs each
 
-// The 128 x 128 outputs from (m0, n0) on, by a block of 256 threads.
+// The 128 x 128 outputs from (m0, n0) on, by a block of 256 threads.  REPAIR: of those only the ones that y holds no
+// finite number for.
+template <bool REPAIR = false>
 __device__ __forceinline__ void f32_tile(const float* __restrict__ x, const float* __restrict__ w,
                                          const float* __restrict__ bias, float* __restrict__ y,
                                          int M, int N, int K, int ldx, int ldy, int m0, int n0) {
@@ -87,7 +89,11 @@ __device__ __forceinline__ void f32_tile(const float* __restrict__ x, const floa
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = acc[i][jh * 4 + j] + ((bias && n + j < N) ? bias[n + j] : 0.f);
             float* out = y + (size_t)m * ldy + n;
-            if (n + 3 < N && (((size_t)out) & 15) == 0) {
+            if (REPAIR) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < N && !(fabsf(out[j]) <= 3.402823466e38f)) out[j] = v[j];
+            } else if (n + 3 < N && (((size_t)out) & 15) == 0) {
                 *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
             } else {
 #pragma unroll

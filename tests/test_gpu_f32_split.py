@@ -120,7 +120,7 @@ def test_split_product_of_infinities():
 
 
 @pytest.mark.parametrize("x_power,w_power", [(-115, 0), (0, -118), (-117, -20), (-75, -75), (-140, 40), (60, -130), (70, -70),
-                                             (40, 0), (63, 63), (90, -90), (-120, 100), (127, -127)])
+                                             (40, 0), (22, 22), (23, 24), (63, 63), (90, -90), (-120, 100), (127, -127)])
 def test_split_product_of_small_and_large_numbers(x_power, w_power):
     """Operands of any size, subnormal numbers and results among them: no further off than FFMA, which rounds at every
     k (a unit of the smallest result beside it); sums that overflow are infinite in both."""
@@ -135,6 +135,25 @@ def test_split_product_of_small_and_large_numbers(x_power, w_power):
     torch.testing.assert_close(got[~finite], plain[~finite], rtol=0, atol=0, equal_nan=True)
     off = [(v.double() - want)[finite].norm().item() for v in (got, plain)]
     assert off[0] <= off[1] + 2.0 ** -150 * got.numel() ** 0.5
+
+
+@pytest.mark.parametrize("bias", [False, True])
+def test_rows_beside_infinities_keep_their_bits(bias):
+    """A row with an infinity, a NaN, an overflow in its sums or in its planes changes no bit of the rows beside it."""
+    torch.manual_seed(4)
+    x, w = torch.randn(260, 320, device="cuda"), torch.randn(300, 320, device="cuda")
+    b = torch.randn(300, device="cuda") if bias else None
+    calm = product(x, w, b)
+    rows = torch.ones(260, dtype=torch.bool, device="cuda")
+    for row, value in ((3, float("inf")), (70, float("nan")), (130, 3e38), (131, 1e25), (259, -float("inf"))):
+        x[row, 9], rows[row] = value, False
+    got = product(x, w, b)
+    assert torch.equal(got[rows], calm[rows])
+    assert not torch.isfinite(got[[3, 70, 259]]).any() and not torch.isfinite(got[130]).all()
+    assert torch.isfinite(got[131]).all()                # beyond the room of the planes, not of float32
+    size = x[131].double().abs() @ w.double().abs().T
+    want = x[131].double() @ w.double().T + (b.double() if bias else 0)
+    assert ((got[131].double() - want).abs() <= 2e-6 * size).all()
 
 
 def test_split_product_refuses():
