@@ -205,10 +205,11 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         if (total > 0 && lane == 0) load();
         for (int it = 0; it < total + F3_STAGES; ++it) {
             const int s = it & 1;
+            // (a warp goes on or gives up as one: the votes and shared reads below wait for all of its lanes)
             if (it >= F3_STAGES) {
                 // ---- stage it - 2 has been multiplied: add its accumulator up
-                if (*(volatile int*)&abort_flag) { ok = false; break; }
-                if (!mbar_wait(&done_bar[s], ((it >> 1) - 1) & 1)) {
+                if (__any_sync(0xffffffffu, *(volatile int*)&abort_flag)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(&done_bar[s], ((it >> 1) - 1) & 1))) {
                     atomicExch(p.error, ERR_F3_WORKER_WAIT); atomicExch(&abort_flag, 1); ok = false; break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -224,7 +225,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             }
             if (it < total) {
-                if (!mbar_wait(&raw_bar[worker], it & 1)) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&raw_bar[worker], it & 1))) {
                     atomicExch(p.error, ERR_F3_WORKER_WAIT); atomicExch(&abort_flag, 1); ok = false; break;
                 }
                 unsigned char* to = smem + s * F3_STAGE;
