@@ -1,7 +1,7 @@
 // True 32-bit matrix products for the float32 path: y[M,N] = x[M,K] * w[N,K]^T (+ bias[N]).
 // Plain FFMA on CUDA cores (the reference instead asks its library for strict fp32,
 // src/cuda/device.cu:322-357); steps of many tokens take the product that splits its operands into three
-// bfloat16 parts, which loses nothing of the 32 bits (gemm_f32_tcgen05.cu).  Three kernels:
+// bfloat16 parts, exactly (gemm_f32_tcgen05.cu), unless k is short.  Three kernels:
 //
 //  * gemm_f32_rows_kernel - steps of few tokens (M <= 48, in tiles of up to 16 rows).  The
 //    product is bound by reading w once from HBM, so a warp owns R rows of w and streams them
@@ -9,7 +9,7 @@
 //    memory and every x value read from there is used for R rows of w.  A lane's partial sums
 //    run over k in ascending order and the 32 lanes are then added in a fixed tree, so an
 //    output does not depend on how many other rows share the launch.
-//  * gemm_f32_tiles_kernel - more rows than that, by name: tiles of 128 x 128 outputs, k in steps of 16 through
+//  * gemm_f32_tiles_kernel - more rows than that, k below about 128: tiles of 128 x 128 outputs, k in steps of 16 through
 //    shared memory, 8 x 8 outputs per thread in registers.  Each output is one thread's sum over
 //    k in ascending order.
 //  * gemm_f32_plain_kernel - any sizes and alignments (k no multiple of 4, unaligned rows).

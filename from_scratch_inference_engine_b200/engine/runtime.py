@@ -24,6 +24,27 @@ def parse_dtype(name) -> torch.dtype:
         raise ValueError(f"unknown dtype '{name}' (bfloat16 or float32)") from None
 
 
+def f32_split_pays(rows: int, n: int, k: int, sm_count: int) -> bool:
+    """Whether a float32 product [rows, k] x [n, k] is one for the tensor cores (three bfloat16 parts per operand) and
+    not for FFMA: faster, and no further off from 64 bits."""
+    if rows > ops.GEMM_F32_FEW_ROWS:
+        # Against FFMA tiles (us, split / FFMA: 49 rows of 192 x 192 24 / 31, of 1,536 x 8,960 245 / 1,045, of 37,888 x
+        # 3,584 229 / 844; 1,668 rows of 1,536 x 8,960 304 / 1,856, of 37,888 x 3,584 1,715 / 11,329).  Its three launches
+        # take 15 to 20 whatever k is, FFMA's one 8 to 9 and 2 for every 16 k-elements: 49 rows of 64 x 16 15 / 9, 2,048 of
+        # 1,024 x 96 23 / 20, x 128 22 / 25; with tiles for many rounds the lines cross sooner: 300 rows of 16,384 x 32
+        # 24 / 23, x 48 26 / 30, 2,048 of 4,096 x 32 26 / 26, x 48 26 / 33.  Errors against 64 bits, over the sums of |x w|
+        # (normal operands; positive ones): k = 4 3.1e-8 / 2.7e-8 (4.7e-8 / 3.6e-8), 48 and up below FFMA's: 64
+        # 1.5e-8 / 2.8e-8 (9.2e-8 / 1.2e-7), 1,536 4.9e-9 / 2.8e-8 (1.1e-7 / 5.3e-7).
+        return k >= 128 or (k >= 48 and rows * n >= 4 << 20)
+    # Against the FFMA kernel for few rows.  A tile of 256 columns takes as long whatever its rows (2 us per 64
+    # k-elements), so it takes columns for half of the pairs of SMs: 17 and 48 rows of 17,920 x 1,536 57 / 119 and
+    # 57 / 179, of 4,096 x 4,096 119 / 64 and 119 / 94; up to 16 rows the FFMA kernel reads w once and is level (16 rows
+    # of 17,920 x 1,536 58 / 66) or ahead.  Errors as above: that kernel's 32 partial sums are shorter, so k = 64 1.5e-8 /
+    # 1.3e-8, 256 8.6e-9 / 8.0e-9, level at 512, 1,536 4.9e-9 / 5.6e-9, 8,960 3.8e-9 / 5.1e-9 (positive operands, whose
+    # truncated sums all err to one side: 1,536 1.1e-7 / 3.7e-8).
+    return rows >= 17 and k >= 512 and 2 * -(-n // ops.GEMM_F32_SPLIT_COLUMNS) >= sm_count // 2
+
+
 class Runtime:
     """Device and precision of one engine, and which kernel multiplies which step.
 
@@ -32,8 +53,8 @@ class Runtime:
     256 x 256 output tiles to fill the GPU take the engine's tiled tcgen05 product, and the
     steps in between take the library product (cuBLAS through torch, bf16 operands, 32-bit
     accumulation), as the reference engine uses the library for its products
-    (src/cuda/device.cu:322-357).  float32: every product by the engine's own FFMA kernel,
-    no tensor-core mode.  Everything that is not a plain matrix product is a kernel of
+    (src/cuda/device.cu:322-357).  float32: every product by the engine's own kernels, FFMA for few
+    tokens and tcgen05 over operands in three bfloat16 parts for many (`f32_split_pays`).  Everything that is not a plain matrix product is a kernel of
     this package in both modes.
     """
 
@@ -211,14 +232,7 @@ class Runtime:
         tokens, else FFMA."""
         rows, (n, k) = x.shape[0], weight.shape
         out = self.buffer(tag, rows, n, torch.float32)
-        # Beyond the rows of the FFMA kernel for few rows the tensor cores won at every size measured (us, split /
-        # FFMA tiles: 49 rows of 192 x 192 16 / 27, of 1,536 x 8,960 245 / 1,045, of 37,888 x 3,584 229 / 844; 1,668
-        # rows of 1,536 x 8,960 304 / 1,856, of 37,888 x 3,584 1,715 / 11,329).  Below, a tile of 256 columns takes as
-        # long whatever its rows (2 us per 64 k-elements), so it takes columns for half of the pairs of SMs: 17 and
-        # 48 rows of 17,920 x 1,536 57 / 119 and 57 / 179, of 4,096 x 4,096 119 / 64 and 119 / 94; up to 16 rows the
-        # FFMA kernel reads w once and is level (16 rows of 17,920 x 1,536 58 / 66) or ahead.
-        least = 17 if 2 * -(-n // ops.GEMM_F32_SPLIT_COLUMNS) >= self.sm_count // 2 else ops.gemm_f32_rows_limit() + 1
-        if rows < least or not ops.gemm_f32_split_takes(x, weight):
+        if not f32_split_pays(rows, n, k, self.sm_count) or not ops.gemm_f32_split_takes(x, weight):
             return ops.gemm_f32(x, weight, bias, out)
         planes, notes = ops.gemm_f32_split_room(rows, n, k)
         return ops.gemm_f32_split(x, weight, bias, out,

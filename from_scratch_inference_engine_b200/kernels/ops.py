@@ -260,6 +260,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]
     return out
 
 
+GEMM_F32_FEW_ROWS = 48            # what `gemm_f32_rows_limit` says, for rules that are asked without a GPU
 GEMM_F32_SPLIT_COLUMNS = 256      # columns of a tile of `gemm_f32_split`
 _gemm_f32_split = None
 

@@ -162,3 +162,20 @@ def test_split_product_refuses():
         product(torch.randn(64, 6, device="cuda"), torch.randn(8, 6, device="cuda"))
     with pytest.raises(KernelError):
         product(torch.randn(64, 13, device="cuda")[:, 1:9], torch.randn(8, 8, device="cuda"))
+
+
+@pytest.mark.parametrize("rows,n,k", [(49, 64, 16), (64, 16384, 4), (300, 5000, 8), (2048, 4096, 32), (17, 17920, 64),
+                                      (48, 17920, 256)])
+@pytest.mark.parametrize("sign", ["normal", "positive"])
+def test_products_over_a_short_k_lose_nothing(rows, n, k, sign):
+    """What a step's product of these sizes gives is no further from 64 bits than FFMA (whichever of its kernels
+    takes the rows), also where the sums of a stage, truncated, would be."""
+    from from_scratch_inference_engine_b200.engine.runtime import Runtime
+    from from_scratch_inference_engine_b200.kernels import ops
+    torch.manual_seed(rows + k)
+    x, w = torch.randn(rows, k, device="cuda"), torch.randn(n, k, device="cuda")
+    if sign == "positive":
+        x, w = x.abs(), w.abs()
+    want = x.double() @ w.double().T
+    got = Runtime(dtype="float32").linear(x, w, None)
+    assert distance(got, want) <= distance(ops.gemm_f32(x, w, None), want)
