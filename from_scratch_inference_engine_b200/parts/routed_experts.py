@@ -12,6 +12,22 @@ from ..weights.tensor_spec import TensorSpec
 from .base import Part, build_part, register_part
 
 
+def streaming_pays(dtype: torch.dtype, pairs: int, experts: int) -> bool:
+    """Whether a step's (token, choice) pairs take the products that stream the experts' matrices, in tiles of 16
+    rows, and not those in tiles of 64.  The host knows the average of rows per expert, not how the router spreads
+    them.  Measured on 64 experts of 1,408 x 2,048 and 16 of 4,096 x 2,048 (both products, us, streaming / tiled), for
+    even routing, for choices by a power law, and for the worst: every token the same six (two) experts.
+
+    bfloat16, 64 experts: 4 rows on average 202 / 286, 178 / 247, 77 / 126; 12 rows 237 / 312, 267 / 327, 167 / 185; 16
+    rows 286 / 325, 317 / 349, 222 / 187; 20 rows 351 / 341, 355 / 368, 284 / 214 - an expert of many rows has its
+    matrices read once per 16 of them.  16 experts, 20 rows: 251 / 316, 259 / 339, 194 / 267.
+    float32, 64 experts: 16 rows 1,206 / 2,957, 1,238 / 3,148, 1,073 / 1,069; 32 rows 2,252 / 2,962, 2,262 / 3,557, 2,106 /
+    1,683, about 65 a row, so level at 40; 16 experts, 32 rows: 1,562 / 2,496, 1,533 / 2,815, 1,457 / 1,613."""
+    if dtype is torch.float32:
+        return pairs <= 32 * experts
+    return pairs <= 12 * experts or (pairs <= 20 * experts and pairs <= 768)
+
+
 @register_part("feed_forward", "routed_experts")
 class RoutedExperts(Part):
     """`experts` gated feed-forwards down(act(gate y) * (up y)) without biases, of which a token
@@ -35,18 +51,13 @@ class RoutedExperts(Part):
     its (token, choice) pairs by expert on the device and runs the two products over tiles of rows
     that share an expert, so it launches the same kernels whatever the router says: tiles of 16
     rows through kernels that stream the experts' matrices while an expert meets few rows on average
-    (`FEW_MAX_ROWS`), tiles of 64 through the mma.sync / FFMA kernels beyond that, or - bfloat16 steps with at least `GROUPED_MIN_ROWS`
+    (`streaming_pays`), tiles of 64 through the mma.sync / FFMA kernels beyond that, or - bfloat16 steps with at least `GROUPED_MIN_ROWS`
     rows per expert on average - the tokens' rows gathered into a layout in which every expert's
     rows start on a multiple of 256, and the grouped form of the tiled tcgen05 product (SwiGLU in
     its epilogue) over it.  `names` gives the tensor names below the prefix ("expert" takes the
     expert's index).
     """
 
-    # Average rows per expert up to which the products that stream the matrices are taken.  Measured on 64
-    # experts of 1,408 x 2,048 (both products, us, streaming / tiled): bfloat16 at 4 rows 185 / 314 (6 rows), at 16 287 /
-    # 342 - 17 rows are two tiles of 16; float32 at 6 rows 631 / 2,964, at 24 1,757 / 2,968 - there the streaming
-    # kernel's time grows by about 65 us a row and meets the tiled one's at about 40.
-    FEW_MAX_ROWS = {torch.bfloat16: 20, torch.float32: 32}
     GROUPED_MIN_ROWS = 32       # average rows per expert from which the tcgen05 form is taken
 
     NAMES = {"expert": "e{index}.", "gate": "gate", "up": "up", "down": "down", "router": "router",
@@ -171,7 +182,7 @@ class RoutedExperts(Part):
             expert_out = rt.buffer("routed.expert_out", rows, self.hidden_size, y.dtype)
             ops.gemm_tiles_grouped(down, act, expert_out, lists[2], lists[4], ctx.error, rt.sm_count)
             return ops.moe_combine(expert_out, weights, shared, out, top, place=lists[5], **identity)
-        few = (pairs <= self.FEW_MAX_ROWS[y.dtype] * self.experts
+        few = (streaming_pays(y.dtype, pairs, self.experts)
                and ops.moe_few_fits(y, self.hidden_size, self.intermediate_size))
         tile = ops.moe_few_tile_rows() if few else ops.moe_tile_rows()
         lists = ops.moe_align(ids, pairs, self.experts,
