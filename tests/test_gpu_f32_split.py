@@ -1,5 +1,5 @@
-"""The float32 product on the tensor cores (operands in three bfloat16 parts) against 64-bit products: no
-further off than the FFMA kernel, at the edges of tiles, stages and rounds of tiles, and with numbers that
+"""The float32 product on the tensor cores (operands in three bfloat16 parts) against 64-bit products: over more than
+one stage of k no further off than the FFMA kernel, at the edges of tiles, stages and rounds of tiles, and with numbers that
 the parts cannot hold."""
 
 import pytest
@@ -52,20 +52,22 @@ def test_split_product(rows, n, k, held):
         x *= torch.exp(4 * torch.randn(rows, 1, device="cuda"))
     want = x.double() @ w.double().T
     got = product(x, w)
-    # Errors are measured against the sums of |x w|: where a sum cancels, what is left of it says nothing.  Never
-    # further off than FFMA; where k is one stage or less and FFMA has next to no error, the four truncated steps
-    # of a stage may show: 4 x 2^-23 at most, half of that on average.
+    # Errors are measured against the sums of |x w|: where a sum cancels, what is left of it says nothing.  Over more
+    # than one stage of k never further off than FFMA; within one, where FFMA has next to no error, the four truncated
+    # steps of the stage may show: 4 x 2^-23 at most, half of that on average.
     size = x.abs().double() @ w.abs().double().T
+    allowed = 2.0 ** -22 if k <= 64 else 0.0
 
     def off(got, want, size):
         return ((got.double() - want).norm() / size.norm()).item()
-    assert off(got, want, size) <= max(off(ffma(x, w), want, size), 2.0 ** -22)
-    # no single output is far off either
-    assert ((got.double() - want).abs() / size).max().item() < 2e-6
+    assert off(got, want, size) <= max(off(ffma(x, w), want, size), allowed)
+    # no single output is far off either: of operands of both signs by the steps of a stage and its sum, of positive ones,
+    # whose stages all err to one side, by a few more roundings of a long sum
+    assert ((got.double() - want).abs() / size).max().item() < (2e-6 if held == "positive" else 5 * 2.0 ** -23)
     size = size + bias.double().abs()
     biased = product(x, w, bias, blocks=6 if rows < 1000 else BLOCKS)   # three pairs: several tiles each
     want += bias.double()
-    assert off(biased, want, size) <= max(off(ffma(x, w, bias), want, size), 2.0 ** -22)
+    assert off(biased, want, size) <= max(off(ffma(x, w, bias), want, size), allowed)
     alone = product(x[rows // 2:rows // 2 + 1].contiguous(), w)
     assert torch.equal(alone[0], got[rows // 2])
 
