@@ -3,8 +3,9 @@
     python -m from_scratch_inference_engine_b200.kernels.microbench KERNEL [options]
 
 KERNEL: attention_decode, attention_prefill, add_rmsnorm, rope_kv_write, swiglu, argmax,
-sample, linear (the library product as the engine calls it), gemm_f32, gemm_decode,
-gemm_decode_swiglu, gemm_tiles, gemm_tiles_swiglu (the engine's own tcgen05 products),
+sample, linear (the library product as the engine calls it), gemm_f32 (the kernel that the engine takes for the
+size, or --f32-kind), gemm_decode, gemm_decode_swiglu, gemm_tiles, gemm_tiles_swiglu (the engine's own tcgen05
+products), gemm_skinny, gemm_skinny_swiglu (steps of few tokens against small matrices),
 sum_layernorm, routed_experts (every kernel of a feed-forward of routed experts, one line for all),
 state_space (every kernel of a state-space mixer, and the same scan with one decay per head beside it),
 stream_norm (a residual of --streams streams settled, gathered and normed), scaled_attention (capped scores
@@ -234,7 +235,9 @@ def run_routed_experts(args, timer, dtype):
     """Every kernel of a feed-forward of routed experts at --tokens, --hidden, --inter (an expert's
     width), --experts, --top, --groups, --keep with a random router: ms, and the share of the
     measured peak that the work a token asks for (no padding rows counted) reaches.  Steps with at
-    least 32 rows per expert take the grouped tcgen05 products, others the tiles of 64 rows."""
+    least 32 rows per expert take the grouped tcgen05 products, others the products that stream the
+    matrices or (`--tiles-of-64`, and where `streaming_pays` says so) the tiles of 64 rows."""
+    from ..parts.routed_experts import streaming_pays
     g = torch.Generator(device="cuda").manual_seed(0)
     rand = lambda *shape: torch.randn(shape, generator=g, device="cuda", dtype=torch.float32)
     elem = 2 if dtype is torch.bfloat16 else 4
@@ -286,18 +289,20 @@ def run_routed_experts(args, timer, dtype):
              (pairs + 2 * tokens) * h * elem, 2.0 * pairs * h)
         extra = {"rows_with_padding": padded}
     else:
-        buffer = torch.zeros(ops.moe_lists_size(pairs, experts), dtype=torch.int32, device="cuda")
-        lists = ops.moe_align(ids, pairs, experts, buffer)
-        note("moe_align", timer(lambda: ops.moe_align(ids, pairs, experts, buffer)), pairs * 8, 0.0)
+        few = streaming_pays(dtype, pairs, experts) and ops.moe_few_fits(y, h, f) and not args.tiles_of_64
+        tile = ops.moe_few_tile_rows() if few else ops.moe_tile_rows()
+        buffer = torch.zeros(ops.moe_lists_size(pairs, experts, tile), dtype=torch.int32, device="cuda")
+        lists = ops.moe_align(ids, pairs, experts, buffer, tile)
+        note("moe_align", timer(lambda: ops.moe_align(ids, pairs, experts, buffer, tile)), pairs * 8, 0.0)
         act = torch.empty(pairs, f, dtype=dtype, device="cuda")
-        note("moe_product gate,up", timer(lambda: ops.moe_product(y, w_gu, act, lists, pairs, top, True, "silu")),
+        note("moe_product gate,up", timer(lambda: ops.moe_product(y, w_gu, act, lists, pairs, top, True, "silu", tile=tile)),
              (used * 2 * f * h + tokens * h + pairs * f) * elem, 2.0 * pairs * 2 * f * h)
         expert_out = torch.empty(pairs, h, dtype=dtype, device="cuda")
-        note("moe_product down", timer(lambda: ops.moe_product(act, w_d, expert_out, lists, pairs, top, False)),
+        note("moe_product down", timer(lambda: ops.moe_product(act, w_d, expert_out, lists, pairs, top, False, tile=tile)),
              (used * f * h + pairs * (h + f)) * elem, 2.0 * pairs * f * h)
         note("moe_combine", timer(lambda: ops.moe_combine(expert_out, weights, shared, out, top)),
              (pairs + 2 * tokens) * h * elem, 2.0 * pairs * h)
-        extra = {}
+        extra = {"rows_per_tile": tile}
     print(json.dumps(dict({"kernel": "routed_experts", "dtype": args.dtype, "tokens": tokens, "hidden": h,
                            "inter": f, "experts": experts, "top": top, "groups": [args.groups, args.keep],
                            "experts_used": used, "error": int(error.item()), "peaks": peak["source"],
@@ -478,7 +483,9 @@ def run(args):
             ones = torch.ones(args.tokens, device="cuda")
             k = torch.full((args.tokens,), args.top_k, dtype=torch.int32, device="cuda")
             u = torch.rand(args.tokens, generator=g, device="cuda")
-            ms = timer(lambda: ops.sample(logits, ones * 0.8, k, ones * args.top_p, u, out))
+            temperature, top_p = ones * 0.8, ones * args.top_p
+            short = 0 < args.top_k <= ops.sample_short_top_k()
+            ms = timer(lambda: ops.sample(logits, temperature, k, top_p, u, out, short_lists=short))
         nbytes, flops = args.tokens * args.vocab * 4, float(args.tokens * args.vocab)
     elif args.kernel in ("gemm_decode", "gemm_decode_swiglu"):
         m, n, k = args.tokens, args.n, args.k
@@ -499,6 +506,12 @@ def run(args):
         out = torch.empty((m, n), dtype=dtype, device="cuda")
         ms = timer(lambda: ops.gemm_skinny(w, x, out, None))
         nbytes, flops = (m * k + n * k + m * n) * elem, 2.0 * m * n * k
+    elif args.kernel == "gemm_skinny_swiglu":
+        m, n, k = args.tokens, args.n, args.k
+        x, w = rand(m, k).to(dtype), (rand(2 * n, k) / math.sqrt(k)).to(dtype)
+        out = torch.empty((m, n), dtype=dtype, device="cuda")
+        ms = timer(lambda: ops.gemm_skinny_swiglu(w, x, out))
+        nbytes, flops = (m * k + 2 * n * k + m * n) * elem, 4.0 * m * n * k
     elif args.kernel in ("gemm_tiles", "gemm_tiles_swiglu"):
         m, n, k = args.tokens, args.n, args.k
         swiglu = args.kernel == "gemm_tiles_swiglu"
@@ -522,10 +535,28 @@ def run(args):
             x, w = rand(m, k).to(dtype), rand(n, k).to(dtype)
             ms = timer(lambda: torch.nn.functional.linear(x, w))
         else:
+            from ..engine.runtime import f32_split_pays
             x, w = rand(m, k), rand(n, k)
-            ms = timer(lambda: ops.gemm_f32(x, w, None, kind=args.f32_kind, rows_per_warp=args.f32_rows_per_warp))
+            if args.bf16_weight:
+                w = w.bfloat16().float()
+            sms = torch.cuda.get_device_properties(0).multi_processor_count
+            kind = args.f32_kind
+            if kind == "auto" and f32_split_pays(m, n, k, sms) and ops.gemm_f32_split_takes(x, w):
+                kind = "split"
+            out = torch.empty((m, n), device="cuda")
             elem = 4
-            extra = {"frac_ffma": round(2.0 * m * n * k / (ms * 1e-3) / 74.4e12, 3), "f32_kind": args.f32_kind}
+            if kind == "split":
+                planes, notes = ops.gemm_f32_split_room(m, n, k)
+                planes = torch.empty(planes, dtype=torch.bfloat16, device="cuda")
+                notes = torch.empty(notes, dtype=torch.int32, device="cuda")
+                error = torch.zeros(1, dtype=torch.int32, device="cuda")
+                ms = timer(lambda: ops.gemm_f32_split(x, w, None, out, planes, notes, error, sms))
+                products = 3 if args.bf16_weight else 6
+                extra = {"f32_kind": kind, "bf16_products": products, "error": int(error.item()),
+                         "frac_split": round(products * 2.0 * m * n * k / (ms * 1e-3) / 1e12 / peaks()["bf16_tflops"], 3)}
+            else:
+                ms = timer(lambda: ops.gemm_f32(x, w, None, out, kind=kind, rows_per_warp=args.f32_rows_per_warp))
+                extra = {"frac_ffma": round(2.0 * m * n * k / (ms * 1e-3) / 74.4e12, 3), "f32_kind": kind}
         nbytes, flops = (m * k + n * k + m * n) * elem, 2.0 * m * n * k
     elif args.kernel == "routed_experts":
         return run_routed_experts(args, timer, dtype)
@@ -576,7 +607,8 @@ def run(args):
               "frac_hbm": round(gbs / peak["hbm_gbs"], 3),
               "frac_bf16": round(tflops / peak["bf16_tflops"], 3), "peaks": peak["source"],
               "sizes": {k: v for k, v in vars(args).items()
-                        if k not in ("kernel", "dtype", "warmup", "iters", "no_flush", "f32_kind", "f32_rows_per_warp")}}
+                        if k not in ("kernel", "dtype", "warmup", "iters", "no_flush", "f32_kind", "f32_rows_per_warp",
+                                     "bf16_weight")}}
     record.update(extra)
     print(json.dumps(record))
 
@@ -620,13 +652,18 @@ def main(argv=None) -> int:
     parser.add_argument("--keep", type=int, default=4)
     parser.add_argument("--no-grouped", action="store_true",
                         help="routed_experts: tiles of 64 rows also where the grouped products would run")
+    parser.add_argument("--tiles-of-64", action="store_true",
+                        help="routed_experts: tiles of 64 rows also where the matrices would be streamed")
     parser.add_argument("--variant", default="mma", choices=["mma", "tc", "rows16", "whole_tiles"],
                         help="bfloat16 attention: mma.sync with cp.async loads, or tcgen05; float32 "
                              "attention: rows16 takes the kernel for tiles of up to 16 rows; gemm_tiles: "
                              "whole_tiles leaves a partial last round of tiles to the pairs it falls to")
-    parser.add_argument("--f32-kind", default="auto", choices=["auto", "rows", "tiles", "plain"],
+    parser.add_argument("--f32-kind", default="auto", choices=["auto", "rows", "tiles", "plain", "split"],
                         help="gemm_f32: which of the float32 kernels (frac_ffma is of the nominal "
-                             "74.4 TFLOP/s: 148 SMs x 128 lanes x 2 x 1.965 GHz)")
+                             "74.4 TFLOP/s: 148 SMs x 128 lanes x 2 x 1.965 GHz; frac_split counts "
+                             "the bfloat16 products of the split form against the bf16 peak)")
+    parser.add_argument("--bf16-weight", action="store_true",
+                        help="gemm_f32: a weight of bfloat16 numbers (three products instead of six)")
     parser.add_argument("--f32-rows-per-warp", type=int, default=0, choices=[0, 1, 2, 4])
     parser.add_argument("--top-k", type=int, default=0)
     parser.add_argument("--top-p", type=float, default=1.0)
