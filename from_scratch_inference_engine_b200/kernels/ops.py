@@ -298,9 +298,9 @@ def gemm_f32_split_room(rows: int, n: int, k: int) -> Tuple[int, int]:
 
 def gemm_f32_split(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
                    planes: torch.Tensor, notes: torch.Tensor, error: torch.Tensor, blocks: int) -> torch.Tensor:
-    """out = x @ weight.T (+ bias), all float32, on the tensor cores: operands as exact sums of three
-    bfloat16 numbers, 64 k-elements at a time summed up in float32 registers (results that are not finite
-    come from the FFMA kernel).  planes and notes of the sizes `gemm_f32_split_room` names; `blocks`:
+    """out = x @ weight.T (+ bias), all float32, on the tensor cores: operands (times 2^40) as exact sums of
+    three bfloat16 numbers, 64 k-elements at a time summed up in float32 registers (results that are not
+    finite come from the FFMA kernel).  planes and notes of the sizes `gemm_f32_split_room` names; `blocks`:
     size of the persistent grid."""
     _need(x, torch.float32, "x", contiguous=False)
     _need(weight, torch.float32, "weight")
