@@ -18,7 +18,7 @@
 // 17,920 x 1,536 376 (244) and 2,258 (41); of 1,536 x 8,960 304 and 1,856 (42 tiles for 74 pairs); 512 rows of
 // 37,888 x 3,584 514 (270) and 3,379.  Where all numbers of w in a stage are bfloat16 numbers (a checkpoint stored
 // as such), the second and third part of w are zero and the three products with them are left out: 295 to 310 us
-// instead of 362 to 386, by the box; every stage finds that out for itself.
+// instead of 362 to 386; every stage finds that out for itself.
 //
 // x is split by a kernel of its own into three planes (it is small and every tile of columns reads it); w,
 // which would be 1.5 times itself as planes, is split on its way into shared memory.  Two blocks (a
