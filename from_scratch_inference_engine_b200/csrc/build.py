@@ -14,13 +14,16 @@ from __future__ import annotations
 import ctypes
 import fcntl
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
+import types
 from pathlib import Path
 from typing import Dict, Iterable, Sequence, Tuple
 
@@ -188,8 +191,80 @@ def load_library(name: str, defines: Sequence[str] = ()) -> ctypes.CDLL:
         return _loaded[key]
 
 
+_host_call = None
+
+
+class _PlainCalls:
+    """What `host_call` gives where it cannot be compiled (no headers of this Python, another processor): the same calls through
+    ctypes, several times slower."""
+
+    @staticmethod
+    def fits(tensor, dtype, contiguous) -> bool:
+        return tensor.is_cuda and (dtype is None or tensor.dtype is dtype) and (not contiguous or tensor.is_contiguous())
+
+
+def host_call():
+    """The extension module host_call.cpp, compiled at first use; `_PlainCalls` where that fails."""
+    global _host_call
+    with _lock:
+        if _host_call is None:
+            try:
+                _host_call = _load_host_call()
+            except (BuildError, ImportError, OSError) as error:
+                _say(f"the calls into the kernels go through ctypes, which costs a short prompt about a quarter of its time: {error}")
+                _host_call = _PlainCalls
+    return _host_call
+
+
+def _load_host_call():
+    source = CSRC / "host_call.cpp"
+    include, suffix = sysconfig.get_paths()["include"], sysconfig.get_config_var("EXT_SUFFIX") or ".so"
+    tag = hashlib.sha256(source.read_bytes() + f"{suffix} {sys.version}".encode()).hexdigest()[:16]
+    out_dir = _build_dir()
+    target = out_dir / f"fsie_host_call-{tag}.so"
+    if not target.exists():
+        compiler = next((c for c in (os.environ.get("CXX"), shutil.which("g++"), shutil.which("c++")) if c), None)
+        if compiler is None:
+            raise BuildError("no C++ compiler")
+        handle, partial = tempfile.mkstemp(suffix=".so", dir=str(out_dir))
+        os.close(handle)
+        try:
+            _run_with_progress([[compiler, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", include, str(source), "-o", partial]],
+                               "host_call")
+            os.chmod(partial, 0o755)
+            os.replace(partial, target)
+        finally:
+            if os.path.exists(partial):
+                os.unlink(partial)
+    spec = importlib.util.spec_from_file_location("host_call", str(target))
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+def fast_calls(lib: ctypes.CDLL):
+    """The entry points of a library whose argument types are declared, as callables that take ints, floats, None and
+    tensors (for their addresses).  One with other argument types stays ctypes' own."""
+    kinds = {ctypes.c_int: "i", ctypes.c_longlong: "i", ctypes.c_void_p: "i", ctypes.c_float: "f"}
+    module, calls = host_call(), types.SimpleNamespace()
+    for name, function in vars(lib).items():
+        if not isinstance(function, lib._FuncPtr):
+            continue
+        signature = "".join(kinds.get(kind, "?") for kind in function.argtypes or ())
+        if function.argtypes is None or "?" in signature or function.restype is not ctypes.c_int:
+            call = function
+        elif module is _PlainCalls:
+            def call(*args, _function=function):
+                return _function(*(arg.data_ptr() if hasattr(arg, "data_ptr") else arg for arg in args))
+        else:
+            call = module.Function(ctypes.cast(function, ctypes.c_void_p).value, signature, name)
+        setattr(calls, name, call)
+    return calls
+
+
 def build_all() -> None:
     """Compile every library in its default form (the build check of the package)."""
+    host_call()
     for name in LIBRARIES:
         for defines in DEFAULT_SPECIALISATIONS.get(name, [()]):
             library_path(name, defines)

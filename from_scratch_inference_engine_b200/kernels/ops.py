@@ -1,8 +1,8 @@
 """Typed Python entry points of the hand-written CUDA kernels.
 
 Each function checks what the kernel assumes (device, dtype, contiguity, sizes),
-passes raw pointers and the current CUDA stream to the C entry point, and raises on
-any non-zero return.  There is no other implementation behind these functions: on a
+passes the tensors' addresses and the current CUDA stream to the C entry point (`build.fast_calls`: without ctypes),
+and raises on any non-zero return.  There is no other implementation behind these functions: on a
 machine without the compiled library or without a GPU they raise.
 """
 
@@ -33,11 +33,6 @@ def _tag(dtype: torch.dtype) -> int:
     raise KernelError(f"kernels take float32 or bfloat16 storage, not {dtype}")
 
 
-def _ptr(tensor: Optional[torch.Tensor]) -> Optional[int]:
-    """The address for a pointer argument (ctypes takes an int or None for c_void_p)."""
-    return None if tensor is None else tensor.data_ptr()
-
-
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
@@ -51,15 +46,17 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+_fits = build.host_call().fits
+
+
 def _need(tensor: torch.Tensor, dtype, name: str, contiguous: bool = True) -> None:
-    if tensor.is_cuda and (dtype is None or tensor.dtype is dtype) and (not contiguous or tensor.is_contiguous()):
+    if _fits(tensor, dtype, contiguous):
         return
     if not tensor.is_cuda:
         raise KernelError(f"{name} must live on the GPU (the engine has no CPU path)")
     if dtype is not None and tensor.dtype is not dtype:
         raise KernelError(f"{name} must be {dtype}, got {tensor.dtype}")
-    if contiguous and not tensor.is_contiguous():
-        raise KernelError(f"{name} must be contiguous")
+    raise KernelError(f"{name} must be contiguous")
 
 
 launches = 0      # kernel launches issued through this module (benchmarks read this)
@@ -112,7 +109,7 @@ def core():
                      "fsie_gemm_f32", "fsie_attn_generic", "fsie_attn_generic_rows",
                      "fsie_argmax", "fsie_argmax_staged", "fsie_sample", "fsie_sample_short_top_k"):
             getattr(lib, name).restype = ctypes.c_int
-        _core = lib
+        _core = build.fast_calls(lib)
     return _core
 
 
@@ -128,8 +125,8 @@ def embed_gather(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor,
     tokens, (vocab, hidden) = ids.numel(), table.shape
     if out.shape[-1] != hidden or out.numel() < tokens * hidden:
         raise KernelError("embed_gather: out is too small")
-    _check(core().fsie_embed_gather(_ptr(ids), _ptr(table), _ptr(out), tokens, hidden, vocab,
-                                    float(scale), _tag(table.dtype), _ptr(error), _stream()), "embed_gather")
+    _check(core().fsie_embed_gather(ids, table, out, tokens, hidden, vocab,
+                                    float(scale), _tag(table.dtype), error, _stream()), "embed_gather")
     return out
 
 
@@ -161,8 +158,8 @@ def add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], gain: torch.Tens
         count = x.numel() // hidden
     if out.numel() < count * hidden:
         raise KernelError("add_rmsnorm: out is too small")
-    _check(core().fsie_add_rmsnorm(_ptr(x), _ptr(delta), _ptr(gain),
-                                   int(gain.dtype is torch.float32), _ptr(out), _ptr(rows), count,
+    _check(core().fsie_add_rmsnorm(x, delta, gain,
+                                   int(gain.dtype is torch.float32), out, rows, count,
                                    hidden, float(eps), int(write_x), _tag(out.dtype), _stream()),
            "add_rmsnorm")
     return out
@@ -192,10 +189,10 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Ten
         _need(slot_of, torch.int32, "slot_of")
         if k_pages.dtype is not qkv.dtype or v_pages.dtype is not qkv.dtype:
             raise KernelError("rope_kv_write: cache dtype differs from the projection dtype")
-    _check(core().fsie_rope_kv_write(_ptr(qkv), ld, _ptr(positions), _ptr(cos_sin),
-                                     cos_sin.shape[0], _ptr(slot_of), _ptr(k_pages), _ptr(v_pages),
+    _check(core().fsie_rope_kv_write(qkv, ld, positions, cos_sin,
+                                     cos_sin.shape[0], slot_of, k_pages, v_pages,
                                      page_stride, page_size, tokens, heads, kv_heads, head_dim,
-                                     rotary_dim, int(write), _tag(qkv.dtype), _ptr(error),
+                                     rotary_dim, int(write), _tag(qkv.dtype), error,
                                      _stream()), "rope_kv_write")
 
 
@@ -208,7 +205,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     inter = two_inter // 2
     if two_inter != 2 * inter or out.numel() < tokens * inter:
         raise KernelError("swiglu: shapes do not fit")
-    _check(core().fsie_swiglu(_ptr(gate_up), _ptr(out), tokens, inter, _tag(out.dtype), _stream()),
+    _check(core().fsie_swiglu(gate_up, out, tokens, inter, _tag(out.dtype), _stream()),
            "swiglu")
     return out
 
@@ -218,8 +215,8 @@ def place_tokens(ids: torch.Tensor, dst_and_row: torch.Tensor, chosen: torch.Ten
     for name, t in (("ids", ids), ("dst_and_row", dst_and_row), ("chosen", chosen)):
         _need(t, torch.int32, name)
     n = dst_and_row.numel() // 2
-    _check(core().fsie_place_tokens(_ptr(ids), _ptr(dst_and_row), _ptr(dst_and_row[n:]),
-                                    _ptr(chosen), n, _stream()), "place_tokens")
+    _check(core().fsie_place_tokens(ids, dst_and_row, dst_and_row[n:],
+                                    chosen, n, _stream()), "place_tokens")
 
 
 # --------------------------------------------------------------------- float32 product
@@ -253,7 +250,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]
     _need(out, torch.float32, "out", contiguous=False)
     if out.shape != (m, n) or out.stride(1) != 1:
         raise KernelError("gemm_f32: out must be [rows of x, rows of weight] with unit inner stride")
-    _check(core().fsie_gemm_f32(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k,
+    _check(core().fsie_gemm_f32(x, weight, bias, out, m, n, k,
                                 x.stride(0), out.stride(0), GEMM_F32_KINDS[kind], int(rows_per_warp),
                                 _stream()),
            "gemm_f32")
@@ -278,7 +275,7 @@ def gemm_f32_split_lib():
         pairs = lib.fsie_gemm_f32_split_pairs()       # also sets the kernel up, outside any capture
         if pairs <= 0:
             raise KernelError(f"gemm_f32_split: pairs of blocks cannot be launched here (code {pairs})")
-        _gemm_f32_split = lib
+        _gemm_f32_split = build.fast_calls(lib)
     return _gemm_f32_split
 
 
@@ -316,8 +313,8 @@ def gemm_f32_split(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
     if bias is not None:
         _need(bias, torch.float32, "bias")
     _check(gemm_f32_split_lib().fsie_gemm_f32_split(
-        _ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(out), out.stride(0), rows, n, k, _ptr(planes),
-        planes.numel(), _ptr(notes), notes.numel(), blocks, _ptr(error), _stream()), "gemm_f32_split")
+        x, x.stride(0), weight, bias, out, out.stride(0), rows, n, k, planes,
+        planes.numel(), notes, notes.numel(), blocks, error, _stream()), "gemm_f32_split")
     return out
 
 
@@ -353,11 +350,11 @@ def attention_generic(q: torch.Tensor, q_ld: int, k_pages: torch.Tensor, v_pages
         if part_o.numel() < nsplit * tokens * heads * head_dim or \
                 part_ml.numel() < nsplit * tokens * heads * 2:
             raise KernelError("attention: split scratch is too small")
-    _check(core().fsie_attn_tiles(_ptr(q), q_ld, _ptr(k_pages), _ptr(v_pages), page_stride,
-                                  page_size, _ptr(block_tables), block_tables.stride(0),
-                                  _ptr(tile_item), _ptr(tile_row0), num_tiles,
-                                  _ptr(item_qstart), _ptr(item_qlen), _ptr(item_pos0),
-                                  _ptr(out), out.stride(0), _ptr(part_o), _ptr(part_ml), tokens,
+    _check(core().fsie_attn_tiles(q, q_ld, k_pages, v_pages, page_stride,
+                                  page_size, block_tables, block_tables.stride(0),
+                                  tile_item, tile_row0, num_tiles,
+                                  item_qstart, item_qlen, item_pos0,
+                                  out, out.stride(0), part_o, part_ml, tokens,
                                   heads, kv_heads, head_dim, window, nsplit, float(scale),
                                   _tag(q.dtype), int(rows16), int(merge), _stream()),
            "attention_generic")
@@ -390,7 +387,7 @@ def attn_mma(head_dim: int):
         lib.fsie_attn_mma.restype = i
         lib.fsie_attn_mma_rows.argtypes = [i]
         lib.fsie_attn_mma_rows.restype = i
-        _attn_mma[head_dim] = lib
+        _attn_mma[head_dim] = build.fast_calls(lib)
     return _attn_mma[head_dim]
 
 
@@ -424,11 +421,11 @@ def attention_mma(row_class: int, q: torch.Tensor, q_ld: int, k_pages: torch.Ten
         if combine_tokens is not None:
             _need(combine_tokens, torch.int32, "combine_tokens")
     _check(attn_mma(head_dim).fsie_attn_mma(
-        row_class, _ptr(q), q_ld, _ptr(k_pages), _ptr(v_pages), page_stride, page_size,
-        _ptr(block_tables), block_tables.stride(0), _ptr(tile_item), _ptr(tile_row0), num_tiles,
-        _ptr(item_qstart), _ptr(item_qlen), _ptr(item_pos0), _ptr(out), out.stride(0),
-        _ptr(part_o), _ptr(part_ml), tokens, heads, kv_heads, head_dim, window, nsplit,
-        float(scale), _ptr(combine_tokens), num_combine, _stream()), "attention_mma")
+        row_class, q, q_ld, k_pages, v_pages, page_stride, page_size,
+        block_tables, block_tables.stride(0), tile_item, tile_row0, num_tiles,
+        item_qstart, item_qlen, item_pos0, out, out.stride(0),
+        part_o, part_ml, tokens, heads, kv_heads, head_dim, window, nsplit,
+        float(scale), combine_tokens, num_combine, _stream()), "attention_mma")
     return out
 
 
@@ -457,7 +454,7 @@ def attn_tc(head_dim: int):
         for name in ("fsie_attn_tc_map_bytes", "fsie_attn_tc_pages_map", "fsie_attn_tc",
                      "fsie_attn_tc_scaled", "fsie_attn_tc_decode", "fsie_attn_tc_decode_rows"):
             getattr(lib, name).restype = i
-        _attn_tc[head_dim] = lib
+        _attn_tc[head_dim] = build.fast_calls(lib)
     return _attn_tc[head_dim]
 
 
@@ -478,8 +475,8 @@ class PagesMap:
         size, encode = lib.fsie_attn_tc_map_bytes(), lib.fsie_attn_tc_pages_map
         self.buffer = ctypes.create_string_buffer(size + 64)
         offset = (-ctypes.addressof(self.buffer)) % 64
-        self.ptr = ctypes.c_void_p(ctypes.addressof(self.buffer) + offset)
-        _check(encode(self.ptr, _ptr(pages), rows, head_dim, page_size), "attention pages map")
+        self.ptr = ctypes.addressof(self.buffer) + offset
+        _check(encode(self.ptr, pages, rows, head_dim, page_size), "attention pages map")
 
 
 def attention_tc(pages_map: PagesMap, entry: int, q: torch.Tensor, q_ld: int,
@@ -505,11 +502,11 @@ def attention_tc(pages_map: PagesMap, entry: int, q: torch.Tensor, q_ld: int,
                 part_ml.numel() < nsplit * tokens * heads * 2:
             raise KernelError("attention_tc: split scratch is too small")
     _check(attn_tc(head_dim).fsie_attn_tc(
-        pages_map.ptr, pages_map.entries, entry, _ptr(q), q_ld, pages_map.page_size,
-        _ptr(block_tables), block_tables.stride(0), _ptr(tile_item), _ptr(tile_row0), num_tiles,
-        _ptr(item_qstart), _ptr(item_qlen), _ptr(item_pos0), _ptr(out), out.stride(0),
-        _ptr(part_o), _ptr(part_ml), tokens, heads, kv_heads, head_dim, window, nsplit,
-        float(scale), _ptr(combine_tokens), num_combine, _ptr(error), _stream()), "attention_tc")
+        pages_map.ptr, pages_map.entries, entry, q, q_ld, pages_map.page_size,
+        block_tables, block_tables.stride(0), tile_item, tile_row0, num_tiles,
+        item_qstart, item_qlen, item_pos0, out, out.stride(0),
+        part_o, part_ml, tokens, heads, kv_heads, head_dim, window, nsplit,
+        float(scale), combine_tokens, num_combine, error, _stream()), "attention_tc")
     return out
 
 
@@ -537,12 +534,12 @@ def attention_tc_scaled(pages_map: PagesMap, entry: int, q: torch.Tensor, q_ld: 
                        part_ml.numel() < nsplit * tokens * heads * 2):
         raise KernelError("attention_tc_scaled: split scratch is too small")
     _check(attn_tc(head_dim).fsie_attn_tc_scaled(
-        pages_map.ptr, pages_map.entries, entry, _ptr(q), q_ld, pages_map.page_size, _ptr(block_tables),
-        block_tables.stride(0), _ptr(tile_item), _ptr(tile_row0), num_tiles, _ptr(item_qstart), _ptr(item_qlen),
-        _ptr(item_pos0), _ptr(out), heads * head_dim, _ptr(part_o), _ptr(part_ml), tokens, heads, kv_heads, head_dim,
-        window, nsplit, _ptr(head_scale), int(chunk), float(softcap), _ptr(gate), gate_ld, _ptr(head_gate),
-        head_gate_ld, _ptr(sink), _ptr(pos_scale), pos_len, int(maps), int(partial), _ptr(combine_tokens),
-        num_combine, _ptr(error), _stream()), "attention_tc_scaled")
+        pages_map.ptr, pages_map.entries, entry, q, q_ld, pages_map.page_size, block_tables,
+        block_tables.stride(0), tile_item, tile_row0, num_tiles, item_qstart, item_qlen,
+        item_pos0, out, heads * head_dim, part_o, part_ml, tokens, heads, kv_heads, head_dim,
+        window, nsplit, head_scale, int(chunk), float(softcap), gate, gate_ld, head_gate,
+        head_gate_ld, sink, pos_scale, pos_len, int(maps), int(partial), combine_tokens,
+        num_combine, error, _stream()), "attention_tc_scaled")
     return out
 
 
@@ -601,11 +598,11 @@ def attention_tc_decode(pages_map: PagesMap, entry: int, q: torch.Tensor, q_ld: 
                 part_ml.numel() < nsplit * tokens * heads * 2:
             raise KernelError("attention_tc_decode: split scratch is too small")
     _check(attn_tc(head_dim).fsie_attn_tc_decode(
-        pages_map.ptr, pages_map.entries, entry, _ptr(q), q_ld, pages_map.page_size,
-        _ptr(block_tables), block_tables.stride(0), _ptr(tile_item), _ptr(tile_row0), num_tiles,
-        _ptr(item_qstart), _ptr(item_qlen), _ptr(item_pos0), _ptr(out), out.stride(0),
-        _ptr(part_o), _ptr(part_ml), tokens, heads, kv_heads, head_dim, window, nsplit,
-        float(scale), _ptr(combine_tokens), num_combine, _ptr(error), _stream()),
+        pages_map.ptr, pages_map.entries, entry, q, q_ld, pages_map.page_size,
+        block_tables, block_tables.stride(0), tile_item, tile_row0, num_tiles,
+        item_qstart, item_qlen, item_pos0, out, out.stride(0),
+        part_o, part_ml, tokens, heads, kv_heads, head_dim, window, nsplit,
+        float(scale), combine_tokens, num_combine, error, _stream()),
         "attention_tc_decode")
     return out
 
@@ -624,7 +621,7 @@ def gemm_decode_lib():
         lib.fsie_gemm_decode.argtypes = [p, p, i, p, i, p, i, i, i, i, i, i, p, p]
         for name in ("fsie_tensor_map_bytes", "fsie_gemm_decode_weight_map", "fsie_gemm_decode"):
             getattr(lib, name).restype = i
-        _gemm_decode = lib
+        _gemm_decode = build.fast_calls(lib)
     return _gemm_decode
 
 
@@ -662,8 +659,8 @@ class DecodeWeight:
         self.n = rows // 2 if swiglu else rows
         self.map = ctypes.create_string_buffer(lib.fsie_tensor_map_bytes() + 64)
         offset = (-ctypes.addressof(self.map)) % 64
-        self.map_ptr = ctypes.c_void_p(ctypes.addressof(self.map) + offset)
-        _check(lib.fsie_gemm_decode_weight_map(self.map_ptr, _ptr(weight), rows, k,
+        self.map_ptr = ctypes.addressof(self.map) + offset
+        _check(lib.fsie_gemm_decode_weight_map(self.map_ptr, weight, rows, k,
                                                64 if swiglu else 128), "gemm_decode weight map")
 
 
@@ -690,8 +687,8 @@ def gemm_decode(weight: DecodeWeight, x: torch.Tensor, out: torch.Tensor,
     if bias is not None:
         _need(bias, torch.bfloat16, "bias")
     _check(gemm_decode_lib().fsie_gemm_decode(
-        weight.map_ptr, _ptr(x), x.stride(0), _ptr(out), out.stride(0), _ptr(bias), tokens,
-        weight.n, k, weight.gate, int(out.dtype is torch.float32), splits, _ptr(error),
+        weight.map_ptr, x, x.stride(0), out, out.stride(0), bias, tokens,
+        weight.n, k, weight.gate, int(out.dtype is torch.float32), splits, error,
         _stream()), "gemm_decode")
     return out
 
@@ -717,7 +714,7 @@ def gemm_skinny_lib():
         lib.fsie_gemm_skinny_qkv_rope.argtypes = [p, p, ll, p, ll, p, i, i, p, p, i, p, p, p, ll, i,
                                                   i, i, i, p, p]
         lib.fsie_gemm_skinny_qkv_rope.restype = i
-        _gemm_skinny = lib
+        _gemm_skinny = build.fast_calls(lib)
     return _gemm_skinny
 
 
@@ -753,9 +750,9 @@ def gemm_skinny_qkv_rope(weight: torch.Tensor, x: torch.Tensor, out: torch.Tenso
         if k_pages.dtype is not torch.bfloat16 or v_pages.dtype is not torch.bfloat16:
             raise KernelError("gemm_skinny_qkv_rope: the cache must be bfloat16")
     _check(lib.fsie_gemm_skinny_qkv_rope(
-        _ptr(weight), _ptr(x), x.stride(0), _ptr(out), out.stride(0), _ptr(bias), tokens, k,
-        _ptr(positions), _ptr(cos_sin), cos_sin.shape[0], _ptr(slot_of), _ptr(k_pages),
-        _ptr(v_pages), page_stride, page_size, heads, kv_heads, head_dim, _ptr(error), _stream()),
+        weight, x, x.stride(0), out, out.stride(0), bias, tokens, k,
+        positions, cos_sin, cos_sin.shape[0], slot_of, k_pages,
+        v_pages, page_stride, page_size, heads, kv_heads, head_dim, error, _stream()),
         "gemm_skinny_qkv_rope")
     return out
 
@@ -778,8 +775,8 @@ def gemm_skinny(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
         raise KernelError("gemm_skinny: out does not fit")
     if bias is not None:
         _need(bias, torch.bfloat16, "bias")
-    _check(_gemm_skinny.fsie_gemm_skinny(_ptr(weight), _ptr(x), x.stride(0), _ptr(out), out.stride(0),
-                                         _ptr(bias), tokens, n, k, int(out.dtype is torch.float32),
+    _check(_gemm_skinny.fsie_gemm_skinny(weight, x, x.stride(0), out, out.stride(0),
+                                         bias, tokens, n, k, int(out.dtype is torch.float32),
                                          int(_epilogue("gemm_skinny", False, "silu", plain_activation) == 3),
                                          _stream()), "gemm_skinny")
     return out
@@ -798,7 +795,7 @@ def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor)
         raise KernelError("gemm_skinny_swiglu: x does not fit the weight, or the sizes are beyond the kernel")
     if out.shape[0] != tokens or out.shape[1] != n or out.stride(1) != 1:
         raise KernelError("gemm_skinny_swiglu: out does not fit")
-    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(_ptr(weight), _ptr(x), x.stride(0), _ptr(out), out.stride(0), tokens, n,
+    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(weight, x, x.stride(0), out, out.stride(0), tokens, n,
                                                 k, _stream()), "gemm_skinny_swiglu")
     return out
 
@@ -824,7 +821,7 @@ def gemm_tiles_lib():
         if pairs <= 0:
             raise KernelError(f"gemm_tiles: pairs of blocks cannot be launched here (code {pairs})")
         lib.pairs = pairs
-        _gemm_tiles = lib
+        _gemm_tiles = build.fast_calls(lib)
     return _gemm_tiles
 
 
@@ -852,8 +849,8 @@ class TiledWeight:
         self.n = rows // 2 if swiglu else rows
         self.map = ctypes.create_string_buffer(lib.fsie_gemm_tiles_map_bytes() + 64)
         offset = (-ctypes.addressof(self.map)) % 64
-        self.map_ptr = ctypes.c_void_p(ctypes.addressof(self.map) + offset)
-        _check(lib.fsie_gemm_tiles_weight_map(self.map_ptr, _ptr(weight), rows, k),
+        self.map_ptr = ctypes.addressof(self.map) + offset
+        _check(lib.fsie_gemm_tiles_weight_map(self.map_ptr, weight, rows, k),
                "gemm_tiles weight map")
 
 
@@ -894,10 +891,10 @@ def gemm_tiles(weight: TiledWeight, x: torch.Tensor, out: torch.Tensor,
         _need(workspace, torch.float32, "workspace")
         _need(counters, torch.int32, "counters")
     _check(gemm_tiles_lib().fsie_gemm_tiles(
-        weight.map_ptr, _ptr(x), x.stride(0), _ptr(out), out.stride(0), _ptr(bias), rows,
+        weight.map_ptr, x, x.stride(0), out, out.stride(0), bias, rows,
         weight.n, k, weight.gate, int(out.dtype is torch.float32), blocks,
-        _ptr(workspace), workspace.numel() if workspace is not None else 0,
-        _ptr(counters), counters.numel() if counters is not None else 0, _ptr(error),
+        workspace, workspace.numel() if workspace is not None else 0,
+        counters, counters.numel() if counters is not None else 0, error,
         _stream()), "gemm_tiles")
     return out
 
@@ -923,8 +920,8 @@ class GroupedTiledWeight:
         self.n = rows // 2 if swiglu else rows
         self.map = ctypes.create_string_buffer(lib.fsie_gemm_tiles_map_bytes() + 64)
         offset = (-ctypes.addressof(self.map)) % 64
-        self.map_ptr = ctypes.c_void_p(ctypes.addressof(self.map) + offset)
-        _check(lib.fsie_gemm_tiles_weight_map(self.map_ptr, _ptr(weight), groups * rows, k),
+        self.map_ptr = ctypes.addressof(self.map) + offset
+        _check(lib.fsie_gemm_tiles_weight_map(self.map_ptr, weight, groups * rows, k),
                "gemm_tiles_grouped weight map")
 
 
@@ -944,8 +941,8 @@ def gemm_tiles_grouped(weight: GroupedTiledWeight, x: torch.Tensor, out: torch.T
             tile_group.numel() < rows // GEMM_TILES_ROWS:
         raise KernelError("gemm_tiles_grouped: shapes do not fit")
     _check(gemm_tiles_lib().fsie_gemm_tiles_grouped(
-        weight.map_ptr, _ptr(x), x.stride(0), _ptr(out), out.stride(0), rows, weight.n, k, weight.gate,
-        blocks, _ptr(tile_group), _ptr(tiles_used), weight.rows, _ptr(error), _stream()),
+        weight.map_ptr, x, x.stride(0), out, out.stride(0), rows, weight.n, k, weight.gate,
+        blocks, tile_group, tiles_used, weight.rows, error, _stream()),
         "gemm_tiles_grouped")
     return out
 
@@ -977,10 +974,10 @@ def argmax(logits: torch.Tensor, out: torch.Tensor,
             raise KernelError("argmax: scratch is too small")
         # enough blocks to fill the GPU several times over, each with more than a few loads per thread
         parts = max(4, min(ARGMAX_PARTS, 2048 // rows))
-        _check(core().fsie_argmax_staged(_ptr(logits), rows, vocab, _ptr(out), _ptr(scratch),
+        _check(core().fsie_argmax_staged(logits, rows, vocab, out, scratch,
                                          parts, _stream()), "argmax")
         return out
-    _check(core().fsie_argmax(_ptr(logits), rows, vocab, _ptr(out), _stream()), "argmax")
+    _check(core().fsie_argmax(logits, rows, vocab, out, _stream()), "argmax")
     return out
 
 
@@ -1000,8 +997,8 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     _need(uniform, torch.float32, "uniform")
     _need(out, torch.int32, "out")
     rows, vocab = logits.shape
-    _check(core().fsie_sample(_ptr(logits), rows, vocab, _ptr(temperature), _ptr(top_k),
-                              _ptr(top_p), _ptr(uniform), _ptr(out), int(short_lists), _stream()), "sample")
+    _check(core().fsie_sample(logits, rows, vocab, temperature, top_k,
+                              top_p, uniform, out, int(short_lists), _stream()), "sample")
     return out
 
 
@@ -1034,7 +1031,7 @@ def scan():
         for name in ("fsie_lightning_scan", "fsie_row_decay", "fsie_head_norm_silu", "fsie_silu_rows", "fsie_gated_rmsnorm", "fsie_ssd_max_taps",
                      "fsie_ssd_prep", "fsie_ssd_tails", "fsie_ssd_gate_norm"):
             getattr(lib, name).restype = i
-        _scan = lib
+        _scan = build.fast_calls(lib)
     return _scan
 
 
@@ -1063,7 +1060,7 @@ def hybrid():
                      "fsie_talking_attention_tile_tokens", "fsie_talking_attention_key_tile",
                      "fsie_talking_attention"):
             getattr(lib, name).restype = i
-        _hybrid = lib
+        _hybrid = build.fast_calls(lib)
     return _hybrid
 
 
@@ -1084,7 +1081,7 @@ def layernorm_rows(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.T
         count = x.numel() // width
     if out.numel() < count * width:
         raise KernelError("layernorm_rows: out is too small")
-    _check(hybrid().fsie_add_layernorm(_ptr(x), _ptr(rows), _ptr(gain), None, _ptr(out), count,
+    _check(hybrid().fsie_add_layernorm(x, rows, gain, None, out, count,
                                        width, float(eps), 0, _tag(out.dtype), _stream()),
            "layernorm_rows")
     return out
@@ -1105,7 +1102,7 @@ def add_layernorm(x: torch.Tensor, delta: torch.Tensor, gain: torch.Tensor, eps:
         _need(copy, delta.dtype, "copy")
         if copy.numel() < x.numel():
             raise KernelError("add_layernorm: copy is too small")
-    _check(hybrid().fsie_add_layernorm(_ptr(delta), None, _ptr(gain), _ptr(x), _ptr(copy), count,
+    _check(hybrid().fsie_add_layernorm(delta, None, gain, x, copy, count,
                                        width, float(eps), 1, _tag(delta.dtype), _stream()),
            "add_layernorm")
 
@@ -1116,7 +1113,7 @@ def cast_rows(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     _need(out, None, "out")
     if out.numel() < x.numel():
         raise KernelError("cast_rows: out is too small")
-    _check(hybrid().fsie_cast_rows(_ptr(x), _ptr(out), x.numel(), _tag(out.dtype), _stream()),
+    _check(hybrid().fsie_cast_rows(x, out, x.numel(), _tag(out.dtype), _stream()),
            "cast_rows")
     return out
 
@@ -1128,7 +1125,7 @@ def silu_rows(proj: torch.Tensor, width: int, act: torch.Tensor) -> torch.Tensor
     tokens, ld = proj.shape
     if width > ld or act.numel() < tokens * width:
         raise KernelError("silu_rows: shapes do not fit")
-    _check(scan().fsie_silu_rows(_ptr(proj), ld, width, _ptr(act), tokens, _tag(proj.dtype),
+    _check(scan().fsie_silu_rows(proj, ld, width, act, tokens, _tag(proj.dtype),
                                    _stream()), "silu_rows")
     return act
 
@@ -1189,11 +1186,11 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
         kept = dim if decay_row is not None else int(decay_tok is not None)     # decays of a chunk, per head
         if chunk_states.numel() < num_segs * heads * (dim * vdim + kept):
             raise KernelError("lightning_scan: chunk_states is too small")
-    _check(scan().fsie_lightning_scan(_ptr(proj), ld, q_off, k_off, v_off, _ptr(item_qstart),
-                                      _ptr(item_qlen), _ptr(item_slots), items, _ptr(state),
-                                      _ptr(decay), _ptr(out), heads, dim, vdim, _ptr(seg_item),
-                                      _ptr(seg_row0), num_segs, seg_tokens, _ptr(chunk_states),
-                                      int(share), _ptr(decay_tok), _ptr(decay_row), float(out_scale),
+    _check(scan().fsie_lightning_scan(proj, ld, q_off, k_off, v_off, item_qstart,
+                                      item_qlen, item_slots, items, state,
+                                      decay, out, heads, dim, vdim, seg_item,
+                                      seg_row0, num_segs, seg_tokens, chunk_states,
+                                      int(share), decay_tok, decay_row, float(out_scale),
                                       _tag(proj.dtype), state_stride, _stream()),
            "lightning_scan")
     return out
@@ -1240,10 +1237,10 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
         stride = state.stride(0)
         if tail_off + (taps - 1) * channels > stride:
             raise KernelError("ssd_prep: the state slots do not hold the convolution's inputs")
-    _check(scan().fsie_ssd_prep(_ptr(proj), ld, conv_off, dt_off, _ptr(item_qstart), _ptr(item_qlen),
-                                _ptr(item_slots), items, _ptr(state), stride, tail_off, _ptr(conv_w),
-                                _ptr(conv_b), taps, channels, _ptr(dt_bias), _ptr(a_log), heads, vdim,
-                                _ptr(act), act.stride(0), _ptr(decay), _ptr(conv_wt), tokens,
+    _check(scan().fsie_ssd_prep(proj, ld, conv_off, dt_off, item_qstart, item_qlen,
+                                item_slots, items, state, stride, tail_off, conv_w,
+                                conv_b, taps, channels, dt_bias, a_log, heads, vdim,
+                                act, act.stride(0), decay, conv_wt, tokens,
                                 _tag(proj.dtype), _stream()), "ssd_prep")
 
 
@@ -1256,8 +1253,8 @@ def ssd_tails(proj: torch.Tensor, conv_off: int, channels: int, taps: int, item_
         return
     _need(proj, None, "proj")
     _need(state, torch.float32, "state", contiguous=False)
-    _check(scan().fsie_ssd_tails(_ptr(proj), proj.shape[1], conv_off, _ptr(item_qstart), _ptr(item_qlen),
-                                 _ptr(item_slots), items, _ptr(state), state.stride(0), tail_off, taps,
+    _check(scan().fsie_ssd_tails(proj, proj.shape[1], conv_off, item_qstart, item_qlen,
+                                 item_slots, items, state, state.stride(0), tail_off, taps,
                                  channels, _tag(proj.dtype), _stream()), "ssd_tails")
 
 
@@ -1276,8 +1273,8 @@ def ssd_gate_norm(o: torch.Tensor, act: torch.Tensor, proj: torch.Tensor, z_off:
     if z_off + inner > proj.shape[1] or gain.numel() != inner or skip.numel() * vdim != inner or \
             out.numel() < tokens * inner or act.shape[1] < inner:
         raise KernelError("ssd_gate_norm: shapes do not fit")
-    _check(scan().fsie_ssd_gate_norm(_ptr(o), _ptr(act), act.stride(0), _ptr(proj), proj.shape[1], z_off,
-                                     _ptr(skip), _ptr(gain), _ptr(out), tokens, inner, vdim, int(parts),
+    _check(scan().fsie_ssd_gate_norm(o, act, act.stride(0), proj, proj.shape[1], z_off,
+                                     skip, gain, out, tokens, inner, vdim, int(parts),
                                      float(eps), _tag(proj.dtype), _stream()), "ssd_gate_norm")
     return out
 
@@ -1293,7 +1290,7 @@ def row_decay(proj: torch.Tensor, low_off: int, rank: int, weight_t: torch.Tenso
     columns = bias.numel()
     if weight_t.shape != (rank, columns) or low_off + rank > ld or out.numel() < tokens * columns:
         raise KernelError("row_decay: shapes do not fit")
-    _check(scan().fsie_row_decay(_ptr(proj), ld, low_off, rank, _ptr(weight_t), _ptr(bias), float(inv_tau), _ptr(out),
+    _check(scan().fsie_row_decay(proj, ld, low_off, rank, weight_t, bias, float(inv_tau), out,
                                  tokens, columns, _tag(proj.dtype), _stream()), "row_decay")
     return out
 
@@ -1310,7 +1307,7 @@ def head_norm_silu(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.
     vdim = gain.numel()
     if heads * vdim != width or g_off + width > proj.shape[1] or out.numel() < tokens * width:
         raise KernelError("head_norm_silu: shapes do not fit")
-    _check(scan().fsie_head_norm_silu(_ptr(o), _ptr(proj), proj.shape[1], g_off, _ptr(gain), _ptr(out), tokens, heads,
+    _check(scan().fsie_head_norm_silu(o, proj, proj.shape[1], g_off, gain, out, tokens, heads,
                                       vdim, float(eps), _tag(proj.dtype), _stream()), "head_norm_silu")
     return out
 
@@ -1325,8 +1322,8 @@ def gated_rmsnorm(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.T
     tokens, width = o.shape
     if g_off + width > proj.shape[1] or gain.numel() != width or out.numel() < tokens * width:
         raise KernelError("gated_rmsnorm: shapes do not fit")
-    _check(scan().fsie_gated_rmsnorm(_ptr(o), _ptr(proj), proj.shape[1], g_off, _ptr(gain),
-                                       _ptr(out), tokens, width, float(eps), _tag(proj.dtype),
+    _check(scan().fsie_gated_rmsnorm(o, proj, proj.shape[1], g_off, gain,
+                                       out, tokens, width, float(eps), _tag(proj.dtype),
                                        _stream()), "gated_rmsnorm")
     return out
 
@@ -1368,12 +1365,12 @@ def conv_norm_rotate(proj: torch.Tensor, items: int, item_qstart: torch.Tensor,
     if q_out.numel() < tokens * heads * dim:
         raise KernelError("conv_norm_rotate: q_out is too small")
     _check(hybrid().fsie_conv_norm_rotate(
-        _ptr(proj), ld, tokens, items, _ptr(item_qstart), _ptr(item_pos0), _ptr(item_slots),
-        _ptr(tails) if taps > 1 else None, _ptr(conv_w), taps, _ptr(q_gain), _ptr(k_gain),
-        _ptr(cos_sin), cos_sin.shape[0], rot_dims, _ptr(slot_of) if has_kv else None,
-        _ptr(k_pages) if has_kv else None, _ptr(v_pages) if has_kv else None, page_stride,
-        page_size, _ptr(q_out), heads, kv_heads, dim, vdim, int(has_kv), float(eps),
-        _tag(proj.dtype), _ptr(error), _stream()), "conv_norm_rotate")
+        proj, ld, tokens, items, item_qstart, item_pos0, item_slots,
+        tails if taps > 1 else None, conv_w, taps, q_gain, k_gain,
+        cos_sin, cos_sin.shape[0], rot_dims, slot_of if has_kv else None,
+        k_pages if has_kv else None, v_pages if has_kv else None, page_stride,
+        page_size, q_out, heads, kv_heads, dim, vdim, int(has_kv), float(eps),
+        _tag(proj.dtype), error, _stream()), "conv_norm_rotate")
     return q_out
 
 
@@ -1385,8 +1382,8 @@ def conv_tails(proj: torch.Tensor, item_qstart: torch.Tensor, item_qlen: torch.T
     width = proj.shape[1]
     if tuple(tails.shape[1:]) != (taps - 1, width):
         raise KernelError("conv_tails: tails must be [slots, taps - 1, width]")
-    _check(hybrid().fsie_conv_tails(_ptr(proj), width, _ptr(item_qstart), _ptr(item_qlen),
-                                    _ptr(item_slots), items, _ptr(tails), taps, width,
+    _check(hybrid().fsie_conv_tails(proj, width, item_qstart, item_qlen,
+                                    item_slots, items, tails, taps, width,
                                     _tag(proj.dtype), _stream()), "conv_tails")
 
 
@@ -1437,11 +1434,11 @@ def talking_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
                 part_out.numel() < nsplit * tokens * heads * vdim:
             raise KernelError("talking_attention: split scratch is too small")
     _check(hybrid().fsie_talking_attention(
-        _ptr(q), _ptr(k_pages), _ptr(v_pages), page_stride, page_size, _ptr(block_tables),
-        block_tables.stride(0), _ptr(tile_item), _ptr(tile_row0), num_tiles, _ptr(item_qstart),
-        _ptr(item_qlen), _ptr(item_pos0), _ptr(item_slots), _ptr(talk), _ptr(out), tokens, heads,
+        q, k_pages, v_pages, page_stride, page_size, block_tables,
+        block_tables.stride(0), tile_item, tile_row0, num_tiles, item_qstart,
+        item_qlen, item_pos0, item_slots, talk, out, tokens, heads,
         kv_heads, dim, vdim, window, keep_first, tile_tokens, float(scale), nsplit,
-        _ptr(part_stats), _ptr(part_out), _tag(k_pages.dtype), _ptr(error), _stream()),
+        part_stats, part_out, _tag(k_pages.dtype), error, _stream()),
         "talking_attention")
     return out
 
@@ -1482,10 +1479,10 @@ def talking_attention_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch
     if partial.numel() < tokens * heads * kv_heads * vdim or talk.numel() != heads * heads:
         raise KernelError("talking_attention_mma: scratch or mixing matrix does not fit")
     _check(hybrid().fsie_talking_attention_mma(
-        _ptr(q), _ptr(k_pages), _ptr(v_pages), page_stride, page_size, _ptr(block_tables),
-        block_tables.stride(0), _ptr(tile_item), _ptr(tile_row0), num_tiles, _ptr(item_qstart),
-        _ptr(item_qlen), _ptr(item_pos0), _ptr(item_slots), _ptr(talk), _ptr(partial), _ptr(out),
-        tokens, heads, kv_heads, dim, vdim, window, keep_first, float(scale), _ptr(error),
+        q, k_pages, v_pages, page_stride, page_size, block_tables,
+        block_tables.stride(0), tile_item, tile_row0, num_tiles, item_qstart,
+        item_qlen, item_pos0, item_slots, talk, partial, out,
+        tokens, heads, kv_heads, dim, vdim, window, keep_first, float(scale), error,
         _stream()), "talking_attention_mma")
     return out
 
@@ -1525,7 +1522,7 @@ def mixers():
                      "fsie_latent_prep", "fsie_head_product", "fsie_norm_rotate_write",
                      "fsie_difference_merge", "fsie_relu_squared", "fsie_scaled_sum_rmsnorm"):
             getattr(lib, name).restype = i
-        _mixers = lib
+        _mixers = build.fast_calls(lib)
     return _mixers
 
 
@@ -1559,8 +1556,8 @@ def norm_add_norm(x: torch.Tensor, delta: Optional[torch.Tensor], delta_gain: Op
         count = x.numel() // hidden
     if out is not None and out.numel() < count * hidden:
         raise KernelError("norm_add_norm: out is too small")
-    _check(mixers().fsie_norm_add_norm(_ptr(x), _ptr(delta), _ptr(delta_gain), _ptr(gain), _ptr(out),
-                                       _ptr(rows), count, hidden, float(delta_eps), float(eps),
+    _check(mixers().fsie_norm_add_norm(x, delta, delta_gain, gain, out,
+                                       rows, count, hidden, float(delta_eps), float(eps),
                                        int(write_x), _tag(dtype), _stream()), "norm_add_norm")
     return out
 
@@ -1573,7 +1570,7 @@ def gated_act(gate_up: torch.Tensor, out: torch.Tensor, kind: str) -> torch.Tens
     inter = two_inter // 2
     if two_inter != 2 * inter or out.numel() < tokens * inter:
         raise KernelError("gated_act: shapes do not fit")
-    _check(mixers().fsie_gated_act(_ptr(gate_up), _ptr(out), tokens, inter, GATE_KINDS[kind],
+    _check(mixers().fsie_gated_act(gate_up, out, tokens, inter, GATE_KINDS[kind],
                                    _tag(out.dtype), _stream()), "gated_act")
     return out
 
@@ -1581,7 +1578,7 @@ def gated_act(gate_up: torch.Tensor, out: torch.Tensor, kind: str) -> torch.Tens
 def relu_squared(x: torch.Tensor) -> torch.Tensor:
     """x <- relu(x)^2 in place (behind products whose kernel has no such epilogue)."""
     _need(x, None, "x")
-    _check(mixers().fsie_relu_squared(_ptr(x), x.numel(), _tag(x.dtype), _stream()), "relu_squared")
+    _check(mixers().fsie_relu_squared(x, x.numel(), _tag(x.dtype), _stream()), "relu_squared")
     return x
 
 
@@ -1603,9 +1600,9 @@ def mingru_scan(proj: torch.Tensor, width: int, item_qstart: torch.Tensor, item_
     if num_segs:
         if seg_ab.numel() < 2 * num_segs * width or seg_start.numel() < num_segs * width:
             raise KernelError("mingru_scan: segment scratch is too small")
-    _check(mixers().fsie_mingru_scan(_ptr(proj), ld, width, _ptr(item_qstart), _ptr(item_qlen),
-                                     _ptr(item_slots), items, _ptr(seg_item), _ptr(seg_row0), num_segs,
-                                     seg_tokens, _ptr(state), _ptr(seg_ab), _ptr(seg_start), _ptr(out),
+    _check(mixers().fsie_mingru_scan(proj, ld, width, item_qstart, item_qlen,
+                                     item_slots, items, seg_item, seg_row0, num_segs,
+                                     seg_tokens, state, seg_ab, seg_start, out,
                                      _tag(proj.dtype), _stream()), "mingru_scan")
     return out
 
@@ -1668,13 +1665,13 @@ def scaled_attention(q: torch.Tensor, q_ld: int, head_scale: torch.Tensor, k_pag
                 part_ml.numel() < nsplit * tokens * heads * 2:
             raise KernelError("scaled_attention: scratch for the key splits is too small")
     _check(mixers().fsie_scaled_attention(
-        _ptr(q), q_ld, _ptr(head_scale), _ptr(k_pages), _ptr(v_pages), page_stride, page_size, key_dim,
-        value_dim, int(values_in_keys), _ptr(block_tables), block_tables.stride(0), _ptr(tile_item),
-        _ptr(tile_row0), tiles, _ptr(item_qstart), _ptr(item_qlen), _ptr(item_pos0), _ptr(item_slots),
-        _ptr(out), heads * value_dim, _ptr(part_o), _ptr(part_ml), tokens, heads, kv_heads, window,
-        int(chunk), float(softcap), _ptr(gate), gate_ld, _ptr(head_gate), head_gate_ld, _ptr(sink), _ptr(pos_scale),
-        pos_len, int(maps), int(partial), nsplit, _ptr(combine_tokens), num_combine, _tag(q.dtype),
-        SCALED_ATTENTION_FORMS[form], _ptr(error), _stream()), "scaled_attention")
+        q, q_ld, head_scale, k_pages, v_pages, page_stride, page_size, key_dim,
+        value_dim, int(values_in_keys), block_tables, block_tables.stride(0), tile_item,
+        tile_row0, tiles, item_qstart, item_qlen, item_pos0, item_slots,
+        out, heads * value_dim, part_o, part_ml, tokens, heads, kv_heads, window,
+        int(chunk), float(softcap), gate, gate_ld, head_gate, head_gate_ld, sink, pos_scale,
+        pos_len, int(maps), int(partial), nsplit, combine_tokens, num_combine, _tag(q.dtype),
+        SCALED_ATTENTION_FORMS[form], error, _stream()), "scaled_attention")
     return out
 
 
@@ -1696,8 +1693,8 @@ def difference_merge(part_o: torch.Tensor, part_ml: torch.Tensor, out: torch.Ten
         if gate.shape != (tokens, heads) or gate.stride(1) != 1:
             raise KernelError("difference_merge: gate must hold one number per head and token")
     _check(mixers().fsie_difference_merge(
-        _ptr(part_o), _ptr(part_ml), _ptr(out), heads * value_dim, tokens, heads, value_dim, nsplit, float(weight),
-        float(eps), float(factor), _ptr(gate), 0 if gate is None else gate.stride(0), _ptr(combine_tokens), num_combine,
+        part_o, part_ml, out, heads * value_dim, tokens, heads, value_dim, nsplit, float(weight),
+        float(eps), float(factor), gate, 0 if gate is None else gate.stride(0), combine_tokens, num_combine,
         _tag(out.dtype), _stream()), "difference_merge")
     return out
 
@@ -1725,11 +1722,11 @@ def rotate_mix_write(proj: torch.Tensor, positions: torch.Tensor, cos_sin: torch
             raise KernelError("rotate_mix_write: v_first is too small")
     if mix_mode == 2:
         _need(mix, torch.float32, "mix")
-    _check(mixers().fsie_rotate_mix_write(_ptr(proj), ld, _ptr(positions), _ptr(cos_sin),
-                                          cos_sin.shape[0], _ptr(slot_of), _ptr(k_pages), _ptr(v_pages),
+    _check(mixers().fsie_rotate_mix_write(proj, ld, positions, cos_sin,
+                                          cos_sin.shape[0], slot_of, k_pages, v_pages,
                                           page_stride, page_size, tokens, heads, kv_heads, dim, vdim,
-                                          rotary_dim, mix_mode, _ptr(mix), _ptr(v_first),
-                                          _tag(proj.dtype), _ptr(error), _stream()), "rotate_mix_write")
+                                          rotary_dim, mix_mode, mix, v_first,
+                                          _tag(proj.dtype), error, _stream()), "rotate_mix_write")
 
 
 def norm_rotate_write(proj: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tensor,
@@ -1762,12 +1759,12 @@ def norm_rotate_write(proj: torch.Tensor, positions: torch.Tensor, cos_sin: torc
                                   f"{'all heads' if whole else 'a head'}")
     if values_from_keys and vdim != dim:
         raise KernelError("norm_rotate_write: values that are the keys are as wide as the keys")
-    _check(mixers().fsie_norm_rotate_write(_ptr(proj), ld, _ptr(positions), _ptr(cos_sin), cos_sin.shape[0],
-                                           _ptr(slot_of), _ptr(k_pages), _ptr(v_pages), page_stride,
+    _check(mixers().fsie_norm_rotate_write(proj, ld, positions, cos_sin, cos_sin.shape[0],
+                                           slot_of, k_pages, v_pages, page_stride,
                                            page_size, tokens, heads, kv_heads, dim, vdim, rotary_dim,
-                                           _ptr(q_gain), _ptr(k_gain), float(eps), int(unit), int(whole),
+                                           q_gain, k_gain, float(eps), int(unit), int(whole),
                                            int(values_from_keys),
-                                           _tag(proj.dtype), _ptr(error), _stream()), "norm_rotate_write")
+                                           _tag(proj.dtype), error, _stream()), "norm_rotate_write")
 
 
 def scaled_sum_rmsnorm(x: torch.Tensor, deltas, scales, gain: Optional[torch.Tensor], eps: float,
@@ -1795,9 +1792,9 @@ def scaled_sum_rmsnorm(x: torch.Tensor, deltas, scales, gain: Optional[torch.Ten
         if out.numel() < count * hidden or gain.numel() != hidden:
             raise KernelError("scaled_sum_rmsnorm: out or gain does not fit")
     second = deltas[1] if len(deltas) > 1 else None
-    _check(mixers().fsie_scaled_sum_rmsnorm(_ptr(x), _ptr(deltas[0]), scales[0], _ptr(second),
-                                            scales[1] if second is not None else 0.0, _ptr(gain), _ptr(out),
-                                            _ptr(rows), count, hidden, float(eps), int(write_x),
+    _check(mixers().fsie_scaled_sum_rmsnorm(x, deltas[0], scales[0], second,
+                                            scales[1] if second is not None else 0.0, gain, out,
+                                            rows, count, hidden, float(eps), int(write_x),
                                             _tag(deltas[0].dtype), _stream()), "scaled_sum_rmsnorm")
     return out
 
@@ -1823,10 +1820,10 @@ def latent_prep(proj: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tens
     if pages.dtype is not proj.dtype or gain.numel() != rank or \
             qa.numel() < tokens * heads * (rank + rope):
         raise KernelError("latent_prep: shapes or dtypes do not fit")
-    _check(mixers().fsie_latent_prep(_ptr(proj), ld, _ptr(positions), _ptr(cos_sin), cos_sin.shape[0],
-                                     _ptr(slot_of), _ptr(pages), page_stride, page_size, _ptr(gain),
-                                     float(eps), _ptr(qa), tokens, heads, dim, rope, rank, rotary_dim,
-                                     int(half_pairs), _tag(proj.dtype), _ptr(error), _stream()), "latent_prep")
+    _check(mixers().fsie_latent_prep(proj, ld, positions, cos_sin, cos_sin.shape[0],
+                                     slot_of, pages, page_stride, page_size, gain,
+                                     float(eps), qa, tokens, heads, dim, rope, rank, rotary_dim,
+                                     int(half_pairs), _tag(proj.dtype), error, _stream()), "latent_prep")
 
 
 def head_product(x: torch.Tensor, x_ld: int, x_head: int, weight: torch.Tensor, out: torch.Tensor,
@@ -1837,7 +1834,7 @@ def head_product(x: torch.Tensor, x_ld: int, x_head: int, weight: torch.Tensor, 
     _need(weight, x.dtype, "weight")
     _need(out, x.dtype, "out", contiguous=False)
     heads, n, k = weight.shape
-    _check(mixers().fsie_head_product(_ptr(x), x_ld, x_head, _ptr(weight), _ptr(out), out_ld, out_head,
+    _check(mixers().fsie_head_product(x, x_ld, x_head, weight, out, out_ld, out_head,
                                       tokens, heads, n, k, _tag(x.dtype), _stream()), "head_product")
     return out
 
@@ -1861,7 +1858,7 @@ def parallel():
         lib.fsie_sigmoid_gate.argtypes = [p, i, p, i, i, i, i, p]
         for name in ("fsie_sum_layernorm", "fsie_settle_concat", "fsie_logit_cap", "fsie_sigmoid_gate"):
             getattr(lib, name).restype = i
-        _parallel = lib
+        _parallel = build.fast_calls(lib)
     return _parallel
 
 
@@ -1882,7 +1879,7 @@ def routed():
         for name in ("fsie_moe_tile_rows", "fsie_moe_few_tile_rows", "fsie_moe_route", "fsie_moe_align",
                      "fsie_moe_gather", "fsie_moe_product", "fsie_moe_combine"):
             getattr(lib, name).restype = i
-        _routed = lib
+        _routed = build.fast_calls(lib)
     return _routed
 
 
@@ -1921,8 +1918,8 @@ def sum_layernorm(x: torch.Tensor, deltas, gain: Optional[torch.Tensor], bias: O
         raise KernelError("sum_layernorm: out is too small")
     d1 = deltas[0] if deltas else None
     d2 = deltas[1] if len(deltas) > 1 else None
-    _check(parallel().fsie_sum_layernorm(_ptr(x), _ptr(d1), _ptr(d2), _ptr(gain), _ptr(bias), _ptr(rows),
-                                       _ptr(out), count, width, float(eps), int(write_x), _tag(dtype),
+    _check(parallel().fsie_sum_layernorm(x, d1, d2, gain, bias, rows,
+                                       out, count, width, float(eps), int(write_x), _tag(dtype),
                                        _stream()), "sum_layernorm")
     return out
 
@@ -1943,7 +1940,7 @@ def settle_concat(x: torch.Tensor, deltas, x0: torch.Tensor, out: torch.Tensor) 
             raise KernelError("settle_concat: a pending output is not of x's shape")
     d1 = deltas[0] if deltas else None
     d2 = deltas[1] if len(deltas) > 1 else None
-    _check(parallel().fsie_settle_concat(_ptr(x), _ptr(d1), _ptr(d2), _ptr(x0), _ptr(out), tokens, width,
+    _check(parallel().fsie_settle_concat(x, d1, d2, x0, out, tokens, width,
                                        _tag(out.dtype), _stream()), "settle_concat")
     return out
 
@@ -1951,7 +1948,7 @@ def settle_concat(x: torch.Tensor, deltas, x0: torch.Tensor, out: torch.Tensor) 
 def logit_cap(logits: torch.Tensor, scale: float, cap: float) -> torch.Tensor:
     """logits <- cap * tanh(logits * scale / cap) in place (cap = 0: logits * scale)."""
     _need(logits, torch.float32, "logits")
-    _check(parallel().fsie_logit_cap(_ptr(logits), logits.numel(), float(scale), float(cap), _stream()),
+    _check(parallel().fsie_logit_cap(logits, logits.numel(), float(scale), float(cap), _stream()),
            "logit_cap")
     return logits
 
@@ -1964,7 +1961,7 @@ def sigmoid_gate(out: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     tokens, width = out.shape
     if gate.shape != out.shape or out.stride(1) != 1 or gate.stride(1) != 1:
         raise KernelError("sigmoid_gate: shapes do not fit")
-    _check(parallel().fsie_sigmoid_gate(_ptr(out), out.stride(0), _ptr(gate), gate.stride(0), tokens, width,
+    _check(parallel().fsie_sigmoid_gate(out, out.stride(0), gate, gate.stride(0), tokens, width,
                                       _tag(out.dtype), _stream()), "sigmoid_gate")
     return out
 
@@ -2019,12 +2016,12 @@ def moe_route(y: Optional[torch.Tensor], w_router: Optional[torch.Tensor], corre
         experts = w_router.shape[0]
         if w_router.shape[1] != width or y.stride(1) != 1:
             raise KernelError("moe_route: shapes do not fit")
-        y_ptr, y_ld, tag, w_ptr = _ptr(y), y.stride(0), _tag(y.dtype), _ptr(w_router)
+        y_ptr, y_ld, tag, w_ptr = y, y.stride(0), _tag(y.dtype), w_router
     if ids.numel() < tokens * top or weights.numel() < tokens * top or \
             any(vector is not None and vector.numel() != experts for vector in (correction, bias)):
         raise KernelError("moe_route: shapes do not fit")
-    _check(routed().fsie_moe_route(y_ptr, y_ld, w_ptr, _ptr(logits), _ptr(bias), _ptr(correction),
-                                   _ptr(ids), _ptr(weights), tokens, width, experts, int(top), int(groups),
+    _check(routed().fsie_moe_route(y_ptr, y_ld, w_ptr, logits, bias, correction,
+                                   ids, weights, tokens, width, experts, int(top), int(groups),
                                    int(keep), float(scale), ROUTER_SCORES[scores], int(normalise),
                                    int(group_score == "max"), tag, _stream()), "moe_route")
 
@@ -2049,9 +2046,9 @@ def moe_align(ids: torch.Tensor, pairs: int, experts: int, lists: torch.Tensor,
         views.append(lists[cut:cut + n])
         cut += n
     offsets, order, tile_expert, tile_row0, meta, place = views
-    _check(routed().fsie_moe_align(_ptr(ids), pairs, experts, tile, int(padded), _ptr(offsets), _ptr(order),
-                                   _ptr(tile_expert), _ptr(tile_row0), _ptr(meta),
-                                   _ptr(place) if padded else None, _stream()), "moe_align")
+    _check(routed().fsie_moe_align(ids, pairs, experts, tile, int(padded), offsets, order,
+                                   tile_expert, tile_row0, meta,
+                                   place if padded else None, _stream()), "moe_align")
     return offsets, order, tile_expert, tile_row0, meta, (place if padded else None)
 
 
@@ -2070,8 +2067,8 @@ def moe_gather(x: torch.Tensor, lists, tile: int, top: int, out: torch.Tensor) -
     rows, k = out.shape
     if x.shape[1] != k or x.stride(1) != 1 or rows > order.numel():
         raise KernelError("moe_gather: shapes do not fit")
-    _check(routed().fsie_moe_gather(_ptr(x), x.stride(0), _ptr(order), _ptr(meta), int(tile), int(top),
-                                    _ptr(out), rows, k, _stream()), "moe_gather")
+    _check(routed().fsie_moe_gather(x, x.stride(0), order, meta, int(tile), int(top),
+                                    out, rows, k, _stream()), "moe_gather")
     return out
 
 
@@ -2092,9 +2089,9 @@ def moe_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, lists,
     if x.shape[1] != k or x.stride(1) != 1 or out.shape[1] != n or out.shape[0] < pairs or \
             (gated and rows % 2):
         raise KernelError("moe_product: shapes do not fit")
-    _check(routed().fsie_moe_product(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), out.stride(0),
-                                     _ptr(offsets), _ptr(order), _ptr(tile_expert), _ptr(tile_row0),
-                                     _ptr(meta), pairs, experts, int(top), n, k, mode,
+    _check(routed().fsie_moe_product(x, x.stride(0), weight, out, out.stride(0),
+                                     offsets, order, tile_expert, tile_row0,
+                                     meta, pairs, experts, int(top), n, k, mode,
                                      GATE_KINDS[activation], _tag(x.dtype), int(tile) or moe_tile_rows(),
                                      _stream()), "moe_product")
     return out
@@ -2127,8 +2124,8 @@ def moe_combine(expert_out: torch.Tensor, weights: torch.Tensor, shared: Optiona
         if ids.numel() < tokens * top or y.shape != out.shape or y.stride(1) != 1:
             raise KernelError("moe_combine: ids or y does not fit")
         y_ld = y.stride(0)
-    _check(routed().fsie_moe_combine(_ptr(expert_out), _ptr(weights), _ptr(shared), _ptr(place), _ptr(out),
-                                     tokens, width, int(top), _ptr(ids), int(experts), _ptr(y), y_ld,
+    _check(routed().fsie_moe_combine(expert_out, weights, shared, place, out,
+                                     tokens, width, int(top), ids, int(experts), y, y_ld,
                                      _tag(out.dtype), _stream()), "moe_combine")
     return out
 
@@ -2145,7 +2142,7 @@ def streams_lib():
         i, f, p = ctypes.c_int, ctypes.c_float, ctypes.c_void_p
         lib.fsie_stream_norm.argtypes = [p, p, p, p, p, p, p, p, p, p, p, i, i, i, f, i, i, i, p]
         lib.fsie_stream_norm.restype = i
-        _streams = lib
+        _streams = build.fast_calls(lib)
     return _streams
 
 
@@ -2195,8 +2192,8 @@ def stream_norm(x: torch.Tensor, start: Optional[torch.Tensor], delta: Optional[
             _need(bias, torch.float32, "bias")
         if gain.numel() != width or (bias is not None and bias.numel() != width) or out.numel() < count * width:
             raise KernelError("stream_norm: gain, bias or out does not fit")
-    _check(streams_lib().fsie_stream_norm(_ptr(x), _ptr(start), _ptr(delta), _ptr(delta_scale), _ptr(mix), _ptr(spread), _ptr(gather),
-                                          _ptr(gain), _ptr(bias), _ptr(rows), _ptr(out), count, streams, width,
+    _check(streams_lib().fsie_stream_norm(x, start, delta, delta_scale, mix, spread, gather,
+                                          gain, bias, rows, out, count, streams, width,
                                           float(eps), int(write_x), int(centred), _tag(dtype), _stream()),
            "stream_norm")
     return out
