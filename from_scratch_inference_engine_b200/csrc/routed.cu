@@ -145,6 +145,34 @@ __global__ void moe_route_kernel(const T* __restrict__ y, int y_ld, const float*
 }
 
 // ------------------------------------------------------------------- pairs sorted by expert
+// By one warp, from the rows of every expert: start[e], the expert's first row (start[experts]: their number; `padded`:
+// every expert's rows start on a multiple of `tile`), and tile_start[e], its first tile.  Returns the number of tiles.
+__device__ __forceinline__ int expert_starts(const int* count, int experts, int tile, int padded, int* start, int* tile_start) {
+    const int lane = threadIdx.x & 31;
+    int rows_before = 0, tiles_before = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+        const int e = e0 + lane, n = e < experts ? count[e] : 0;
+        int rows = n, tiles = (n + tile - 1) / tile;
+        const int own_tiles = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int r = __shfl_up_sync(0xffffffffu, rows, o), t = __shfl_up_sync(0xffffffffu, tiles, o);
+            if (lane >= o) { rows += r; tiles += t; }
+        }
+        if (e < experts) {
+            tile_start[e] = tiles_before + tiles - own_tiles;
+            start[e] = padded ? tile_start[e] * tile : rows_before + rows - n;
+        }
+        rows_before += __shfl_sync(0xffffffffu, rows, 31);
+        tiles_before += __shfl_sync(0xffffffffu, tiles, 31);
+    }
+    if (lane == 0) {
+        start[experts] = padded ? tiles_before * tile : rows_before;
+        tile_start[experts] = tiles_before;
+    }
+    return tiles_before;
+}
+
 // One block.  Compact layout: offsets[e] .. offsets[e + 1] are the rows of expert e in `sorted`
 // (pair = token * top + choice); tiles: (expert, first row) of every tile of `tile` rows; meta[0] =
 // their number.  Padded layout (`padded`): every expert's rows start on a multiple of `tile`, rows
@@ -165,17 +193,9 @@ __global__ void moe_align_kernel(const int* __restrict__ ids, int pairs, int exp
         if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int rows = 0, tiles = 0;
-        for (int e = 0; e < experts; ++e) {
-            start[e] = padded ? tiles * tile : rows;
-            tile_start[e] = tiles;
-            rows += count[e];
-            tiles += (count[e] + tile - 1) / tile;
-        }
-        start[experts] = padded ? tiles * tile : rows;
-        tile_start[experts] = tiles;
-        meta[0] = tiles;
+    if (threadIdx.x < 32) {
+        const int tiles = expert_starts(count, experts, tile, padded, start, tile_start);
+        if (threadIdx.x == 0) meta[0] = tiles;
     }
     __syncthreads();
     for (int e = threadIdx.x; e <= experts; e += blockDim.x) offsets[e] = start[e];
@@ -198,6 +218,169 @@ __global__ void moe_align_kernel(const int* __restrict__ ids, int pairs, int exp
         const int at = start[e] + atomicAdd(&count[e], 1);
         sorted[at] = p;
         if (place) place[p] = at;
+    }
+}
+
+// ------------------------------------------------- choice and lists of a step in one launch
+// The choice of one token by one warp, its experts' scores in registers (expert lane + 32 j in the lane's j-th): what
+// moe_route_kernel computes from the router's logits, the same bits.  Lane k < top receives choice k and its weight.
+// `choice_smem`: room of this warp for `experts` floats.
+template <int EPL>
+__device__ __forceinline__ int lane_argmax(const float (&v)[EPL], unsigned taken, int lane) {
+    float best = -INFINITY;
+    int at = -1;
+#pragma unroll
+    for (int j = 0; j < EPL; ++j)
+        if (!(taken >> j & 1) && (at < 0 || v[j] > best)) { best = v[j]; at = lane + 32 * j; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+        if (oa >= 0 && (at < 0 || ob > best || (ob == best && oa < at))) { best = ob; at = oa; }
+    }
+    return __shfl_sync(0xffffffffu, at, 0);
+}
+
+template <int EPL>
+__device__ __forceinline__ void choose_experts(const float* __restrict__ logits, const float* __restrict__ bias,
+                                               const float* __restrict__ correction, float* choice_smem, int experts,
+                                               int top, int groups, int keep, float scale, int score_kind, int normalise,
+                                               int group_max, int lane, int& my_expert, float& my_weight) {
+    float s[EPL], c[EPL];
+    unsigned taken = 0;
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        const int e = lane + 32 * j;
+        s[j] = e < experts ? logits[e] + (bias ? bias[e] : 0.f) : -INFINITY;
+        if (e >= experts) taken |= 1u << j;
+    }
+    if (score_kind == SCORES_SOFTMAX) {
+        float m = -INFINITY, sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) if (lane + 32 * j < experts) m = fmaxf(m, s[j]);
+        m = warp_max(m);
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) if (lane + 32 * j < experts) sum += expf(s[j] - m);
+        sum = warp_sum(sum);
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) s[j] = expf(s[j] - m) / sum;
+    } else if (score_kind == SCORES_SIGMOID) {
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) s[j] = 1.0f / (1.0f + expf(-s[j]));
+    }
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        const int e = lane + 32 * j;
+        c[j] = s[j] + (correction && e < experts ? correction[e] : 0.f);
+    }
+    if (groups > 1 && keep < groups) {
+        const int per = experts / groups;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) if (lane + 32 * j < experts) choice_smem[lane + 32 * j] = c[j];
+        __syncwarp();
+        float score[EPL];
+        unsigned kept = 0;                               // of the groups lane + 32 j
+        unsigned none = 0;                               // ... those that do not exist
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+            const int g = lane + 32 * j;
+            float first = -INFINITY, second = -INFINITY;
+            if (g < groups)
+                for (int i = 0; i < per; ++i) {
+                    const float v = choice_smem[g * per + i];
+                    if (v > first) { second = first; first = v; }
+                    else if (v > second) second = v;
+                }
+            else none |= 1u << j;
+            score[j] = (per > 1 && !group_max) ? first + second : first;
+        }
+        for (int k = 0; k < keep; ++k) {
+            const int g = lane_argmax<EPL>(score, kept | none, lane);
+            if (g >= 0 && (g & 31) == lane) kept |= 1u << (g >> 5);
+        }
+        __syncwarp();                                    // every lane has read the choices: the room holds marks now
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) if (lane + 32 * j < groups) choice_smem[lane + 32 * j] = kept >> j & 1 ? 1.f : 0.f;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < EPL; ++j)
+            if (lane + 32 * j < experts && choice_smem[(lane + 32 * j) / per] == 0.f) taken |= 1u << j;
+    }
+    float sum = 0.f, largest = -INFINITY, my_score = 0.f;
+    my_expert = 0;
+    for (int k = 0; k < top; ++k) {
+        const int found = lane_argmax<EPL>(c, taken, lane), e = found < 0 ? 0 : found;
+        float v = 0.f;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) if (j == e >> 5) v = s[j];
+        v = __shfl_sync(0xffffffffu, v, e & 31);
+        if (found >= 0) {
+            sum += v;
+            largest = fmaxf(largest, v);
+            if ((e & 31) == lane) taken |= 1u << (e >> 5);
+        }
+        if (lane == k) { my_expert = e; my_score = v; }
+    }
+    if (score_kind == SCORES_CHOSEN_SOFTMAX) {
+        const float part = expf(my_score - largest);
+        float total = 0.f;
+        for (int k = 0; k < top; ++k) total += __shfl_sync(0xffffffffu, part, k);
+        my_weight = part / total * scale;
+    } else {
+        my_weight = normalise ? my_score / (sum + 1e-20f) * scale : my_score * scale;
+    }
+}
+
+// One block, a warp per token: the choice from the router's logits, then the lists of moe_align_kernel (compact layout) from
+// the choices in shared memory.  Nothing here is more than a chain of dependent steps, so what
+// counts is their number: as two launches that met in global memory, with the scores in shared memory and one
+// thread walking the experts' counts, 8 tokens of 64 experts in 8 groups took 16 us of a decode step's layer.
+constexpr int CHOOSE_TOKENS = 32;
+template <int EPL>
+__global__ void __launch_bounds__(32 * CHOOSE_TOKENS)
+moe_route_align_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
+                       const float* __restrict__ correction, int* __restrict__ ids,
+                       float* __restrict__ weights, int routed, int top, int groups, int keep,
+                       float scale, int score_kind, int normalise, int group_max, int experts, int tile,
+                       int* __restrict__ offsets, int* __restrict__ sorted, int* __restrict__ tile_expert,
+                       int* __restrict__ tile_row0, int* __restrict__ meta) {
+    extern __shared__ float choose_smem[];
+    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31, tokens = blockDim.x >> 5;
+    float* room = choose_smem + (size_t)t * routed;                                    // [tokens][routed]
+    int* count = reinterpret_cast<int*>(choose_smem + (size_t)tokens * routed);         // [experts]
+    int* start = count + experts;                                                      // [experts + 1]
+    int* tile_start = start + experts + 1;                                             // [experts + 1]
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
+    grid_dependency_wait();
+    grid_dependents_go();
+    int expert;
+    float weight;
+    choose_experts<EPL>(logits + (size_t)t * routed, bias, correction, room, routed, top, groups, keep, scale, score_kind,
+                        normalise, group_max, lane, expert, weight);
+    __syncthreads();                                     // the counts are zero
+    // choices at or beyond `experts` are identity experts: no rows.  A pair's place among its expert's rows is the
+    // order the lanes arrive in: each row of a product is summed on its own, so it changes no result.
+    const bool chosen = lane < top, listed = chosen && expert < experts;
+    int place = 0;
+    if (chosen) {
+        ids[t * top + lane] = expert;
+        weights[t * top + lane] = weight;
+    }
+    if (listed) place = atomicAdd(&count[expert], 1);
+    __syncthreads();
+    if (t == 0) {
+        const int tiles = expert_starts(count, experts, tile, 0, start, tile_start);
+        if (lane == 0) meta[0] = tiles;
+    }
+    __syncthreads();
+    if (listed) sorted[start[expert] + place] = t * top + lane;
+    for (int e = threadIdx.x; e <= experts; e += blockDim.x) {
+        offsets[e] = start[e];
+        if (e == experts) break;
+        for (int i = tile_start[e]; i < tile_start[e + 1]; ++i) {
+            tile_expert[i] = e;
+            tile_row0[i] = start[e] + (i - tile_start[e]) * tile;
+        }
     }
 }
 
@@ -716,19 +899,30 @@ __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float
     grid_dependents_go();
     const size_t t = blockIdx.x;
     // a choice at or beyond `experts` is an identity expert: its output is the token's input row
-    if (VEC) {          // eight columns per thread, 16-byte accesses; the sums run in the same order
+    // eight columns per thread, 16-byte accesses; the sums run in the same order.  Four choices' rows travel together: one after
+    // the other, each behind its id and place, they were the launch's time.
+    if (VEC) {
+        constexpr int AHEAD = 4;
         for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
             float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, v[8];
-            for (int j = 0; j < top; ++j) {
-                const float w = weights[t * top + j];
-                if (ids && ids[t * top + j] >= experts) {
-                    load8(y + t * y_ld + c, v);
-                } else {
-                    const size_t row = place ? (size_t)place[t * top + j] : t * top + j;
-                    load8(expert_out + row * width + c, v);
+            for (int j0 = 0; j0 < top; j0 += AHEAD) {
+                const T* src[AHEAD];
+                float w[AHEAD], rows[AHEAD][8];
+#pragma unroll
+                for (int j = 0; j < AHEAD; ++j) {
+                    const size_t at = t * top + min(j0 + j, top - 1);
+                    const bool own = ids && ids[at] >= experts;
+                    w[j] = weights[at];
+                    src[j] = own ? y + t * y_ld : expert_out + (place ? (own ? 0 : (size_t)place[at]) : at) * width;
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, v[i], acc[i]);
+                for (int j = 0; j < AHEAD; ++j) load8(src[j] + c, rows[j]);
+#pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                    if (j0 + j < top) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[i] = fmaf(w[j], rows[j][i], acc[i]);
+                    }
             }
             if (shared) {
                 load8(shared + t * width + c, v);
@@ -803,6 +997,33 @@ int fsie_moe_align(const int* ids, int pairs, int experts, int tile, int padded,
     const int threads = pairs >= 4096 ? 1024 : (pairs >= 512 ? 256 : 64);
     return launch_dependent(moe_align_kernel, 1, threads, smem, stream, ids, pairs, experts, tile, padded, offsets,
                             sorted, tile_expert, tile_row0, meta, place);
+}
+
+// The choice from the router's logits [tokens, routed] and the lists of the compact layout in one launch (arguments as above;
+// experts <= routed: choices from `experts` on are identity experts).  Up to CHOOSE_TOKENS tokens, 256
+// experts and 32 choices.
+int fsie_moe_route_align_tokens() { return CHOOSE_TOKENS; }
+
+int fsie_moe_route_align(const float* logits, const float* bias, const float* correction, int* ids, float* weights, int tokens,
+                         int routed, int top, int groups, int keep, float scale, int score_kind, int normalise,
+                         int group_max, int experts, int tile, int* offsets, int* sorted, int* tile_expert,
+                         int* tile_row0, int* meta, cudaStream_t stream) {
+    if (tokens <= 0) return 0;
+    if (!logits || routed <= 0 || top <= 0 || top > routed || groups <= 0 || routed % groups || experts <= 0 || experts > routed ||
+        score_kind < SCORES_SIGMOID || score_kind > SCORES_CHOSEN_SOFTMAX || keep <= 0 || keep > groups ||
+        top > keep * (routed / groups) || (tile != MOE_TILE && tile != MOE_FEW_TILE))
+        return ERR_BAD_ARGUMENT;
+    if (tokens > CHOOSE_TOKENS || routed > 256 || top > 32) return ERR_UNSUPPORTED;
+    const size_t smem = ((size_t)tokens * routed + 3 * (size_t)experts + 2) * 4;     // 35 KB at most
+#define FSIE_ROUTE_ALIGN(EPL)                                                                                       \
+    launch_dependent(moe_route_align_kernel<EPL>, 1, 32 * tokens, smem, stream, logits, bias, correction, ids, weights, \
+                     routed, top, groups, keep, scale, score_kind, normalise, group_max, experts, tile, offsets, sorted, \
+                     tile_expert, tile_row0, meta)
+    if (routed <= 32) return FSIE_ROUTE_ALIGN(1);
+    if (routed <= 64) return FSIE_ROUTE_ALIGN(2);
+    if (routed <= 128) return FSIE_ROUTE_ALIGN(4);
+    return FSIE_ROUTE_ALIGN(8);
+#undef FSIE_ROUTE_ALIGN
 }
 
 // out [rows of the padded layout, k] bf16 = the tokens' rows of x in that order; `rows` is the room

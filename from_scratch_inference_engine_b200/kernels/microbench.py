@@ -294,6 +294,10 @@ def run_routed_experts(args, timer, dtype):
         buffer = torch.zeros(ops.moe_lists_size(pairs, experts, tile), dtype=torch.int32, device="cuda")
         lists = ops.moe_align(ids, pairs, experts, buffer, tile)
         note("moe_align", timer(lambda: ops.moe_align(ids, pairs, experts, buffer, tile)), pairs * 8, 0.0)
+        if ops.moe_route_align_fits(tokens, experts, top):
+            note("moe_route_align", timer(lambda: ops.moe_route_align(
+                logits, None, correction, ids, weights, top, args.groups, args.keep, 2.5, "sigmoid", True, "top2", experts,
+                buffer, tile)), tokens * (experts * 4 + top * 12), 0.0)
         act = torch.empty(pairs, f, dtype=dtype, device="cuda")
         note("moe_product gate,up", timer(lambda: ops.moe_product(y, w_gu, act, lists, pairs, top, True, "silu", tile=tile)),
              (used * 2 * f * h + tokens * h + pairs * f) * elem, 2.0 * pairs * 2 * f * h)

@@ -1873,11 +1873,13 @@ def routed():
         lib.fsie_moe_few_tile_rows.argtypes = []
         lib.fsie_moe_route.argtypes = [p, i, p, p, p, p, p, p, i, i, i, i, i, i, f, i, i, i, i, p]
         lib.fsie_moe_align.argtypes = [p, i, i, i, i, p, p, p, p, p, p, p]
+        lib.fsie_moe_route_align.argtypes = [p, p, p, p, p, i, i, i, i, i, f, i, i, i, i, i, p, p, p, p, p, p]
+        lib.fsie_moe_route_align_tokens.argtypes = []
         lib.fsie_moe_gather.argtypes = [p, ll, p, p, i, i, p, i, i, p]
         lib.fsie_moe_product.argtypes = [p, ll, p, p, ll, p, p, p, p, p, i, i, i, i, i, i, i, i, i, p]
         lib.fsie_moe_combine.argtypes = [p, p, p, p, p, i, i, i, p, i, p, ll, i, p]
         for name in ("fsie_moe_tile_rows", "fsie_moe_few_tile_rows", "fsie_moe_route", "fsie_moe_align",
-                     "fsie_moe_gather", "fsie_moe_product", "fsie_moe_combine"):
+                     "fsie_moe_route_align", "fsie_moe_route_align_tokens", "fsie_moe_gather", "fsie_moe_product", "fsie_moe_combine"):
             getattr(lib, name).restype = i
         _routed = build.fast_calls(lib)
     return _routed
@@ -2050,6 +2052,47 @@ def moe_align(ids: torch.Tensor, pairs: int, experts: int, lists: torch.Tensor,
                                    tile_expert, tile_row0, meta,
                                    place if padded else None, _stream()), "moe_align")
     return offsets, order, tile_expert, tile_row0, meta, (place if padded else None)
+
+
+MOE_ROUTE_ALIGN_TOKENS = 32       # what the kernel's `fsie_moe_route_align_tokens` says, for rules asked without a GPU
+
+
+def moe_route_align_fits(tokens: int, routed: int, top: int) -> bool:
+    """Whether `moe_route_align` takes a step: a warp per token of one block, its choices in the warp's lanes."""
+    return tokens <= MOE_ROUTE_ALIGN_TOKENS and routed <= 256 and top <= 32
+
+
+def moe_route_align(logits: torch.Tensor, bias: Optional[torch.Tensor], correction: Optional[torch.Tensor],
+                    ids: torch.Tensor, weights: torch.Tensor, top: int, groups: int, keep: int, scale: float,
+                    scores: str, normalise: bool, group_score: str, experts: int, lists: torch.Tensor,
+                    tile: int) -> Tuple[torch.Tensor, ...]:
+    """`moe_route` from the router's logits and `moe_align` (compact layout) in one launch, for steps of few tokens:
+    ids and weights as the one, the views of `lists` as the other.  `experts` <= logits' columns: choices
+    from there on are identity experts."""
+    for tensor, dtype, name in ((logits, torch.float32, "logits"), (ids, torch.int32, "ids"),
+                                (weights, torch.float32, "weights"), (lists, torch.int32, "lists")):
+        _need(tensor, dtype, name)
+    tokens, routed_experts = logits.shape
+    for name, vector in (("correction", correction), ("bias", bias)):
+        if vector is not None:
+            _need(vector, torch.float32, name)
+            if vector.numel() != routed_experts:
+                raise KernelError("moe_route_align: shapes do not fit")
+    if scores not in ROUTER_SCORES or group_score not in ("top2", "max"):
+        raise KernelError(f"moe_route_align: scores must be one of {', '.join(ROUTER_SCORES)}, group_score 'top2' or 'max'")
+    pairs = tokens * top
+    tiles = pairs // tile + experts
+    if ids.numel() < pairs or weights.numel() < pairs or lists.numel() < moe_lists_size(pairs, experts, tile):
+        raise KernelError("moe_route_align: working memory is too small")
+    views, cut = [], 0
+    for n in (experts + 1, pairs, tiles, tiles, 1):
+        views.append(lists[cut:cut + n])
+        cut += n
+    _check(routed().fsie_moe_route_align(logits, bias, correction, ids, weights, tokens,
+                                         routed_experts, int(top), int(groups), int(keep), float(scale),
+                                         ROUTER_SCORES[scores], int(normalise), int(group_score == "max"), experts, tile,
+                                         *views, _stream()), "moe_route_align")
+    return (*views, None)
 
 
 def moe_lists_size(pairs: int, experts: int, tile: int = 0, padded: bool = False) -> int:

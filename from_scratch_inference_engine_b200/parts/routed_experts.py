@@ -155,9 +155,6 @@ class RoutedExperts(Part):
         ids = rt.buffer("routed.ids", tokens, top, torch.int32)
         weights = rt.buffer("routed.weights", tokens, top, torch.float32)
         logits = rt.linear_f32_out(y, self.w_router, "routed.logits")
-        ops.moe_route(None, None, self.correction, ids, weights, top, self.groups, self.keep,
-                      self.scale, self.scores, self.normalise, logits=logits, group_score=self.group_score,
-                      bias=self.router_bias)
         # choices at or beyond `experts` are identity experts: no rows in the products, and the
         # weighted sum takes the token's own row for them
         identity = dict(ids=ids, experts=self.experts, y=y) if self.identity else {}
@@ -168,8 +165,16 @@ class RoutedExperts(Part):
                    and pairs >= self.GROUPED_MIN_ROWS * self.experts
                    and self.hidden_size % 8 == 0 and self.intermediate_size % 8 == 0
                    and y.stride(0) % 8 == 0 and y.data_ptr() % 16 == 0)
+        few = not grouped and (streaming_pays(y.dtype, pairs, self.experts)
+                               and ops.moe_few_fits(y, self.hidden_size, self.intermediate_size))
+        tile = ops.GEMM_TILES_ROWS if grouped else (ops.moe_few_tile_rows() if few else ops.moe_tile_rows())
+        # steps of few tokens: choice and lists in one launch
+        at_once = not grouped and ops.moe_route_align_fits(tokens, self.routed, top)
+        if not at_once:
+            ops.moe_route(None, None, self.correction, ids, weights, top, self.groups, self.keep,
+                          self.scale, self.scores, self.normalise, logits=logits, group_score=self.group_score,
+                          bias=self.router_bias)
         if grouped:
-            tile = ops.GEMM_TILES_ROWS
             rows = (pairs // tile + self.experts) * tile
             lists = ops.moe_align(ids, pairs, self.experts,
                                   rt.buffer("routed.lists", 1, ops.moe_lists_size(pairs, self.experts, tile, True),
@@ -182,12 +187,13 @@ class RoutedExperts(Part):
             expert_out = rt.buffer("routed.expert_out", rows, self.hidden_size, y.dtype)
             ops.gemm_tiles_grouped(down, act, expert_out, lists[2], lists[4], ctx.error, rt.sm_count)
             return ops.moe_combine(expert_out, weights, shared, out, top, place=lists[5], **identity)
-        few = (streaming_pays(y.dtype, pairs, self.experts)
-               and ops.moe_few_fits(y, self.hidden_size, self.intermediate_size))
-        tile = ops.moe_few_tile_rows() if few else ops.moe_tile_rows()
-        lists = ops.moe_align(ids, pairs, self.experts,
-                              rt.buffer("routed.lists", 1, ops.moe_lists_size(pairs, self.experts, tile),
-                                        torch.int32).view(-1), tile)
+        room = rt.buffer("routed.lists", 1, ops.moe_lists_size(pairs, self.experts, tile), torch.int32).view(-1)
+        if at_once:
+            lists = ops.moe_route_align(logits, self.router_bias, self.correction, ids, weights, top, self.groups,
+                                        self.keep, self.scale, self.scores, self.normalise, self.group_score,
+                                        self.experts, room, tile)
+        else:
+            lists = ops.moe_align(ids, pairs, self.experts, room, tile)
         act = rt.buffer("routed.act", pairs, self.intermediate_size, y.dtype)
         ops.moe_product(y, self.w_gate_up, act, lists, pairs, top, self.gated, self.activation, first=True,
                         tile=tile)
