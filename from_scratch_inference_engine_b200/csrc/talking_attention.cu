@@ -135,6 +135,124 @@ __global__ void conv_norm_rotate_kernel(const T* __restrict__ proj, int ld, int 
     }
 }
 
+// The same with eight neighbouring channels per thread, all of a row in one go (up to CONV_VEC_WIDTH channels): 16-byte loads,
+// everything a row needs on its way at once (weights, gains, angles and lists before the kernel that makes
+// the projection has finished), and one barrier before the norms.  A decode step's rows are few, so the chain of trips to
+// memory is what it takes: with a channel per thread and turn, and the tails in a launch behind it, 4 tokens of 3,072
+// channels took 22 + 10 us of the step's chain.
+// FOLD (every request brings one token): the row's own channels move the request's tail on as well, which conv_tails
+// does otherwise (a longer portion's first tokens still read the old tail when its last one is done).
+constexpr int CONV_VEC_WIDTH = 6144;
+template <typename T, int TAPS, bool FOLD>
+__global__ void __launch_bounds__(CONV_VEC_WIDTH / 8)
+conv_norm_rotate_vec_kernel(const T* __restrict__ proj, int ld, int items, const int* __restrict__ item_qstart,
+                            const int* __restrict__ item_pos0, const int* __restrict__ item_slots,
+                            float* tails, const float* __restrict__ conv_w,
+                            const float* __restrict__ q_gain, const float* __restrict__ k_gain,
+                            const float* __restrict__ cos_sin, int table_len, int rot_dims,
+                            const int* __restrict__ slot_of, T* __restrict__ k_pages, T* __restrict__ v_pages,
+                            long long page_stride, int page_size, float* __restrict__ q_out, int heads, int kv_heads,
+                            int dim, int vdim, int has_kv, float eps, int* error) {
+    __shared__ float sums[2][32];                       // per warp: squares of q, of k
+    __shared__ float eights[CONV_VEC_WIDTH / 8];        // squares of every thread's channels
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int wq = heads * dim, wk = has_kv ? kv_heads * dim : 0, wv = has_kv ? kv_heads * vdim : 0;
+    const int width = wq + wk + wv, c0 = threadIdx.x * 8;
+    const bool active = c0 < width, is_q = c0 < wq, is_k = !is_q && c0 < wq + wk, is_v = active && !is_q && !is_k;
+    // neither the lists nor the constants come from the kernel before
+    const int item = item_of_token(item_qstart, items, t);
+    const int slot = item_slots[item], start = item_qstart[item], pos0 = item_pos0[item], pos = pos0 + (t - start);
+    const int slot_kv = has_kv && slot >= 0 ? slot_of[t] : -1;
+    float w[TAPS * 8];                                  // [channel][tap]
+    float gain[8], co[4], si[4];
+    const int local = is_q ? c0 : c0 - wq, head = is_v ? (local - wk) / vdim : local / dim;
+    const int d0 = is_v ? local - wk - head * vdim : local - head * dim;
+    const bool refused = rot_dims > 0 && (pos < 0 || pos >= table_len);
+    if (active) {
+#pragma unroll
+        for (int i = 0; i < TAPS; ++i) {
+            float part[8];
+            load8(conv_w + (size_t)c0 * TAPS + 8 * i, part);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[8 * i + e] = part[e];
+        }
+        if (!is_v) {
+            load8((is_q ? q_gain : k_gain) + local, gain);
+            const float* cs = cos_sin + (size_t)(refused ? 0 : pos) * rot_dims;      // [cos (half) | sin (half)]
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool turned = d0 + 2 * i < rot_dims;
+                co[i] = turned ? cs[d0 / 2 + i] : 1.f;
+                si[i] = turned ? cs[rot_dims / 2 + d0 / 2 + i] : 0.f;
+            }
+        }
+    }
+    grid_dependency_wait();
+    grid_dependents_go();
+    if (slot < 0) return;                               // a padding entry of a fixed-size batch
+    if (refused && threadIdx.x == 0) atomicExch(error, 2);
+    float* tail = tails + (size_t)slot * (TAPS - 1) * width + c0;
+    float u[TAPS][8], y[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) y[e] = 0.f;
+    float sq = 0.f;
+    if (active) {
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const int p = pos - TAPS + 1 + j;
+            if (p >= pos0) load8(proj + (size_t)(start + p - pos0) * ld + c0, u[j]);
+            else load8(tail + (size_t)(p - pos0 + TAPS - 1) * width, u[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            if (pos - TAPS + 1 + j < 0) continue;       // before the sequence starts
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] += w[e * TAPS + j] * u[j][e];
+        }
+        if (FOLD) {
+#pragma unroll
+            for (int j = 1; j < TAPS; ++j) store8(tail + (size_t)(j - 1) * width, u[j]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sq += y[e] * y[e];
+    }
+    eights[threadIdx.x] = sq;
+    const float q_sum = warp_sum(is_q ? sq : 0.f), k_sum = warp_sum(is_k ? sq : 0.f);
+    if (lane == 0) { sums[0][warp] = q_sum; sums[1][warp] = k_sum; }
+    __syncthreads();
+    if (!active) return;
+    float total = 0.f;
+    if (is_v) {
+        const int first = threadIdx.x - d0 / 8;
+        for (int i = 0; i < vdim / 8; ++i) total += eights[first + i];
+    } else {
+        for (int i = 0; i < warps; ++i) total += sums[is_k ? 1 : 0][i];
+    }
+    const float inv = 1.0f / sqrtf(total / (float)(is_v ? vdim : (is_q ? wq : wk)) + eps);
+    if (!is_v) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y[e] = y[e] * inv * gain[e];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (d0 + 2 * i >= rot_dims) continue;
+            const float a = y[2 * i], b = y[2 * i + 1];
+            y[2 * i] = a * co[i] - b * si[i];
+            y[2 * i + 1] = b * co[i] + a * si[i];
+        }
+        if (is_q) {
+            store8(q_out + (size_t)t * wq + c0, y);
+            return;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y[e] *= inv;
+    }
+    if (slot_kv < 0) return;
+    const long long page = slot_kv / page_size;
+    const int offset = slot_kv - (int)page * page_size, row = is_v ? vdim : dim;
+    store8((is_v ? v_pages : k_pages) + page * page_stride + ((size_t)head * page_size + offset) * row + d0, y);
+}
+
 // ------------------------------------------------------------------------------- tails
 // One block per request: row r of its new tail is the projected row of position
 // end - (taps - 1) + r, which is a row of this step or, when the step brought fewer than
@@ -168,17 +286,44 @@ using namespace fsie;
 
 extern "C" {
 
+// fold_tails != 0 (every request brings one token): the kernel also moves the requests' tails on where it can; *folded
+// (host memory) says whether it does, else conv_tails has to follow.
 int fsie_conv_norm_rotate(const void* proj, int ld, int tokens, int items, const int* item_qstart,
-                          const int* item_pos0, const int* item_slots, const float* tails,
+                          const int* item_pos0, const int* item_slots, float* tails,
                           const float* conv_w, int taps, const float* q_gain, const float* k_gain,
                           const float* cos_sin, int table_len, int rot_dims, const int* slot_of,
                           void* k_pages, void* v_pages, long long page_stride, int page_size,
                           float* q_out, int heads, int kv_heads, int dim, int vdim, int has_kv,
-                          float eps, int dtype, int* error, cudaStream_t stream) {
+                          float eps, int dtype, int* error, int fold_tails, int* folded, cudaStream_t stream) {
+    if (folded) *folded = 0;
     if (tokens <= 0) return 0;
-    if (items <= 0 || taps <= 0 || (taps > 1 && !tails) || rot_dims < 0 || rot_dims > dim || (rot_dims & 1))
+    if (items <= 0 || taps <= 0 || (taps > 1 && !tails) || rot_dims < 0 || rot_dims > dim || (rot_dims & 1) ||
+        (fold_tails && (tokens != items || !folded)))
         return ERR_BAD_ARGUMENT;
     const int width = heads * dim + (has_kv ? kv_heads * (dim + vdim) : 0);
+    const int per = dtype == DTYPE_F32 ? 4 : 8;
+    const bool vec = taps >= 2 && taps <= 4 && dim % 8 == 0 && vdim % 8 == 0 && width <= CONV_VEC_WIDTH && ld % per == 0 &&
+        (!has_kv || !k_pages || (page_stride % per == 0 && ((((size_t)k_pages) | ((size_t)v_pages)) & 15) == 0)) &&
+        ((((size_t)proj) | ((size_t)tails) | ((size_t)conv_w) | ((size_t)q_gain) | ((size_t)k_gain) | ((size_t)q_out)) & 15) == 0;
+    if (vec) {
+        const int threads = ((width / 8 + 31) / 32) * 32;
+        if (folded) *folded = fold_tails;
+#define FSIE_PREPARE_VEC(T, N, F)                                                                                       \
+        launch_dependent(conv_norm_rotate_vec_kernel<T, N, F>, tokens, threads, 0, stream, (const T*)proj, ld, items,   \
+                         item_qstart, item_pos0, item_slots, tails, conv_w, q_gain, k_gain, cos_sin, table_len, rot_dims, \
+                         slot_of, (T*)k_pages, (T*)v_pages, page_stride, page_size, q_out, heads, kv_heads, dim, vdim, \
+                         has_kv, eps, error)
+#define FSIE_PREPARE_TAPS(T)                                                                                            \
+        switch (taps) {                                                                                                 \
+            case 2: return fold_tails ? FSIE_PREPARE_VEC(T, 2, true) : FSIE_PREPARE_VEC(T, 2, false);                    \
+            case 3: return fold_tails ? FSIE_PREPARE_VEC(T, 3, true) : FSIE_PREPARE_VEC(T, 3, false);                    \
+            default: return fold_tails ? FSIE_PREPARE_VEC(T, 4, true) : FSIE_PREPARE_VEC(T, 4, false);                   \
+        }
+        if (dtype == DTYPE_F32) FSIE_PREPARE_TAPS(float)
+        FSIE_PREPARE_TAPS(bf16)
+#undef FSIE_PREPARE_TAPS
+#undef FSIE_PREPARE_VEC
+    }
     const size_t smem = (size_t)(width + kv_heads) * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
     const int threads = width >= 1024 ? 512 : 256;

@@ -1,0 +1,151 @@
+"""Mixed-heads attention and its preparation for steps of one token per request: the two launches against the tiled kernel
+and 64 bits, and the row in one go against the general kernel."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DTYPES = [torch.float32, torch.bfloat16]
+
+
+def device(values):
+    return torch.tensor(values, dtype=torch.int32, device="cuda")
+
+
+# one key; the edges of a range of 64 keys and of 256 weights; a window with kept first tokens, kept ones alone; a padding entry; one
+# head per key/value head and eight; columns that are no multiple of 64 or 32; pages of other sizes
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,page,window,keep,lengths", [
+    (16, 4, 128, 128, 16, 1024, 4, (1, 64, 65, 916)), (4, 4, 8, 40, 16, 0, 0, (255, 256, 257, 513)),
+    (8, 1, 72, 24, 8, 100, 3, (1, 99, 103, 700)), (6, 2, 256, 256, 32, 33, 64, (63, 200, 0, 32)), (64, 8, 64, 136, 16, 1, 2, (5, 1, 2, 300))])
+def test_scores_then_values(heads, kv_heads, dim, vdim, page, window, keep, lengths, dtype):
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(heads * 100 + dim)
+    rand = lambda *shape: torch.randn(shape, generator=generator, device="cuda")
+    items, group = len(lengths), heads // kv_heads
+    blocks = -(-max(lengths) // page) + 1
+    keys, values = rand(items * blocks, kv_heads, page, dim).to(dtype), rand(items * blocks, kv_heads, page, vdim).to(dtype)
+    width = kv_heads * page * (dim + vdim)
+    pages = torch.cat([keys.flatten(1), values.flatten(1)], dim=1).contiguous()
+    k_pages, v_pages = pages[:, :kv_heads * page * dim], pages[:, kv_heads * page * dim:]
+    tables = torch.randperm(items * blocks, generator=generator, device="cuda").int().view(items, blocks)
+    q, talk = rand(items, heads * dim), rand(heads, heads) * heads ** -0.5
+    scale = dim ** -0.5
+    pos0, slots = device([max(n - 1, 0) for n in lengths]), device([-1 if n == 0 else i for i, n in enumerate(lengths)])
+    qstart, qlen, error = device(list(range(items))), device([1] * items), device([0])
+    sees = max(lengths) if window == 0 else min(max(lengths), window + keep)
+    nsplit = ops.talking_decode_splits(items, sees, heads, kv_heads, dim, vdim, width, dtype)
+    assert nsplit == -(-sees // ops.TALKING_DECODE_KEYS) and ops.hybrid().fsie_talking_decode_keys() == ops.TALKING_DECODE_KEYS
+    out = torch.full((items, heads * vdim), float("nan"), device="cuda", dtype=dtype)
+    scores = torch.full((items * heads * nsplit * 64,), float("nan"), device="cuda")
+    stats = torch.full((items * nsplit * heads * 2,), float("nan"), device="cuda")
+    ops.talking_decode(q, k_pages, v_pages, width, page, tables, qstart, qlen, pos0, slots, items, talk, out, heads, kv_heads,
+                       dim, vdim, window, keep, scale, error, nsplit, scores, stats)
+    tiled = torch.full_like(out, float("nan"))
+    if ops.talking_attention_key_tile(heads, kv_heads, dim, vdim, dtype) > 0:
+        ops.talking_attention(q, k_pages, v_pages, width, page, tables, device(list(range(items))), device([0] * items), items,
+                              qstart, qlen, pos0, slots, talk, tiled, heads, kv_heads, dim, vdim, window, keep, 1, scale, error)
+    assert int(error.item()) == 0
+    for i, n in enumerate(lengths):
+        if n == 0:
+            assert torch.isnan(out[i]).all()                 # a padding entry writes nothing
+            continue
+        seen = [j for j in range(n) if window == 0 or n - 1 - j < window or j < keep]
+        rows = [(int(tables[i, j // page]), j % page) for j in seen]
+        k = torch.stack([keys[p, :, s] for p, s in rows]).double()                 # [keys, kv heads, dim]
+        v = torch.stack([values[p, :, s] for p, s in rows]).double()
+        s = torch.einsum("hd,jhd->hj", q[i].view(heads, dim).double(), k.repeat_interleave(group, 1)) * scale
+        mixed = talk.double() @ torch.softmax(s, dim=1)
+        want = torch.einsum("hj,jhv->hv", mixed, v.repeat_interleave(group, 1)).flatten()
+        size = torch.einsum("hj,jhv->hv", talk.double().abs() @ torch.softmax(s, dim=1), v.abs().repeat_interleave(group, 1)).flatten()
+        # 32-bit: a score of dim products moves its weight by dim 2^-24 of the products' sum (up to 64 here), then sums over
+        # keys and heads; the result rounded to the storage type
+        bound = size * (dim + heads + 64) * 64 * 2.0 ** -24 + (want.abs() + size * 1e-3) * (2.0 ** -8 if dtype is torch.bfloat16 else 0.0)
+        assert ((out[i].double() - want).abs() <= bound).all()
+        if not torch.isnan(tiled[i]).all():
+            assert ((out[i].double() - tiled[i].double()).abs() <= 2 * bound).all()
+
+
+def test_a_page_that_was_given_back():
+    """Its keys count as zeros and the step fails, as in the tiled kernel."""
+    from from_scratch_inference_engine_b200.kernels import ops
+    pages = torch.randn(4, 2 * 8 * 16, device="cuda")
+    error, one = device([0]), device([0])
+    out, tiled = torch.empty(1, 16, device="cuda"), torch.empty(1, 16, device="cuda")
+    common = (torch.randn(1, 16, device="cuda"), pages[:, :128], pages[:, 128:], 256, 16, device([[2, -1, 0, 3]]))
+    lists, sizes = (one, device([1]), device([60]), one), (2, 1, 8, 8, 0, 0)
+    talk = torch.randn(2, 2, device="cuda")
+    ops.talking_decode(*common, *lists, 1, talk, out, *sizes, 0.3, error, 1, torch.empty(128, device="cuda"), torch.empty(4, device="cuda"))
+    assert int(error.item()) == 3
+    ops.talking_attention(*common, one, one, 1, *lists, talk, tiled, *sizes, 1, 0.3, error)
+    assert torch.allclose(out, tiled, rtol=1e-4, atol=1e-5)
+
+
+# tokens of one request each (tails move in the launch) and longer portions beside them; before the sequence's start; taps 2 to
+# 4 and a count the row form does not take; without keys of its own; a refused position; a padding entry
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps,rot,qlens", [
+    (16, 4, 128, 128, 4, 128, (1, 1, 1, 1)), (16, 4, 128, 128, 4, 64, (1, 5, 2, 30)), (2, 1, 16, 24, 2, 10, (1, 1, 1, 1)),
+    (3, 1, 40, 8, 3, 0, (1, 1, 3, 1)), (4, 2, 8, 8, 5, 4, (1, 1, 1, 1)), (4, 0, 24, 8, 4, 24, (1, 1, 1, 1))])
+def test_rows_in_one_go(heads, kv_heads, dim, vdim, taps, rot, qlens, dtype):
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(dim + taps)
+    rand = lambda *shape: torch.randn(shape, generator=generator, device="cuda")
+    has_kv, kvh, page, items = kv_heads > 0, max(kv_heads, 1), 16, len(qlens)
+    width = heads * dim + (kvh * (dim + vdim) if has_kv else 0)
+    tokens, starts = sum(qlens), [sum(qlens[:i]) for i in range(items)]
+    pos0 = [0, 1, 40, 7]
+    slots = [2, 0, -1, 3]
+    proj, conv_w, q_gain, k_gain = rand(tokens, width).to(dtype), rand(width, taps), rand(heads * dim), rand(kvh * dim)
+    tails = rand(5, taps - 1, width)
+    tails[2], tails[0, :-1] = 0.0, 0.0                        # nothing before the sequence starts
+    table = rand(64, max(rot, 1))
+    error = device([0])
+    pages = torch.zeros(8, kvh * page * (dim + vdim), device="cuda", dtype=dtype)
+    slot_of = device([16 * i + 3 if i != 1 else -1 for i in range(tokens)]) if tokens <= 8 else device([-1] * tokens)
+
+    def run(proj, pages, tails, qlen):
+        q = torch.full((tokens, heads * dim), float("nan"), device="cuda")
+        ops.conv_norm_rotate(proj, items, device(starts), device(pos0), device(slots), tails, conv_w, taps, q_gain,
+                             k_gain if has_kv else None, table, rot, slot_of if has_kv else None,
+                             pages[:, :kvh * page * dim] if has_kv else None, pages[:, kvh * page * dim:] if has_kv else None,
+                             pages.stride(0), page, q, heads, kv_heads, dim, vdim, has_kv, 1e-6, error, qlen)
+        return q
+    got_pages, got_tails = pages.clone(), tails.clone()
+    got = run(proj, got_pages, got_tails, device(list(qlens)))
+    # the general kernel takes what does not start on 16 bytes: the same projection four bytes further on
+    shifted = torch.empty(proj.numel() + 8, device="cuda", dtype=dtype)[8 // proj.element_size() // 2:][:proj.numel()].view_as(proj)
+    shifted.copy_(proj)
+    assert shifted.data_ptr() % 16
+    want_pages, want_tails = pages.clone(), tails.clone()
+    want = run(shifted, want_pages, want_tails, None)
+    ops.conv_tails(proj, device(starts), device(list(qlens)), device(slots), items, want_tails, taps)
+    assert torch.equal(got_tails, want_tails) and int(error.item()) == 0
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    known = ~torch.isnan(want)
+    # norms summed in another order: dim 2^-24 and a few roundings of numbers around one (times the gain)
+    assert ((got - want).abs()[known] <= 1e-5 * (1 + want.abs()[known]) * 4).all()
+    step = 2.0 ** -7 if dtype is torch.bfloat16 else 1e-5 * 4        # a rounding to the storage type may fall the other way
+    assert ((got_pages.float() - want_pages.float()).abs() <= step * (1e-2 + want_pages.float().abs())).all()
+    run(proj, got_pages, got_tails, None)
+    assert int(error.item()) == 0
+    pos0[3] = 64                                              # beyond the table
+    run(proj, got_pages, got_tails, None)
+    assert int(error.item()) == (2 if rot else 0)
+
+
+@pytest.mark.parametrize("width", [8, 264, 2048, 8192, 8200])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_layer_norm_rows(width, dtype):
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(width)
+    src, gain, x = (torch.randn(shape, generator=generator, device="cuda") * 3 + 1.5 for shape in ((5, width), (width,), (5, width)))
+    norm = lambda v: torch.nn.functional.layer_norm(v.double(), (width,), eps=1e-6) * gain.double()
+    rows, half = device([4, 0, 2]), 2.0 ** -8 if dtype is torch.bfloat16 else 0.0
+    want = norm(src)[rows.long()]
+    got = ops.layernorm_rows(src, gain, 1e-6, torch.empty(3, width, device="cuda", dtype=dtype), rows=rows)
+    assert ((got.double() - want).abs() <= (1e-5 + half) * (1 + want.abs())).all()
+    delta, copy, sum_ = src.to(dtype), torch.empty(5, width, device="cuda", dtype=dtype), x.clone()
+    ops.add_layernorm(sum_, delta, gain, 1e-6, copy)
+    want = x.double() + norm(delta)
+    assert ((sum_.double() - want).abs() <= 1e-5 * (1 + want.abs())).all()      # the sum stays 32-bit
+    assert torch.equal(copy, sum_.to(dtype))
