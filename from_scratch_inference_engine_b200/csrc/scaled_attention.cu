@@ -353,14 +353,18 @@ __global__ void __launch_bounds__(SA_WARPS * 32) scaled_attention_mma_kernel(con
     // blocks start in the order of the grid: the last tiles of a prompt see the most keys and go first
     const int kvh = blockIdx.x, tile = gridDim.y - 1 - blockIdx.y, split = blockIdx.z;
     const int group = p.heads / p.kv_heads;
-    grid_dependency_wait();
-    grid_dependents_go();
+    // The lists and block tables were staged before the step, and keys older than the request's new tokens were written by
+    // earlier steps: they are read and asked for while the kernel before (which makes the queries and this step's
+    // keys) still runs.  Nobody leaves before that kernel is done: the one behind waits for this one only.
     const int item = p.tile_item[tile];
-    if (p.item_slots && p.item_slots[item] < 0) return;
     const int row0 = p.tile_row0[tile];
     const int qstart = p.item_qstart[item], qlen = p.item_qlen[item], pos0 = p.item_pos0[item];
     const int nrows = min(SA_ROWS, qlen * group - row0);
-    if (nrows <= 0) return;
+    if ((p.item_slots && p.item_slots[item] < 0) || nrows <= 0) {
+        grid_dependency_wait();
+        grid_dependents_go();
+        return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int mi = warp >> 2, vi = warp & 3;             // which 16 rows; which quarter of keys / value columns
     const int g = lane >> 2, t = lane & 3;
@@ -409,8 +413,13 @@ __global__ void __launch_bounds__(SA_WARPS * 32) scaled_attention_mma_kernel(con
         if (part == 0) key_ok[stage * TM_KT + j] = ok;
         cp_async_commit();
     };
-    if (kbegin < kend) issue_tile(0, kbegin, page_of(kbegin));
+    const int first_page = page_of(kbegin);
     int page_ahead = page_of(kbegin + TM_KT);
+    const bool early = kbegin < kend && kbegin + TM_KT <= pos0;
+    if (early) issue_tile(0, kbegin, first_page);
+    grid_dependency_wait();
+    grid_dependents_go();
+    if (!early && kbegin < kend) issue_tile(0, kbegin, first_page);
 
     // the tile's query rows as they are (the head's scale meets the scores), zero beyond the tile
     for (int r = warp; r < SA_ROWS; r += SA_WARPS) {
@@ -623,14 +632,18 @@ __global__ void __launch_bounds__(TR_WARPS * 32) scaled_attention_rows_kernel(co
     // blocks start in the order of the grid: the last tiles of a prompt see the most keys and go first
     const int kvh = blockIdx.x, tile = gridDim.y - 1 - blockIdx.y, split = blockIdx.z;
     const int group = p.heads / p.kv_heads;
-    grid_dependency_wait();
-    grid_dependents_go();
+    // The lists and block tables were staged before the step, and keys older than the request's new tokens were written by
+    // earlier steps: they are read and asked for while the kernel before (which makes the queries and this step's
+    // keys) still runs.  Nobody leaves before that kernel is done: the one behind waits for this one only.
     const int item = p.tile_item[tile];
-    if (p.item_slots && p.item_slots[item] < 0) return;
     const int row0 = p.tile_row0[tile];
     const int qstart = p.item_qstart[item], qlen = p.item_qlen[item], pos0 = p.item_pos0[item];
     const int nrows = min(ROWS, qlen * group - row0);
-    if (nrows <= 0) return;
+    if ((p.item_slots && p.item_slots[item] < 0) || nrows <= 0) {
+        grid_dependency_wait();
+        grid_dependents_go();
+        return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int wrow = FEW ? 0 : warp * 16, wkey = FEW ? warp * WK : 0;    // this warp's first row and key of a tile
@@ -685,11 +698,20 @@ __global__ void __launch_bounds__(TR_WARPS * 32) scaled_attention_rows_kernel(co
         int pages[SLOTS - 1];
 #pragma unroll
         for (int s = 0; s < SLOTS - 1; ++s) pages[s] = page_of(kbegin + s * TM_KT);
-#pragma unroll
-        for (int s = 0; s < SLOTS - 1; ++s) {
+        auto ask = [&](int s) {
             if (kbegin + s * TM_KT < kend) issue_tile(s, kbegin + s * TM_KT, pages[s]);
             else cp_async_commit();
+        };
+        bool early[SLOTS - 1];
+#pragma unroll
+        for (int s = 0; s < SLOTS - 1; ++s) {
+            early[s] = kbegin + (s + 1) * TM_KT <= pos0;
+            if (early[s]) ask(s);
         }
+        grid_dependency_wait();
+        grid_dependents_go();
+#pragma unroll
+        for (int s = 0; s < SLOTS - 1; ++s) if (!early[s]) ask(s);
     }
     int page_ahead = page_of(kbegin + (SLOTS - 1) * TM_KT);
 
@@ -914,7 +936,7 @@ template <typename T> __device__ __forceinline__ void sa_store(T* p, const float
 
 // o = sum_z acc_z e^(m_z - M) / sum_z l_z e^(m_z - M) over the key ranges z of one (token, head).  The
 // weights of 32 ranges at a time are worked out by the lanes of every warp and handed round by shuffles;
-// a range's values are asked for eight ranges at a time.
+// the values are asked for sixteen ranges at a time, the first before the weights are known.
 template <typename T>
 __global__ void sa_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                   T* __restrict__ out, int out_ld, int tokens, int heads, int dv,
@@ -933,29 +955,34 @@ __global__ void sa_combine_kernel(const float* __restrict__ part_o, const float*
         const bool mine = d < dv;
         float mmax = -INFINITY, denom = 0.f, o = 0.f;
         for (int z0 = 0; z0 < nsplit; z0 += 32) {
-            const int zl = z0 + lane;
+            const int zl = z0 + lane, n = min(32, nsplit - z0);
             float mz = -INFINITY, lz = 0.f;
             if (zl < nsplit) {
                 const float2 ml = *reinterpret_cast<const float2*>(part_ml + ((size_t)zl * stride + slot) * 2);
                 mz = ml.x;
                 lz = ml.y;
             }
+            // the first half of the ranges' values travel beside the maxima and sums: they do not depend on them
+            float ahead[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                ahead[j] = mine ? part_o[((size_t)(z0 + min(j, n - 1)) * stride + slot) * dv + d] : 0.f;
             const float m_new = fmaxf(mmax, warp_max(mz));
             const float corr = mmax == -INFINITY ? 0.f : expf(mmax - m_new);
             const float w = mz == -INFINITY ? 0.f : expf(mz - m_new);
             mmax = m_new;
             denom = denom * corr + warp_sum(lz * w);
             o *= corr;
-            const int n = min(32, nsplit - z0);
-            for (int j0 = 0; j0 < n; j0 += 8) {
-                float v[8];
+            for (int j0 = 0; j0 < n; j0 += 16) {
+                if (j0) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    v[j] = mine ? part_o[((size_t)(z0 + min(j0 + j, n - 1)) * stride + slot) * dv + d] : 0.f;
+                    for (int j = 0; j < 16; ++j)
+                        ahead[j] = mine ? part_o[((size_t)(z0 + min(j0 + j, n - 1)) * stride + slot) * dv + d] : 0.f;
+                }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < 16; ++j) {
                     const float wj = __shfl_sync(0xffffffffu, w, min(j0 + j, 31));
-                    if (j0 + j < n && wj != 0.f) o += v[j] * wj;        // a range without keys may hold anything
+                    if (j0 + j < n && wj != 0.f) o += ahead[j] * wj;        // a range without keys may hold anything
                 }
             }
         }
