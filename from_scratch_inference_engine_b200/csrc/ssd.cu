@@ -103,6 +103,67 @@ __global__ void ssd_prep_kernel(const T* __restrict__ proj, int ld, int conv_off
     }
 }
 
+// The same for a step of one token per request, eight channels per thread and a block for every 1,024 of a token's: nothing
+// waits for another thread (a thread works out its head's step size itself), what the model and the lists hold is asked
+// for before the kernel that makes the projection has finished, and a thread moves its channels' tails on (ssd_tails'
+// work).  With one block per token, a search behind a barrier and the tails in a launch of their own a token of 4,352 channels
+// took 16 + 8 us of the step's chain.
+constexpr int SSD_ROW_THREADS = 128;
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(SSD_ROW_THREADS) ssd_prep_rows_kernel(
+        const T* __restrict__ proj, int ld, int conv_off, int dt_off, const int* __restrict__ item_qstart,
+        const int* __restrict__ item_slots, int items, float* state, long long state_stride, long long tail_off,
+        const float* __restrict__ conv_wt, const float* __restrict__ conv_b, int channels, const float* __restrict__ dt_bias,
+        const float* __restrict__ a_log, int heads, int vdim, float* __restrict__ act, int act_ld, float* __restrict__ decay) {
+    const int t = blockIdx.x, c = (blockIdx.y * SSD_ROW_THREADS + threadIdx.x) * 8, inner = heads * vdim;
+    int item = t;
+    if (item_qstart[t] != t) {                          // requests in another order than their tokens
+        item = -1;
+        for (int i = 0; i < items; ++i) if (item_qstart[i] == t) item = i;
+    }
+    const int slot = item < 0 ? -1 : item_slots[item];
+    const bool active = c < channels, has_head = active && c < inner;
+    float w[TAPS][8], sum[8], bias = 0.f, rate = 0.f;
+    const int h = has_head ? c / vdim : 0;
+    if (active) {
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) load8(conv_wt + (size_t)j * channels + c, w[j]);
+        if (conv_b) load8(conv_b + c, sum);
+        else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sum[i] = 0.f;
+        }
+        if (has_head) { bias = dt_bias[h]; rate = a_log[h]; }
+    }
+    grid_dependency_wait();
+    grid_dependents_go();
+    if (slot < 0 || !active) return;                    // a padding entry of a fixed-size batch
+    const T* row = proj + (size_t)t * ld;
+    float* tail = state + (size_t)slot * state_stride + tail_off + c;
+    float u[TAPS][8];
+#pragma unroll
+    for (int j = 0; j + 1 < TAPS; ++j) load8(tail + (size_t)j * channels, u[j]);
+    load8(row + conv_off + c, u[TAPS - 1]);
+    const float z = has_head ? to_float(row[dt_off + h]) : 0.f;
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum[i] = fmaf(w[j][i], u[j][i], sum[i]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum[i] = ssd_silu(sum[i]);
+    float* out = act + (size_t)t * act_ld;
+    store8(out + c, sum);
+    if (has_head) {
+        const float dt = ssd_softplus(z + bias);
+        if (c == h * vdim) decay[(size_t)t * heads + h] = expf(-expf(rate) * dt);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum[i] *= dt;
+        store8(out + channels + c, sum);
+    }
+#pragma unroll
+    for (int j = 1; j < TAPS; ++j) store8(tail + (size_t)(j - 1) * channels, u[j]);
+}
+
 // One block per request: the last taps - 1 inputs of (what the slot held, then the step's tokens).
 template <typename T>
 __global__ void ssd_tails_kernel(const T* __restrict__ proj, int ld, int conv_off,
@@ -159,6 +220,43 @@ __global__ void ssd_gate_norm_kernel(const float* __restrict__ o, const float* _
         y[t * inner + c0 + i] = from_float<T>(ssd_row[i] * inv * gain[c0 + i]);
 }
 
+// The same with eight neighbouring values per thread and the row in registers (up to 8,192 values): one trip to memory and one
+// sum over the block (a token of 4,096: 14.5 us of the step's chain with a value per thread and turn).
+template <typename T>
+__global__ void __launch_bounds__(1024) ssd_gate_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ act,
+                                                                 int act_ld, const T* __restrict__ proj, int ld, int z_off,
+                                                                 const float* __restrict__ skip, const float* __restrict__ gain,
+                                                                 T* __restrict__ y, int inner, int vdim, int parts, float eps) {
+    __shared__ float scratch[32];
+    const size_t t = blockIdx.x;
+    const int width = inner / parts, c = blockIdx.y * width + threadIdx.x * 8;
+    const bool active = (int)threadIdx.x * 8 < width;
+    float g[8], d = 0.f;
+    if (active) {
+        load8(gain + c, g);
+        d = skip[c / vdim];
+    }
+    grid_dependency_wait();
+    grid_dependents_go();
+    float v[8], sq = 0.f;
+    if (active) {
+        float x[8], z[8];
+        load8(o + t * inner + c, v);
+        load8(act + t * act_ld + c, x);
+        load8(proj + t * ld + z_off + c, z);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            v[i] = (v[i] + d * x[i]) * ssd_silu(z[i]);
+            sq += v[i] * v[i];
+        }
+    }
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+    if (!active) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = v[i] * inv * g[i];
+    store8(y + t * inner + c, v);
+}
+
 }  // namespace fsie
 
 using namespace fsie;
@@ -171,13 +269,17 @@ int fsie_ssd_max_taps() { return SSD_MAX_TAPS; }
 // the last taps - 1 tokens at tail_off; conv_w [channels, taps], conv_b [channels] or null, dt_bias,
 // a_log [heads] float; act [tokens, act_ld >= channels + heads * vdim] and decay [tokens, heads] float;
 // conv_wt [taps, channels] float or null: conv_w transposed, for the form that takes eight channels at once.
+// fold_tails != 0 (every request brings one token): the kernel also moves the requests' tails on where it can; *folded
+// (host memory) says whether it does, else ssd_tails has to follow.
 int fsie_ssd_prep(const void* proj, int ld, int conv_off, int dt_off, const int* item_qstart,
-                  const int* item_qlen, const int* item_slots, int items, const float* state,
+                  const int* item_qlen, const int* item_slots, int items, float* state,
                   long long state_stride, long long tail_off, const float* conv_w, const float* conv_b,
                   int taps, int channels, const float* dt_bias, const float* a_log, int heads, int vdim,
                   float* act, int act_ld, float* decay, const float* conv_wt, int tokens, int dtype,
-                  cudaStream_t stream) {
+                  int fold_tails, int* folded, cudaStream_t stream) {
+    if (folded) *folded = 0;
     if (tokens <= 0 || items <= 0) return 0;
+    if (fold_tails && (tokens != items || !folded)) return ERR_BAD_ARGUMENT;
     if (taps < 1 || taps > SSD_MAX_TAPS || channels < heads * vdim || heads <= 0 || vdim <= 0 ||
         act_ld < channels + heads * vdim || (taps > 1 && !state))
         return ERR_BAD_ARGUMENT;
@@ -186,6 +288,18 @@ int fsie_ssd_prep(const void* proj, int ld, int conv_off, int dt_off, const int*
     const bool vec = conv_wt && channels % 8 == 0 && vdim % 8 == 0 && conv_off % 8 == 0 && ld % 8 == 0 && act_ld % 8 == 0 &&
         (taps == 1 || (state_stride % 8 == 0 && tail_off % 8 == 0)) &&
         ((((size_t)proj) | ((size_t)act) | ((size_t)state) | ((size_t)conv_b) | ((size_t)conv_wt)) & 31) == 0;
+    if (vec && fold_tails && taps >= 2 && taps <= 4) {
+        *folded = 1;
+        const dim3 grid(tokens, (channels / 8 + SSD_ROW_THREADS - 1) / SSD_ROW_THREADS);
+#define FSIE_SSD_ROWS(T, N)                                                                                               \
+        launch_dependent(ssd_prep_rows_kernel<T, N>, grid, SSD_ROW_THREADS, 0, stream, (const T*)proj, ld, conv_off, dt_off, \
+                         item_qstart, item_slots, items, state, state_stride, tail_off, conv_wt, conv_b, channels, dt_bias, \
+                         a_log, heads, vdim, act, act_ld, decay)
+        if (dtype == DTYPE_F32)
+            return taps == 2 ? FSIE_SSD_ROWS(float, 2) : (taps == 3 ? FSIE_SSD_ROWS(float, 3) : FSIE_SSD_ROWS(float, 4));
+        return taps == 2 ? FSIE_SSD_ROWS(bf16, 2) : (taps == 3 ? FSIE_SSD_ROWS(bf16, 3) : FSIE_SSD_ROWS(bf16, 4));
+#undef FSIE_SSD_ROWS
+    }
     const int threads = vec ? (channels >= 2048 ? 256 : (channels >= 1024 ? 128 : 64))
                             : (channels >= 2048 ? 512 : (channels >= 512 ? 256 : 128));
 #define FSIE_SSD_PREP(T, V)                                                                                        \
@@ -220,10 +334,19 @@ int fsie_ssd_gate_norm(const float* o, const float* act, int act_ld, const void*
     if (inner <= 0 || vdim <= 0 || inner % vdim || parts <= 0 || inner % parts || parts > 65535)
         return ERR_BAD_ARGUMENT;
     const int width = inner / parts;
+    const dim3 grid(tokens, parts);
+    if (width % 8 == 0 && vdim % 8 == 0 && width <= 8192 && act_ld % 8 == 0 && ld % 8 == 0 && z_off % 8 == 0 &&
+        ((((size_t)o) | ((size_t)act) | ((size_t)proj) | ((size_t)gain) | ((size_t)y)) & 15) == 0) {
+        const int threads = ((width / 8 + 31) / 32) * 32;
+        if (dtype == DTYPE_F32)
+            return launch_dependent(ssd_gate_norm_vec_kernel<float>, grid, threads, 0, stream, o, act, act_ld, (const float*)proj,
+                                    ld, z_off, skip, gain, (float*)y, inner, vdim, parts, eps);
+        return launch_dependent(ssd_gate_norm_vec_kernel<bf16>, grid, threads, 0, stream, o, act, act_ld, (const bf16*)proj, ld,
+                                z_off, skip, gain, (bf16*)y, inner, vdim, parts, eps);
+    }
     const size_t smem = (size_t)width * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    const dim3 grid(tokens, parts);
     if (dtype == DTYPE_F32) {
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(ssd_gate_norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

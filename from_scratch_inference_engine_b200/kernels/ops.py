@@ -1110,7 +1110,7 @@ def scan():
         lib.fsie_gated_rmsnorm.argtypes = [p, p, i, i, p, p, i, i, f, i, p]
         lib.fsie_ssd_max_taps.argtypes = []
         lib.fsie_ssd_prep.argtypes = [p, i, i, i, p, p, p, i, p, ll, ll, p, p, i, i, p, p, i, i, p, i, p,
-                                      p, i, i, p]
+                                      p, i, i, i, p, p]
         lib.fsie_ssd_tails.argtypes = [p, i, i, p, p, p, i, p, ll, ll, i, i, i, p]
         lib.fsie_ssd_gate_norm.argtypes = [p, p, i, p, i, i, p, p, p, i, i, i, i, f, i, p]
         for name in ("fsie_lightning_scan", "fsie_row_decay", "fsie_head_norm_silu", "fsie_silu_rows", "fsie_gated_rmsnorm", "fsie_ssd_max_taps",
@@ -1294,7 +1294,7 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
              state: Optional[torch.Tensor], tail_off: int, conv_w: torch.Tensor,
              conv_b: Optional[torch.Tensor], dt_bias: torch.Tensor, a_log: torch.Tensor, heads: int,
              vdim: int, act: torch.Tensor, decay: torch.Tensor,
-             conv_wt: Optional[torch.Tensor] = None) -> None:
+             conv_wt: Optional[torch.Tensor] = None, move_tails: bool = False) -> None:
     """What a state-space mixer's scan reads, per token of proj [tokens, ld] (the stored projection
     with the convolution's input columns at conv_off and the step sizes at dt_off):
     act [tokens, channels + heads * vdim] float32 = [silu(causal convolution + bias) | dt * x] with x
@@ -1303,7 +1303,8 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
     the inputs of the taps - 1 tokens before a step's first live in the request's slot of `state`
     [slots, n] (float32) from float tail_off on, oldest first (`ssd_tails` moves them on).  conv_wt:
     conv_w transposed ([taps, channels], contiguous), with which sizes in multiples of 8 take eight
-    channels per thread."""
+    channels per thread.  `move_tails`: the slots move on too, as by `ssd_tails`: in the same launch where every
+    request brings one token and the kernel for these sizes can, else by a call of it."""
     _need(proj, None, "proj")
     _need(conv_w, torch.float32, "conv_w")
     _need(dt_bias, torch.float32, "dt_bias")
@@ -1326,11 +1327,15 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
         stride = state.stride(0)
         if tail_off + (taps - 1) * channels > stride:
             raise KernelError("ssd_prep: the state slots do not hold the convolution's inputs")
+    moved = ctypes.c_int(0)
     _check(scan().fsie_ssd_prep(proj, ld, conv_off, dt_off, item_qstart, item_qlen,
                                 item_slots, items, state, stride, tail_off, conv_w,
                                 conv_b, taps, channels, dt_bias, a_log, heads, vdim,
                                 act, act.stride(0), decay, conv_wt, tokens,
-                                _tag(proj.dtype), _stream()), "ssd_prep")
+                                _tag(proj.dtype), int(move_tails and taps > 1 and tokens == items),
+                                ctypes.addressof(moved), _stream()), "ssd_prep")
+    if move_tails and taps > 1 and not moved.value:
+        ssd_tails(proj, conv_off, channels, taps, item_qstart, item_qlen, item_slots, items, state, tail_off)
 
 
 def ssd_tails(proj: torch.Tensor, conv_off: int, channels: int, taps: int, item_qstart: torch.Tensor,
