@@ -58,8 +58,10 @@ template <int DR> __device__ __forceinline__ int scan_row_at(int d) {
 // from a zero state (`chunk_states` receives the sum, nothing else is written), a second kernel
 // chains the sums into the state at every chunk's start, and every chunk then runs again from
 // that state and writes the outputs.
-// ROWS: a decay per state row (decay_row); the outputs are multiplied by out_scale.
-template <int DR, typename T, bool ROWS>
+// ROWS: a decay per state row (decay_row); the outputs are multiplied by out_scale.  SILU: q, k and v are the SiLU of what proj
+// holds, taken as they are staged (a launch less in a decode step; chunks, which stage every value eight
+// times, read what silu_rows left).
+template <int DR, typename T, bool ROWS, bool SILU>
 __global__ void __launch_bounds__(SCAN_COLS / 4 * SCAN_ROW_GROUPS)
 lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off,
                       const int* __restrict__ item_qstart, const int* __restrict__ item_qlen,
@@ -97,6 +99,12 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
     float* mine = (phase == 0 ? state + (size_t)slot * state_stride + ((size_t)head * dim) * vdim
                               : chunk_states + (((size_t)blockIdx.z * heads + head) * dim) * vdim);
     const float head_decay = decay ? decay[head] : 1.f;
+    auto one = [&](const T* at) { const float v = to_float(*at); return SILU ? silu_f(v) : v; };
+    auto four = [&](const T* at) {
+        float4 v = scan_load4(at);
+        if (SILU) v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+        return v;
+    };
     const int qk_head = head / share;                  // `share` heads read the same q and k columns
     float through = 1.f;                               // the product of the chunk's decays (phase 1)
     float s[DR][4];
@@ -125,8 +133,8 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
                 const int at = t * ROW_LEN + scan_row_at<DR>(d);
                 const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (write_out)
-                    *reinterpret_cast<float4*>(qs + at) = d < dim ? scan_load4(row + q_off) : zero;
-                *reinterpret_cast<float4*>(ks + at) = d < dim ? scan_load4(row + k_off) : zero;
+                    *reinterpret_cast<float4*>(qs + at) = d < dim ? four(row + q_off) : zero;
+                *reinterpret_cast<float4*>(ks + at) = d < dim ? four(row + k_off) : zero;
                 if (ROWS)
                     *reinterpret_cast<float4*>(as + at) = d < dim ? scan_load4(decay_row + ((size_t)(start + t0 + t) * heads + head) * dim + d) : zero;
             }
@@ -135,15 +143,15 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
                 const int t = idx / (SCAN_ROW_GROUPS * DR), d = idx - t * (SCAN_ROW_GROUPS * DR);
                 const T* row = proj + (size_t)(start + t0 + t) * ld + qk_head * dim + d;
                 const int at = t * ROW_LEN + scan_row_at<DR>(d);
-                if (write_out) qs[at] = d < dim ? to_float(row[q_off]) : 0.f;
-                ks[at] = d < dim ? to_float(row[k_off]) : 0.f;
+                if (write_out) qs[at] = d < dim ? one(row + q_off) : 0.f;
+                ks[at] = d < dim ? one(row + k_off) : 0.f;
                 if (ROWS) as[at] = d < dim ? decay_row[((size_t)(start + t0 + t) * heads + head) * dim + d] : 0.f;
             }
         }
         for (int idx = threadIdx.x; idx < n * SCAN_COLS; idx += blockDim.x) {
             const int t = idx / SCAN_COLS, c = idx - t * SCAN_COLS;
             const int cc = blockIdx.x * SCAN_COLS + c;
-            vs[idx] = cc < vdim ? to_float(proj[(size_t)(start + t0 + t) * ld + v_off + head * vdim + cc]) : 0.f;
+            vs[idx] = cc < vdim ? one(proj + (size_t)(start + t0 + t) * ld + v_off + head * vdim + cc) : 0.f;
         }
         if (!ROWS && threadIdx.x < n)
             ls[threadIdx.x] = decay_tok ? decay_tok[(size_t)(start + t0 + threadIdx.x) * heads + head] : head_decay;
@@ -267,16 +275,34 @@ __global__ void lightning_chain_kernel(const int* __restrict__ item_qstart, cons
     const float lambda = decay ? decay[head] : 1.f;
     const int row = (int)((e - head * per_head) / vdim);
     float s = state[(size_t)slot * state_stride + e];
-    for (int c = 0; c < chunks; ++c) {
-        const int len = min(seg_tokens, count - c * seg_tokens);
-        float* at = chunk_states + (size_t)(first + c) * per_state + e;
-        const float sum = *at;
-        *at = s;
-        float power = 1.f;                                 // decay^len by the same products as the scan
-        if (by_row) power = chunk_decay[((size_t)(first + c) * heads + head) * dim + row];
-        else if (chunk_decay) power = chunk_decay[(size_t)(first + c) * heads + head];     // (what the chunk's walk multiplied)
-        else for (int t = 0; t < len; ++t) power *= lambda;
-        s = power * s + sum;
+    float* mine = chunk_states + (size_t)first * per_state + e;
+    // decay^len by the same products as the scan; all chunks but the last are of seg_tokens
+    float whole = 1.f, rest = 1.f;
+    if (!by_row && !chunk_decay) {
+        for (int t = 0; t < seg_tokens; ++t) whole *= lambda;
+        for (int t = (chunks - 1) * seg_tokens; t < count; ++t) rest *= lambda;
+    }
+    auto power_of = [&](int c) {
+        if (by_row) return chunk_decay[((size_t)(first + c) * heads + head) * dim + row];
+        if (chunk_decay) return chunk_decay[(size_t)(first + c) * heads + head];     // (what the chunk's walk multiplied)
+        return c + 1 < chunks ? whole : rest;
+    };
+    // eight chunks' sums travel together: one by one a prompt's chunks were as many trips to memory in a row
+    constexpr int AHEAD = 8;
+    for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+        float sum[AHEAD], power[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+            const int c = min(c0 + j, chunks - 1);
+            sum[j] = mine[(size_t)c * per_state];
+            power[j] = power_of(c);
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+            if (c0 + j >= chunks) break;
+            mine[(size_t)(c0 + j) * per_state] = s;
+            s = power[j] * s + sum[j];
+        }
     }
     state[(size_t)slot * state_stride + e] = s;
 }
@@ -397,6 +423,33 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __res
     }
 }
 
+// The same with eight neighbouring values per thread and the row in registers (up to 8,192 values): one trip to memory and one
+// sum over the block in a decode step's chain (4 tokens of 2,048: 5.4 us with a value per thread and turn).
+template <typename T>
+__global__ void __launch_bounds__(1024) gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ proj, int ld,
+                                                                 int g_off, const float* __restrict__ gain, T* __restrict__ y,
+                                                                 int width, float eps) {
+    __shared__ float scratch[32];
+    const size_t t = blockIdx.x;
+    const int c = threadIdx.x * 8;
+    const bool active = c < width;
+    float w[8], v[8], g[8], sq = 0.f;
+    if (active) load8(gain + c, w);
+    grid_dependency_wait();
+    grid_dependents_go();
+    if (active) {
+        load8(o + t * width + c, v);
+        load8(proj + t * ld + g_off + c, g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sq += v[i] * v[i];
+    }
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+    if (!active) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = v[i] * inv * w[i] * (1.0f / (1.0f + expf(-g[i])));
+    store8(y + t * width + c, v);
+}
+
 }  // namespace fsie
 
 using namespace fsie;
@@ -423,18 +476,18 @@ int fsie_silu_rows(const void* proj, int ld, int width, float* act, int tokens, 
 // With seg_item / seg_row0 (num_segs chunks of seg_tokens tokens, listed request by request) and
 // chunk_states [num_segs, heads, dim, vdim] (with decay_tok: and num_segs * heads floats more, with decay_row
 // num_segs * heads * dim more) the requests run chunk-parallel in three launches.  decay_row [tokens, heads *
-// dim]: a decay per state row in place of the others; proj may then be of either storage type (`dtype`), else it
-// is float.  The outputs are multiplied by out_scale.
+// dim]: a decay per state row in place of the others.  With that or with silu != 0 (q, k and v are the SiLU of what proj
+// holds; not both) proj may be of either storage type (`dtype`), else it is float.  The outputs are multiplied by out_scale.
 int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_off,
                         const int* item_qstart, const int* item_qlen, const int* item_slots,
                         int items, float* state, const float* decay, float* out, int heads,
                         int dim, int vdim, const int* seg_item, const int* seg_row0, int num_segs,
                         int seg_tokens, float* chunk_states, int share, const float* decay_tok,
-                        const float* decay_row, float out_scale, int dtype, long long state_stride,
+                        const float* decay_row, float out_scale, int dtype, long long state_stride, int silu,
                         cudaStream_t stream) {
     if (items <= 0) return 0;
     if (heads <= 0 || dim <= 0 || vdim <= 0 || heads > 65535 || items > 65535 || share <= 0 ||
-        heads % share || (!decay && !decay_tok && !decay_row) || (dtype != DTYPE_F32 && !decay_row) || state_stride < (long long)heads * dim * vdim)
+        heads % share || (!decay && !decay_tok && !decay_row) || (dtype != DTYPE_F32 && !decay_row && !silu) || (silu && decay_row) || state_stride < (long long)heads * dim * vdim)
         return ERR_BAD_ARGUMENT;
     if (dim > SCAN_ROW_GROUPS * 16) return ERR_UNSUPPORTED;
     const bool chunked = seg_item != nullptr;
@@ -447,24 +500,26 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
     const int threads = SCAN_COLS / 4 * SCAN_ROW_GROUPS;
     const int per_thread = (dim + SCAN_ROW_GROUPS - 1) / SCAN_ROW_GROUPS;
     int launch_code = 0;
-#define FSIE_SCAN(T, R, DPT)                                                                     \
-    launch_code = launch_dependent(lightning_scan_kernel<DPT, T, R>, grid, threads, 0, stream,   \
+#define FSIE_SCAN(T, R, S, DPT)                                                                  \
+    launch_code = launch_dependent(lightning_scan_kernel<DPT, T, R, S>, grid, threads, 0, stream,   \
         (const T*)proj, ld, q_off, k_off, v_off, item_qstart, item_qlen, item_slots, state,      \
         decay, out, heads, dim, vdim, seg_item, seg_row0, seg_tokens, chunk_states, phase, share, \
         decay_tok, decay_row, out_scale, state_stride, chunk_decay)
-#define FSIE_SCAN_SIZES(T, R)                                                                    \
+#define FSIE_SCAN_SIZES(T, R, S)                                                                 \
     do {                                                                                         \
-        if (per_thread <= 1) FSIE_SCAN(T, R, 1);                                                 \
-        else if (per_thread <= 2) FSIE_SCAN(T, R, 2);                                            \
-        else if (per_thread <= 4) FSIE_SCAN(T, R, 4);                                            \
-        else if (per_thread <= 8) FSIE_SCAN(T, R, 8);                                            \
-        else FSIE_SCAN(T, R, 16);                                                                \
+        if (per_thread <= 1) FSIE_SCAN(T, R, S, 1);                                              \
+        else if (per_thread <= 2) FSIE_SCAN(T, R, S, 2);                                         \
+        else if (per_thread <= 4) FSIE_SCAN(T, R, S, 4);                                         \
+        else if (per_thread <= 8) FSIE_SCAN(T, R, S, 8);                                         \
+        else FSIE_SCAN(T, R, S, 16);                                                             \
     } while (0)
 #define FSIE_SCAN_BY_SIZE()                                                                      \
     do {                                                                                         \
-        if (!decay_row) FSIE_SCAN_SIZES(float, false);                                           \
-        else if (dtype == DTYPE_F32) FSIE_SCAN_SIZES(float, true);                               \
-        else FSIE_SCAN_SIZES(bf16, true);                                                        \
+        if (silu && dtype == DTYPE_F32) FSIE_SCAN_SIZES(float, false, true);                     \
+        else if (silu) FSIE_SCAN_SIZES(bf16, false, true);                                       \
+        else if (!decay_row) FSIE_SCAN_SIZES(float, false, false);                               \
+        else if (dtype == DTYPE_F32) FSIE_SCAN_SIZES(float, true, false);                        \
+        else FSIE_SCAN_SIZES(bf16, true, false);                                                 \
     } while (0)
     FSIE_SCAN_BY_SIZE();
     if (launch_code) return launch_code;
@@ -520,6 +575,15 @@ int fsie_head_norm_silu(const float* o, const void* proj, int ld, int g_off, con
 int fsie_gated_rmsnorm(const float* o, const void* proj, int ld, int g_off, const float* gain,
                        void* y, int tokens, int width, float eps, int dtype, cudaStream_t stream) {
     if (tokens <= 0) return 0;
+    if (width % 8 == 0 && width <= 8192 && ld % 8 == 0 && g_off % 8 == 0 &&
+        ((((size_t)o) | ((size_t)proj) | ((size_t)gain) | ((size_t)y)) & 15) == 0) {
+        const int threads = ((width / 8 + 31) / 32) * 32;
+        if (dtype == DTYPE_F32)
+            return launch_dependent(gated_rmsnorm_vec_kernel<float>, tokens, threads, 0, stream, o, (const float*)proj, ld, g_off,
+                                    gain, (float*)y, width, eps);
+        return launch_dependent(gated_rmsnorm_vec_kernel<bf16>, tokens, threads, 0, stream, o, (const bf16*)proj, ld, g_off, gain,
+                                (bf16*)y, width, eps);
+    }
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
     if (dtype == DTYPE_F32)
         return launch_dependent(gated_rmsnorm_kernel<float>, tokens, threads, 0, stream, o,

@@ -1103,7 +1103,7 @@ def scan():
         lib = build.load_library("scan")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_lightning_scan.argtypes = [p, i, i, i, i, p, p, p, i, p, p, p, i, i, i, p, p, i, i, p,
-                                            i, p, p, f, i, ll, p]
+                                            i, p, p, f, i, ll, i, p]
         lib.fsie_row_decay.argtypes = [p, i, i, i, p, p, f, p, i, i, i, p]
         lib.fsie_head_norm_silu.argtypes = [p, p, i, i, p, p, i, i, i, f, i, p]
         lib.fsie_silu_rows.argtypes = [p, i, i, p, i, i, p]
@@ -1226,7 +1226,7 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                    seg_row0: Optional[torch.Tensor] = None, num_segs: int = 0, seg_tokens: int = 0,
                    chunk_states: Optional[torch.Tensor] = None, share: int = 1,
                    decay_tok: Optional[torch.Tensor] = None, decay_row: Optional[torch.Tensor] = None,
-                   out_scale: float = 1.0) -> torch.Tensor:
+                   out_scale: float = 1.0, silu: bool = False) -> torch.Tensor:
     """Per request and head, token by token: S = decay * S + k v^T, o = S^T q.  proj [tokens, ld]
     (float32) holds the ACTIVATED projections (`silu_rows`) at the given column offsets; state
     [slots, heads, dim, vdim] (float32; or [slots, n] with the heads' matrices in the first
@@ -1234,14 +1234,17 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     float32.  `decay_tok` (float32 [tokens, heads]) gives a decay per token and head in place of
     `decay`; `decay_row` (float32 [tokens, heads * dim]) one per token, head and state row - proj may then be
     of either storage type; the outputs are multiplied by `out_scale`; `share` heads in a row read the same q and k columns (q and k then hold heads / share
-    column groups of `dim`).
+    column groups of `dim`).  `silu` (no `decay_row`): proj of either storage type holds the projections as they are, the
+    activation is taken as they are read.
 
     With `seg_item` / `seg_row0` (int32, one entry per chunk of `seg_tokens` tokens, listed
     request by request) and `chunk_states` (float32, num_segs * heads * dim * vdim at least; with
     `decay_tok` num_segs * heads more, with `decay_row` num_segs * heads * dim more) the
     chunks of long prompts run side by side: each sums its own tokens, the sums are chained into
     the state at every chunk's start, and each chunk runs again from there for its outputs."""
-    _need(proj, torch.float32 if decay_row is None else None, "proj")
+    _need(proj, torch.float32 if decay_row is None and not silu else None, "proj")
+    if silu and decay_row is not None:
+        raise KernelError("lightning_scan: a decay per state row comes with activated projections")
     _need(state, torch.float32, "state")
     if decay is not None:
         _need(decay, torch.float32, "decay")
@@ -1280,7 +1283,7 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                                       decay, out, heads, dim, vdim, seg_item,
                                       seg_row0, num_segs, seg_tokens, chunk_states,
                                       int(share), decay_tok, decay_row, float(out_scale),
-                                      _tag(proj.dtype), state_stride, _stream()),
+                                      _tag(proj.dtype), state_stride, int(silu), _stream()),
            "lightning_scan")
     return out
 

@@ -76,12 +76,13 @@ class LightningAttention(Mixer):
                           seg_tokens=self.CHUNK_TOKENS,
                           chunk_states=ctx.scratch("lightning.chunk_states",
                                                    tiles.count * self.heads * self.dim * self.vdim))
-        # the activations of q, k and v once, in 32-bit: the scan reads each of them several times
-        width = 2 * self.qk_width + self.v_width
-        act = ops.silu_rows(proj, width, rt.buffer("lightning.act", tokens, width, torch.float32))
+        act = proj
+        if chunks:      # the activations of q, k and v once, in 32-bit: chunks read each of them several times
+            width = 2 * self.qk_width + self.v_width
+            act = ops.silu_rows(proj, width, rt.buffer("lightning.act", tokens, width, torch.float32))
         ops.lightning_scan(act, 0, self.qk_width, 2 * self.qk_width, ctx.item_qstart,
                            ctx.item_qlen, ctx.item_slots, ctx.num_items, cache.state, self.decay, o,
-                           self.heads, self.dim, self.vdim, **chunks)
+                           self.heads, self.dim, self.vdim, silu=not chunks, **chunks)
         gated = rt.buffer("lightning.gated", tokens, self.v_width, proj.dtype)
         ops.gated_rmsnorm(o, proj, 2 * self.qk_width + self.v_width, self.gain, self.eps, gated)
         return rt.linear(gated, self.w_o, None, "lightning.out")
