@@ -27,9 +27,10 @@ __global__ void latent_prep_kernel(const T* __restrict__ proj, int ld, const int
                                    int rotary_dim, int half_pairs, int* __restrict__ error) {
     __shared__ float scratch[32];
     const int t = blockIdx.x;
+    // position and slot were staged before the step: read while the kernel before still runs
+    const int pos = positions[t], slot = slot_of ? slot_of[t] : -1;
     grid_dependency_wait();
     grid_dependents_go();
-    const int pos = positions[t];
     if (rotary_dim > 0 && (pos < 0 || pos >= table_len)) {
         if (threadIdx.x == 0) atomicExch(error, 2);
         return;
@@ -54,7 +55,6 @@ __global__ void latent_prep_kernel(const T* __restrict__ proj, int ld, const int
         }
         qa[((size_t)t * heads + h) * row_width + rank + d] = from_float<T>(val);
     }
-    const int slot = slot_of ? slot_of[t] : -1;
     const T* lat = row + heads * qd;
     float ss = 0.f;
     for (int d = threadIdx.x; d < rank; d += blockDim.x) {
@@ -222,6 +222,84 @@ __device__ __forceinline__ void hm_cp16(void* dst, const void* src, bool valid) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(hm_smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
+// ---- the same for few tokens of bfloat16 on the tensor cores: a warp owns 16 output rows of one head (M of m16n8k16; the
+// tokens are N), and KW warps share the k range.  What bounds it is the chain from the kernel before to its result, so
+// there is no staging: a lane's 16 bytes of two weight rows are its fragments as they are (the order of k does
+// not matter to a dot product), asked for before that kernel has finished, and x gives the matching 16 bytes.
+constexpr int HQ_WARPS = 4, HQ_AHEAD = 4;                      // chunks of 32 k-elements asked for together
+template <int TT, int KW>
+__global__ void __launch_bounds__(HQ_WARPS * 32) head_product_rows_kernel(
+        const bf16* __restrict__ x, long long x_ld, int x_head, const bf16* __restrict__ w, bf16* __restrict__ out,
+        long long out_ld, int out_head, int tokens, int n, int k) {
+    constexpr int TILES = HQ_WARPS / KW;                        // tiles of 16 rows per block
+    __shared__ float parts[KW > 1 ? KW - 1 : 1][TILES][16][8 * TT + 1];
+    const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int part = warp % KW, tile = warp / KW, g = lane >> 2, t = lane & 3;
+    const int row0 = (blockIdx.x * TILES + tile) * 16;
+    const int chunks = k / 32, per = (chunks + KW - 1) / KW, c_begin = part * per, c_end = min(chunks, c_begin + per);
+    const bf16* w_lo = w + ((size_t)h * n + min(row0 + g, n - 1)) * k + 8 * t;
+    const bf16* w_hi = w + ((size_t)h * n + min(row0 + 8 + g, n - 1)) * k + 8 * t;
+    uint4 lo[HQ_AHEAD], hi[HQ_AHEAD];
+    auto weights = [&](int c0) {
+#pragma unroll
+        for (int j = 0; j < HQ_AHEAD; ++j) {
+            const bool in = c0 + j < c_end;
+            lo[j] = in ? __ldg(reinterpret_cast<const uint4*>(w_lo + (c0 + j) * 32)) : make_uint4(0, 0, 0, 0);
+            hi[j] = in ? __ldg(reinterpret_cast<const uint4*>(w_hi + (c0 + j) * 32)) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    weights(c_begin);
+    grid_dependency_wait();
+    grid_dependents_go();
+    float acc[TT][4];
+#pragma unroll
+    for (int m = 0; m < TT; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+    for (int c0 = c_begin; c0 < c_end; c0 += HQ_AHEAD) {
+        uint4 b[HQ_AHEAD][TT];
+#pragma unroll
+        for (int j = 0; j < HQ_AHEAD; ++j)
+#pragma unroll
+            for (int m = 0; m < TT; ++m)
+                b[j][m] = c0 + j < c_end && 8 * m + g < tokens
+                    ? *reinterpret_cast<const uint4*>(x + (size_t)(8 * m + g) * x_ld + (size_t)h * x_head + (c0 + j) * 32 + 8 * t)
+                    : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int j = 0; j < HQ_AHEAD; ++j) {
+            const uint32_t a0[4] = {lo[j].x, hi[j].x, lo[j].y, hi[j].y}, a1[4] = {lo[j].z, hi[j].z, lo[j].w, hi[j].w};
+#pragma unroll
+            for (int m = 0; m < TT; ++m) {
+                hm_mma(acc[m], a0, b[j][m].x, b[j][m].y);
+                hm_mma(acc[m], a1, b[j][m].z, b[j][m].w);
+            }
+        }
+        if (c0 + HQ_AHEAD < c_end) weights(c0 + HQ_AHEAD);
+    }
+    // acc[m]: rows g (0, 1) and g + 8 (2, 3), tokens 8 m + 2 t and 8 m + 2 t + 1; the parts of k are added in order
+    if (KW > 1) {
+        if (part > 0) {
+#pragma unroll
+            for (int m = 0; m < TT; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) parts[part - 1][tile][g + (e >> 1) * 8][8 * m + 2 * t + (e & 1)] = acc[m][e];
+        }
+        __syncthreads();
+        if (part > 0) return;
+#pragma unroll
+        for (int q = 0; q + 1 < KW; ++q)
+#pragma unroll
+            for (int m = 0; m < TT; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][e] += parts[q][tile][g + (e >> 1) * 8][8 * m + 2 * t + (e & 1)];
+    }
+#pragma unroll
+    for (int m = 0; m < TT; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int token = 8 * m + 2 * t + (e & 1), c = row0 + g + (e >> 1) * 8;
+            if (token < tokens && c < n) out[(size_t)token * out_ld + (size_t)h * out_head + c] = __float2bfloat16_rn(acc[m][e]);
+        }
+}
+
 __global__ void __launch_bounds__(128) head_product_mma_kernel(
         const bf16* __restrict__ x, long long x_ld, int x_head, const bf16* __restrict__ w,
         bf16* __restrict__ out, long long out_ld, int out_head, int tokens, int n, int k) {
@@ -327,6 +405,17 @@ int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, 
                 cudaFuncSetAttribute(head_product_few_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             return launch_dependent(head_product_few_kernel<float>, few, dim3(HF_WARPS * 32), smem, stream, (const float*)x,
                                     x_ld, x_head, (const float*)w, (float*)out, out_ld, out_head, tokens, n, k);
+        }
+        // on the tensor cores where rows start on 16 bytes; a warp takes up to four chunks of k, so that all of its
+        // weights are on their way before x is there
+        if (k % 32 == 0 && x_ld % 8 == 0 && x_head % 8 == 0 && ((((size_t)x) | ((size_t)w)) & 15) == 0) {
+#define FSIE_HEAD_ROWS(T, W)                                                                                       \
+            launch_dependent(head_product_rows_kernel<T, W>, dim3((n + 16 * HQ_WARPS / W - 1) / (16 * HQ_WARPS / W), heads), \
+                             dim3(HQ_WARPS * 32), 0, stream, (const bf16*)x, x_ld, x_head, (const bf16*)w, (bf16*)out, \
+                             out_ld, out_head, tokens, n, k)
+            if (tokens <= 8) return k >= 512 ? FSIE_HEAD_ROWS(1, 4) : (k >= 256 ? FSIE_HEAD_ROWS(1, 2) : FSIE_HEAD_ROWS(1, 1));
+            return k >= 512 ? FSIE_HEAD_ROWS(2, 4) : (k >= 256 ? FSIE_HEAD_ROWS(2, 2) : FSIE_HEAD_ROWS(2, 1));
+#undef FSIE_HEAD_ROWS
         }
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(head_product_few_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

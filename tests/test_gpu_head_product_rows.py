@@ -1,0 +1,26 @@
+"""Products per head of few tokens on the tensor cores against 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# one token and the edges of 8 and 16; rows that end inside a warp's 16; k in one, two and four parts, with parts of unequal
+# length; k that the kernel does not take, and rows that do not start on 16 bytes
+@pytest.mark.parametrize("tokens", [1, 8, 9, 16])
+@pytest.mark.parametrize("heads,n,k,gap", [(16, 512, 128, 8), (2, 40, 32, 0), (3, 129, 288, 16), (5, 128, 512, 8), (1, 17, 1056, 8),
+                                           (2, 24, 40, 8), (2, 32, 64, 4)])
+def test_head_product(tokens, heads, n, k, gap):
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(n + k)
+    rand = lambda *shape: torch.randn(shape, generator=generator, device="cuda").to(torch.bfloat16)
+    x_head, out_head = k + gap, n + 3
+    x, w = rand(tokens, heads * x_head + gap), rand(heads, n, k) * k ** -0.5
+    out = torch.full((tokens, heads * out_head), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.head_product(x, x.stride(0), x_head, w, out, out.stride(0), out_head, tokens)
+    rows = torch.stack([x[:, h * x_head:h * x_head + k] for h in range(heads)]).double()           # [heads, tokens, k]
+    want = rows @ w.double().transpose(1, 2)
+    got = torch.stack([out[:, h * out_head:h * out_head + n] for h in range(heads)]).double()
+    size = rows.abs() @ w.double().abs().transpose(1, 2)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + size * k * 2.0 ** -24).all()
+    assert torch.isnan(torch.stack([out[:, h * out_head + n:(h + 1) * out_head] for h in range(heads)])).all()
