@@ -24,6 +24,16 @@ __global__ void sum_layernorm_kernel(float* __restrict__ x, const T* __restrict_
                                      T* __restrict__ y, int width, float eps, int write_x) {
     extern __shared__ __align__(16) float row_cache[];
     __shared__ float scratch[32];
+    // gain and bias of the thread's first trip along the row (a short row's only one) are asked for before the kernel before
+    // has finished, not behind the sums
+    const int first = threadIdx.x * 8;
+    float gain_first[VEC ? 8 : 1], bias_first[VEC ? 8 : 1];
+    if constexpr (VEC) {
+        if (y && first < width) {
+            load8(gain + first, gain_first);
+            if (bias) load8(bias + first, bias_first);
+        }
+    }
     grid_dependency_wait();
     grid_dependents_go();
     const int r = blockIdx.x;
@@ -72,15 +82,17 @@ __global__ void sum_layernorm_kernel(float* __restrict__ x, const T* __restrict_
     const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
     T* yr = y + (size_t)r * width;
     for (int c = threadIdx.x * STEP; c < width; c += blockDim.x * STEP) {
-        if (VEC) {
-            float v[8], g[8], o[8];
+        if constexpr (VEC) {
+            float v[8];
             load8(row_cache + c, v);
-            load8(gain + c, g);
-            if (bias) load8(bias + c, o);
+            if (c != first) {
+                load8(gain + c, gain_first);
+                if (bias) load8(bias + c, bias_first);
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                v[i] = (v[i] - mean) * inv * g[i];
-                if (bias) v[i] += o[i];
+                v[i] = (v[i] - mean) * inv * gain_first[i];
+                if (bias) v[i] += bias_first[i];
             }
             store8(yr + c, v);
         } else {

@@ -58,8 +58,11 @@ __device__ __forceinline__ void store4(bf16* p, const float (&v)[1]) { *p = __fl
 // S: the number of streams, or 0: any number, a thread's old values wait in shared memory.
 // STEP: columns per thread and trip (4: the width is a multiple of 4 and every row starts on 16
 // bytes, or 8 for bfloat16).
-template <typename T, int S, int STEP>
-__global__ void __launch_bounds__(512, S > 0 && S <= 4 ? 2 : 1) stream_norm_kernel(const StreamNormParams p) {
+// FEW: a step of few rows, whose blocks need not share an SM: the gain, the bias and the output's scale of the thread's first
+// trip along the row (the only one where the row is short) are asked for before the kernel before has finished, not behind
+// the sums, where they were one more trip to memory in the chain.
+template <typename T, int S, int STEP, bool FEW>
+__global__ void __launch_bounds__(512, !FEW && S > 0 && S <= 4 ? 2 : 1) stream_norm_kernel(const StreamNormParams p) {
     extern __shared__ __align__(16) float sn_smem[];
     __shared__ float scratch[32];
     const int streams = S > 0 ? S : p.streams, width = p.width;
@@ -74,6 +77,13 @@ __global__ void __launch_bounds__(512, S > 0 && S <= 4 ? 2 : 1) stream_norm_kern
     for (int i = threadIdx.x; i < streams; i += blockDim.x) {
         out[i] = settle ? p.out[i] : 0.f;
         in[i] = p.in ? p.in[i] : 1.f;
+    }
+    const int first = FEW ? threadIdx.x * STEP : -1;
+    float gain_first[STEP], bias_first[STEP], scale_first[STEP];
+    if (FEW && first < width) {
+        if (p.z) load4(p.gain + first, gain_first);
+        if (p.z && p.bias) load4(p.bias + first, bias_first);
+        if (settle && p.y_scale) load4(p.y_scale + first, scale_first);
     }
     __syncthreads();
     grid_dependency_wait();
@@ -93,9 +103,9 @@ __global__ void __launch_bounds__(512, S > 0 && S <= 4 ? 2 : 1) stream_norm_kern
             if (settle) {
                 load4(yr + c, y);
                 if (p.y_scale) {
-                    load4(p.y_scale + c, v);
+                    if (c != first) load4(p.y_scale + c, scale_first);
 #pragma unroll
-                    for (int i = 0; i < STEP; ++i) y[i] *= v[i];
+                    for (int i = 0; i < STEP; ++i) y[i] *= scale_first[i];
                 }
             }
             if (sr) {
@@ -168,17 +178,26 @@ __global__ void __launch_bounds__(512, S > 0 && S <= 4 ? 2 : 1) stream_norm_kern
     const float inv = 1.0f / sqrtf(var + p.eps);
     T* zr = (T*)p.z + (size_t)r * width;
     for (int c = threadIdx.x * STEP; c < width; c += blockDim.x * STEP) {
-        float v[STEP], g[STEP], b[STEP];
+        float v[STEP];
         load4(u + c, v);
-        load4(p.gain + c, g);
-        if (p.bias) load4(p.bias + c, b);
+        if (c != first) {
+            load4(p.gain + c, gain_first);
+            if (p.bias) load4(p.bias + c, bias_first);
+        }
 #pragma unroll
         for (int i = 0; i < STEP; ++i) {
-            v[i] = (v[i] - mean) * inv * g[i];
-            if (p.bias) v[i] += b[i];
+            v[i] = (v[i] - mean) * inv * gain_first[i];
+            if (p.bias) v[i] += bias_first[i];
         }
         store4(zr + c, v);
     }
+}
+
+template <typename T, int S, int STEP, bool FEW>
+static int stream_norm_launch_as(const StreamNormParams& p, int num_rows, int threads, size_t smem, cudaStream_t stream) {
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(stream_norm_kernel<T, S, STEP, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_dependent(stream_norm_kernel<T, S, STEP, FEW>, num_rows, threads, smem, stream, p);
 }
 
 template <typename T, int S, int STEP>
@@ -191,9 +210,8 @@ static int stream_norm_launch(const StreamNormParams& p, int num_rows, cudaStrea
                           (S == 0 ? (size_t)p.streams * threads : 0);
     const size_t smem = floats * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(stream_norm_kernel<T, S, STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_dependent(stream_norm_kernel<T, S, STEP>, num_rows, threads, smem, stream, p);
+    return S > 0 && num_rows <= 64 ? stream_norm_launch_as<T, S, STEP, (S > 0)>(p, num_rows, threads, smem, stream)
+                                   : stream_norm_launch_as<T, S, STEP, false>(p, num_rows, threads, smem, stream);
 }
 
 template <typename T, int STEP>
