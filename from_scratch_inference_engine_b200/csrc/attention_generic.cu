@@ -169,23 +169,40 @@ template <typename T>
 __global__ void attn_combine_kernel(const float* __restrict__ part_o,
                                     const float* __restrict__ part_ml, T* __restrict__ out,
                                     int out_ld, int tokens, int heads, int hd, int nsplit) {
+    extern __shared__ float combine_smem[];              // [3][nsplit]: maxima, sums, weights
+    float *m = combine_smem, *l = m + nsplit, *w = l + nsplit;
     const int tok = blockIdx.x, h = blockIdx.y;
-    float mmax = -INFINITY;
-    for (int z = 0; z < nsplit; ++z)
-        mmax = fmaxf(mmax, part_ml[(((size_t)z * tokens + tok) * heads + h) * 2]);
-    float denom = 0.f;
-    for (int z = 0; z < nsplit; ++z) {
-        const size_t idx = ((size_t)z * tokens + tok) * heads + h;
-        const float mz = part_ml[idx * 2];
-        if (mz != -INFINITY) denom += part_ml[idx * 2 + 1] * expf(mz - mmax);
+    const size_t stride = (size_t)tokens * heads, slot = (size_t)tok * heads + h;
+    grid_dependency_wait();
+    grid_dependents_go();
+    // maxima, sums and the first eight splits' values travel together: none of their addresses depends on another
+    for (int z = threadIdx.x; z < nsplit; z += blockDim.x) {
+        m[z] = part_ml[(z * stride + slot) * 2];
+        l[z] = part_ml[(z * stride + slot) * 2 + 1];
     }
+    constexpr int AHEAD = 8;
+    float ahead[AHEAD];
+    auto ask = [&](int z0, int d) {
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) ahead[j] = part_o[(min(z0 + j, nsplit - 1) * stride + slot) * hd + min(d, hd - 1)];
+    };
+    ask(0, threadIdx.x);
+    __syncthreads();
+    float mmax = -INFINITY;
+    for (int z = 0; z < nsplit; ++z) mmax = fmaxf(mmax, m[z]);
+    for (int z = threadIdx.x; z < nsplit; z += blockDim.x) w[z] = m[z] == -INFINITY ? 0.f : expf(m[z] - mmax);
+    __syncthreads();
+    float denom = 0.f;
+    for (int z = 0; z < nsplit; ++z)
+        if (m[z] != -INFINITY) denom += l[z] * w[z];
     const float inv = denom > 0.f ? 1.0f / denom : 0.f;
     for (int d = threadIdx.x; d < hd; d += blockDim.x) {
         float o = 0.f;
-        for (int z = 0; z < nsplit; ++z) {
-            const size_t idx = ((size_t)z * tokens + tok) * heads + h;
-            const float mz = part_ml[idx * 2];
-            if (mz != -INFINITY) o += part_o[idx * hd + d] * expf(mz - mmax);
+        for (int z0 = 0; z0 < nsplit; z0 += AHEAD) {
+            if (z0 > 0 || d != (int)threadIdx.x) ask(z0, d);
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j)
+                if (z0 + j < nsplit && m[z0 + j] != -INFINITY) o += ahead[j] * w[z0 + j];     // a split without keys may hold anything
         }
         out[(size_t)tok * out_ld + h * hd + d] = from_float<T>(o * inv);
     }
@@ -246,17 +263,6 @@ attn_rows16_kernel(const AttnParams p) {
     const float* vp = (const float*)p.v_pages;
     const int* bt = p.block_tables + (size_t)item * p.bt_stride;
 
-    for (int e = tid; e < FR * hd; e += FTHREADS) {
-        const int r = e / hd, d = e - r * hd;
-        float v = 0.f;
-        if (r < nrows) {
-            const int row = row0 + r;
-            const int tok = qstart + row / group, h = kvh * group + row % group;
-            v = q[(size_t)tok * p.q_ld + h * hd + d] * p.scale;
-        }
-        qs[e] = v;
-    }
-
     const int pos_first = pos0 + row0 / group;
     const int pos_last = pos0 + (row0 + nrows - 1) / group;
     int kbegin = p.window > 0 ? max(0, pos_first - p.window + 1) : 0;
@@ -309,10 +315,26 @@ attn_rows16_kernel(const AttnParams p) {
         row_on[i] = has_values && rg + i * row_groups < nrows;
     }
 
+    // The lists and block tables were staged before the step, and keys older than the request's new tokens were written by
+    // earlier steps: a first chunk of only such keys is asked for while the kernel before still runs.
     find_rows(0);
-    __syncthreads();                                   // qs and key_base[0] are in place
-    if (chunks > 0) fetch(0);
+    __syncthreads();                                   // key_base[0] is in place
+    const bool early = chunks > 0 && kbegin + FK <= pos0;
+    if (early) fetch(0);
     find_rows(1);
+    grid_dependency_wait();
+    grid_dependents_go();
+    if (!early && chunks > 0) fetch(0);
+    for (int e = tid; e < FR * hd; e += FTHREADS) {
+        const int r = e / hd, d = e - r * hd;
+        float v = 0.f;
+        if (r < nrows) {
+            const int row = row0 + r;
+            const int tok = qstart + row / group, h = kvh * group + row % group;
+            v = q[(size_t)tok * p.q_ld + h * hd + d] * p.scale;
+        }
+        qs[e] = v;
+    }
     for (int c = 0; c < chunks; ++c) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                               // chunk c has landed; the last chunk's weights are used up
@@ -699,7 +721,7 @@ int fsie_attn_tiles(const void* q, int q_ld, const void* k_pages, const void* v_
 #define FSIE_ROWS16(HDV)                                                                                        \
     case HDV:                                                                                                   \
         cudaFuncSetAttribute(attn_rows16_kernel<HDV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-        attn_rows16_kernel<HDV><<<grid, FTHREADS, smem, stream>>>(p);                                           \
+        rc = launch_dependent(attn_rows16_kernel<HDV>, grid, dim3(FTHREADS), smem, stream, p);                  \
         break;
             switch (head_dim) {
                 FSIE_ROWS16(32) FSIE_ROWS16(64) FSIE_ROWS16(96) FSIE_ROWS16(128) FSIE_ROWS16(256)
@@ -726,16 +748,18 @@ int fsie_attn_tiles(const void* q, int q_ld, const void* k_pages, const void* v_
                 attn_generic_kernel<bf16><<<grid, WARPS * 32, smem, stream>>>(p);
             }
         }
-        rc = FSIE_LAUNCH_CHECK();
+        if (rc == 0) rc = FSIE_LAUNCH_CHECK();
     }
     if (rc != 0 || nsplit == 1 || !merge) return rc;
     dim3 cgrid(tokens, heads);
     const int threads = head_dim >= 128 ? 128 : (head_dim >= 64 ? 64 : 32);
+    const size_t room = 3 * (size_t)nsplit * sizeof(float);
+    if (room > 48 * 1024) return ERR_UNSUPPORTED;        // (4,096 splits; the grid's z dimension takes 65,535)
     if (dtype == DTYPE_F32)
-        attn_combine_kernel<float><<<cgrid, threads, 0, stream>>>(part_o, part_ml, (float*)out, out_ld, tokens, heads, head_dim, nsplit);
-    else
-        attn_combine_kernel<bf16><<<cgrid, threads, 0, stream>>>(part_o, part_ml, (bf16*)out, out_ld, tokens, heads, head_dim, nsplit);
-    return FSIE_LAUNCH_CHECK();
+        return launch_dependent(attn_combine_kernel<float>, cgrid, dim3(threads), room, stream, part_o, part_ml, (float*)out,
+                                out_ld, tokens, heads, head_dim, nsplit);
+    return launch_dependent(attn_combine_kernel<bf16>, cgrid, dim3(threads), room, stream, part_o, part_ml, (bf16*)out, out_ld,
+                            tokens, heads, head_dim, nsplit);
 }
 
 // The launch as callers outside the engine know it: tiles of up to 32 rows, merged at once.
