@@ -19,7 +19,6 @@
 // Every wait on an mbarrier is bounded: when it runs out the kernel records where in
 // *error, drains what it started, frees its tensor memory and returns.
 #include "common.cuh"
-#include "late_norm.cuh"
 #include "tma.cuh"
 #include <cooperative_groups.h>
 #include <math.h>
@@ -37,15 +36,13 @@ enum { ERR_TMA_WAIT = 11, ERR_MMA_WAIT = 12, ERR_EPILOGUE_WAIT = 13 };
 
 struct GemmParams {
     void* y; int ldy;               // [T, ldy] bf16 or float
-    const bf16* bias;               // [N] or null (SwiGLU: [2 N], the gate rows' and then the up rows')
+    const bf16* bias;               // [N] or null
     int T, N, K;                    // N = output features (SwiGLU: intermediate size)
     int up_row0;                    // SwiGLU: row of w where the up rows start
     int gate;                       // gated epilogue: 1 = SiLU on the gate, 2 = GELU (tanh form); plain epilogue: 3 = the square of relu on the result
     int kblocks_per_split;
     int out_f32;
     int* error;
-    LateNorm norm;                  // x is rows that are still to be normed (parts == nullptr: they are not)
-    LateResidual into;              // plain epilogue: the result goes into the residual stream (x == nullptr: into y)
 };
 
 // Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzle: rows of 128
@@ -95,8 +92,6 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __shared__ uint64_t full_bar[L::STAGES], empty_bar[L::STAGES], acc_bar;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
-    constexpr bool LATE = TN <= 32;                   // pending norms are for few tokens
-    __shared__ float factor[LATE ? TN : 1];           // of each token's norm
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x, split = blockIdx.y, splits = gridDim.y;
@@ -192,11 +187,6 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (warp >= 2) {
         const int quarter = warp & 3;                // the tensor-memory lanes this warp may read
         const int row = quarter * 32 + lane;         // weight row inside the tile = accumulator lane
-        // the factors of a pending norm, while the weights stream
-        for (int t = LATE ? warp - 2 : TN; t < TN; t += 4) {
-            const float f = p.norm.parts && t < p.T ? late_factor(p.norm.parts + (size_t)t * p.norm.count, p.norm, lane) : 1.f;
-            if (lane == 0) factor[t] = f;
-        }
         bool ok = kb1 > kb0 ? mbar_wait(&acc_bar, 0) : true;
         if (!ok) { atomicExch(p.error, ERR_EPILOGUE_WAIT); atomicExch(&abort_flag, 1); }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -242,11 +232,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     for (int e = threadIdx.x; e < rows_per_rank * TN; e += blockDim.x) {
         const int r = r_begin + e % rows_per_rank, t = e / rows_per_rank;
         const int n = n0 + r;
-        const bool in = t < p.T && n < p.N;
-        // (into the residual stream: the 16 lanes of a part stay together; rows per rank and threads are multiples of 16)
-        if (!in && !(LATE && EPI == EPI_PLAIN && p.into.x)) continue;
-        float old = 0.f, gain = 0.f;
-        if (LATE && EPI == EPI_PLAIN && p.into.x) late_fetch(p.into, t, n, in, old, gain);
+        if (t >= p.T || n >= p.N) continue;
         float acc = 0.f, acc_up = 0.f;
         if (splits > 1) {
             cg::cluster_group cluster = cg::this_cluster();
@@ -259,19 +245,9 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             acc = red[r * L::RED_LD + t];
             if (EPI == EPI_SWIGLU) acc_up = red[(r + BM / 2) * L::RED_LD + t];
         }
-        if constexpr (LATE) {
-            acc *= factor[t];
-            if (EPI == EPI_SWIGLU) acc_up *= factor[t];
-        }
         float out;
-        if (LATE && EPI == EPI_PLAIN && p.into.x) {
-            out = acc + (p.bias && in ? __bfloat162float(p.bias[n]) : 0.f);
-            late_store(p.into, out, old, gain, t, n, in, lane);
-            continue;
-        }
         if (EPI == EPI_SWIGLU) {
             // the library path rounds gate and up to bfloat16 before the activation; do the same
-            if (p.bias) { acc += __bfloat162float(p.bias[n]); acc_up += __bfloat162float(p.bias[p.N + n]); }
             const float g = __bfloat162float(__float2bfloat16_rn(acc));
             const float u = __bfloat162float(__float2bfloat16_rn(acc_up));
             out = (p.gate == 2 ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)))
@@ -356,15 +332,9 @@ int fsie_gemm_decode_weight_map(void* map_out, const void* w, long long rows, lo
 
 // y[T, N] = x[T, K] * w^T (+ bias), or for swiglu != 0 y[T, N] = act(x w_gate^T) * (x w_up^T) with
 // w = [gate rows (N); up rows (N)], act = SiLU (swiglu = 1) or the tanh form of GELU (2); swiglu = 3: no gate, y = relu(x w^T)^2.  T <= 64.  `splits` (1, 2, 4 or 8) cuts K over a cluster.
-// norm_* and into_*: norms without a launch of their own, as in fsie_gemm_skinny (late_norm.cuh), up to 32 tokens.
 int fsie_gemm_decode(const void* weight_map, const void* x, int ldx, void* y, int ldy, const void* bias,
-                     int T, int N, int K, int swiglu, int out_f32, int splits, int* error, const float* norm_parts,
-                     int norm_count, float norm_eps, float* into_x, long long into_ldx, const void* into_gain,
-                     int into_gain_f32, void* into_z, long long into_ldz, float* into_parts, cudaStream_t stream) {
+                     int T, int N, int K, int swiglu, int out_f32, int splits, int* error, cudaStream_t stream) {
     if (T <= 0 || N <= 0) return 0;
-    if (((norm_parts || into_x) && T > 32) || (norm_parts && norm_count <= 0) ||
-        (into_x && (!into_gain || !into_z || !into_parts || out_f32 || swiglu)))
-        return ERR_BAD_ARGUMENT;
     if (T > 64 || K <= 0 || K % 8 != 0 || ldx % 8 != 0 || (splits != 1 && splits != 2 && splits != 4 && splits != 8) ||
         swiglu < 0 || swiglu > 3)
         return ERR_BAD_ARGUMENT;
@@ -377,9 +347,6 @@ int fsie_gemm_decode(const void* weight_map, const void* x, int ldx, void* y, in
     GemmParams p;
     p.y = y; p.ldy = ldy; p.bias = (const bf16*)bias; p.T = T; p.N = N; p.K = K;
     p.up_row0 = N; p.out_f32 = out_f32; p.error = error; p.gate = swiglu;
-    p.norm = LateNorm{norm_parts, norm_count, K, norm_eps};
-    p.into = LateResidual{into_x, into_ldx, into_gain, into_gain_f32, (bf16*)into_z, into_ldz, into_parts,
-                          (N + LATE_COLS - 1) / LATE_COLS};
     const int total_kblocks = (K + BK - 1) / BK;
     p.kblocks_per_split = (total_kblocks + splits - 1) / splits;
     const int tiles = gated ? (N + BM / 2 - 1) / (BM / 2) : (N + BM - 1) / BM;

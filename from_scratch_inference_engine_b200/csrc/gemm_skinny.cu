@@ -16,7 +16,6 @@
 // Launched as a programmatic dependent: the first weights are asked for before the kernel that
 // produces x has finished.
 #include "common.cuh"
-#include "late_norm.cuh"
 
 namespace fsie {
 
@@ -25,14 +24,10 @@ constexpr int SK_WARPS = 16;
 constexpr int SK_CHUNK = 32;         // k elements per warp and step: 4 lanes x 16 bytes per row
 constexpr int SK_AHEAD = 4;          // chunks whose weights a warp has asked for (a ring of 4 KB per warp)
 
-constexpr size_t SK_PARTS_BYTES = 32 * 1024;     // room for the parts of a pending norm: two blocks still fit an SM
-
 struct SkinnyParams {
     const bf16* w; const bf16* x; long long ldx;
     void* y; long long ldy; const bf16* bias;
     int T, N, K, out_f32, relu2;
-    LateNorm norm;                   // x is a row that is still to be normed (parts == nullptr: it is not)
-    LateResidual into;               // plain epilogue: the result goes into the residual stream (x == nullptr: into y)
 };
 
 // The q, k, v product of an attention layer with what follows it on the way to the cache: w
@@ -56,10 +51,6 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
 __device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -76,7 +67,6 @@ __global__ void __launch_bounds__(32 * SK_WARPS, 2)       // two blocks per SM: 
 gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     extern __shared__ __align__(16) unsigned char sk_ring[];
     __shared__ float red[SK_WARPS * SK_ROWS * 8 * TT];            // [warp][16 rows][8 * TT]
-    __shared__ float factor[8 * TT];                              // of each token's norm
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int chunks = p.K / SK_CHUNK;
@@ -137,18 +127,6 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
 #pragma unroll
     for (int n = 0; n < TT; ++n) x_of[n] = (8 * n + g < p.T) ? p.x + (size_t)(8 * n + g) * p.ldx + 8 * t : nullptr;
 
-    // the parts of a pending norm's factor, a token per warp: on their way while the weights are (they join the
-    // group of the first refill)
-    float* my_parts = reinterpret_cast<float*>(sk_ring + SK_WARPS * SK_AHEAD * 1024) + (size_t)warp * p.norm.count;
-    const bool pending = p.norm.parts && warp < p.T;
-    if (pending)
-        for (int i = lane; i < p.norm.count; i += 32) cp_async_4(my_parts + i, p.norm.parts + (size_t)warp * p.norm.count + i);
-    // what the result is added to, by the thread that will
-    float early_x = 0.f, early_gain = 0.f;
-    if (!ROPE && !GATED && p.into.x) {
-        const int token = threadIdx.x / SK_ROWS, n = row0 + threadIdx.x % SK_ROWS;
-        late_fetch(p.into, token, n, token < p.T && n < p.N, early_x, early_gain);
-    }
     float acc[TT][4];
 #pragma unroll
     for (int n = 0; n < TT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
@@ -184,11 +162,7 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
             if (c < chunks) multiply(b[j], c);
         }
     }
-    cp_async_wait_all();
-    if (warp < 8 * TT) {                                          // (8 TT <= SK_WARPS)
-        const float f = pending ? late_factor(my_parts, p.norm, lane) : 1.f;     // a lane reads what it asked for itself
-        if (lane == 0) factor[warp] = f;
-    }
+    cp_async_wait<0>();
     // acc[n]: rows g (0, 1) and g + 8 (2, 3), tokens 8 n + 2 t and 8 n + 2 t + 1
 #pragma unroll
     for (int n = 0; n < TT; ++n) {
@@ -212,9 +186,7 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 lo += red[((size_t)w * SK_ROWS + r) * TP + token];
                 hi += red[((size_t)w * SK_ROWS + r + 8) * TP + token];
             }
-            // (e is this thread's own pair: see above)
-            lo = lo * factor[token] + early_bias_lo;
-            hi = hi * factor[token] + early_bias_hi;
+            lo += early_bias_lo; hi += early_bias_hi;             // (e is this thread's own pair: see above)
             // the unfused path stores the product as bfloat16 before it rotates: the same rounding here
             lo = __bfloat162float(__float2bfloat16_rn(lo));
             hi = __bfloat162float(__float2bfloat16_rn(hi));
@@ -255,23 +227,9 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 gate += red[((size_t)w * SK_ROWS + r) * TP + token];
                 up += red[((size_t)w * SK_ROWS + r + 8) * TP + token];
             }
-            gate *= factor[token]; up *= factor[token];
-            if (p.bias) { gate += __bfloat162float(p.bias[n]); up += __bfloat162float(p.bias[p.N + n]); }
             gate = __bfloat162float(__float2bfloat16_rn(gate));
             up = __bfloat162float(__float2bfloat16_rn(up));
             reinterpret_cast<bf16*>(p.y)[(size_t)token * p.ldy + n] = __float2bfloat16_rn((gate / (1.0f + expf(-gate))) * up);
-        }
-    } else if (p.into.x) {
-        static_assert(SK_ROWS == LATE_COLS && SK_ROWS * TP <= 32 * SK_WARPS, "a part per block and token, an output per thread");
-        if (threadIdx.x < SK_ROWS * TP) {                         // whole warps
-            const int token = threadIdx.x / SK_ROWS, r = threadIdx.x - token * SK_ROWS, n = row0 + r;
-            const bool in = token < p.T && n < p.N;
-            float sum = 0.f;
-#pragma unroll
-            for (int w = 0; w < SK_WARPS; ++w) sum += red[((size_t)w * SK_ROWS + r) * TP + token];
-            sum *= factor[token];
-            if (p.bias && in) sum += __bfloat162float(p.bias[n]);
-            late_store(p.into, sum, early_x, early_gain, token, n, in, lane);
         }
     } else {
     for (int e = threadIdx.x; e < SK_ROWS * TP; e += blockDim.x) {
@@ -281,7 +239,6 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
         float sum = 0.f;
 #pragma unroll
         for (int w = 0; w < SK_WARPS; ++w) sum += red[((size_t)w * SK_ROWS + r) * TP + token];
-        sum *= factor[token];
         if (p.bias) sum += __bfloat162float(p.bias[n]);
         if (p.relu2) {                        // the square of relu, on the value as bfloat16 would store it
             const float r = fmaxf(__bfloat162float(__float2bfloat16_rn(sum)), 0.f);
@@ -295,12 +252,10 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
 
 template <int TT, bool ROPE, bool GATED = false>
 static int launch_skinny(const SkinnyParams& p, const SkinnyRope& rope, cudaStream_t stream) {
-    constexpr size_t ring = (size_t)SK_WARPS * SK_AHEAD * 1024;
-    const size_t smem = ring + (p.norm.parts ? (size_t)p.T * p.norm.count * sizeof(float) : 0);
-    if (smem > ring + SK_PARTS_BYTES) return ERR_UNSUPPORTED;
+    constexpr size_t smem = (size_t)SK_WARPS * SK_AHEAD * 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TT, ROPE, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ring + SK_PARTS_BYTES));
+        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TT, ROPE, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -315,43 +270,29 @@ extern "C" {
 
 // y[T, N] = x[T, K] * w^T (+ bias); T <= 16, K a multiple of 32, rows of x and w on 16-byte boundaries.
 // relu2 != 0: the square of relu of the result, taken as bfloat16 would store it.
-// Norms without a launch of their own (late_norm.cuh): norm_parts != null: x is z, the product's sums are multiplied by the
-// factor of norm_parts [T, norm_count]; into_x != null: the result is added to into_x [T, into_ldx] instead of
-// stored, into_z [T, into_ldz] and into_parts [T, N / 16 rounded up] are what the next product reads.
 int fsie_gemm_skinny(const void* w, const void* x, long long ldx, void* y, long long ldy, const void* bias,
-                     int T, int N, int K, int out_f32, int relu2, const float* norm_parts, int norm_count,
-                     float norm_eps, float* into_x, long long into_ldx, const void* into_gain, int into_gain_f32,
-                     void* into_z, long long into_ldz, float* into_parts, cudaStream_t stream) {
+                     int T, int N, int K, int out_f32, int relu2, cudaStream_t stream) {
     if (T <= 0 || N <= 0) return 0;
-    if ((norm_parts && norm_count <= 0) || (into_x && (!into_gain || !into_z || !into_parts || out_f32 || relu2)))
-        return ERR_BAD_ARGUMENT;
     if (T > 16 || K <= 0 || K % SK_CHUNK != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(w) & 15) ||
         (reinterpret_cast<uintptr_t>(x) & 15))
         return ERR_BAD_ARGUMENT;
     SkinnyParams p;
     p.w = (const bf16*)w; p.x = (const bf16*)x; p.ldx = ldx; p.y = y; p.ldy = ldy; p.bias = (const bf16*)bias;
     p.T = T; p.N = N; p.K = K; p.out_f32 = out_f32; p.relu2 = relu2;
-    p.norm = LateNorm{norm_parts, norm_count, K, norm_eps};
-    p.into = LateResidual{into_x, into_ldx, into_gain, into_gain_f32, (bf16*)into_z, into_ldz, into_parts,
-                          (N + LATE_COLS - 1) / LATE_COLS};
     SkinnyRope none = {};
     return T <= 8 ? launch_skinny<1, false>(p, none, stream) : launch_skinny<2, false>(p, none, stream);
 }
 
-// y[T, N] = silu(x w_gate^T) * (x w_up^T) for w = [gate rows (N); up rows (N)] (bias [2 N] or null, stacked alike), y
-// bfloat16; else as above.
-int fsie_gemm_skinny_swiglu(const void* w, const void* x, long long ldx, void* y, long long ldy, const void* bias, int T,
-                            int N, int K, const float* norm_parts, int norm_count, float norm_eps, cudaStream_t stream) {
+// y[T, N] = silu(x w_gate^T) * (x w_up^T) for w = [gate rows (N); up rows (N)], y bfloat16; else as above.
+int fsie_gemm_skinny_swiglu(const void* w, const void* x, long long ldx, void* y, long long ldy, int T, int N, int K,
+                            cudaStream_t stream) {
     if (T <= 0 || N <= 0) return 0;
-    if (norm_parts && norm_count <= 0) return ERR_BAD_ARGUMENT;
     if (T > 16 || K <= 0 || K % SK_CHUNK != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(w) & 15) ||
         (reinterpret_cast<uintptr_t>(x) & 15))
         return ERR_BAD_ARGUMENT;
     SkinnyParams p;
-    p.w = (const bf16*)w; p.x = (const bf16*)x; p.ldx = ldx; p.y = y; p.ldy = ldy; p.bias = (const bf16*)bias;
+    p.w = (const bf16*)w; p.x = (const bf16*)x; p.ldx = ldx; p.y = y; p.ldy = ldy; p.bias = nullptr;
     p.T = T; p.N = N; p.K = K; p.out_f32 = 0; p.relu2 = 0;
-    p.norm = LateNorm{norm_parts, norm_count, K, norm_eps};
-    p.into = LateResidual{};
     SkinnyRope none = {};
     return T <= 8 ? launch_skinny<1, false, true>(p, none, stream) : launch_skinny<2, false, true>(p, none, stream);
 }
@@ -363,10 +304,8 @@ int fsie_gemm_skinny_swiglu(const void* w, const void* x, long long ldx, void* y
 int fsie_gemm_skinny_qkv_rope(const void* w, const void* x, long long ldx, void* q_out, long long ldq, const void* bias,
                               int T, int K, const int* positions, const float* cos_sin, int table_len,
                               const int* slot_of, void* k_pages, void* v_pages, long long page_stride, int page_size,
-                              int heads, int kv_heads, int head_dim, int* error,
-                              const float* norm_parts, int norm_count, float norm_eps, cudaStream_t stream) {
+                              int heads, int kv_heads, int head_dim, int* error, cudaStream_t stream) {
     if (T <= 0) return 0;
-    if (norm_parts && norm_count <= 0) return ERR_BAD_ARGUMENT;
     if (T > 16 || K <= 0 || K % SK_CHUNK != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(w) & 15) ||
         (reinterpret_cast<uintptr_t>(x) & 15) || heads <= 0 || kv_heads <= 0 || head_dim <= 0 || head_dim % 16 != 0 ||
         !positions || !cos_sin || !error || page_size <= 0)
@@ -374,8 +313,6 @@ int fsie_gemm_skinny_qkv_rope(const void* w, const void* x, long long ldx, void*
     SkinnyParams p;
     p.w = (const bf16*)w; p.x = (const bf16*)x; p.ldx = ldx; p.y = q_out; p.ldy = ldq; p.bias = (const bf16*)bias;
     p.T = T; p.N = (heads + 2 * kv_heads) * head_dim; p.K = K; p.out_f32 = 0; p.relu2 = 0;
-    p.norm = LateNorm{norm_parts, norm_count, K, norm_eps};
-    p.into = LateResidual{};
     SkinnyRope rope;
     rope.positions = positions; rope.cos_sin = cos_sin; rope.table_len = table_len;
     rope.slot_of = k_pages ? slot_of : nullptr; rope.k_pages = (bf16*)k_pages; rope.v_pages = (bf16*)v_pages;

@@ -91,7 +91,6 @@ class StepContext:
         # what one part leaves for a later part of the same step (values of the step's tokens that
         # another layer blends with its own, for instance)
         self.shared: Dict[str, torch.Tensor] = {}
-        self.next_norm = None        # the norm that the call behind the running one takes pending (DecoderModel.forward)
         self.num_tokens = T = len(token_ids)
         self.num_items = I = len(q_len)
         self.h_qstart = np.asarray(q_start, dtype=np.int32)

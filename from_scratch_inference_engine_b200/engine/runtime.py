@@ -106,8 +106,6 @@ class Runtime:
                                           else int(decode_tcgen05_min_blocks))
         # steps of few tokens rotate q, k and write k, v in the q, k, v product's epilogue
         self.fused_qkv_rope = True
-        # ... and norm the residual stream around the products (`late_kind`)
-        self.late_norms = True
         # the tiled product shares a partial last round of tiles out among all pairs of blocks
         self.share_tiles = bool(share_tiles)
         # its counters (eight per shared tile, fewer tiles than pairs of SMs): made now, so that a
@@ -168,20 +166,18 @@ class Runtime:
         return self._tables[key]
 
     def prepare_weight(self, weight: torch.Tensor, swiglu: bool = False,
-                       activation: str = "silu", plain_activation: Optional[str] = None,
-                       biased: bool = False) -> None:
+                       activation: str = "silu", plain_activation: Optional[str] = None) -> None:
         """Called by a part at bind for a matrix it will multiply activations with.  Large
         bfloat16 matrices get a TMA descriptor for the tcgen05 product that steps of few
         tokens use (the library product is kept where it measured faster: small matrices).
-        `plain_activation`: the weight is for `linear_activated` only.  `biased`: a SwiGLU weight that comes with a
-        bias, which the few-token products add; the tiled one is plain then, with the activation behind it."""
+        `plain_activation`: the weight is for `linear_activated` only."""
         if self.dtype is not torch.bfloat16 or weight.dtype is not torch.bfloat16:
             return
         rows, k = weight.shape
         if k % 8 or (swiglu and rows % 2):
             return
         if self.products == "own":
-            self._tiled_weights[weight.data_ptr()] = (weight, swiglu and not biased, activation, plain_activation)
+            self._tiled_weights[weight.data_ptr()] = (weight, swiglu, activation, plain_activation)
         if rows * k >= self.few_token_min_elements:
             self._few_token_weights[weight.data_ptr()] = ops.DecodeWeight(weight, swiglu, activation,
                                                                           plain_activation)
@@ -224,39 +220,11 @@ class Runtime:
         limit = self.few_token_limit_fused if prepared.swiglu else self.few_token_limit
         return prepared if x.shape[0] <= limit else None
 
-    def _few_token_product(self, prepared, x, bias, out_dtype, tag=None, norm=None, into=None) -> Optional[torch.Tensor]:
-        out = None if into is not None else self.buffer(tag, x.shape[0], prepared.n, out_dtype)
+    def _few_token_product(self, prepared, x, bias, out_dtype, tag=None) -> torch.Tensor:
+        out = self.buffer(tag, x.shape[0], prepared.n, out_dtype)
         tiles = -(-prepared.n // (64 if prepared.swiglu else 128))
         splits = ops.gemm_decode_splits(tiles, prepared.k, self.sm_count)
-        return ops.gemm_decode(prepared, x, out, bias, self.error, splits, norm, into)
-
-    def late_kind(self, weight: torch.Tensor, tokens: int) -> str:
-        """Which of the engine's own products multiplies `weight` in a step of so few tokens that norms go without
-        launches of their own ("" where another product does, or more tokens come): "few", the tcgen05
-        product, or "skinny", the one without set-up."""
-        if self.dtype is not torch.bfloat16 or self.products != "own" or tokens > ops.GEMM_SKINNY_MAX_TOKENS \
-                or not self.late_norms:
-            return ""
-        prepared = self._few_token_weights.get(weight.data_ptr())
-        if prepared is not None:
-            return "few" if tokens <= (self.few_token_limit_fused if prepared.swiglu else self.few_token_limit) else ""
-        k = weight.shape[1]
-        return "skinny" if (ops.gemm_skinny_fits(tokens, k) and weight.dtype is torch.bfloat16 and weight.is_contiguous()
-                            and tokens * -(-k // ops.LATE_COLUMNS) * 4 <= ops.LATE_PARTS_BYTES) else ""
-
-    def linear_into(self, x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], residual: torch.Tensor,
-                    gain: torch.Tensor, eps: float, tag: str) -> "ops.LateRows":
-        """residual += x @ weight.T (+ bias), by a product that `late_kind` names; returns the new rows with their norm
-        (gain, eps) pending."""
-        tokens, n = residual.shape
-        late = ops.LateRows(self.buffer(tag, tokens, n, torch.bfloat16),
-                            self.buffer(tag + ".parts", tokens, -(-n // ops.LATE_COLUMNS), torch.float32), eps)
-        into = ops.LateResidual(residual, gain, late)
-        if self.late_kind(weight, tokens) == "few":
-            self._few_token_product(self._few_token_weights[weight.data_ptr()], x, bias, None, None, None, into)
-        else:
-            ops.gemm_skinny(weight, x, None, bias, None, None, into)
-        return late
+        return ops.gemm_decode(prepared, x, out, bias, self.error, splits)
 
     def _product_f32(self, x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor],
                      tag: Optional[str]) -> torch.Tensor:
@@ -276,10 +244,6 @@ class Runtime:
                bias: Optional[torch.Tensor], tag: Optional[str] = None) -> torch.Tensor:
         """x @ weight.T (+ bias) in the compute dtype.  `tag`: see `buffer` (the result may then
         live where the last result under that tag lived)."""
-        if isinstance(x, ops.LateRows):              # rows with a pending norm, for a product that `late_kind` names
-            if self.late_kind(weight, x.shape[0]) == "few":
-                return self._few_token_product(self._few_token_weights[weight.data_ptr()], x.rows, bias, torch.bfloat16, tag, x)
-            return ops.gemm_skinny(weight, x.rows, self.buffer(tag, x.shape[0], weight.shape[0], torch.bfloat16), bias, None, x)
         if self.dtype is torch.float32:
             return self._product_f32(x, weight, bias, tag)
         prepared = self._few_tokens(x, weight)
@@ -330,11 +294,7 @@ class Runtime:
         the write of k and v into the pages, where one kernel does all three (steps of few
         tokens against a matrix that the set-up-free product takes, whole heads rotated);
         else None, and the caller runs the product and `ops.rope_kv_write` one after the other.
-        Returns [tokens, q + k + v width] of which only the query columns are filled.  x may be rows with a
-        pending norm."""
-        norm = x if isinstance(x, ops.LateRows) else None
-        if norm is not None:
-            x = norm.rows
+        Returns [tokens, q + k + v width] of which only the query columns are filled."""
         if not (self.dtype is torch.bfloat16 and self.fused_qkv_rope and rotary_dim == head_dim
                 and head_dim % 16 == 0 and self._few_tokens(x, weight) is None
                 and self._skinny(x, weight)
@@ -343,29 +303,17 @@ class Runtime:
         out = self.buffer("qkv", x.shape[0], weight.shape[0], torch.bfloat16)
         return ops.gemm_skinny_qkv_rope(weight, x, out, bias, positions, cos_sin, slot_of, k_pages,
                                         v_pages, page_stride, page_size, heads, kv_heads, head_dim,
-                                        self.error, norm)
+                                        self.error)
 
     def linear_swiglu(self, x: torch.Tensor, gate_up: torch.Tensor,
                       tag: Optional[str] = None, bias: Optional[torch.Tensor] = None,
                       activation: str = "silu") -> torch.Tensor:
         """silu(x @ gate.T) * (x @ up.T) for the stacked weight [gate rows; up rows]: one fused
         kernel for steps of few tokens, else the library product and the SwiGLU kernel.  With a
-        `bias` (stacked like the weight) a product beyond few tokens adds it and the SwiGLU kernel follows.
-        x may be rows with a pending norm (no bias then).
+        `bias` (stacked like the weight) the product adds it and the SwiGLU kernel follows.
         `activation` names what the gate passes through (the fused kernels were told at
         `prepare_weight`; the unfused path runs the kernel of gated activations)."""
-        if isinstance(x, ops.LateRows):
-            if self.late_kind(gate_up, x.shape[0]) == "few":
-                return self._few_token_product(self._few_token_weights[gate_up.data_ptr()], x.rows, None, torch.bfloat16, tag, x)
-            return ops.gemm_skinny_swiglu(gate_up, x.rows, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2, torch.bfloat16), x)
         if bias is not None:
-            prepared = self._few_tokens(x, gate_up) if self.dtype is torch.bfloat16 else None
-            if prepared is not None and prepared.swiglu:
-                return self._few_token_product(prepared, x, bias, torch.bfloat16, tag)
-            if (self.dtype is torch.bfloat16 and prepared is None and activation == "silu"
-                    and gate_up.shape[0] % 2 == 0 and self._skinny(x, gate_up)):
-                return ops.gemm_skinny_swiglu(gate_up, x, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2,
-                                                                      torch.bfloat16), None, bias)
             both = self.linear(x, gate_up, bias, None if tag is None else tag + ".gate_up")
             return self._gated(both, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2, both.dtype),
                                activation)

@@ -618,7 +618,7 @@ def gemm_decode_lib():
         i, ll, p = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_tensor_map_bytes.argtypes = []
         lib.fsie_gemm_decode_weight_map.argtypes = [p, p, ll, ll, i]
-        lib.fsie_gemm_decode.argtypes = [p, p, i, p, i, p, i, i, i, i, i, i, p, p, i, ctypes.c_float, p, ll, p, i, p, ll, p, p]
+        lib.fsie_gemm_decode.argtypes = [p, p, i, p, i, p, i, i, i, i, i, i, p, p]
         for name in ("fsie_tensor_map_bytes", "fsie_gemm_decode_weight_map", "fsie_gemm_decode"):
             getattr(lib, name).restype = i
         _gemm_decode = build.fast_calls(lib)
@@ -638,62 +638,6 @@ def _epilogue(what: str, swiglu: bool, activation: str, plain_activation: Option
     if swiglu and activation not in FUSED_GATES:
         raise KernelError(f"{what}: the gate is one of {', '.join(FUSED_GATES)}")
     return 1 + GATE_KINDS[activation] if swiglu else 0
-
-
-LATE_COLUMNS = 16                # columns of one part of a pending norm
-LATE_PARTS_BYTES = 32 * 1024     # parts that the product without set-up has room for
-
-
-class LateRows:
-    """Rows [T, K] of a residual stream whose RMS norm is pending: `rows` (bfloat16) holds them times the norm's
-    gain, `parts` (float32 [T, K / 16 rounded up]) the squares' sums over 16 columns each; whoever multiplies the rows
-    multiplies its sums by 1 / sqrt(sum of the parts / K + eps)."""
-
-    __slots__ = ("rows", "parts", "eps")
-
-    def __init__(self, rows: torch.Tensor, parts: torch.Tensor, eps: float):
-        self.rows, self.parts, self.eps = rows, parts, float(eps)
-
-    @property
-    def shape(self):
-        return self.rows.shape
-
-
-class LateResidual:
-    """Where a product leaves its result instead of in a matrix of its own: added to `x` (float32 [T, N]), with the
-    rows that the next product reads in `late` (x times `gain`, and the squares' sums)."""
-
-    __slots__ = ("x", "gain", "late")
-
-    def __init__(self, x: torch.Tensor, gain: torch.Tensor, late: LateRows):
-        self.x, self.gain, self.late = x, gain, late
-
-
-def _late_arguments(norm: Optional[LateRows], x: torch.Tensor, what: str):
-    if norm is None:
-        return None, 0, 0.0
-    _need(norm.parts, torch.float32, "parts")
-    tokens, k = x.shape
-    count = -(-k // LATE_COLUMNS)
-    if norm.rows is not x or norm.parts.shape[0] < tokens or norm.parts.shape[1] != count:
-        raise KernelError(f"{what}: the pending norm's parts do not fit x")
-    return norm.parts, count, norm.eps
-
-
-def _into_arguments(into: Optional[LateResidual], tokens: int, n: int, what: str):
-    if into is None:
-        return None, 0, None, 0, None, 0, None
-    late = into.late
-    _need(into.x, torch.float32, "x", contiguous=False)
-    _need(late.rows, torch.bfloat16, "rows", contiguous=False)
-    _need(late.parts, torch.float32, "parts")
-    _need(into.gain, None, "gain")
-    if into.x.shape != (tokens, n) or into.x.stride(1) != 1 or late.rows.shape != (tokens, n) or late.rows.stride(1) != 1 or \
-            late.parts.shape != (tokens, -(-n // LATE_COLUMNS)) or into.gain.numel() != n or \
-            into.gain.dtype not in (torch.float32, torch.bfloat16):
-        raise KernelError(f"{what}: the residual stream, its gain or its rows do not fit the result")
-    return (into.x, into.x.stride(0), into.gain, int(into.gain.dtype is torch.float32), late.rows,
-            late.rows.stride(0), late.parts)
 
 
 class DecodeWeight:
@@ -728,36 +672,24 @@ def gemm_decode_splits(tiles: int, k: int, sm_count: int) -> int:
     return splits
 
 
-def gemm_decode(weight: DecodeWeight, x: torch.Tensor, out: Optional[torch.Tensor],
-                bias: Optional[torch.Tensor], error: torch.Tensor, splits: int = 1,
-                norm: Optional[LateRows] = None, into: Optional[LateResidual] = None) -> Optional[torch.Tensor]:
-    """out[T, N] = x[T, K] @ w.T (+ bias), or silu(x @ gate.T) * (x @ up.T) (bias: the gate rows', then the up rows');
-    T <= 64; out is bfloat16 or float32.  Up to 32 tokens: `norm`, x are the rows of a pending norm; `into`, the
-    result is added to the residual stream there (out is None)."""
+def gemm_decode(weight: DecodeWeight, x: torch.Tensor, out: torch.Tensor,
+                bias: Optional[torch.Tensor], error: torch.Tensor, splits: int = 1) -> torch.Tensor:
+    """out[T, N] = x[T, K] @ w.T (+ bias), or silu(x @ gate.T) * (x @ up.T); T <= 64; out is
+    bfloat16 or float32."""
     _need(x, torch.bfloat16, "x", contiguous=False)
+    _need(out, None, "out")
     tokens, k = x.shape
     if k != weight.k or x.stride(1) != 1 or tokens > GEMM_DECODE_MAX_TOKENS:
         raise KernelError("gemm_decode: x does not fit the weight (or more than 64 tokens)")
-    if (out is None) != (into is not None) or (into is not None and weight.gate):
-        raise KernelError("gemm_decode: either out or a residual stream takes a plain product's result")
-    if bias is not None:
-        _need(bias, torch.bfloat16, "bias")
-        if bias.numel() != weight.n * (2 if weight.swiglu else 1):
-            raise KernelError("gemm_decode: the bias does not fit the weight")
-    late = (*_late_arguments(norm, x, "gemm_decode"), *_into_arguments(into, tokens, weight.n, "gemm_decode"))
-    if into is not None:
-        _check(gemm_decode_lib().fsie_gemm_decode(
-            weight.map_ptr, x, x.stride(0), None, 0, bias, tokens, weight.n, k, weight.gate, 0, splits,
-            error, *late, _stream()), "gemm_decode")
-        return None
-    _need(out, None, "out")
     if out.shape[0] < tokens or out.shape[1] != weight.n or out.dtype not in (torch.bfloat16,
                                                                             torch.float32):
         raise KernelError("gemm_decode: out does not fit")
+    if bias is not None:
+        _need(bias, torch.bfloat16, "bias")
     _check(gemm_decode_lib().fsie_gemm_decode(
         weight.map_ptr, x, x.stride(0), out, out.stride(0), bias, tokens,
         weight.n, k, weight.gate, int(out.dtype is torch.float32), splits, error,
-        *late, _stream()), "gemm_decode")
+        _stream()), "gemm_decode")
     return out
 
 
@@ -775,14 +707,12 @@ def gemm_skinny_lib():
     if _gemm_skinny is None:
         lib = build.load_library("gemm_skinny")
         i, ll, p = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p
-        f = ctypes.c_float
-        late, into = [p, i, f], [p, ll, p, i, p, ll, p]
-        lib.fsie_gemm_skinny.argtypes = [p, p, ll, p, ll, p, i, i, i, i, i, *late, *into, p]
+        lib.fsie_gemm_skinny.argtypes = [p, p, ll, p, ll, p, i, i, i, i, i, p]
         lib.fsie_gemm_skinny.restype = i
-        lib.fsie_gemm_skinny_swiglu.argtypes = [p, p, ll, p, ll, p, i, i, i, *late, p]
+        lib.fsie_gemm_skinny_swiglu.argtypes = [p, p, ll, p, ll, i, i, i, p]
         lib.fsie_gemm_skinny_swiglu.restype = i
         lib.fsie_gemm_skinny_qkv_rope.argtypes = [p, p, ll, p, ll, p, i, i, p, p, i, p, p, p, ll, i,
-                                                  i, i, i, p, *late, p]
+                                                  i, i, i, p, p]
         lib.fsie_gemm_skinny_qkv_rope.restype = i
         _gemm_skinny = build.fast_calls(lib)
     return _gemm_skinny
@@ -793,7 +723,7 @@ def gemm_skinny_qkv_rope(weight: torch.Tensor, x: torch.Tensor, out: torch.Tenso
                          cos_sin: torch.Tensor, slot_of: Optional[torch.Tensor],
                          k_pages: Optional[torch.Tensor], v_pages: Optional[torch.Tensor],
                          page_stride: int, page_size: int, heads: int, kv_heads: int,
-                         head_dim: int, error: torch.Tensor, norm: Optional[LateRows] = None) -> torch.Tensor:
+                         head_dim: int, error: torch.Tensor) -> torch.Tensor:
     """The q, k, v product of up to 16 tokens with the rotation of q and k and the cache write in
     its epilogue: rotated queries into out[:, :heads * head_dim] (bfloat16; the key and value
     columns of `out` are not written), rotated keys and the values into the pages (not when
@@ -822,50 +752,39 @@ def gemm_skinny_qkv_rope(weight: torch.Tensor, x: torch.Tensor, out: torch.Tenso
     _check(lib.fsie_gemm_skinny_qkv_rope(
         weight, x, x.stride(0), out, out.stride(0), bias, tokens, k,
         positions, cos_sin, cos_sin.shape[0], slot_of, k_pages,
-        v_pages, page_stride, page_size, heads, kv_heads, head_dim, error, *_late_arguments(norm, x, "gemm_skinny_qkv_rope"), _stream()),
+        v_pages, page_stride, page_size, heads, kv_heads, head_dim, error, _stream()),
         "gemm_skinny_qkv_rope")
     return out
 
 
-def gemm_skinny(weight: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor],
-                bias: Optional[torch.Tensor], plain_activation: Optional[str] = None,
-                norm: Optional[LateRows] = None, into: Optional[LateResidual] = None) -> Optional[torch.Tensor]:
+def gemm_skinny(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
+                bias: Optional[torch.Tensor], plain_activation: Optional[str] = None) -> torch.Tensor:
     """out[T, N] = x[T, K] @ weight.T (+ bias) for T <= 16: no pipeline to fill, every lane asks
     for its weights straight from global memory (for matrices so small that set-up would
-    dominate).  out is bfloat16 or float32.  `plain_activation` "relu2": the square of relu of the result.
-    `norm`: x are the rows of a pending norm; `into`: the result is added to the residual stream there (out is None)."""
+    dominate).  out is bfloat16 or float32.  `plain_activation` "relu2": the square of relu of the result."""
     gemm_skinny_lib()
     _need(weight, torch.bfloat16, "weight")
     _need(x, torch.bfloat16, "x", contiguous=False)
+    _need(out, None, "out", contiguous=False)
     tokens, k = x.shape
     n = weight.shape[0]
     if weight.shape[1] != k or x.stride(1) != 1 or not gemm_skinny_fits(tokens, k):
         raise KernelError("gemm_skinny: x does not fit the weight, or the sizes are beyond the kernel")
-    if (out is None) != (into is not None) or (into is not None and plain_activation):
-        raise KernelError("gemm_skinny: either out or a residual stream takes a plain product's result")
-    if bias is not None:
-        _need(bias, torch.bfloat16, "bias")
-    late = (*_late_arguments(norm, x, "gemm_skinny"), *_into_arguments(into, tokens, n, "gemm_skinny"))
-    if into is not None:
-        _check(_gemm_skinny.fsie_gemm_skinny(weight, x, x.stride(0), None, 0, bias, tokens, n, k, 0, 0, *late, _stream()),
-               "gemm_skinny")
-        return None
-    _need(out, None, "out", contiguous=False)
     if out.shape[0] != tokens or out.shape[1] != n or out.stride(1) != 1 or \
             out.dtype not in (torch.bfloat16, torch.float32):
         raise KernelError("gemm_skinny: out does not fit")
+    if bias is not None:
+        _need(bias, torch.bfloat16, "bias")
     _check(_gemm_skinny.fsie_gemm_skinny(weight, x, x.stride(0), out, out.stride(0),
                                          bias, tokens, n, k, int(out.dtype is torch.float32),
                                          int(_epilogue("gemm_skinny", False, "silu", plain_activation) == 3),
-                                         *late, _stream()), "gemm_skinny")
+                                         _stream()), "gemm_skinny")
     return out
 
 
-def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
-                       norm: Optional[LateRows] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out[T, N] = silu(x @ gate.T) * (x @ up.T) for T <= 16 and weight = [gate rows (N); up rows (N)] (`bias` stacked
-    alike): the bits of `gemm_skinny` and `swiglu` one after the other, in one launch.  `norm`: x are the rows of a
-    pending norm."""
+def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out[T, N] = silu(x @ gate.T) * (x @ up.T) for T <= 16 and weight = [gate rows (N); up rows (N)]: the bits of
+    `gemm_skinny` and `swiglu` one after the other, in one launch."""
     gemm_skinny_lib()
     _need(weight, torch.bfloat16, "weight")
     _need(x, torch.bfloat16, "x", contiguous=False)
@@ -876,12 +795,8 @@ def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
         raise KernelError("gemm_skinny_swiglu: x does not fit the weight, or the sizes are beyond the kernel")
     if out.shape[0] != tokens or out.shape[1] != n or out.stride(1) != 1:
         raise KernelError("gemm_skinny_swiglu: out does not fit")
-    if bias is not None:
-        _need(bias, torch.bfloat16, "bias")
-        if bias.numel() != 2 * n:
-            raise KernelError("gemm_skinny_swiglu: the bias holds the gate rows' and as many for the up rows")
-    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(weight, x, x.stride(0), out, out.stride(0), bias, tokens, n,
-                                                k, *_late_arguments(norm, x, "gemm_skinny_swiglu"), _stream()), "gemm_skinny_swiglu")
+    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(weight, x, x.stride(0), out, out.stride(0), tokens, n,
+                                                k, _stream()), "gemm_skinny_swiglu")
     return out
 
 

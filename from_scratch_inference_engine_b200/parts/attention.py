@@ -113,16 +113,7 @@ class GqaAttention(Mixer):
         runtime.prepare_weight(self.w_o)
         self.position.bind(tensors, runtime)
 
-    def takes_late(self, tokens: int) -> bool:
-        """Whether the q, k, v product of a step of `tokens` tokens takes rows whose norm is pending."""
-        return bool(self.runtime.late_kind(self.w_qkv, tokens))
-
-    def gives_late(self, tokens: int) -> bool:
-        """Whether the output projection of such a step can add to the residual stream itself."""
-        return bool(self.runtime.late_kind(self.w_o, tokens))
-
-    def forward(self, ctx, y, cache: LayerCache, into=None):
-        """`into` (residual stream, norm): the output is added there, and its rows with that norm pending are returned."""
+    def forward(self, ctx, y: torch.Tensor, cache: LayerCache) -> torch.Tensor:
         rt = self.runtime
         tokens = y.shape[0]
         group = ctx.groups[cache.group]
@@ -140,9 +131,6 @@ class GqaAttention(Mixer):
         # attention output are dead when the next attention layer runs
         out = rt.buffer("attention.out", tokens, self.q_width, qkv.dtype)
         self._attend(ctx, qkv, group, cache, out)
-        if into is not None:
-            residual, norm = into
-            return rt.linear_into(out, self.w_o, None, residual, norm.gain, norm.eps, "prenorm.feed_forward_in")
         return rt.linear(out, self.w_o, None, "attention.o")
 
     def _attend(self, ctx, qkv: torch.Tensor, group, cache: LayerCache, out: torch.Tensor) -> None:

@@ -56,34 +56,16 @@ class PreNormBlock(Part):
         for part in self.parts():
             part.bind(tensors, runtime)
 
-    def late_norm(self, tokens: int) -> Optional[RMSNorm]:
-        """The norm that the block before may leave pending in a step of `tokens` tokens (the mixer's first product
-        finishes it), or None."""
-        takes = getattr(self.mixer, "takes_late", None)
-        return self.mixer_norm if takes is not None and isinstance(self.mixer_norm, RMSNorm) and takes(tokens) else None
-
-    def forward(self, ctx, x: torch.Tensor, delta, cache: LayerCache):
-        """In steps of few tokens the products around a norm do its work (`ops.LateRows`): the output projection and
-        the down projection add to x themselves.  `ctx.next_norm` is the norm that the block behind this one
-        takes pending, if any; `delta` and the result may then be rows with their norm pending."""
+    def forward(self, ctx, x: torch.Tensor, delta: Optional[torch.Tensor],
+                cache: LayerCache) -> torch.Tensor:
         ctx.residual_copy = None      # this block changes x without keeping a copy of it up to date
-        tokens = x.shape[0]
         # the normed rows are read by the sublayer that follows and by nothing after it
-        y = delta if isinstance(delta, ops.LateRows) else self._normed(self.mixer_norm, x, delta, "prenorm.mixer_in")
-        feed_forward = self.feed_forward
-        if feed_forward is None:
-            return self.mixer.forward(ctx, y, cache)
-        gives, takes = getattr(self.mixer, "gives_late", None), getattr(feed_forward, "takes_late", None)
-        if gives is not None and takes is not None and isinstance(self.feed_forward_norm, RMSNorm) \
-                and gives(tokens) and takes(tokens):
-            y = self.mixer.forward(ctx, y, cache, (x, self.feed_forward_norm))
-        else:
-            mixed = self.mixer.forward(ctx, y, cache)     # a tensor, or what the norms add as a whole
-            y = self._normed(self.feed_forward_norm, x, mixed, "prenorm.feed_forward_in")
-        gives = getattr(feed_forward, "gives_late", None)
-        if gives is not None and ctx.next_norm is not None and gives(tokens):
-            return feed_forward.forward(ctx, y, (x, ctx.next_norm))
-        return feed_forward.forward(ctx, y)
+        y = self._normed(self.mixer_norm, x, delta, "prenorm.mixer_in")
+        mixed = self.mixer.forward(ctx, y, cache)     # a tensor, or what the norms add as a whole
+        if self.feed_forward is None:
+            return mixed
+        y = self._normed(self.feed_forward_norm, x, mixed, "prenorm.feed_forward_in")
+        return self.feed_forward.forward(ctx, y)
 
     @staticmethod
     def _normed(norm, x, delta, tag):

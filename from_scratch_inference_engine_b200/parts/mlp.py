@@ -62,29 +62,16 @@ class SwiGluMlp(Part):
             self.b_gate_up = torch.cat([tensors[self._name("gate", "bias")],
                                         tensors[self._name("up", "bias")]]).to(runtime.dtype).contiguous()
             self.b_down = tensors[self._name("down", "bias")].to(runtime.dtype).contiguous()
-        # of the fused SwiGLU products only those of few tokens take a bias: beyond them the stacked product
-        # adds it and a kernel of its own applies the activation
-        runtime.prepare_weight(self.w_gate_up, swiglu=True, activation=self.activation, biased=self.bias)
+        # the fused SwiGLU products take no bias: with one, the stacked product adds it and a
+        # kernel of its own applies the activation
+        runtime.prepare_weight(self.w_gate_up, swiglu=not self.bias, activation=self.activation)
         runtime.prepare_weight(self.w_down)
 
-    def takes_late(self, tokens: int) -> bool:
-        """Whether the gate and up product of a step of `tokens` tokens takes rows whose norm is pending."""
-        kind = "" if self.bias else self.runtime.late_kind(self.w_gate_up, tokens)
-        return kind == "few" or (kind == "skinny" and self.activation == "silu")
-
-    def gives_late(self, tokens: int) -> bool:
-        """Whether the down projection of such a step can add to the residual stream itself."""
-        return not self.bias and bool(self.runtime.late_kind(self.w_down, tokens))
-
-    def forward(self, ctx, y, into=None):
-        """`into` (residual stream, norm): the output is added there, and its rows with that norm pending are returned."""
+    def forward(self, ctx, y: torch.Tensor) -> torch.Tensor:
         rt = self.runtime
         # the activation and the result are dead when the next feed-forward of the model runs
         act = rt.linear_swiglu(y, self.w_gate_up, "swiglu.act", bias=self.b_gate_up,
                                activation=self.activation)
-        if into is not None:
-            residual, norm = into
-            return rt.linear_into(act, self.w_down, None, residual, norm.gain, norm.eps, "prenorm.mixer_in")
         return rt.linear(act, self.w_down, self.b_down, "swiglu.down")
 
 

@@ -123,13 +123,6 @@ class DecoderModel:
         """State each call of the run order keeps per request (None for most mixers)."""
         return [self.blocks[layer].mixer.state_need() for layer, _, _ in self.schedule]
 
-    def _next_norm(self, index: int, tokens: int):
-        """The norm that call `index` of the run order takes pending from the call before it, or None."""
-        if index >= len(self.schedule) or self.inlet_before[index] is not None:
-            return None
-        late_norm = getattr(self.blocks[self.schedule[index][0]], "late_norm", None)
-        return None if late_norm is None else late_norm(tokens)
-
     # ------------------------------------------------------------------ forward
     def forward(self, ctx, caches: List[LayerCache], want_rows: Optional[torch.Tensor]):
         """Run the step's tokens; returns float32 logits [len(want_rows), vocab] (None if
@@ -158,7 +151,6 @@ class DecoderModel:
             if self.inlet_before[index] is not None:
                 x, delta = self.inlets[self.inlet_before[index]].forward(ctx, x, delta, x0), None
                 ctx.residual_copy = None
-            ctx.next_norm = self._next_norm(index + 1, ctx.num_tokens)
             delta = self.blocks[layer].forward(ctx, x, delta, caches[index])
         if want_rows is None or want_rows.numel() == 0:
             return None
