@@ -15,7 +15,7 @@ def test_one_launch_is_the_two(tokens, routed, experts, top, groups, keep, score
     from from_scratch_inference_engine_b200.kernels import ops
     generator = torch.Generator(device="cuda").manual_seed(tokens * 1000 + routed)
     logits = torch.randn(tokens, routed, generator=generator, device="cuda") * 3
-    logits[0, routed // 2:] = logits[0, 0]                                  # ties
+    logits[0, routed // 2:] = logits[0, 0].item()                                  # ties
     correction, bias = (torch.randn(routed, generator=generator, device="cuda") for _ in range(2))
     if scores == "chosen_softmax":
         correction = None
