@@ -47,47 +47,63 @@ __global__ void add_layernorm_kernel(const S* __restrict__ src, const int* __res
     }
 }
 
-// The same with eight neighbouring values per thread and the row in registers (a row of up to 8,192 values, a
-// multiple of 8): a step of few tokens is a chain of such rows, each two sums over a block, and nothing but their
-// trips to memory and barriers bounds it (4 rows of 2,048 took 6.9 us of the step's chain with a value per thread and turn); the gain, a
-// constant, is asked for before the kernel before has finished.
-template <typename S, typename T>
-__global__ void __launch_bounds__(1024) add_layernorm_vec_kernel(const S* __restrict__ src, const int* __restrict__ rows,
+// The same, to the bit, with the row in registers (at most PER values of a thread, all asked for at once): a step of few
+// tokens is a chain of such rows, each two sums over a block, and nothing but their trips to memory and barriers bounds it
+// (4 rows of 2,048 took 6.9 us of the step's chain, a turn through shared memory for each value, and LN_TIME now); the gain, a
+// constant, is asked for before the kernel before has finished.  A thread keeps the values that it has above, neighbours apart by
+// the block: eight neighbours of a thread would be one load, but another order of the sums.
+template <typename S, typename T, int PER>
+__global__ void __launch_bounds__(512) add_layernorm_regs_kernel(const S* __restrict__ src, const int* __restrict__ rows,
                                                                  const float* __restrict__ gain, float* __restrict__ x,
                                                                  T* __restrict__ y, int width, float eps) {
     __shared__ float scratch[32];
-    const int r = blockIdx.x, c = threadIdx.x * 8;
-    const bool active = c < width;
-    float g[8], v[8], old[8];
-    if (active) load8(gain + c, g);
+    const int r = blockIdx.x;
+    float g[PER], v[PER], old[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        g[i] = c < width ? gain[c] : 0.f;
+    }
     grid_dependency_wait();
     grid_dependents_go();
     const size_t s = rows ? (size_t)rows[r] : (size_t)r;
-    float sum = 0.f;
-    if (active) {
-        load8(src + s * width + c, v);
-        if (x) load8(x + (size_t)r * width + c, old);
+    const S* in = src + s * width;
+    float* xr = x ? x + (size_t)r * width : nullptr;
+    T* yr = y ? y + (size_t)r * width : nullptr;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sum += v[i];
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        v[i] = c < width ? to_float(in[c]) : 0.f;
     }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        old[i] = xr && c < width ? xr[c] : 0.f;
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+        if (threadIdx.x + i * blockDim.x < width) sum += v[i];
     const float mean = block_sum(sum, scratch) / (float)width;
     float sq = 0.f;
-    if (active) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] -= mean;
-            sq += v[i] * v[i];
+    for (int i = 0; i < PER; ++i)
+        if (threadIdx.x + i * blockDim.x < width) {
+            const float d = v[i] - mean;
+            sq += d * d;
         }
-    }
     const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
-    if (!active) return;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        v[i] = v[i] * inv * g[i];
-        if (x) v[i] += old[i];
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c >= width) break;
+        float n = (v[i] - mean) * inv * g[i];
+        if (xr) {
+            n += old[i];
+            xr[c] = n;
+        }
+        if (yr) yr[c] = from_float<T>(n);
     }
-    if (x) store8(x + (size_t)r * width + c, v);
-    if (y) store8(y + (size_t)r * width + c, v);
 }
 
 template <typename T>
@@ -114,16 +130,17 @@ int fsie_add_layernorm(const void* src, const int* rows, const float* gain, floa
     if (width <= 0 || (!accumulate && !y) || (accumulate && !x)) return ERR_BAD_ARGUMENT;
     const size_t smem = (size_t)width * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
-    if (width % 8 == 0 && width <= 8192 && ((((size_t)src) | ((size_t)gain) | ((size_t)x) | ((size_t)y)) & 15) == 0) {
-        const int threads = ((width / 8 + 31) / 32) * 32;
-#define FSIE_LN_VEC(S, T)                                                                                           \
-        launch_dependent(add_layernorm_vec_kernel<S, T>, num_rows, threads, 0, stream, (const S*)src, rows, gain,   \
-                         accumulate ? x : nullptr, (T*)y, width, eps)
-        if (dtype == DTYPE_F32) return FSIE_LN_VEC(float, float);
-        return accumulate ? FSIE_LN_VEC(bf16, bf16) : FSIE_LN_VEC(float, bf16);
-#undef FSIE_LN_VEC
-    }
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
+    if (width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
+#define FSIE_LN_REGS(S, T, PER)                                                                                     \
+        launch_dependent(add_layernorm_regs_kernel<S, T, PER>, num_rows, threads, 0, stream, (const S*)src, rows, gain, \
+                         accumulate ? x : nullptr, (T*)y, width, eps)
+        const bool four = width <= 4 * threads;
+        if (dtype == DTYPE_F32) return four ? FSIE_LN_REGS(float, float, 4) : FSIE_LN_REGS(float, float, 8);
+        if (accumulate) return four ? FSIE_LN_REGS(bf16, bf16, 4) : FSIE_LN_REGS(bf16, bf16, 8);
+        return four ? FSIE_LN_REGS(float, bf16, 4) : FSIE_LN_REGS(float, bf16, 8);
+#undef FSIE_LN_REGS
+    }
     int code = 0;
 #define FSIE_LN(S, T)                                                                           \
     do {                                                                                        \

@@ -423,31 +423,39 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __res
     }
 }
 
-// The same with eight neighbouring values per thread and the row in registers (up to 8,192 values): one trip to memory and one
-// sum over the block in a decode step's chain (4 tokens of 2,048: 5.4 us with a value per thread and turn).
-template <typename T>
-__global__ void __launch_bounds__(1024) gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ proj, int ld,
+// The same, to the bit, with the row in registers (at most PER values of a thread, all asked for at once): one trip to memory
+// and one sum over the block in a decode step's chain (4 tokens of 2,048: 5.4 us with a turn through memory for each value,
+// RN_TIME now).
+template <typename T, int PER>
+__global__ void __launch_bounds__(512) gated_rmsnorm_regs_kernel(const float* __restrict__ o, const T* __restrict__ proj, int ld,
                                                                  int g_off, const float* __restrict__ gain, T* __restrict__ y,
                                                                  int width, float eps) {
     __shared__ float scratch[32];
     const size_t t = blockIdx.x;
-    const int c = threadIdx.x * 8;
-    const bool active = c < width;
-    float w[8], v[8], g[8], sq = 0.f;
-    if (active) load8(gain + c, w);
+    float w[PER], v[PER], g[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        w[i] = c < width ? gain[c] : 0.f;
+    }
     grid_dependency_wait();
     grid_dependents_go();
-    if (active) {
-        load8(o + t * width + c, v);
-        load8(proj + t * ld + g_off + c, g);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sq += v[i] * v[i];
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        v[i] = c < width ? o[t * width + c] : 0.f;
+        g[i] = c < width ? to_float(proj[t * ld + g_off + c]) : 0.f;
     }
-    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
-    if (!active) return;
+    float sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = v[i] * inv * w[i] * (1.0f / (1.0f + expf(-g[i])));
-    store8(y + t * width + c, v);
+    for (int i = 0; i < PER; ++i)
+        if (threadIdx.x + i * blockDim.x < width) sq += v[i] * v[i];
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < width) y[t * width + c] = from_float<T>(v[i] * inv * w[i] * (1.0f / (1.0f + expf(-g[i]))));
+    }
 }
 
 }  // namespace fsie
@@ -575,16 +583,15 @@ int fsie_head_norm_silu(const float* o, const void* proj, int ld, int g_off, con
 int fsie_gated_rmsnorm(const float* o, const void* proj, int ld, int g_off, const float* gain,
                        void* y, int tokens, int width, float eps, int dtype, cudaStream_t stream) {
     if (tokens <= 0) return 0;
-    if (width % 8 == 0 && width <= 8192 && ld % 8 == 0 && g_off % 8 == 0 &&
-        ((((size_t)o) | ((size_t)proj) | ((size_t)gain) | ((size_t)y)) & 15) == 0) {
-        const int threads = ((width / 8 + 31) / 32) * 32;
-        if (dtype == DTYPE_F32)
-            return launch_dependent(gated_rmsnorm_vec_kernel<float>, tokens, threads, 0, stream, o, (const float*)proj, ld, g_off,
-                                    gain, (float*)y, width, eps);
-        return launch_dependent(gated_rmsnorm_vec_kernel<bf16>, tokens, threads, 0, stream, o, (const bf16*)proj, ld, g_off, gain,
-                                (bf16*)y, width, eps);
-    }
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
+    if (width <= 8 * threads) {             // (longer rows would spill: they are read twice)
+        const bool four = width <= 4 * threads;
+        if (dtype == DTYPE_F32)
+            return launch_dependent(four ? gated_rmsnorm_regs_kernel<float, 4> : gated_rmsnorm_regs_kernel<float, 8>, tokens, threads,
+                                    0, stream, o, (const float*)proj, ld, g_off, gain, (float*)y, width, eps);
+        return launch_dependent(four ? gated_rmsnorm_regs_kernel<bf16, 4> : gated_rmsnorm_regs_kernel<bf16, 8>, tokens, threads, 0,
+                                stream, o, (const bf16*)proj, ld, g_off, gain, (bf16*)y, width, eps);
+    }
     if (dtype == DTYPE_F32)
         return launch_dependent(gated_rmsnorm_kernel<float>, tokens, threads, 0, stream, o,
                                 (const float*)proj, ld, g_off, gain, (float*)y, width, eps);

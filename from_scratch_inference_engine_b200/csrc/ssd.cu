@@ -220,41 +220,46 @@ __global__ void ssd_gate_norm_kernel(const float* __restrict__ o, const float* _
         y[t * inner + c0 + i] = from_float<T>(ssd_row[i] * inv * gain[c0 + i]);
 }
 
-// The same with eight neighbouring values per thread and the row in registers (up to 8,192 values): one trip to memory and one
-// sum over the block (a token of 4,096: 14.5 us of the step's chain with a value per thread and turn).
-template <typename T>
-__global__ void __launch_bounds__(1024) ssd_gate_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ act,
+// The same, to the bit, with the row in registers (at most PER values of a thread, all asked for at once): one trip to memory
+// and one sum over the block (a token of 4,096: 14.5 us of the step's chain with a turn through memory for each value,
+// GN_TIME now).
+template <typename T, int PER>
+__global__ void __launch_bounds__(512) ssd_gate_norm_regs_kernel(const float* __restrict__ o, const float* __restrict__ act,
                                                                  int act_ld, const T* __restrict__ proj, int ld, int z_off,
                                                                  const float* __restrict__ skip, const float* __restrict__ gain,
                                                                  T* __restrict__ y, int inner, int vdim, int parts, float eps) {
     __shared__ float scratch[32];
     const size_t t = blockIdx.x;
-    const int width = inner / parts, c = blockIdx.y * width + threadIdx.x * 8;
-    const bool active = (int)threadIdx.x * 8 < width;
-    float g[8], d = 0.f;
-    if (active) {
-        load8(gain + c, g);
-        d = skip[c / vdim];
+    const int width = inner / parts, c0 = blockIdx.y * width;
+    float g[PER], d[PER], v[PER], x[PER], z[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        g[k] = i < width ? gain[c0 + i] : 0.f;
+        d[k] = i < width ? skip[(c0 + i) / vdim] : 0.f;
     }
     grid_dependency_wait();
     grid_dependents_go();
-    float v[8], sq = 0.f;
-    if (active) {
-        float x[8], z[8];
-        load8(o + t * inner + c, v);
-        load8(act + t * act_ld + c, x);
-        load8(proj + t * ld + z_off + c, z);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = (v[i] + d * x[i]) * ssd_silu(z[i]);
-            sq += v[i] * v[i];
-        }
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * blockDim.x, c = c0 + i;
+        z[k] = i < width ? to_float(proj[t * ld + z_off + c]) : 0.f;
+        v[k] = i < width ? o[t * inner + c] : 0.f;
+        x[k] = i < width ? act[t * act_ld + c] : 0.f;
     }
-    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
-    if (!active) return;
+    float sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = v[i] * inv * g[i];
-    store8(y + t * inner + c, v);
+    for (int k = 0; k < PER; ++k)
+        if (threadIdx.x + k * blockDim.x < width) {
+            v[k] = (v[k] + d[k] * x[k]) * ssd_silu(z[k]);
+            sq += v[k] * v[k];
+        }
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < width) y[t * inner + c0 + i] = from_float<T>(v[k] * inv * g[k]);
+    }
 }
 
 }  // namespace fsie
@@ -335,18 +340,19 @@ int fsie_ssd_gate_norm(const float* o, const float* act, int act_ld, const void*
         return ERR_BAD_ARGUMENT;
     const int width = inner / parts;
     const dim3 grid(tokens, parts);
-    if (width % 8 == 0 && vdim % 8 == 0 && width <= 8192 && act_ld % 8 == 0 && ld % 8 == 0 && z_off % 8 == 0 &&
-        ((((size_t)o) | ((size_t)act) | ((size_t)proj) | ((size_t)gain) | ((size_t)y)) & 15) == 0) {
-        const int threads = ((width / 8 + 31) / 32) * 32;
+    const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
+    if (width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
+        const bool four = width <= 4 * threads;
         if (dtype == DTYPE_F32)
-            return launch_dependent(ssd_gate_norm_vec_kernel<float>, grid, threads, 0, stream, o, act, act_ld, (const float*)proj,
-                                    ld, z_off, skip, gain, (float*)y, inner, vdim, parts, eps);
-        return launch_dependent(ssd_gate_norm_vec_kernel<bf16>, grid, threads, 0, stream, o, act, act_ld, (const bf16*)proj, ld,
-                                z_off, skip, gain, (bf16*)y, inner, vdim, parts, eps);
+            return launch_dependent(four ? ssd_gate_norm_regs_kernel<float, 4> : ssd_gate_norm_regs_kernel<float, 8>, grid,
+                                    dim3(threads), 0, stream, o, act, act_ld, (const float*)proj, ld, z_off, skip, gain, (float*)y,
+                                    inner, vdim, parts, eps);
+        return launch_dependent(four ? ssd_gate_norm_regs_kernel<bf16, 4> : ssd_gate_norm_regs_kernel<bf16, 8>, grid,
+                                dim3(threads), 0, stream, o, act, act_ld, (const bf16*)proj, ld, z_off, skip, gain, (bf16*)y,
+                                inner, vdim, parts, eps);
     }
     const size_t smem = (size_t)width * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
-    const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
     if (dtype == DTYPE_F32) {
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(ssd_gate_norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
