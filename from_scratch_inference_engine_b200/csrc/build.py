@@ -50,7 +50,7 @@ LIBRARIES: Dict[str, Sequence[str]] = {
     # parts of hybrid decoders: layer norm on a sublayer's output, and windowed attention with mixed
     # heads behind a short convolution
     "hybrid": ("layernorm.cu", "talking_attention.cu", "talking_attention_bf16.cu",
-               "talking_attention_f32.cu", "talking_attention_mma.cu", "talking_decode.cu"),
+               "talking_attention_f32.cu", "talking_attention_mma.cu"),
     # recurrences over per-request state of the form S <- a S + k v^T, o = S^T q: decaying linear
     # attention, and a state-space mixer with its convolution, step sizes and gated norm
     "scan": ("lightning.cu", "ssd.cu"),

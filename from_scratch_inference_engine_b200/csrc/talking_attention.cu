@@ -137,12 +137,14 @@ __global__ void conv_norm_rotate_kernel(const T* __restrict__ proj, int ld, int 
 
 // The same with eight neighbouring channels per thread, all of a row in one go (up to CONV_VEC_WIDTH channels): 16-byte loads,
 // everything a row needs on its way at once (weights, gains, angles and lists before the kernel that makes
-// the projection has finished), and one barrier before the norms.  A decode step's rows are few, so the chain of trips to
-// memory is what it takes: with a channel per thread and turn, and the tails in a launch behind it, 4 tokens of 3,072
-// channels took 22 + 10 us of the step's chain.
+// the projection has finished).  A decode step's rows are few, so the chain of trips to memory is what it takes: with a
+// channel per thread and turn, and the tails in a launch behind it, 4 tokens of 3,072 channels took 22 + 10 us of
+// the step's chain, CV_TIME now.  The squares are added up from shared memory as the general kernel's threads and warps
+// do it, so that both leave the same bits.
 // FOLD (every request brings one token): the row's own channels move the request's tail on as well, which conv_tails
 // does otherwise (a longer portion's first tokens still read the old tail when its last one is done).
 constexpr int CONV_VEC_WIDTH = 6144;
+__host__ __device__ constexpr int conv_threads(int width) { return width >= 1024 ? 512 : 256; }     // of the general kernel
 template <typename T, int TAPS, bool FOLD>
 __global__ void __launch_bounds__(CONV_VEC_WIDTH / 8)
 conv_norm_rotate_vec_kernel(const T* __restrict__ proj, int ld, int items, const int* __restrict__ item_qstart,
@@ -153,8 +155,9 @@ conv_norm_rotate_vec_kernel(const T* __restrict__ proj, int ld, int items, const
                             const int* __restrict__ slot_of, T* __restrict__ k_pages, T* __restrict__ v_pages,
                             long long page_stride, int page_size, float* __restrict__ q_out, int heads, int kv_heads,
                             int dim, int vdim, int has_kv, float eps, int* error) {
-    __shared__ float sums[2][32];                       // per warp: squares of q, of k
-    __shared__ float eights[CONV_VEC_WIDTH / 8];        // squares of every thread's channels
+    __shared__ __align__(16) float all[CONV_VEC_WIDTH]; // the convolved row
+    __shared__ float sums[2][16];                       // squares of q, of k: one for each warp of the general kernel
+    extern __shared__ float v_scale[];                  // of every head's values
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int wq = heads * dim, wk = has_kv ? kv_heads * dim : 0, wv = has_kv ? kv_heads * vdim : 0;
     const int width = wq + wk + wv, c0 = threadIdx.x * 8;
@@ -195,7 +198,6 @@ conv_norm_rotate_vec_kernel(const T* __restrict__ proj, int ld, int items, const
     float u[TAPS][8], y[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) y[e] = 0.f;
-    float sq = 0.f;
     if (active) {
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) {
@@ -213,22 +215,36 @@ conv_norm_rotate_vec_kernel(const T* __restrict__ proj, int ld, int items, const
 #pragma unroll
             for (int j = 1; j < TAPS; ++j) store8(tail + (size_t)(j - 1) * width, u[j]);
         }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sq += y[e] * y[e];
+        store8(all + c0, y);
     }
-    eights[threadIdx.x] = sq;
-    const float q_sum = warp_sum(is_q ? sq : 0.f), k_sum = warp_sum(is_k ? sq : 0.f);
-    if (lane == 0) { sums[0][warp] = q_sum; sums[1][warp] = k_sum; }
+    __syncthreads();
+    const int stride = conv_threads(width);
+    for (int g = warp; g < stride / 32; g += warps) {
+        float sq = 0.f;
+        for (int c = g * 32 + lane; c < wq; c += stride) sq += all[c] * all[c];
+        sq = warp_sum(sq);
+        float sk = 0.f;
+        for (int c = g * 32 + lane; c < wk; c += stride) sk += all[wq + c] * all[wq + c];
+        sk = warp_sum(sk);
+        if (lane == 0) { sums[0][g] = sq; sums[1][g] = sk; }
+    }
+    for (int g = warp; g < (has_kv ? kv_heads : 0); g += warps) {
+        const float* values = all + wq + wk + g * vdim;
+        float s = 0.f;
+        for (int c = lane; c < vdim; c += 32) s += values[c] * values[c];
+        s = warp_sum(s);
+        if (lane == 0) v_scale[g] = 1.0f / sqrtf(s / (float)vdim + eps);
+    }
     __syncthreads();
     if (!active) return;
-    float total = 0.f;
+    float inv;
     if (is_v) {
-        const int first = threadIdx.x - d0 / 8;
-        for (int i = 0; i < vdim / 8; ++i) total += eights[first + i];
+        inv = v_scale[head];
     } else {
-        for (int i = 0; i < warps; ++i) total += sums[is_k ? 1 : 0][i];
+        float total = 0.f;
+        for (int i = 0; i < stride / 32; ++i) total += sums[is_k ? 1 : 0][i];
+        inv = 1.0f / sqrtf(total / (float)(is_q ? wq : wk) + eps);
     }
-    const float inv = 1.0f / sqrtf(total / (float)(is_v ? vdim : (is_q ? wq : wk)) + eps);
     if (!is_v) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) y[e] = y[e] * inv * gain[e];
@@ -309,7 +325,7 @@ int fsie_conv_norm_rotate(const void* proj, int ld, int tokens, int items, const
         const int threads = ((width / 8 + 31) / 32) * 32;
         if (folded) *folded = fold_tails;
 #define FSIE_PREPARE_VEC(T, N, F)                                                                                       \
-        launch_dependent(conv_norm_rotate_vec_kernel<T, N, F>, tokens, threads, 0, stream, (const T*)proj, ld, items,   \
+        launch_dependent(conv_norm_rotate_vec_kernel<T, N, F>, tokens, threads, kv_heads * sizeof(float), stream, (const T*)proj, ld, items, \
                          item_qstart, item_pos0, item_slots, tails, conv_w, q_gain, k_gain, cos_sin, table_len, rot_dims, \
                          slot_of, (T*)k_pages, (T*)v_pages, page_stride, page_size, q_out, heads, kv_heads, dim, vdim, \
                          has_kv, eps, error)
@@ -326,7 +342,7 @@ int fsie_conv_norm_rotate(const void* proj, int ld, int tokens, int items, const
     }
     const size_t smem = (size_t)(width + kv_heads) * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
-    const int threads = width >= 1024 ? 512 : 256;
+    const int threads = conv_threads(width);
     int code = 0;
 #define FSIE_PREPARE(T)                                                                          \
     do {                                                                                         \

@@ -36,6 +36,7 @@ struct TalkingArgs {
     float* part_stats;             // [tiles][nsplit][TA_ROWS][2]
     float* part_out;               // [nsplit][tokens][heads * vdim]
     int tokens;
+    int ahead;                     // values have a buffer of their own and are asked for together with the keys
 };
 
 __device__ __forceinline__ void load2(const float* p, float& a, float& b) {
@@ -66,8 +67,13 @@ struct TalkingLayout {
 };
 
 // One tile of keys (or values) of every key/value head from the pages into shared memory
-// [g][key][ld], zero beyond `width` and for keys without a page: a warp copies a row, 16 bytes
-// per lane where the rows allow it.
+// [g][key][ld], zero beyond `width` and for keys without a page: asynchronous copies of 16 bytes
+// where the rows allow it, all of a tile's on their way together (a warp that copied a row at a time
+// through registers waited for memory once a row, 32 times for 4 heads of 64 keys).
+__device__ __forceinline__ void talking_copy16(void* to, const void* from, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from), "r"(bytes)
+                 : "memory");
+}
 template <typename T>
 __device__ __forceinline__ void copy_tile(T* __restrict__ dst, const T* __restrict__ pages,
                                           const int* key_page, const int* key_off, int G, int keys,
@@ -76,28 +82,39 @@ __device__ __forceinline__ void copy_tile(T* __restrict__ dst, const T* __restri
     constexpr int PER = 16 / (int)sizeof(T);                 // elements of one 16-byte piece
     const bool wide = width % PER == 0 && page_stride % PER == 0 &&
                       (reinterpret_cast<uintptr_t>(pages) & 15) == 0;
-    for (int row = warp; row < G * keys; row += TA_WARPS) {
-        const int g = row / keys, jj = row - g * keys;
-        const int page = key_page[jj];
-        T* to = dst + (size_t)row * ld;
-        const T* from = page < 0 ? nullptr :
-            pages + page * page_stride + ((size_t)g * page_size + key_off[jj]) * width;
-        if (wide) {
-            for (int piece = lane; piece * PER < width8; piece += 32) {
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (from && piece * PER < width) v = *reinterpret_cast<const uint4*>(from + piece * PER);
-                *reinterpret_cast<uint4*>(to + piece * PER) = v;
-            }
-        } else {
+    if (wide) {
+        const int pieces = width8 / PER, total = G * keys * pieces;
+        for (int i = warp * 32 + lane; i < total; i += TA_WARPS * 32) {
+            const int row = i / pieces, d = (i - row * pieces) * PER, g = row / keys, jj = row - g * keys;
+            const int page = key_page[jj];
+            const bool there = page >= 0 && d < width;
+            talking_copy16(dst + (size_t)row * ld + d,
+                           there ? pages + page * page_stride + ((size_t)g * page_size + key_off[jj]) * width + d : pages,
+                           there ? 16 : 0);
+        }
+    } else {
+        for (int row = warp; row < G * keys; row += TA_WARPS) {
+            const int g = row / keys, jj = row - g * keys;
+            const int page = key_page[jj];
+            T* to = dst + (size_t)row * ld;
+            const T* from = page < 0 ? nullptr :
+                pages + page * page_stride + ((size_t)g * page_size + key_off[jj]) * width;
             for (int d = lane; d < width8; d += 32)
                 to[d] = (from && d < width) ? from[d] : from_float<T>(0.f);
         }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
+// all but the newest `N` of a thread's copies have arrived
+template <int N>
+__device__ __forceinline__ void talking_copies_done() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Warp w owns heads w, w + 8, ... (HS = 8 / TOK of them at most) and, of each, the tile's TOK
 // tokens: rows that share their keys and values, so one load of a key or value serves TOK rows.
 // Lane l owns keys l (+ 32) of a tile for the scores and value columns 2 l, 2 l + 1 (+ 64 c).
+// A split tile's block has one or two tiles of keys: it is a chain of trips to memory.  The lists, the first tile's pages
+// and the mixing matrix are read before the kernel before has finished, and by the second walk also the queries, keys
+// and values, which the first walk only read (4 requests of 1,024 keys: TA_TIME).
 template <typename T, int TOK, int VC2, int KPL>
 __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const TalkingArgs a) {
     constexpr int HS = 8 / TOK;
@@ -107,9 +124,11 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
     const int group = H / G;
     const int tile = blockIdx.x, split = blockIdx.y;
     const int item = a.tile_item[tile], tok0 = a.tile_row0[tile];
-    if (a.item_slots[item] < 0) return;                 // a padding entry of a fixed-size batch
     const int n_tok = min(TOK, a.item_qlen[item] - tok0);
-    if (n_tok <= 0) return;
+    if (a.item_slots[item] < 0 || n_tok <= 0) {         // a padding entry of a fixed-size batch
+        grid_dependency_wait();
+        return;
+    }
     const int R = n_tok * H;
     const int p_first = a.item_pos0[item] + tok0, p_last = p_first + n_tok - 1;
     const int lo = a.window > 0 ? max(0, p_first - a.window + 1) : 0;
@@ -128,6 +147,7 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
     float* talk = P2 + TA_ROWS * TK;
     int* key_page = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(talk) + L.talk_bytes);
     int* key_off = key_page + TK;
+    T* vbuf = a.ahead ? reinterpret_cast<T*>(smem_raw + L.total) : kv;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* k_pages = reinterpret_cast<const T*>(a.k_pages);
@@ -135,12 +155,49 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
     const int* table = a.block_tables + (size_t)item * a.table_stride;
     const int token0 = a.item_qstart[item] + tok0;
 
+    bool gone = false;                                  // a visible key's page was given back
+    const auto find_keys = [&](int u0) {
+        if ((int)threadIdx.x >= TK) return;
+        int page = -1, off = 0;
+        if (u0 + (int)threadIdx.x < u_end) {
+            const int u = u0 + threadIdx.x;
+            const int j = u < kept ? u : lo + (u - kept);
+            page = table[j / a.page_size];
+            off = j - (j / a.page_size) * a.page_size;
+            gone |= page < 0;
+        }
+        key_page[threadIdx.x] = page;
+        key_off[threadIdx.x] = off;
+    };
+    // keys or values of every key/value head: [g][key][dim8], zero beyond dim and beyond the tile
+    const auto copy_keys = [&]() {
+        copy_tile<T>(kv, k_pages, key_page, key_off, G, TK, dim, L.dim8, L.kv_ld, a.page_stride, a.page_size, warp, lane);
+    };
+    const auto copy_values = [&]() {
+        copy_tile<T>(vbuf, v_pages, key_page, key_off, G, TK, vdim, L.vdim8, L.kv_ld, a.page_stride, a.page_size, warp, lane);
+    };
+    const bool early = a.mode == 2;                     // what the keys' writer left is older than the kernel before
+    for (int idx = threadIdx.x; idx < H * H; idx += blockDim.x) talk[idx] = a.talk[idx];
+    if (u_begin < u_end) find_keys(u_begin);
+    if (!early) {
+        grid_dependency_wait();
+        grid_dependents_go();                           // (not before the wait: the second walk's early reads rest on it)
+    } else {
+        __syncthreads();                                // the first tile's pages
+        if (u_begin < u_end) {
+            copy_keys();
+            if (a.ahead) copy_values();
+        }
+    }
     // q rows [tok * H + h], zero beyond dim and beyond the tile's tokens
     for (int idx = threadIdx.x; idx < TOK * H * L.dim8; idx += blockDim.x) {
         const int r = idx / L.dim8, d = idx - r * L.dim8;
         qs[r * L.q_ld + d] = (r < R && d < dim) ? a.q[((size_t)token0 * H + r) * dim + d] : 0.f;
     }
-    for (int idx = threadIdx.x; idx < H * H; idx += blockDim.x) talk[idx] = a.talk[idx];
+    if (early) {
+        grid_dependency_wait();
+        grid_dependents_go();
+    }
 
     float row_max[HS][TOK], row_sum[HS][TOK], acc[HS][TOK][VC2][2];
 #pragma unroll
@@ -154,26 +211,45 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
         }
 
     if (a.mode == 2) {
-        // maximum and sum over all key ranges, from what the first launch left
-        __syncthreads();
+        // maximum and sum over all key ranges, from what the first launch left: a lane reads a range's, the sum is
+        // taken range by range
         const float* stats = a.part_stats + (size_t)tile * a.nsplit * TA_ROWS * 2;
+        float range_max[HS][TOK], range_sum[HS][TOK];
+        const auto read_ranges = [&](int s0) {
 #pragma unroll
-        for (int hs = 0; hs < HS; ++hs) {
-            const int h = warp + TA_WARPS * hs;
+            for (int hs = 0; hs < HS; ++hs)
 #pragma unroll
-            for (int t = 0; t < TOK; ++t) {
-                if (h >= H || t >= n_tok) continue;
-                const int r = t * H + h;
-                float m = -INFINITY;
-                for (int s = 0; s < a.nsplit; ++s) m = fmaxf(m, stats[((size_t)s * TA_ROWS + r) * 2]);
-                float l = 0.f;
-                for (int s = 0; s < a.nsplit; ++s) {
-                    const float ms = stats[((size_t)s * TA_ROWS + r) * 2];
-                    if (ms > -INFINITY) l += stats[((size_t)s * TA_ROWS + r) * 2 + 1] * expf(ms - m);
+                for (int t = 0; t < TOK; ++t) {
+                    const int h = warp + TA_WARPS * hs, s = s0 + lane;
+                    const bool in = h < H && t < n_tok && s < a.nsplit;
+                    const float2 v = in ? *reinterpret_cast<const float2*>(stats + ((size_t)s * TA_ROWS + t * H + h) * 2)
+                                        : make_float2(-INFINITY, 0.f);
+                    range_max[hs][t] = v.x;
+                    range_sum[hs][t] = v.y;
                 }
-                row_max[hs][t] = m;
-                row_sum[hs][t] = l;
-            }
+        };
+        for (int s0 = 0; s0 < a.nsplit; s0 += 32) {
+            read_ranges(s0);
+#pragma unroll
+            for (int hs = 0; hs < HS; ++hs)
+#pragma unroll
+                for (int t = 0; t < TOK; ++t) row_max[hs][t] = fmaxf(row_max[hs][t], warp_max(range_max[hs][t]));
+        }
+        for (int s0 = 0; s0 < a.nsplit; s0 += 32) {
+            if (a.nsplit > 32) read_ranges(s0);
+#pragma unroll
+            for (int hs = 0; hs < HS; ++hs)
+#pragma unroll
+                for (int t = 0; t < TOK; ++t) {
+                    if (warp + TA_WARPS * hs >= H || t >= n_tok) continue;
+                    const float factor = expf(range_max[hs][t] - row_max[hs][t]);
+                    for (int s = 0; s < min(32, a.nsplit - s0); ++s) {
+                        const float ms = __shfl_sync(0xffffffffu, range_max[hs][t], s);
+                        const float sum = __shfl_sync(0xffffffffu, range_sum[hs][t], s);
+                        const float e = __shfl_sync(0xffffffffu, factor, s);
+                        if (ms > -INFINITY) row_sum[hs][t] += sum * e;
+                    }
+                }
         }
     }
 
@@ -181,23 +257,15 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
     for (int pass = first_pass; pass <= last_pass; ++pass) {
         for (int u0 = u_begin; u0 < u_end; u0 += TK) {
             const int n = min(TK, u_end - u0);
-            __syncthreads();                             // the tile before is done with kv, P, P2
-            if (threadIdx.x < TK) {
-                int page = -1, off = 0;
-                if ((int)threadIdx.x < n) {
-                    const int u = u0 + threadIdx.x;
-                    const int j = u < kept ? u : lo + (u - kept);
-                    page = table[j / a.page_size];
-                    off = j - (j / a.page_size) * a.page_size;
-                    if (page < 0) atomicExch(a.error, 3);      // a visible key's page was given back
-                }
-                key_page[threadIdx.x] = page;
-                key_off[threadIdx.x] = off;
+            if (!(early && u0 == u_begin)) {
+                __syncthreads();                         // the tile before is done with kv, P, P2
+                if (u0 != u_begin || pass != first_pass) find_keys(u0);
+                __syncthreads();
+                copy_keys();
+                if (pass == 1 && a.ahead) copy_values();
             }
-            __syncthreads();
-            // keys of every key/value head: [g][key][dim8], zero beyond dim and beyond the tile
-            copy_tile<T>(kv, k_pages, key_page, key_off, G, TK, dim, L.dim8, L.kv_ld, a.page_stride,
-                         a.page_size, warp, lane);
+            if (pass == 1 && a.ahead) talking_copies_done<1>();
+            else talking_copies_done<0>();
             __syncthreads();
 #pragma unroll
             for (int hs = 0; hs < HS; ++hs) {
@@ -259,6 +327,7 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
             }
             if (pass == 0) continue;
             __syncthreads();                             // P holds every head's weights of this tile
+            if (!a.ahead) copy_values();
             for (int idx = threadIdx.x; idx < R * TK; idx += blockDim.x) {
                 const int r = idx / TK, jj = idx - r * TK;
                 const int t = r / H, h = r - t * H;
@@ -268,15 +337,13 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
                 for (int h2 = 0; h2 < H; ++h2) m += mix[h2] * col[h2 * TK];
                 P2[idx] = m;
             }
-            // values of every key/value head: [g][key][vdim8], zero beyond vdim and beyond the tile
-            copy_tile<T>(kv, v_pages, key_page, key_off, G, TK, vdim, L.vdim8, L.kv_ld, a.page_stride,
-                         a.page_size, warp, lane);
+            talking_copies_done<0>();
             __syncthreads();
 #pragma unroll
             for (int hs = 0; hs < HS; ++hs) {
                 const int h = warp + TA_WARPS * hs;
                 if (h >= H) continue;
-                const T* vg = kv + (size_t)(h / group) * TK * L.kv_ld;
+                const T* vg = vbuf + (size_t)(h / group) * TK * L.kv_ld;
                 for (int jj = 0; jj < TK; jj += 4) {
                     if (jj >= n) break;
                     float4 p[TOK];
@@ -302,6 +369,7 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
         }
     }
 
+    if (gone) atomicExch(a.error, 3);
     if (a.mode == 1) {
         float* stats = a.part_stats + ((size_t)tile * a.nsplit + split) * TA_ROWS * 2;
 #pragma unroll
@@ -341,9 +409,12 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
 template <typename T>
 __global__ void talking_attention_merge_kernel(const float* __restrict__ part, T* __restrict__ out,
                                                long long count, int nsplit) {
+    grid_dependency_wait();
+    grid_dependents_go();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count;
          i += (long long)gridDim.x * blockDim.x) {
         float v = 0.f;
+#pragma unroll 16
         for (int s = 0; s < nsplit; ++s) v += part[(size_t)s * count + i];
         out[i] = from_float<T>(v);
     }
@@ -358,20 +429,26 @@ inline int talking_key_tile(int heads, int kv_heads, int dim, int vdim, int elem
     return 0;
 }
 
+// Values get a buffer of their own where every block has an SM to itself anyway (148 of them): a second block on the SM hides
+// more than that where there are more.
+constexpr int TA_AHEAD_BLOCKS = 148;
+constexpr size_t TA_AHEAD_BYTES = 220 * 1024;
+
 template <typename T, int TOK, int VC2>
-int talking_attention_launch_tile(const TalkingArgs& a, int num_tiles, int key_tile, size_t smem,
+int talking_attention_launch_tile(TalkingArgs a, int num_tiles, int key_tile, size_t smem,
                                   cudaStream_t stream) {
     const dim3 grid(num_tiles, a.nsplit);
+    const size_t both = smem + TalkingLayout(a.heads, a.kv_heads, a.dim, a.vdim, key_tile, (int)sizeof(T)).kv_bytes;
+    a.ahead = a.mode != 1 && (long long)num_tiles * a.nsplit <= TA_AHEAD_BLOCKS && both <= TA_AHEAD_BYTES;
+    if (a.ahead) smem = both;
     if (key_tile == 64) {
         cudaFuncSetAttribute(talking_attention_kernel<T, TOK, VC2, 2>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        talking_attention_kernel<T, TOK, VC2, 2><<<grid, TA_WARPS * 32, smem, stream>>>(a);
-    } else {
-        cudaFuncSetAttribute(talking_attention_kernel<T, TOK, VC2, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        talking_attention_kernel<T, TOK, VC2, 1><<<grid, TA_WARPS * 32, smem, stream>>>(a);
+        return launch_dependent(talking_attention_kernel<T, TOK, VC2, 2>, grid, TA_WARPS * 32, smem, stream, a);
     }
-    return FSIE_LAUNCH_CHECK();
+    cudaFuncSetAttribute(talking_attention_kernel<T, TOK, VC2, 1>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch_dependent(talking_attention_kernel<T, TOK, VC2, 1>, grid, TA_WARPS * 32, smem, stream, a);
 }
 
 template <typename T, int TOK>
@@ -411,9 +488,8 @@ int talking_attention_launch(TalkingArgs a, int num_tiles, cudaStream_t stream) 
     if (a.nsplit > 1) {
         const long long count = (long long)a.tokens * a.heads * a.vdim;
         const long long wanted = (count + 255) / 256;
-        talking_attention_merge_kernel<T><<<(unsigned)(wanted > 2048 ? 2048 : wanted), 256, 0, stream>>>(
-            a.part_out, reinterpret_cast<T*>(a.out), count, a.nsplit);
-        return FSIE_LAUNCH_CHECK();
+        return launch_dependent(talking_attention_merge_kernel<T>, (unsigned)(wanted > 2048 ? 2048 : wanted), 256, 0, stream,
+                                a.part_out, reinterpret_cast<T*>(a.out), count, a.nsplit);
     }
     return 0;
 }

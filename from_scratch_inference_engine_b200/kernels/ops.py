@@ -1049,10 +1049,6 @@ def hybrid():
         lib.fsie_conv_tails.argtypes = [p, i, p, p, p, i, p, i, i, i, p]
         lib.fsie_talking_attention_tile_tokens.argtypes = [i]
         lib.fsie_talking_attention_key_tile.argtypes = [i, i, i, i, i]
-        lib.fsie_talking_decode.argtypes = [p, p, p, ll, i, p, i, p, p, p, p, i, p, p, i, i, i, i, i, i, f, p, i, p, p, i, p]
-        lib.fsie_talking_decode_keys.argtypes = []
-        lib.fsie_talking_decode_keys.restype = i
-        lib.fsie_talking_decode.restype = i
         lib.fsie_talking_attention.argtypes = [p, p, p, ll, i, p, i, p, p, i, p, p, p, p, p, p,
                                                i, i, i, i, i, i, i, i, f, i, p, p, i, p, p]
         lib.fsie_talking_attention_mma_takes.argtypes = [i, i, i, i]
@@ -1459,49 +1455,6 @@ def talking_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         kv_heads, dim, vdim, window, keep_first, tile_tokens, float(scale), nsplit,
         part_stats, part_out, _tag(k_pages.dtype), error, _stream()),
         "talking_attention")
-    return out
-
-
-TALKING_DECODE_KEYS = 64           # what `fsie_talking_decode_keys` says: keys of one range of `talking_decode`
-TALKING_DECODE_SCORES = 1 << 24    # floats of scores at most (64 MB)
-
-
-def talking_decode_splits(items: int, keys: int, heads: int, kv_heads: int, dim: int, vdim: int, page_stride: int,
-                          dtype: torch.dtype) -> int:
-    """Ranges of keys with which `talking_decode` takes a step of one token per request that sees up to `keys` keys;
-    0 where it does not take it."""
-    per = 4 if dtype is torch.float32 else 8
-    nsplit = max(1, -(-keys // TALKING_DECODE_KEYS))
-    takes = (heads // kv_heads <= 8 and heads <= 64 and dim % 8 == 0 and vdim % 8 == 0 and dim <= 256 and vdim <= 256
-             and page_stride % per == 0 and items * heads * nsplit * TALKING_DECODE_KEYS <= TALKING_DECODE_SCORES)
-    return nsplit if takes else 0
-
-
-def talking_decode(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, page_stride: int, page_size: int,
-                   block_tables: torch.Tensor, item_qstart: torch.Tensor, item_qlen: torch.Tensor,
-                   item_pos0: torch.Tensor, item_slots: torch.Tensor, items: int, talk: torch.Tensor, out: torch.Tensor,
-                   heads: int, kv_heads: int, dim: int, vdim: int, window: int, keep_first: int, scale: float,
-                   error: torch.Tensor, nsplit: int, scores: torch.Tensor, stats: torch.Tensor) -> torch.Tensor:
-    """`talking_attention` for a step of one token per request, in two launches.  `nsplit` from
-    `talking_decode_splits`; float32 scratch scores [items * heads * nsplit * 64] and stats [items * nsplit * heads * 2]."""
-    _need(q, torch.float32, "q")
-    _need(talk, torch.float32, "talk")
-    _need(out, k_pages.dtype, "out")
-    _need(scores, torch.float32, "scores")
-    _need(stats, torch.float32, "stats")
-    _need(error, torch.int32, "error")
-    for name, t in (("block_tables", block_tables), ("item_qstart", item_qstart), ("item_qlen", item_qlen),
-                    ("item_pos0", item_pos0), ("item_slots", item_slots)):
-        _need(t, torch.int32, name)
-    if v_pages.dtype is not k_pages.dtype or talk.numel() != heads * heads:
-        raise KernelError("talking_decode: keys and values differ in dtype, or the mixing matrix is not [heads, heads]")
-    if q.shape[0] != items or q.numel() < items * heads * dim or out.numel() < items * heads * vdim or \
-            scores.numel() < items * heads * nsplit * TALKING_DECODE_KEYS or stats.numel() < items * nsplit * heads * 2:
-        raise KernelError("talking_decode: one token per request, and scratch for all of its keys")
-    _check(hybrid().fsie_talking_decode(
-        q, k_pages, v_pages, page_stride, page_size, block_tables, block_tables.stride(0), item_qstart, item_qlen, item_pos0,
-        item_slots, items, talk, out, heads, kv_heads, dim, vdim, window, keep_first, float(scale), error, nsplit, scores,
-        stats, _tag(k_pages.dtype), _stream()), "talking_decode")
     return out
 
 

@@ -146,19 +146,6 @@ class TalkingWindowAttention(Mixer):
                                       self.kv_heads, self.dim, self.vdim, self.window,
                                       self.keep_first, self.scale, ctx.error)
             return rt.linear(out, self.w_o, None, "talking.o")
-        if ctx.num_tokens == ctx.num_items:
-            # one token per request: scores first, then mixed weights and values
-            keys = ctx.max_context if self.window <= 0 else min(ctx.max_context, self.window + self.keep_first)
-            nsplit = ops.talking_decode_splits(ctx.num_items, keys, self.heads, self.kv_heads, self.dim, self.vdim,
-                                               cache.page_stride, rt.dtype)
-            if nsplit:
-                scores = ctx.scratch("talking.scores", tokens * self.heads * nsplit * ops.TALKING_DECODE_KEYS)
-                stats = ctx.scratch("talking.part_stats", tokens * nsplit * self.heads * 2)
-                ops.talking_decode(q, cache.k_pages, cache.v_pages, cache.page_stride, group.page_size,
-                                   group.block_tables, ctx.item_qstart, ctx.item_qlen, ctx.item_pos0, ctx.item_slots,
-                                   ctx.num_items, self.talk, out, self.heads, self.kv_heads, self.dim, self.vdim,
-                                   self.window, self.keep_first, self.scale, ctx.error, nsplit, scores, stats)
-                return rt.linear(out, self.w_o, None, "talking.o")
         # a step of single tokens takes tiles of one token, a step with prompt portions the
         # largest tile a block holds for this many heads
         tile_tokens = 1 if ctx.num_tokens == ctx.num_items else self.tile_tokens
