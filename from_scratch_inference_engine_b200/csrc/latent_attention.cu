@@ -222,82 +222,78 @@ __device__ __forceinline__ void hm_cp16(void* dst, const void* src, bool valid) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(hm_smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// ---- the same for few tokens of bfloat16 on the tensor cores: a warp owns 16 output rows of one head (M of m16n8k16; the
-// tokens are N), and KW warps share the k range.  What bounds it is the chain from the kernel before to its result, so
-// there is no staging: a lane's 16 bytes of two weight rows are its fragments as they are (the order of k does
-// not matter to a dot product), asked for before that kernel has finished, and x gives the matching 16 bytes.
-constexpr int HQ_WARPS = 4, HQ_AHEAD = 4;                      // chunks of 32 k-elements asked for together
-template <int TT, int KW>
+// ---- the same for few tokens of bfloat16 where rows start on 16 bytes and k is up to 1,024: a lane's weights of HQ_ROWS rows
+// are on their way before the kernel before has finished and x comes straight to the lanes that use it.  What bounds it is the
+// chain from that kernel to its result: staging x as floats in shared memory, a value at a time and behind a barrier, for 8
+// rows a block took 10.5 us (4 tokens, 16 heads of 512 x 128), HQ_TIME now.  A row has LANES lanes (16 where k <= 128 would leave
+// the others idle), which add up what they had above in the same order: the same bits.
+constexpr int HQ_WARPS = 4, HQ_ROWS = 4;
+template <int LANES, int CHUNKS, int TOK>
 __global__ void __launch_bounds__(HQ_WARPS * 32) head_product_rows_kernel(
         const bf16* __restrict__ x, long long x_ld, int x_head, const bf16* __restrict__ w, bf16* __restrict__ out,
         long long out_ld, int out_head, int tokens, int n, int k) {
-    constexpr int TILES = HQ_WARPS / KW;                        // tiles of 16 rows per block
-    __shared__ float parts[KW > 1 ? KW - 1 : 1][TILES][16][8 * TT + 1];
-    const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int part = warp % KW, tile = warp / KW, g = lane >> 2, t = lane & 3;
-    const int row0 = (blockIdx.x * TILES + tile) * 16;
-    const int chunks = k / 32, per = (chunks + KW - 1) / KW, c_begin = part * per, c_end = min(chunks, c_begin + per);
-    const bf16* w_lo = w + ((size_t)h * n + min(row0 + g, n - 1)) * k + 8 * t;
-    const bf16* w_hi = w + ((size_t)h * n + min(row0 + 8 + g, n - 1)) * k + 8 * t;
-    uint4 lo[HQ_AHEAD], hi[HQ_AHEAD];
-    auto weights = [&](int c0) {
+    const int h = blockIdx.y, lane = threadIdx.x % LANES, owner = threadIdx.x / LANES;
+    const int row0 = (blockIdx.x * (HQ_WARPS * 32 / LANES) + owner) * HQ_ROWS;
+    uint4 raw[HQ_ROWS][CHUNKS];
 #pragma unroll
-        for (int j = 0; j < HQ_AHEAD; ++j) {
-            const bool in = c0 + j < c_end;
-            lo[j] = in ? __ldg(reinterpret_cast<const uint4*>(w_lo + (c0 + j) * 32)) : make_uint4(0, 0, 0, 0);
-            hi[j] = in ? __ldg(reinterpret_cast<const uint4*>(w_hi + (c0 + j) * 32)) : make_uint4(0, 0, 0, 0);
+    for (int r = 0; r < HQ_ROWS; ++r)
+#pragma unroll
+        for (int j = 0; j < CHUNKS; ++j) {
+            const int kk = (j * LANES + lane) * 8;
+            raw[r][j] = kk < k ? __ldg(reinterpret_cast<const uint4*>(w + ((size_t)h * n + min(row0 + r, n - 1)) * k + kk))
+                               : make_uint4(0u, 0u, 0u, 0u);
         }
-    };
-    weights(c_begin);
     grid_dependency_wait();
     grid_dependents_go();
-    float acc[TT][4];
+    for (int t0 = 0; t0 < tokens; t0 += TOK) {
+        uint4 xs[TOK][CHUNKS];
 #pragma unroll
-    for (int m = 0; m < TT; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
-    for (int c0 = c_begin; c0 < c_end; c0 += HQ_AHEAD) {
-        uint4 b[HQ_AHEAD][TT];
+        for (int t = 0; t < TOK; ++t)
 #pragma unroll
-        for (int j = 0; j < HQ_AHEAD; ++j)
+            for (int j = 0; j < CHUNKS; ++j) {
+                const int kk = (j * LANES + lane) * 8;
+                xs[t][j] = t0 + t < tokens && kk < k
+                    ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + t) * x_ld + (size_t)h * x_head + kk)
+                    : make_uint4(0u, 0u, 0u, 0u);
+            }
+        float acc[HQ_ROWS][TOK];
 #pragma unroll
-            for (int m = 0; m < TT; ++m)
-                b[j][m] = c0 + j < c_end && 8 * m + g < tokens
-                    ? *reinterpret_cast<const uint4*>(x + (size_t)(8 * m + g) * x_ld + (size_t)h * x_head + (c0 + j) * 32 + 8 * t)
-                    : make_uint4(0, 0, 0, 0);
+        for (int r = 0; r < HQ_ROWS; ++r)
 #pragma unroll
-        for (int j = 0; j < HQ_AHEAD; ++j) {
-            const uint32_t a0[4] = {lo[j].x, hi[j].x, lo[j].y, hi[j].y}, a1[4] = {lo[j].z, hi[j].z, lo[j].w, hi[j].w};
+            for (int t = 0; t < TOK; ++t) acc[r][t] = 0.f;
 #pragma unroll
-            for (int m = 0; m < TT; ++m) {
-                hm_mma(acc[m], a0, b[j][m].x, b[j][m].y);
-                hm_mma(acc[m], a1, b[j][m].z, b[j][m].w);
+        for (int j = 0; j < CHUNKS; ++j) {
+            if ((j * LANES + lane) * 8 >= k) break;
+            float wv[HQ_ROWS][8];
+#pragma unroll
+            for (int r = 0; r < HQ_ROWS; ++r) load8(reinterpret_cast<const bf16*>(&raw[r][j]), wv[r]);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) {
+                float a[8];
+                load8(reinterpret_cast<const bf16*>(&xs[t][j]), a);
+#pragma unroll
+                for (int r = 0; r < HQ_ROWS; ++r)
+                    acc[r][t] += wv[r][0] * a[0] + wv[r][1] * a[1] + wv[r][2] * a[2] + wv[r][3] * a[3] +
+                                 wv[r][4] * a[4] + wv[r][5] * a[5] + wv[r][6] * a[6] + wv[r][7] * a[7];
             }
         }
-        if (c0 + HQ_AHEAD < c_end) weights(c0 + HQ_AHEAD);
+#pragma unroll
+        for (int r = 0; r < HQ_ROWS; ++r)
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) {
+                float v = acc[r][t];
+#pragma unroll
+                for (int o = LANES / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                acc[r][t] = v;
+            }
+        // every lane has every sum: lane r * TOK + t writes one (LANES = 16 of HQ_ROWS * TOK sums go round)
+#pragma unroll
+        for (int r = 0; r < HQ_ROWS; ++r)
+#pragma unroll
+            for (int t = 0; t < TOK; ++t)
+                if (lane == (r * TOK + t) % LANES && t0 + t < tokens && row0 + r < n)
+                    out[(size_t)(t0 + t) * out_ld + (size_t)h * out_head + row0 + r] = __float2bfloat16_rn(acc[r][t]);
     }
-    // acc[m]: rows g (0, 1) and g + 8 (2, 3), tokens 8 m + 2 t and 8 m + 2 t + 1; the parts of k are added in order
-    if (KW > 1) {
-        if (part > 0) {
-#pragma unroll
-            for (int m = 0; m < TT; ++m)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) parts[part - 1][tile][g + (e >> 1) * 8][8 * m + 2 * t + (e & 1)] = acc[m][e];
-        }
-        __syncthreads();
-        if (part > 0) return;
-#pragma unroll
-        for (int q = 0; q + 1 < KW; ++q)
-#pragma unroll
-            for (int m = 0; m < TT; ++m)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[m][e] += parts[q][tile][g + (e >> 1) * 8][8 * m + 2 * t + (e & 1)];
-    }
-#pragma unroll
-    for (int m = 0; m < TT; ++m)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int token = 8 * m + 2 * t + (e & 1), c = row0 + g + (e >> 1) * 8;
-            if (token < tokens && c < n) out[(size_t)token * out_ld + (size_t)h * out_head + c] = __float2bfloat16_rn(acc[m][e]);
-        }
 }
 
 __global__ void __launch_bounds__(128) head_product_mma_kernel(
@@ -406,15 +402,17 @@ int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, 
             return launch_dependent(head_product_few_kernel<float>, few, dim3(HF_WARPS * 32), smem, stream, (const float*)x,
                                     x_ld, x_head, (const float*)w, (float*)out, out_ld, out_head, tokens, n, k);
         }
-        // on the tensor cores where rows start on 16 bytes; a warp takes up to four chunks of k, so that all of its
-        // weights are on their way before x is there
-        if (k % 32 == 0 && x_ld % 8 == 0 && x_head % 8 == 0 && ((((size_t)x) | ((size_t)w)) & 15) == 0) {
-#define FSIE_HEAD_ROWS(T, W)                                                                                       \
-            launch_dependent(head_product_rows_kernel<T, W>, dim3((n + 16 * HQ_WARPS / W - 1) / (16 * HQ_WARPS / W), heads), \
+        // all of a row's weights in registers: up to 1,024 of them
+        if (k % 8 == 0 && k <= 1024 && x_ld % 8 == 0 && x_head % 8 == 0 && ((((size_t)x) | ((size_t)w)) & 15) == 0) {
+#define FSIE_HEAD_ROWS(L, C, T)                                                                                    \
+            launch_dependent(head_product_rows_kernel<L, C, T>,                                                    \
+                             dim3((n + HQ_ROWS * HQ_WARPS * 32 / L - 1) / (HQ_ROWS * HQ_WARPS * 32 / L), heads),   \
                              dim3(HQ_WARPS * 32), 0, stream, (const bf16*)x, x_ld, x_head, (const bf16*)w, (bf16*)out, \
                              out_ld, out_head, tokens, n, k)
-            if (tokens <= 8) return k >= 512 ? FSIE_HEAD_ROWS(1, 4) : (k >= 256 ? FSIE_HEAD_ROWS(1, 2) : FSIE_HEAD_ROWS(1, 1));
-            return k >= 512 ? FSIE_HEAD_ROWS(2, 4) : (k >= 256 ? FSIE_HEAD_ROWS(2, 2) : FSIE_HEAD_ROWS(2, 1));
+            if (k <= 128) return tokens <= 4 ? FSIE_HEAD_ROWS(16, 1, 4) : FSIE_HEAD_ROWS(16, 1, 8);
+            if (k <= 256) return tokens <= 4 ? FSIE_HEAD_ROWS(32, 1, 4) : FSIE_HEAD_ROWS(32, 1, 8);
+            if (k <= 512) return tokens <= 4 ? FSIE_HEAD_ROWS(32, 2, 4) : FSIE_HEAD_ROWS(32, 2, 8);
+            return FSIE_HEAD_ROWS(32, 4, 4);
 #undef FSIE_HEAD_ROWS
         }
         if (smem > 48 * 1024)
