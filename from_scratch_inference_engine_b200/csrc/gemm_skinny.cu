@@ -26,7 +26,7 @@ constexpr int SK_AHEAD = 4;          // chunks whose weights a warp has asked fo
 
 struct SkinnyParams {
     const bf16* w; const bf16* x; long long ldx;
-    void* y; long long ldy; const bf16* bias;
+    void* y; long long ldy; const bf16* bias;      // GATED: of the gate rows, then of the up rows
     int T, N, K, out_f32, relu2;
 };
 
@@ -118,6 +118,10 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
             if (head >= rope.heads && rope.slot_of) early_slot = rope.slot_of[token];
             if (p.bias) { early_bias_lo = __bfloat162float(p.bias[row0 + r]); early_bias_hi = __bfloat162float(p.bias[row8 + r]); }
         }
+    }
+    if (GATED && p.bias && threadIdx.x < 8 * TP) {                // the pair of outputs this thread finishes
+        const int n = min(row0 + (int)(threadIdx.x & 7), p.N - 1);
+        early_bias_lo = __bfloat162float(p.bias[n]); early_bias_hi = __bfloat162float(p.bias[p.N + n]);
     }
     grid_dependency_wait();
     grid_dependents_go();
@@ -227,6 +231,7 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 gate += red[((size_t)w * SK_ROWS + r) * TP + token];
                 up += red[((size_t)w * SK_ROWS + r + 8) * TP + token];
             }
+            if (p.bias) { gate += early_bias_lo; up += early_bias_hi; }     // (e is this thread's own pair: see above)
             gate = __bfloat162float(__float2bfloat16_rn(gate));
             up = __bfloat162float(__float2bfloat16_rn(up));
             reinterpret_cast<bf16*>(p.y)[(size_t)token * p.ldy + n] = __float2bfloat16_rn((gate / (1.0f + expf(-gate))) * up);
@@ -283,15 +288,15 @@ int fsie_gemm_skinny(const void* w, const void* x, long long ldx, void* y, long 
     return T <= 8 ? launch_skinny<1, false>(p, none, stream) : launch_skinny<2, false>(p, none, stream);
 }
 
-// y[T, N] = silu(x w_gate^T) * (x w_up^T) for w = [gate rows (N); up rows (N)], y bfloat16; else as above.
-int fsie_gemm_skinny_swiglu(const void* w, const void* x, long long ldx, void* y, long long ldy, int T, int N, int K,
-                            cudaStream_t stream) {
+// y[T, N] = silu(x w_gate^T) * (x w_up^T) for w = [gate rows (N); up rows (N)] (bias alike, or null), y bfloat16; else as above.
+int fsie_gemm_skinny_swiglu(const void* w, const void* x, long long ldx, void* y, long long ldy, const void* bias, int T, int N,
+                            int K, cudaStream_t stream) {
     if (T <= 0 || N <= 0) return 0;
     if (T > 16 || K <= 0 || K % SK_CHUNK != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(w) & 15) ||
         (reinterpret_cast<uintptr_t>(x) & 15))
         return ERR_BAD_ARGUMENT;
     SkinnyParams p;
-    p.w = (const bf16*)w; p.x = (const bf16*)x; p.ldx = ldx; p.y = y; p.ldy = ldy; p.bias = nullptr;
+    p.w = (const bf16*)w; p.x = (const bf16*)x; p.ldx = ldx; p.y = y; p.ldy = ldy; p.bias = (const bf16*)bias;
     p.T = T; p.N = N; p.K = K; p.out_f32 = 0; p.relu2 = 0;
     SkinnyRope none = {};
     return T <= 8 ? launch_skinny<1, false, true>(p, none, stream) : launch_skinny<2, false, true>(p, none, stream);

@@ -309,11 +309,18 @@ class Runtime:
                       tag: Optional[str] = None, bias: Optional[torch.Tensor] = None,
                       activation: str = "silu") -> torch.Tensor:
         """silu(x @ gate.T) * (x @ up.T) for the stacked weight [gate rows; up rows]: one fused
-        kernel for steps of few tokens, else the library product and the SwiGLU kernel.  With a
-        `bias` (stacked like the weight) the product adds it and the SwiGLU kernel follows.
+        kernel for steps of few tokens, else the library product and the SwiGLU kernel.  A `bias`
+        (stacked like the weight) is added by the product; of the fused kernels the one of the
+        smallest steps takes it, otherwise the SwiGLU kernel follows.
         `activation` names what the gate passes through (the fused kernels were told at
         `prepare_weight`; the unfused path runs the kernel of gated activations)."""
         if bias is not None:
+            if (self.dtype is torch.bfloat16 and activation == "silu" and gate_up.shape[0] % 2 == 0
+                    and bias.dtype is torch.bfloat16 and self._few_tokens(x, gate_up) is None
+                    and self._tiled(x, gate_up) is None and self._skinny(x, gate_up)):
+                # the product that `linear` would take, with the activation in its epilogue
+                return ops.gemm_skinny_swiglu(gate_up, x, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2,
+                                                                      torch.bfloat16), bias)
             both = self.linear(x, gate_up, bias, None if tag is None else tag + ".gate_up")
             return self._gated(both, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2, both.dtype),
                                activation)

@@ -709,7 +709,7 @@ def gemm_skinny_lib():
         i, ll, p = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_gemm_skinny.argtypes = [p, p, ll, p, ll, p, i, i, i, i, i, p]
         lib.fsie_gemm_skinny.restype = i
-        lib.fsie_gemm_skinny_swiglu.argtypes = [p, p, ll, p, ll, i, i, i, p]
+        lib.fsie_gemm_skinny_swiglu.argtypes = [p, p, ll, p, ll, p, i, i, i, p]
         lib.fsie_gemm_skinny_swiglu.restype = i
         lib.fsie_gemm_skinny_qkv_rope.argtypes = [p, p, ll, p, ll, p, i, i, p, p, i, p, p, p, ll, i,
                                                   i, i, i, p, p]
@@ -782,9 +782,10 @@ def gemm_skinny(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
     return out
 
 
-def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out[T, N] = silu(x @ gate.T) * (x @ up.T) for T <= 16 and weight = [gate rows (N); up rows (N)]: the bits of
-    `gemm_skinny` and `swiglu` one after the other, in one launch."""
+def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor,
+                       bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """out[T, N] = silu(x @ gate.T) * (x @ up.T) for T <= 16 and weight = [gate rows (N); up rows (N)], each product
+    with its half of `bias` where there is one: the bits of `gemm_skinny` and `swiglu` one after the other, in one launch."""
     gemm_skinny_lib()
     _need(weight, torch.bfloat16, "weight")
     _need(x, torch.bfloat16, "x", contiguous=False)
@@ -795,7 +796,11 @@ def gemm_skinny_swiglu(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor)
         raise KernelError("gemm_skinny_swiglu: x does not fit the weight, or the sizes are beyond the kernel")
     if out.shape[0] != tokens or out.shape[1] != n or out.stride(1) != 1:
         raise KernelError("gemm_skinny_swiglu: out does not fit")
-    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(weight, x, x.stride(0), out, out.stride(0), tokens, n,
+    if bias is not None:
+        _need(bias, torch.bfloat16, "bias")
+        if bias.numel() != 2 * n:
+            raise KernelError("gemm_skinny_swiglu: the bias does not fit the weight")
+    _check(_gemm_skinny.fsie_gemm_skinny_swiglu(weight, x, x.stride(0), out, out.stride(0), bias, tokens, n,
                                                 k, _stream()), "gemm_skinny_swiglu")
     return out
 
