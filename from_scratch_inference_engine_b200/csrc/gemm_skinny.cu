@@ -23,6 +23,8 @@ constexpr int SK_ROWS = 16;          // rows of w per block (MMA M)
 constexpr int SK_WARPS = 16;
 constexpr int SK_CHUNK = 32;         // k elements per warp and step: 4 lanes x 16 bytes per row
 constexpr int SK_AHEAD = 4;          // chunks whose weights a warp has asked for (a ring of 4 KB per warp)
+constexpr int SK_DEEP = 8;           // the same where an SM has one block at most and a warp more chunks than SK_AHEAD
+constexpr int SK_SMS = 148;
 
 struct SkinnyParams {
     const bf16* w; const bf16* x; long long ldx;
@@ -62,42 +64,60 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // GATED: w holds N gate rows and then N up rows, the block's 16 rows are 8 gate rows and the 8 up rows of the
 // same outputs, and the epilogue is silu(gate) * up on the two as bfloat16 would store them: the bits of a
 // product and the SwiGLU kernel behind it, without that launch (1 token of 8,960 x 1,536 14.0 -> 11.4 us, 16 tokens of 2,816 x 2,048 11.4 -> 8.6).
-template <int TT, bool ROPE, bool GATED>
-__global__ void __launch_bounds__(32 * SK_WARPS, 2)       // two blocks per SM: 64 registers at most
+// A matrix of more tiles of 16 rows than the GPU holds blocks has the blocks stay and go on to their next tile: the ring runs on
+// across tiles, where a block of its own for every tile of, say, 8,960 x 1,536 (three chunks per warp) was asked, waited and gone
+// (SK_STAY_TIME).  With one block per SM or less the ring is twice as deep (SK_DEEP_TIME).
+// Neither changes which warp adds up what: the same bits.
+template <int TT, bool ROPE, bool GATED, int AHEAD>
+__global__ void __launch_bounds__(32 * SK_WARPS, AHEAD == SK_AHEAD ? 2 : 1)       // two blocks per SM: 64 registers at most
 gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     extern __shared__ __align__(16) unsigned char sk_ring[];
-    __shared__ float red[SK_WARPS * SK_ROWS * 8 * TT];            // [warp][16 rows][8 * TT]
+    constexpr int RED = SK_WARPS * SK_ROWS * 8 * TT;              // [warp][16 rows][8 * TT]
+    __shared__ float reds[ROPE ? 1 : 2][RED];                     // a tile's, while the tile before is still added up
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int chunks = p.K / SK_CHUNK;
-    // rows of w behind rows 0-7 and 8-15 of the block's tile
+    // rows of w behind rows 0-7 and 8-15 of a tile (clamped at the matrix's end; those results are not stored)
+    constexpr int TILE_ROWS = GATED ? SK_ROWS / 2 : SK_ROWS;
+    const int tiles = (p.N + TILE_ROWS - 1) / TILE_ROWS;
     int row0, row8;
-    if (ROPE) {
-        const int per_head = rope.head_dim / 16;                  // blocks per head
-        const int head = blockIdx.x / per_head, d0 = (blockIdx.x - head * per_head) * 8;
-        row0 = head * rope.head_dim + d0;
-        row8 = row0 + rope.head_dim / 2;
-    } else if (GATED) {
-        row0 = blockIdx.x * (SK_ROWS / 2);
-        row8 = p.N + row0;
-    } else {
-        row0 = blockIdx.x * SK_ROWS;
-        row8 = row0 + 8;
-    }
-    // this lane's two rows (clamped at the matrix's end; those results are not stored)
-    const bf16* w_lo = p.w + (size_t)min(row0 + g, p.N - 1) * p.K + 8 * t;
-    const bf16* w_hi = p.w + (size_t)min(row8 + g, (GATED ? 2 : 1) * p.N - 1) * p.K + 8 * t;
-    unsigned char* mine = sk_ring + (size_t)warp * SK_AHEAD * 1024 + lane * 16;     // slot s: + s * 1024; second row: + 512
+    auto rows_of = [&](int tile) {
+        if (ROPE) {
+            const int per_head = rope.head_dim / 16;              // blocks per head
+            const int head = tile / per_head, d0 = (tile - head * per_head) * 8;
+            row0 = head * rope.head_dim + d0;
+            row8 = row0 + rope.head_dim / 2;
+        } else {
+            row0 = tile * TILE_ROWS;
+            row8 = GATED ? p.N + row0 : row0 + 8;
+        }
+    };
+    unsigned char* mine = sk_ring + (size_t)warp * AHEAD * 1024 + lane * 16;        // slot s: + s * 1024; second row: + 512
 
-    auto ask = [&](int slot, int c) {                             // this lane's 32 bytes of chunk c
-        if (c < chunks) {
-            cp_async_16(mine + slot * 1024, w_lo + c * SK_CHUNK);
-            cp_async_16(mine + slot * 1024 + 512, w_hi + c * SK_CHUNK);
+    // the next chunk to ask for: of which tile, which chunk, this lane's two rows there
+    int ask_tile = blockIdx.x, ask_c = warp;
+    const bf16 *w_lo, *w_hi;
+    auto ask_rows = [&]() {
+        rows_of(ask_tile);
+        w_lo = p.w + (size_t)min(row0 + g, p.N - 1) * p.K + 8 * t;
+        w_hi = p.w + (size_t)min(row8 + g, (GATED ? 2 : 1) * p.N - 1) * p.K + 8 * t;
+    };
+    ask_rows();
+    auto ask = [&](int slot) {                                    // this lane's 32 bytes of it
+        if (ask_c < chunks) {
+            cp_async_16(mine + slot * 1024, w_lo + ask_c * SK_CHUNK);
+            cp_async_16(mine + slot * 1024 + 512, w_hi + ask_c * SK_CHUNK);
+            ask_c += SK_WARPS;
+            if (!ROPE && ask_c >= chunks && ask_tile + (int)gridDim.x < tiles) {
+                ask_tile += gridDim.x;
+                ask_c = warp;
+                ask_rows();
+            }
         }
         cp_async_commit();                                        // one group per slot, also when empty
     };
 #pragma unroll
-    for (int j = 0; j < SK_AHEAD; ++j) ask(j, warp + j * SK_WARPS);    // weights do not depend on the kernel before
+    for (int j = 0; j < AHEAD; ++j) ask(j);                       // weights do not depend on the kernel before
     // Nor does what the epilogue's rotation needs: the token's position and slot were staged before
     // the step, the table and the bias are constants.  A thread of the epilogue owns one rotation
     // pair of one token (the block has more threads than such pairs) and fetches its angle now.
@@ -106,6 +126,7 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     int early_pos = 0, early_slot = -1;
     float early_cos = 1.f, early_sin = 0.f, early_bias_lo = 0.f, early_bias_hi = 0.f;
     if (ROPE) {
+        rows_of(blockIdx.x);
         const int token = threadIdx.x >> 3, r = threadIdx.x & 7;
         if (threadIdx.x < 8 * TP && token < p.T) {
             const int per_head = rope.head_dim / 16;
@@ -119,10 +140,6 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
             if (p.bias) { early_bias_lo = __bfloat162float(p.bias[row0 + r]); early_bias_hi = __bfloat162float(p.bias[row8 + r]); }
         }
     }
-    if (GATED && p.bias && threadIdx.x < 8 * TP) {                // the pair of outputs this thread finishes
-        const int n = min(row0 + (int)(threadIdx.x & 7), p.N - 1);
-        early_bias_lo = __bfloat162float(p.bias[n]); early_bias_hi = __bfloat162float(p.bias[p.N + n]);
-    }
     grid_dependency_wait();
     grid_dependents_go();
     // x: token 8 n + g, the same 16 bytes of k as this lane's weights (tokens beyond T read as zero);
@@ -131,28 +148,12 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
 #pragma unroll
     for (int n = 0; n < TT; ++n) x_of[n] = (8 * n + g < p.T) ? p.x + (size_t)(8 * n + g) * p.ldx + 8 * t : nullptr;
 
-    float acc[TT][4];
-#pragma unroll
-    for (int n = 0; n < TT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    int slot = 0;
-    auto multiply = [&](const uint4 (&b)[TT], int c) {              // chunk c of the weights (this slot) times the tokens' chunk
-        cp_async_wait<SK_AHEAD - 1>();                            // the oldest group - this slot - has landed
-        const uint4 a_lo = *reinterpret_cast<const uint4*>(mine + slot * 1024);
-        const uint4 a_hi = *reinterpret_cast<const uint4*>(mine + slot * 1024 + 512);
-#pragma unroll
-        for (int n = 0; n < TT; ++n) {
-            mma_16x8x16(acc[n], a_lo.x, a_hi.x, a_lo.y, a_hi.y, b[n].x, b[n].y);
-            mma_16x8x16(acc[n], a_lo.z, a_hi.z, a_lo.w, a_hi.w, b[n].z, b[n].w);
-        }
-        ask(slot, c + SK_WARPS * SK_AHEAD);                       // refill what has just been used
-        slot = slot + 1 == SK_AHEAD ? 0 : slot + 1;
-    };
     // the x values of four of the warp's chunks are asked for together: a trip to L2 per four chunks
     // instead of one per chunk (two chunks with more than 8 tokens: the registers of four would
-    // cost the second block that an SM holds)
+    // cost the second block that an SM holds); where a warp has no more than that they stay for all tiles
     constexpr int X_AHEAD = TT == 1 ? 4 : 2;
-    for (int c0 = warp; c0 < chunks; c0 += X_AHEAD * SK_WARPS) {
-        uint4 b[X_AHEAD][TT];
+    uint4 b[X_AHEAD][TT];
+    auto ask_x = [&](int c0) {
 #pragma unroll
         for (int j = 0; j < X_AHEAD; ++j) {
             const int c = c0 + j * SK_WARPS;
@@ -160,23 +161,47 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
             for (int n = 0; n < TT; ++n)
                 b[j][n] = (c < chunks && x_of[n]) ? *reinterpret_cast<const uint4*>(x_of[n] + c * SK_CHUNK) : make_uint4(0, 0, 0, 0);
         }
+    };
+    const bool x_stays = !ROPE && chunks <= X_AHEAD * SK_WARPS;
+    if (x_stays) ask_x(warp);
+    int slot = 0, turn = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, turn ^= 1) {
+    float acc[TT][4];
+#pragma unroll
+    for (int n = 0; n < TT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    if (GATED && p.bias && threadIdx.x < 8 * TP) {                // of the pair of outputs this thread finishes
+        const int n = min(tile * TILE_ROWS + (int)(threadIdx.x & 7), p.N - 1);
+        early_bias_lo = __bfloat162float(p.bias[n]); early_bias_hi = __bfloat162float(p.bias[p.N + n]);
+    }
+    for (int c0 = warp; c0 < chunks; c0 += X_AHEAD * SK_WARPS) {
+        if (!x_stays) ask_x(c0);
 #pragma unroll
         for (int j = 0; j < X_AHEAD; ++j) {
-            const int c = c0 + j * SK_WARPS;
-            if (c < chunks) multiply(b[j], c);
+            if (c0 + j * SK_WARPS >= chunks) break;
+            cp_async_wait<AHEAD - 1>();                           // the oldest group - this slot - has landed
+            const uint4 a_lo = *reinterpret_cast<const uint4*>(mine + slot * 1024);
+            const uint4 a_hi = *reinterpret_cast<const uint4*>(mine + slot * 1024 + 512);
+#pragma unroll
+            for (int n = 0; n < TT; ++n) {
+                mma_16x8x16(acc[n], a_lo.x, a_hi.x, a_lo.y, a_hi.y, b[j][n].x, b[j][n].y);
+                mma_16x8x16(acc[n], a_lo.z, a_hi.z, a_lo.w, a_hi.w, b[j][n].z, b[j][n].w);
+            }
+            ask(slot);                                            // refill what has just been used
+            slot = slot + 1 == AHEAD ? 0 : slot + 1;
         }
     }
-    cp_async_wait<0>();
     // acc[n]: rows g (0, 1) and g + 8 (2, 3), tokens 8 n + 2 t and 8 n + 2 t + 1
+    float* red = reds[ROPE ? 0 : turn];
 #pragma unroll
     for (int n = 0; n < TT; ++n) {
-        float* mine = red + ((size_t)warp * SK_ROWS) * TP + 8 * n + 2 * t;
-        mine[(size_t)g * TP] = acc[n][0];
-        mine[(size_t)g * TP + 1] = acc[n][1];
-        mine[(size_t)(g + 8) * TP] = acc[n][2];
-        mine[(size_t)(g + 8) * TP + 1] = acc[n][3];
+        float* part = red + ((size_t)warp * SK_ROWS) * TP + 8 * n + 2 * t;
+        part[(size_t)g * TP] = acc[n][0];
+        part[(size_t)g * TP + 1] = acc[n][1];
+        part[(size_t)(g + 8) * TP] = acc[n][2];
+        part[(size_t)(g + 8) * TP + 1] = acc[n][3];
     }
     __syncthreads();
+    const int first = tile * TILE_ROWS;
     if constexpr (ROPE) {
         const int half = rope.head_dim / 2;
         const int per_head = rope.head_dim / 16;
@@ -223,7 +248,7 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     } else if constexpr (GATED) {
         for (int e = threadIdx.x; e < 8 * TP; e += blockDim.x) {
             const int token = e >> 3, r = e & 7;
-            const int n = row0 + r;
+            const int n = first + r;
             if (token >= p.T || n >= p.N) continue;
             float gate = 0.f, up = 0.f;
 #pragma unroll
@@ -239,7 +264,7 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     } else {
     for (int e = threadIdx.x; e < SK_ROWS * TP; e += blockDim.x) {
         const int token = e / SK_ROWS, r = e - token * SK_ROWS;   // consecutive threads: consecutive outputs of a token
-        const int n = row0 + r;
+        const int n = first + r;
         if (token >= p.T || n >= p.N) continue;
         float sum = 0.f;
 #pragma unroll
@@ -253,18 +278,31 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
         else reinterpret_cast<bf16*>(p.y)[(size_t)token * p.ldy + n] = __float2bfloat16_rn(sum);
     }
     }
+    }
+    cp_async_wait<0>();
+}
+
+template <int TT, bool ROPE, bool GATED, int AHEAD>
+static int launch_skinny_ring(const SkinnyParams& p, const SkinnyRope& rope, int blocks, cudaStream_t stream) {
+    constexpr size_t smem = (size_t)SK_WARPS * AHEAD * 1024;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TT, ROPE, GATED, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return launch_dependent(gemm_skinny_kernel<TT, ROPE, GATED, AHEAD>, dim3(blocks), dim3(32 * SK_WARPS), smem, stream, p, rope);
 }
 
 template <int TT, bool ROPE, bool GATED = false>
 static int launch_skinny(const SkinnyParams& p, const SkinnyRope& rope, cudaStream_t stream) {
-    constexpr size_t smem = (size_t)SK_WARPS * SK_AHEAD * 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TT, ROPE, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
+    const int tiles = (p.N + (GATED ? SK_ROWS / 2 : SK_ROWS) - 1) / (GATED ? SK_ROWS / 2 : SK_ROWS);
+    if constexpr (!ROPE) {
+        if (tiles <= SK_SMS && p.K > SK_CHUNK * SK_WARPS * SK_AHEAD)
+            return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP>(p, rope, tiles, stream);
+        return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD>(p, rope, tiles < 2 * SK_SMS ? tiles : 2 * SK_SMS, stream);
     }
-    return launch_dependent(gemm_skinny_kernel<TT, ROPE, GATED>, dim3((p.N + (GATED ? SK_ROWS / 2 : SK_ROWS) - 1) / (GATED ? SK_ROWS / 2 : SK_ROWS)), dim3(32 * SK_WARPS), smem, stream, p, rope);
+    return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD>(p, rope, tiles, stream);
 }
 
 }  // namespace fsie
