@@ -252,8 +252,9 @@ conv_norm_rotate_vec_kernel(const T* __restrict__ proj, int ld, int items, const
         for (int i = 0; i < 4; ++i) {
             if (d0 + 2 * i >= rot_dims) continue;
             const float a = y[2 * i], b = y[2 * i + 1];
-            y[2 * i] = a * co[i] - b * si[i];
-            y[2 * i + 1] = b * co[i] + a * si[i];
+            // which product is rounded is written out: the general kernel's, and so its bits
+            y[2 * i] = fmaf(a, co[i], -__fmul_rn(b, si[i]));
+            y[2 * i + 1] = fmaf(b, co[i], __fmul_rn(a, si[i]));
         }
         if (is_q) {
             store8(q_out + (size_t)t * wq + c0, y);
