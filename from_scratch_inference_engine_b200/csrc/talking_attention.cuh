@@ -36,7 +36,6 @@ struct TalkingArgs {
     float* part_stats;             // [tiles][nsplit][TA_ROWS][2]
     float* part_out;               // [nsplit][tokens][heads * vdim]
     int tokens;
-    int ahead;                     // values have a buffer of their own and are asked for together with the keys
 };
 
 __device__ __forceinline__ void load2(const float* p, float& a, float& b) {
@@ -53,14 +52,14 @@ struct TalkingLayout {
     int dim8, vdim8, q_ld, kv_ld;
     size_t q_bytes, kv_bytes, p_bytes, talk_bytes, total;
     __host__ __device__ TalkingLayout(int heads, int kv_heads, int dim, int vdim, int key_tile,
-                                      int elem_bytes) {
+                                      int elem_bytes, int rows = TA_ROWS) {
         dim8 = (dim + 7) & ~7;
         vdim8 = (vdim + 7) & ~7;
         q_ld = dim8 + 4;
         kv_ld = (dim8 > vdim8 ? dim8 : vdim8) + 16 / elem_bytes;     // rows 16 bytes apart in banks
-        q_bytes = (size_t)TA_ROWS * q_ld * sizeof(float);
+        q_bytes = (size_t)rows * q_ld * sizeof(float);
         kv_bytes = (size_t)kv_heads * key_tile * kv_ld * elem_bytes;
-        p_bytes = (size_t)TA_ROWS * key_tile * sizeof(float);
+        p_bytes = (size_t)rows * key_tile * sizeof(float);
         talk_bytes = (((size_t)heads * heads * sizeof(float)) + 15) & ~(size_t)15;
         total = q_bytes + kv_bytes + 2 * p_bytes + talk_bytes + 2 * key_tile * sizeof(int);
     }
@@ -105,16 +104,15 @@ __device__ __forceinline__ void copy_tile(T* __restrict__ dst, const T* __restri
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
-// all but the newest `N` of a thread's copies have arrived
-template <int N>
-__device__ __forceinline__ void talking_copies_done() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void talking_copies_done() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Warp w owns heads w, w + 8, ... (HS = 8 / TOK of them at most) and, of each, the tile's TOK
 // tokens: rows that share their keys and values, so one load of a key or value serves TOK rows.
 // Lane l owns keys l (+ 32) of a tile for the scores and value columns 2 l, 2 l + 1 (+ 64 c).
 // A split tile's block has one or two tiles of keys: it is a chain of trips to memory.  The lists, the first tile's pages
-// and the mixing matrix are read before the kernel before has finished, and by the second walk also the queries, keys
-// and values, which the first walk only read (4 requests of 1,024 keys: TA_TIME).
+// and the mixing matrix are read before the kernel before has finished, and the second walk gets as far as its first tile's
+// scores and values then: the first walk only read the queries, keys and values.  Shared memory is laid out for the
+// tile's own rows, so that blocks of both walks fit an SM (4 requests of 1,024 keys, the three launches: 56 us, TA_TIME now).
 template <typename T, int TOK, int VC2, int KPL>
 __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const TalkingArgs a) {
     constexpr int HS = 8 / TOK;
@@ -139,15 +137,14 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
     const int u_begin = min(n_keys, split * per_split * TK);
     const int u_end = min(n_keys, (split + 1) * per_split * TK);
 
-    const TalkingLayout L(H, G, dim, vdim, TK, (int)sizeof(T));
+    const TalkingLayout L(H, G, dim, vdim, TK, (int)sizeof(T), TOK * H);
     float* qs = reinterpret_cast<float*>(smem_raw);
     T* kv = reinterpret_cast<T*>(smem_raw + L.q_bytes);
     float* P = reinterpret_cast<float*>(smem_raw + L.q_bytes + L.kv_bytes);
-    float* P2 = P + TA_ROWS * TK;
-    float* talk = P2 + TA_ROWS * TK;
+    float* P2 = P + TOK * H * TK;
+    float* talk = P2 + TOK * H * TK;
     int* key_page = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(talk) + L.talk_bytes);
     int* key_off = key_page + TK;
-    T* vbuf = a.ahead ? reinterpret_cast<T*>(smem_raw + L.total) : kv;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* k_pages = reinterpret_cast<const T*>(a.k_pages);
@@ -174,7 +171,7 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
         copy_tile<T>(kv, k_pages, key_page, key_off, G, TK, dim, L.dim8, L.kv_ld, a.page_stride, a.page_size, warp, lane);
     };
     const auto copy_values = [&]() {
-        copy_tile<T>(vbuf, v_pages, key_page, key_off, G, TK, vdim, L.vdim8, L.kv_ld, a.page_stride, a.page_size, warp, lane);
+        copy_tile<T>(kv, v_pages, key_page, key_off, G, TK, vdim, L.vdim8, L.kv_ld, a.page_stride, a.page_size, warp, lane);
     };
     const bool early = a.mode == 2;                     // what the keys' writer left is older than the kernel before
     for (int idx = threadIdx.x; idx < H * H; idx += blockDim.x) talk[idx] = a.talk[idx];
@@ -184,21 +181,13 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
         grid_dependents_go();                           // (not before the wait: the second walk's early reads rest on it)
     } else {
         __syncthreads();                                // the first tile's pages
-        if (u_begin < u_end) {
-            copy_keys();
-            if (a.ahead) copy_values();
-        }
+        if (u_begin < u_end) copy_keys();
     }
     // q rows [tok * H + h], zero beyond dim and beyond the tile's tokens
     for (int idx = threadIdx.x; idx < TOK * H * L.dim8; idx += blockDim.x) {
         const int r = idx / L.dim8, d = idx - r * L.dim8;
         qs[r * L.q_ld + d] = (r < R && d < dim) ? a.q[((size_t)token0 * H + r) * dim + d] : 0.f;
     }
-    if (early) {
-        grid_dependency_wait();
-        grid_dependents_go();
-    }
-
     float row_max[HS][TOK], row_sum[HS][TOK], acc[HS][TOK][VC2][2];
 #pragma unroll
     for (int hs = 0; hs < HS; ++hs)
@@ -210,7 +199,7 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
             for (int c = 0; c < VC2; ++c) acc[hs][t][c][0] = acc[hs][t][c][1] = 0.f;
         }
 
-    if (a.mode == 2) {
+    const auto read_statistics = [&]() {
         // maximum and sum over all key ranges, from what the first launch left: a lane reads a range's, the sum is
         // taken range by range
         const float* stats = a.part_stats + (size_t)tile * a.nsplit * TA_ROWS * 2;
@@ -251,9 +240,14 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
                     }
                 }
         }
-    }
+    };
 
     const int first_pass = a.mode == 2 ? 1 : 0, last_pass = a.mode == 1 ? 0 : 1;
+    // whether the tile's token t sees this lane's key in the tile of n keys from u0
+    const auto sees = [&](int u0, int n, int t, int kp) {
+        const int u = u0 + lane + 32 * kp, j = u < kept ? u : lo + (u - kept), p_i = p_first + t;
+        return lane + 32 * kp < n && j <= p_i && (a.window <= 0 || p_i - j < a.window || j < a.keep_first);
+    };
     for (int pass = first_pass; pass <= last_pass; ++pass) {
         for (int u0 = u_begin; u0 < u_end; u0 += TK) {
             const int n = min(TK, u_end - u0);
@@ -262,10 +256,8 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
                 if (u0 != u_begin || pass != first_pass) find_keys(u0);
                 __syncthreads();
                 copy_keys();
-                if (pass == 1 && a.ahead) copy_values();
             }
-            if (pass == 1 && a.ahead) talking_copies_done<1>();
-            else talking_copies_done<0>();
+            talking_copies_done();
             __syncthreads();
 #pragma unroll
             for (int hs = 0; hs < HS; ++hs) {
@@ -295,15 +287,11 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
 #pragma unroll
                 for (int t = 0; t < TOK; ++t) {
                     if (t >= n_tok) continue;
-                    const int p_i = p_first + t;
                     bool see[KPL];
                     float tile_max = -INFINITY;
 #pragma unroll
                     for (int kp = 0; kp < KPL; ++kp) {
-                        const int u = u0 + lane + 32 * kp;
-                        const int j = u < kept ? u : lo + (u - kept);
-                        see[kp] = lane + 32 * kp < n && j <= p_i &&
-                            (a.window <= 0 || p_i - j < a.window || j < a.keep_first);
+                        see[kp] = sees(u0, n, t, kp);
                         s[t][kp] = see[kp] ? s[t][kp] * a.scale : -INFINITY;
                         tile_max = fmaxf(tile_max, s[t][kp]);
                     }
@@ -317,17 +305,36 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
                             row_max[hs][t] = m_new;
                         }
                     } else {
-                        const float inv = 1.0f / row_sum[hs][t];
 #pragma unroll
-                        for (int kp = 0; kp < KPL; ++kp)
-                            P[(t * H + h) * TK + lane + 32 * kp] =
-                                see[kp] ? expf(s[t][kp] - row_max[hs][t]) * inv : 0.f;
+                        for (int kp = 0; kp < KPL; ++kp) P[(t * H + h) * TK + lane + 32 * kp] = s[t][kp];
                     }
                 }
             }
             if (pass == 0) continue;
+            __syncthreads();                             // everybody is done with the keys
+            copy_values();
+            if (early && u0 == u_begin) {
+                grid_dependency_wait();
+                grid_dependents_go();
+                read_statistics();
+            }
+            // weights from the scores that this lane has just left there
+#pragma unroll
+            for (int hs = 0; hs < HS; ++hs) {
+                const int h = warp + TA_WARPS * hs;
+                if (h >= H) continue;
+#pragma unroll
+                for (int t = 0; t < TOK; ++t) {
+                    if (t >= n_tok) continue;
+                    const float inv = 1.0f / row_sum[hs][t];
+#pragma unroll
+                    for (int kp = 0; kp < KPL; ++kp) {
+                        float* at = P + (t * H + h) * TK + lane + 32 * kp;
+                        *at = sees(u0, n, t, kp) ? expf(*at - row_max[hs][t]) * inv : 0.f;
+                    }
+                }
+            }
             __syncthreads();                             // P holds every head's weights of this tile
-            if (!a.ahead) copy_values();
             for (int idx = threadIdx.x; idx < R * TK; idx += blockDim.x) {
                 const int r = idx / TK, jj = idx - r * TK;
                 const int t = r / H, h = r - t * H;
@@ -337,13 +344,13 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
                 for (int h2 = 0; h2 < H; ++h2) m += mix[h2] * col[h2 * TK];
                 P2[idx] = m;
             }
-            talking_copies_done<0>();
+            talking_copies_done();
             __syncthreads();
 #pragma unroll
             for (int hs = 0; hs < HS; ++hs) {
                 const int h = warp + TA_WARPS * hs;
                 if (h >= H) continue;
-                const T* vg = vbuf + (size_t)(h / group) * TK * L.kv_ld;
+                const T* vg = kv + (size_t)(h / group) * TK * L.kv_ld;
                 for (int jj = 0; jj < TK; jj += 4) {
                     if (jj >= n) break;
                     float4 p[TOK];
@@ -369,6 +376,10 @@ __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const 
         }
     }
 
+    if (early && u_begin >= u_end) {                    // a range without keys
+        grid_dependency_wait();
+        grid_dependents_go();
+    }
     if (gone) atomicExch(a.error, 3);
     if (a.mode == 1) {
         float* stats = a.part_stats + ((size_t)tile * a.nsplit + split) * TA_ROWS * 2;
@@ -429,18 +440,10 @@ inline int talking_key_tile(int heads, int kv_heads, int dim, int vdim, int elem
     return 0;
 }
 
-// Values get a buffer of their own where every block has an SM to itself anyway (148 of them): a second block on the SM hides
-// more than that where there are more.
-constexpr int TA_AHEAD_BLOCKS = 148;
-constexpr size_t TA_AHEAD_BYTES = 220 * 1024;
-
 template <typename T, int TOK, int VC2>
-int talking_attention_launch_tile(TalkingArgs a, int num_tiles, int key_tile, size_t smem,
+int talking_attention_launch_tile(const TalkingArgs& a, int num_tiles, int key_tile, size_t smem,
                                   cudaStream_t stream) {
     const dim3 grid(num_tiles, a.nsplit);
-    const size_t both = smem + TalkingLayout(a.heads, a.kv_heads, a.dim, a.vdim, key_tile, (int)sizeof(T)).kv_bytes;
-    a.ahead = a.mode != 1 && (long long)num_tiles * a.nsplit <= TA_AHEAD_BLOCKS && both <= TA_AHEAD_BYTES;
-    if (a.ahead) smem = both;
     if (key_tile == 64) {
         cudaFuncSetAttribute(talking_attention_kernel<T, TOK, VC2, 2>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -471,7 +474,8 @@ int talking_attention_launch(TalkingArgs a, int num_tiles, cudaStream_t stream) 
     if (a.vdim > 256) return ERR_UNSUPPORTED;
     const int key_tile = talking_key_tile(a.heads, a.kv_heads, a.dim, a.vdim, (int)sizeof(T));
     if (key_tile == 0) return ERR_UNSUPPORTED;
-    const size_t smem = TalkingLayout(a.heads, a.kv_heads, a.dim, a.vdim, key_tile, (int)sizeof(T)).total;
+    const size_t smem = TalkingLayout(a.heads, a.kv_heads, a.dim, a.vdim, key_tile, (int)sizeof(T),
+                                      a.tile_tokens * a.heads).total;
     if (a.nsplit > 1 && (!a.part_stats || !a.part_out)) return ERR_BAD_ARGUMENT;
     const int first = a.nsplit > 1 ? 1 : 0, last = a.nsplit > 1 ? 2 : 0;
     for (int mode = first; mode <= last; ++mode) {
