@@ -650,17 +650,23 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
         const bf16* __restrict__ x, long long x_ld, const bf16* __restrict__ w, bf16* __restrict__ out,
         long long out_ld, const int* __restrict__ offsets, const int* __restrict__ sorted,
         const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ meta,
-        int top, int n, int k, int gate_kind) {
+        int top, int n, int k, int gate_kind, int early) {
     constexpr bool GATED = MODE == 1, FIRST = MODE != 0;
     constexpr int COLS = GATED ? 16 : 32;                    // outputs per row and item
     extern __shared__ __align__(128) unsigned char few_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    grid_dependency_wait();
-    grid_dependents_go();
+    // early: the lists are older than the kernel before, and the first slots of w are asked for while it still runs
+    if (MODE != 0 || !early) {
+        grid_dependency_wait();
+        grid_dependents_go();
+    }
     const int tiles = meta[0];
     // neighbouring items are the tiles of the same columns: an expert's further tiles find its rows in L2
     const int items = tiles * ((n + COLS - 1) / COLS);
-    if ((int)blockIdx.x >= items) return;
+    if ((int)blockIdx.x >= items) {
+        if (MODE == 0 && early) grid_dependency_wait();
+        return;
+    }
     const int per = (k + FEW_K - 1) / FEW_K;                 // slots per item
     const int step_tile = gridDim.x % tiles, step_n0 = (gridDim.x / tiles) * COLS;
     auto advance = [&](int& tile, int& n0) {                 // the block's next item
@@ -686,15 +692,17 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
         const bool met = row < min(MOE_FEW_TILE, offsets[e + 1] - r0);
         xr = met ? x + (size_t)(FIRST ? sorted[r0 + row] / top : r0 + row) * x_ld + piece * 8 : nullptr;
     };
-    auto ask = [&]() {
+    auto ask = [&](bool of_w = true, bool of_x = true) {
         const int k0 = ask_j * FEW_K;
         if (ask_n0 < n && k0 + piece * 8 < k) {
             unsigned char* slot = few_smem + ask_slot * FEW_SLOT;
+            if (of_w) {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) mm_cp16(slot + few_place(16 * i + row, piece), wr[i] + k0, true);
-            if (xr) mm_cp16(slot + few_place(FEW_ROWS + row, piece), xr + k0, true);
+                for (int i = 0; i < 2; ++i) mm_cp16(slot + few_place(16 * i + row, piece), wr[i] + k0, true);
+            }
+            if (of_x && xr) mm_cp16(slot + few_place(FEW_ROWS + row, piece), xr + k0, true);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");            // one group per slot, also when empty
+        if (of_x) asm volatile("cp.async.commit_group;" ::: "memory");  // one group per slot, also when empty
         ask_slot = ask_slot + 1 == FEW_SLOTS ? 0 : ask_slot + 1;
         if (++ask_j == per) {
             ask_j = 0;
@@ -704,8 +712,16 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
     };
     static_assert(FEW_THREADS == MOE_FEW_TILE * FEW_PIECES && FEW_ROWS == 2 * MOE_FEW_TILE, "a thread's pieces");
     point();
+    if (MODE == 0 && early) {
 #pragma unroll
-    for (int j = 0; j < FEW_SLOTS - 1; ++j) ask();
+        for (int j = 0; j < FEW_SLOTS - 1; ++j) ask(true, false);
+        grid_dependency_wait();
+        grid_dependents_go();
+        ask_tile = blockIdx.x % tiles; ask_n0 = (blockIdx.x / tiles) * COLS; ask_j = ask_slot = 0;     // once more for x
+        point();
+    }
+#pragma unroll
+    for (int j = 0; j < FEW_SLOTS - 1; ++j) ask(MODE != 0 || !early, true);
 
     // ---- multiplying: warp = (16 rows of w, 8 rows of x)
     const int half = warp & 1, eight = warp >> 1;
@@ -868,7 +884,7 @@ static int allow_smem(F* kernel, size_t bytes, bool& done) {
 template <int MODE>
 static int launch_few(const void* x, long long x_ld, const void* w, void* out, long long out_ld, const int* offsets,
                       const int* sorted, const int* tile_expert, const int* tile_row0, const int* meta, int tiles,
-                      int top, int n, int k, int gate_kind, int dtype, cudaStream_t stream) {
+                      int top, int n, int k, int gate_kind, int dtype, int early, cudaStream_t stream) {
     static bool allowed[2] = {false, false};
     if (dtype == DTYPE_F32) {
         if (int e = allow_smem(moe_product_few_f32_kernel<MODE>, FEW32_SMEM, allowed[0])) return e;
@@ -886,7 +902,7 @@ static int launch_few(const void* x, long long x_ld, const void* w, void* out, l
     const long long most = (long long)tiles * ((n + cols - 1) / cols);
     return launch_dependent(moe_product_few_kernel<MODE>, dim3((unsigned)(most < 3 * sms ? most : 3 * sms)),
                             dim3(FEW_THREADS), FEW_SMEM, stream, (const bf16*)x, x_ld, (const bf16*)w, (bf16*)out,
-                            out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind);
+                            out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind, early);
 }
 
 // -------------------------------------------------------------------------------- combine
@@ -1044,7 +1060,7 @@ int fsie_moe_gather(const void* x, long long x_ld, const int* sorted, const int*
 int fsie_moe_product(const void* x, long long x_ld, const void* w, void* out, long long out_ld,
                      const int* offsets, const int* sorted, const int* tile_expert, const int* tile_row0,
                      const int* meta, int pairs, int experts, int top, int n, int k, int gated, int gate_kind,
-                     int dtype, int tile, cudaStream_t stream) {
+                     int dtype, int tile, int early, cudaStream_t stream) {
     if (pairs <= 0 || n <= 0) return 0;
     if (k <= 0 || experts <= 0 || top <= 0 || gated < 0 || gated > 2) return ERR_BAD_ARGUMENT;
     if (tile == MOE_FEW_TILE) {
@@ -1053,7 +1069,7 @@ int fsie_moe_product(const void* x, long long x_ld, const void* w, void* out, lo
             return ERR_BAD_ARGUMENT;
 #define FSIE_MOE_FEW(M)                                                                                           \
         launch_few<M>(x, x_ld, w, out, out_ld, offsets, sorted, tile_expert, tile_row0, meta, pairs / tile + experts, \
-                      top, n, k, gate_kind, dtype, stream)
+                      top, n, k, gate_kind, dtype, early, stream)
         return gated == 1 ? FSIE_MOE_FEW(1) : (gated == 2 ? FSIE_MOE_FEW(2) : FSIE_MOE_FEW(0));
 #undef FSIE_MOE_FEW
     }

@@ -1896,7 +1896,7 @@ def routed():
         lib.fsie_moe_route_align.argtypes = [p, p, p, p, p, i, i, i, i, i, f, i, i, i, i, i, p, p, p, p, p, p]
         lib.fsie_moe_route_align_tokens.argtypes = []
         lib.fsie_moe_gather.argtypes = [p, ll, p, p, i, i, p, i, i, p]
-        lib.fsie_moe_product.argtypes = [p, ll, p, p, ll, p, p, p, p, p, i, i, i, i, i, i, i, i, i, p]
+        lib.fsie_moe_product.argtypes = [p, ll, p, p, ll, p, p, p, p, p, i, i, i, i, i, i, i, i, i, i, p]
         lib.fsie_moe_combine.argtypes = [p, p, p, p, p, i, i, i, p, i, p, ll, i, p]
         for name in ("fsie_moe_tile_rows", "fsie_moe_few_tile_rows", "fsie_moe_route", "fsie_moe_align",
                      "fsie_moe_route_align", "fsie_moe_route_align_tokens", "fsie_moe_gather", "fsie_moe_product", "fsie_moe_combine"):
@@ -2136,12 +2136,14 @@ def moe_gather(x: torch.Tensor, lists, tile: int, top: int, out: torch.Tensor) -
 
 
 def moe_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, lists, pairs: int, top: int,
-                gated: bool, activation: str = "silu", first: Optional[bool] = None, tile: int = 0) -> torch.Tensor:
+                gated: bool, activation: str = "silu", first: Optional[bool] = None, tile: int = 0,
+                early: bool = False) -> torch.Tensor:
     """The experts' products over the sorted pairs (`tile`: what the lists were made with).  gated: weight [experts, 2 n, k] (gate rows, then up
     rows), x [tokens, k] read at pair // top, out [pairs, n] = f(gate) * up in sorted order.  Not gated:
     weight [experts, n, k], x [pairs, k] in sorted order, out [pairs, n] at each pair's own row - or,
     `first` (an expert without a gate: its first product), x [tokens, k] read at pair // top and
-    out [pairs, n] = f(x w^T) in sorted order."""
+    out [pairs, n] = f(x w^T) in sorted order.  `early`: the lists are older than the stream's last kernel (another
+    product of theirs, say), so that matrices may be asked for while that one still runs."""
     mode = 1 if gated else (2 if first else 0)
     _need(x, None, "x", contiguous=False)
     _need(weight, x.dtype, "weight")
@@ -2156,7 +2158,7 @@ def moe_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, lists,
                                      offsets, order, tile_expert, tile_row0,
                                      meta, pairs, experts, int(top), n, k, mode,
                                      GATE_KINDS[activation], _tag(x.dtype), int(tile) or moe_tile_rows(),
-                                     _stream()), "moe_product")
+                                     int(early), _stream()), "moe_product")
     return out
 
 

@@ -198,5 +198,5 @@ class RoutedExperts(Part):
         ops.moe_product(y, self.w_gate_up, act, lists, pairs, top, self.gated, self.activation, first=True,
                         tile=tile)
         expert_out = rt.buffer("routed.expert_out", pairs, self.hidden_size, y.dtype)
-        ops.moe_product(act, self.w_down, expert_out, lists, pairs, top, False, tile=tile)
+        ops.moe_product(act, self.w_down, expert_out, lists, pairs, top, False, tile=tile, early=True)
         return ops.moe_combine(expert_out, weights, shared, out, top, **identity)
