@@ -36,7 +36,7 @@ enum { ERR_TMA_WAIT = 11, ERR_MMA_WAIT = 12, ERR_EPILOGUE_WAIT = 13 };
 
 struct GemmParams {
     void* y; int ldy;               // [T, ldy] bf16 or float
-    const bf16* bias;               // [N] or null
+    const bf16* bias;               // [N] or null (gated: [2 N], the gate rows' first)
     int T, N, K;                    // N = output features (SwiGLU: intermediate size)
     int up_row0;                    // SwiGLU: row of w where the up rows start
     int gate;                       // gated epilogue: 1 = SiLU on the gate, 2 = GELU (tanh form); plain epilogue: 3 = the square of relu on the result
@@ -247,6 +247,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         float out;
         if (EPI == EPI_SWIGLU) {
+            if (p.bias) { acc += __bfloat162float(p.bias[n]); acc_up += __bfloat162float(p.bias[p.N + n]); }
             // the library path rounds gate and up to bfloat16 before the activation; do the same
             const float g = __bfloat162float(__float2bfloat16_rn(acc));
             const float u = __bfloat162float(__float2bfloat16_rn(acc_up));
@@ -331,7 +332,7 @@ int fsie_gemm_decode_weight_map(void* map_out, const void* w, long long rows, lo
 }
 
 // y[T, N] = x[T, K] * w^T (+ bias), or for swiglu != 0 y[T, N] = act(x w_gate^T) * (x w_up^T) with
-// w = [gate rows (N); up rows (N)], act = SiLU (swiglu = 1) or the tanh form of GELU (2); swiglu = 3: no gate, y = relu(x w^T)^2.  T <= 64.  `splits` (1, 2, 4 or 8) cuts K over a cluster.
+// w = [gate rows (N); up rows (N)] (a bias alike), act = SiLU (swiglu = 1) or the tanh form of GELU (2); swiglu = 3: no gate, y = relu(x w^T)^2.  T <= 64.  `splits` (1, 2, 4 or 8) cuts K over a cluster.
 int fsie_gemm_decode(const void* weight_map, const void* x, int ldx, void* y, int ldy, const void* bias,
                      int T, int N, int K, int swiglu, int out_f32, int splits, int* error, cudaStream_t stream) {
     if (T <= 0 || N <= 0) return 0;

@@ -166,21 +166,23 @@ class Runtime:
         return self._tables[key]
 
     def prepare_weight(self, weight: torch.Tensor, swiglu: bool = False,
-                       activation: str = "silu", plain_activation: Optional[str] = None) -> None:
+                       activation: str = "silu", plain_activation: Optional[str] = None, biased: bool = False) -> None:
         """Called by a part at bind for a matrix it will multiply activations with.  Large
         bfloat16 matrices get a TMA descriptor for the tcgen05 product that steps of few
         tokens use (the library product is kept where it measured faster: small matrices).
-        `plain_activation`: the weight is for `linear_activated` only."""
+        `plain_activation`: the weight is for `linear_activated` only.  `biased`: the gated product is
+        called with a bias, which the fused product of few tokens takes and the tiled one does not."""
         if self.dtype is not torch.bfloat16 or weight.dtype is not torch.bfloat16:
             return
         rows, k = weight.shape
         if k % 8 or (swiglu and rows % 2):
             return
         if self.products == "own":
-            self._tiled_weights[weight.data_ptr()] = (weight, swiglu, activation, plain_activation)
+            self._tiled_weights[weight.data_ptr()] = (weight, swiglu and not biased, activation, plain_activation)
         if rows * k >= self.few_token_min_elements:
             self._few_token_weights[weight.data_ptr()] = ops.DecodeWeight(weight, swiglu, activation,
                                                                           plain_activation)
+            self._few_token_weights[weight.data_ptr()].biased = swiglu and biased
 
     def _tiled(self, x: torch.Tensor, weight: torch.Tensor) -> Optional["ops.TiledWeight"]:
         """The weight's descriptor for the tiled product when this step is one for it: more
@@ -217,7 +219,7 @@ class Runtime:
         prepared = self._few_token_weights.get(weight.data_ptr())
         if prepared is None:
             return None
-        limit = self.few_token_limit_fused if prepared.swiglu else self.few_token_limit
+        limit = self.few_token_limit_fused if prepared.swiglu and not prepared.biased else self.few_token_limit
         return prepared if x.shape[0] <= limit else None
 
     def _few_token_product(self, prepared, x, bias, out_dtype, tag=None) -> torch.Tensor:
@@ -310,13 +312,16 @@ class Runtime:
                       activation: str = "silu") -> torch.Tensor:
         """silu(x @ gate.T) * (x @ up.T) for the stacked weight [gate rows; up rows]: one fused
         kernel for steps of few tokens, else the library product and the SwiGLU kernel.  A `bias`
-        (stacked like the weight) is added by the product; of the fused kernels the one of the
-        smallest steps takes it, otherwise the SwiGLU kernel follows.
+        (stacked like the weight) is added by the product; the fused kernels of few tokens take it
+        (a large matrix: if `prepare_weight` was told), otherwise the SwiGLU kernel follows.
         `activation` names what the gate passes through (the fused kernels were told at
         `prepare_weight`; the unfused path runs the kernel of gated activations)."""
         if bias is not None:
+            prepared = self._few_tokens(x, gate_up) if self.dtype is torch.bfloat16 else None
+            if prepared is not None and prepared.swiglu:
+                return self._few_token_product(prepared, x, bias, torch.bfloat16, tag)
             if (self.dtype is torch.bfloat16 and activation == "silu" and gate_up.shape[0] % 2 == 0
-                    and bias.dtype is torch.bfloat16 and self._few_tokens(x, gate_up) is None
+                    and bias.dtype is torch.bfloat16 and prepared is None
                     and self._tiled(x, gate_up) is None and self._skinny(x, gate_up)):
                 # the product that `linear` would take, with the activation in its epilogue
                 return ops.gemm_skinny_swiglu(gate_up, x, self.buffer(tag, x.shape[0], gate_up.shape[0] // 2,

@@ -655,7 +655,7 @@ class DecodeWeight:
         if swiglu and rows % 2:
             raise KernelError("gemm_decode: a SwiGLU weight holds gate rows and as many up rows")
         lib = gemm_decode_lib()
-        self.weight, self.swiglu, self.k = weight, swiglu, k
+        self.weight, self.swiglu, self.k, self.biased = weight, swiglu, k, False
         self.n = rows // 2 if swiglu else rows
         self.map = ctypes.create_string_buffer(lib.fsie_tensor_map_bytes() + 64)
         offset = (-ctypes.addressof(self.map)) % 64
@@ -674,8 +674,8 @@ def gemm_decode_splits(tiles: int, k: int, sm_count: int) -> int:
 
 def gemm_decode(weight: DecodeWeight, x: torch.Tensor, out: torch.Tensor,
                 bias: Optional[torch.Tensor], error: torch.Tensor, splits: int = 1) -> torch.Tensor:
-    """out[T, N] = x[T, K] @ w.T (+ bias), or silu(x @ gate.T) * (x @ up.T); T <= 64; out is
-    bfloat16 or float32."""
+    """out[T, N] = x[T, K] @ w.T (+ bias), or silu(x @ gate.T) * (x @ up.T), each product with its half of the
+    bias; T <= 64; out is bfloat16 or float32."""
     _need(x, torch.bfloat16, "x", contiguous=False)
     _need(out, None, "out")
     tokens, k = x.shape
@@ -686,6 +686,8 @@ def gemm_decode(weight: DecodeWeight, x: torch.Tensor, out: torch.Tensor,
         raise KernelError("gemm_decode: out does not fit")
     if bias is not None:
         _need(bias, torch.bfloat16, "bias")
+        if weight.swiglu and bias.numel() != 2 * weight.n:
+            raise KernelError("gemm_decode: the bias does not fit the weight")
     _check(gemm_decode_lib().fsie_gemm_decode(
         weight.map_ptr, x, x.stride(0), out, out.stride(0), bias, tokens,
         weight.n, k, weight.gate, int(out.dtype is torch.float32), splits, error,

@@ -62,9 +62,10 @@ class SwiGluMlp(Part):
             self.b_gate_up = torch.cat([tensors[self._name("gate", "bias")],
                                         tensors[self._name("up", "bias")]]).to(runtime.dtype).contiguous()
             self.b_down = tensors[self._name("down", "bias")].to(runtime.dtype).contiguous()
-        # the fused SwiGLU products of prepared weights take no bias: with one, the stacked product adds it
-        # and a kernel of its own applies the activation
-        runtime.prepare_weight(self.w_gate_up, swiglu=not self.bias, activation=self.activation)
+        # of the fused SwiGLU products those of few tokens take a bias (with another activation than SiLU, and
+        # beyond few tokens, the stacked product adds it and a kernel of its own applies the activation)
+        runtime.prepare_weight(self.w_gate_up, swiglu=not self.bias or self.activation == "silu",
+                               activation=self.activation, biased=self.bias)
         runtime.prepare_weight(self.w_down)
 
     def forward(self, ctx, y: torch.Tensor) -> torch.Tensor:
