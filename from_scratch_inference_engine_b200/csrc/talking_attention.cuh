@@ -106,16 +106,15 @@ __device__ __forceinline__ void copy_tile(T* __restrict__ dst, const T* __restri
 }
 __device__ __forceinline__ void talking_copies_done() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// Warp w owns heads w, w + 8, ... (HS = 8 / TOK of them at most) and, of each, the tile's TOK
+// Warp w owns heads w, w + 8, ... (HS of them at most: 8 / TOK, two where 16 heads of single tokens need no more code and registers) and, of each, the tile's TOK
 // tokens: rows that share their keys and values, so one load of a key or value serves TOK rows.
 // Lane l owns keys l (+ 32) of a tile for the scores and value columns 2 l, 2 l + 1 (+ 64 c).
 // A split tile's block has one or two tiles of keys: it is a chain of trips to memory.  The lists, the first tile's pages
 // and the mixing matrix are read before the kernel before has finished, and the second walk gets as far as its first tile's
 // scores and values then: the first walk only read the queries, keys and values.  Shared memory is laid out for the
 // tile's own rows, so that blocks of both walks fit an SM (4 requests of 1,024 keys, the three launches: 56 us, TA_TIME now).
-template <typename T, int TOK, int VC2, int KPL>
+template <typename T, int TOK, int VC2, int KPL, int HS>
 __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const TalkingArgs a) {
-    constexpr int HS = 8 / TOK;
     constexpr int TK = 32 * KPL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int H = a.heads, G = a.kv_heads, dim = a.dim, vdim = a.vdim;
@@ -444,14 +443,15 @@ template <typename T, int TOK, int VC2>
 int talking_attention_launch_tile(const TalkingArgs& a, int num_tiles, int key_tile, size_t smem,
                                   cudaStream_t stream) {
     const dim3 grid(num_tiles, a.nsplit);
-    if (key_tile == 64) {
-        cudaFuncSetAttribute(talking_attention_kernel<T, TOK, VC2, 2>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return launch_dependent(talking_attention_kernel<T, TOK, VC2, 2>, grid, TA_WARPS * 32, smem, stream, a);
+    const auto go = [&](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return launch_dependent(kernel, grid, TA_WARPS * 32, smem, stream, a);
+    };
+    if constexpr (TOK == 1) {
+        if (a.heads <= 2 * TA_WARPS)
+            return key_tile == 64 ? go(talking_attention_kernel<T, TOK, VC2, 2, 2>) : go(talking_attention_kernel<T, TOK, VC2, 1, 2>);
     }
-    cudaFuncSetAttribute(talking_attention_kernel<T, TOK, VC2, 1>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_dependent(talking_attention_kernel<T, TOK, VC2, 1>, grid, TA_WARPS * 32, smem, stream, a);
+    return key_tile == 64 ? go(talking_attention_kernel<T, TOK, VC2, 2, 8 / TOK>) : go(talking_attention_kernel<T, TOK, VC2, 1, 8 / TOK>);
 }
 
 template <typename T, int TOK>
