@@ -70,7 +70,7 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
                       int vdim, const int* __restrict__ seg_item, const int* __restrict__ seg_row0,
                       int seg_tokens, float* __restrict__ chunk_states, int phase, int share,
                       const float* __restrict__ decay_tok, const float* __restrict__ decay_row,
-                      float out_scale, long long state_stride, float* __restrict__ chunk_decay) {
+                      float out_scale, long long state_stride, float* __restrict__ chunk_decay, int early) {
     // tokens staged in shared memory at a time (fewer where q, k and the rows' decays of large heads are staged)
     constexpr int SCAN_TOKENS = ROWS && DR > 8 ? 8 : 16;
     constexpr int PAD = DR > 4 ? DR + 4 : DR;
@@ -80,9 +80,8 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
     __shared__ __align__(16) float vs[SCAN_TOKENS * SCAN_COLS];
     __shared__ float ls[SCAN_TOKENS];                  // the decay of each staged token
     __shared__ __align__(16) float as[ROWS ? SCAN_TOKENS * ROW_LEN : 4];     // ... or of each of its state rows
-    // The lists were staged before the step, and a request's state (phase 0) was left by the step before: both are on their way
-    // while the kernel that makes q, k and v still runs (4 requests of 16 heads of 128 x 128: 19.9 us of a decode step's chain
-    // with all of it behind the wait, SCAN_TIME now).
+    // The lists were staged before the step and are read while the kernel before still runs; so is a request's state (phase 0)
+    // where the caller knows that kernel not to write it (early).
     const int item = seg_item ? seg_item[blockIdx.z] : blockIdx.z, head = blockIdx.y;
     const int slot = item_slots[item];
     if (slot < 0) {                                    // a padding entry of a fixed-size batch
@@ -111,7 +110,7 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
     };
     const int qk_head = head / share;                  // `share` heads read the same q and k columns
     float through = 1.f;                               // the product of the chunk's decays (phase 1)
-    if (phase != 0) grid_dependency_wait();            // chunk_states is the kernel before's
+    if (phase != 0 || !early) grid_dependency_wait();  // (chunk_states is the kernel before's)
     float s[DR][4];
 #pragma unroll
     for (int i = 0; i < DR; ++i) {
@@ -127,7 +126,7 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
             for (int x = 0; x < 4; ++x) if (col0 + x < vdim) s[i][x] = at[x];
         }
     }
-    if (phase == 0) grid_dependency_wait();
+    if (phase == 0 && early) grid_dependency_wait();
     grid_dependents_go();
     for (int t0 = 0; t0 < count; t0 += SCAN_TOKENS) {
         const int n = min(SCAN_TOKENS, count - t0);
@@ -499,7 +498,7 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
                         int dim, int vdim, const int* seg_item, const int* seg_row0, int num_segs,
                         int seg_tokens, float* chunk_states, int share, const float* decay_tok,
                         const float* decay_row, float out_scale, int dtype, long long state_stride, int silu,
-                        cudaStream_t stream) {
+                        int early, cudaStream_t stream) {
     if (items <= 0) return 0;
     if (heads <= 0 || dim <= 0 || vdim <= 0 || heads > 65535 || items > 65535 || share <= 0 ||
         heads % share || (!decay && !decay_tok && !decay_row) || (dtype != DTYPE_F32 && !decay_row && !silu) || (silu && decay_row) || state_stride < (long long)heads * dim * vdim)
@@ -519,7 +518,7 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
     launch_code = launch_dependent(lightning_scan_kernel<DPT, T, R, S>, grid, threads, 0, stream,   \
         (const T*)proj, ld, q_off, k_off, v_off, item_qstart, item_qlen, item_slots, state,      \
         decay, out, heads, dim, vdim, seg_item, seg_row0, seg_tokens, chunk_states, phase, share, \
-        decay_tok, decay_row, out_scale, state_stride, chunk_decay)
+        decay_tok, decay_row, out_scale, state_stride, chunk_decay, early)
 #define FSIE_SCAN_SIZES(T, R, S)                                                                 \
     do {                                                                                         \
         if (per_thread <= 1) FSIE_SCAN(T, R, S, 1);                                              \

@@ -1025,7 +1025,7 @@ def scan():
         lib = build.load_library("scan")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_lightning_scan.argtypes = [p, i, i, i, i, p, p, p, i, p, p, p, i, i, i, p, p, i, i, p,
-                                            i, p, p, f, i, ll, i, p]
+                                            i, p, p, f, i, ll, i, i, p]
         lib.fsie_row_decay.argtypes = [p, i, i, i, p, p, f, p, i, i, i, p]
         lib.fsie_head_norm_silu.argtypes = [p, p, i, i, p, p, i, i, i, f, i, p]
         lib.fsie_silu_rows.argtypes = [p, i, i, p, i, i, p]
@@ -1144,7 +1144,7 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                    seg_row0: Optional[torch.Tensor] = None, num_segs: int = 0, seg_tokens: int = 0,
                    chunk_states: Optional[torch.Tensor] = None, share: int = 1,
                    decay_tok: Optional[torch.Tensor] = None, decay_row: Optional[torch.Tensor] = None,
-                   out_scale: float = 1.0, silu: bool = False) -> torch.Tensor:
+                   out_scale: float = 1.0, silu: bool = False, early: bool = False) -> torch.Tensor:
     """Per request and head, token by token: S = decay * S + k v^T, o = S^T q.  proj [tokens, ld]
     (float32) holds the ACTIVATED projections (`silu_rows`) at the given column offsets; state
     [slots, heads, dim, vdim] (float32; or [slots, n] with the heads' matrices in the first
@@ -1159,7 +1159,8 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     request by request) and `chunk_states` (float32, num_segs * heads * dim * vdim at least; with
     `decay_tok` num_segs * heads more, with `decay_row` num_segs * heads * dim more) the
     chunks of long prompts run side by side: each sums its own tokens, the sums are chained into
-    the state at every chunk's start, and each chunk runs again from there for its outputs."""
+    the state at every chunk's start, and each chunk runs again from there for its outputs.
+    `early`: the stream's last kernel does not write the state, which may be read while it still runs."""
     _need(proj, torch.float32 if decay_row is None and not silu else None, "proj")
     if silu and decay_row is not None:
         raise KernelError("lightning_scan: a decay per state row comes with activated projections")
@@ -1201,7 +1202,7 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                                       decay, out, heads, dim, vdim, seg_item,
                                       seg_row0, num_segs, seg_tokens, chunk_states,
                                       int(share), decay_tok, decay_row, float(out_scale),
-                                      _tag(proj.dtype), state_stride, int(silu), _stream()),
+                                      _tag(proj.dtype), state_stride, int(silu), int(early), _stream()),
            "lightning_scan")
     return out
 

@@ -100,7 +100,7 @@ class GatedLinearAttention(Mixer):
         o = rt.buffer("gated_linear.o", tokens, self.v_width, torch.float32)
         ops.lightning_scan(proj, 0, self.qk_width, 2 * self.qk_width, ctx.item_qstart, ctx.item_qlen, ctx.item_slots,
                            ctx.num_items, cache.state, None, o, self.heads, self.dim, self.vdim, decay_row=decay,
-                           out_scale=self.dim ** -0.5, **chunks)
+                           out_scale=self.dim ** -0.5, early=True, **chunks)
         gated = rt.buffer("gated_linear.gated", tokens, self.v_width, proj.dtype)
         ops.head_norm_silu(o, proj, gate0, self.gain, self.eps, gated, self.heads)
         return rt.linear(gated, self.w_o, None, "gated_linear.out")

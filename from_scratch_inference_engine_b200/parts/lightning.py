@@ -82,7 +82,7 @@ class LightningAttention(Mixer):
             act = ops.silu_rows(proj, width, rt.buffer("lightning.act", tokens, width, torch.float32))
         ops.lightning_scan(act, 0, self.qk_width, 2 * self.qk_width, ctx.item_qstart,
                            ctx.item_qlen, ctx.item_slots, ctx.num_items, cache.state, self.decay, o,
-                           self.heads, self.dim, self.vdim, silu=not chunks, **chunks)
+                           self.heads, self.dim, self.vdim, silu=not chunks, early=True, **chunks)
         gated = rt.buffer("lightning.gated", tokens, self.v_width, proj.dtype)
         ops.gated_rmsnorm(o, proj, 2 * self.qk_width + self.v_width, self.gain, self.eps, gated)
         return rt.linear(gated, self.w_o, None, "lightning.out")

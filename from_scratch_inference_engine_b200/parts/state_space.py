@@ -118,7 +118,7 @@ class StateSpaceDuality(Mixer):
         # q = C, k = B, v = dt * x; the heads of a group share its B and C
         ops.lightning_scan(act, inner + gn, inner, self.channels, ctx.item_qstart, ctx.item_qlen,
                            ctx.item_slots, ctx.num_items, cache.state, None, o, self.heads, self.state,
-                           self.vdim, share=self.heads // self.groups, decay_tok=decay, **chunks)
+                           self.vdim, share=self.heads // self.groups, decay_tok=decay, early=True, **chunks)
         gated = rt.buffer("state_space.gated", tokens, inner, proj.dtype)
         ops.ssd_gate_norm(o, act, proj, 0, self.skip, self.gain, gated, self.vdim, self.norm_groups, self.eps)
         return rt.linear(gated, self.w_o, None, "state_space.out")
