@@ -257,6 +257,93 @@ __global__ void silu_rows_kernel(const T* __restrict__ proj, int ld, int width, 
     }
 }
 
+// The same for steps of one token per request, heads of 33 to 128 rows and rows of the state on 16 bytes: every q, k and v value
+// is one thread's, asked for at once, and nothing of the segments is left in the code.  A launch is a chain that a few
+// warps per SM walk alone, so its instructions count: STEP_TIME.  Sums run in the order above: the same bits.
+template <int DR, typename T, bool ROWS, bool SILU>
+__global__ void __launch_bounds__(SCAN_COLS / 4 * SCAN_ROW_GROUPS)
+lightning_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off,
+                      const int* __restrict__ item_qstart, const int* __restrict__ item_qlen,
+                      const int* __restrict__ item_slots, float* __restrict__ state, const float* __restrict__ decay,
+                      float* __restrict__ out, int heads, int dim, int vdim, int share, const float* __restrict__ decay_tok,
+                      const float* __restrict__ decay_row, float out_scale, long long state_stride, int early) {
+    constexpr int PAD = DR > 4 ? DR + 4 : DR, ROW_LEN = SCAN_ROW_GROUPS * PAD;
+    static_assert(DR % 4 == 0 && DR * SCAN_ROW_GROUPS <= SCAN_COLS / 4 * SCAN_ROW_GROUPS, "a thread's one value of q and k");
+    __shared__ __align__(16) float qs[ROW_LEN], ks[ROW_LEN], vs[SCAN_COLS], as[ROWS ? ROW_LEN : 4];
+    const int item = blockIdx.z, head = blockIdx.y, tid = threadIdx.x;
+    const int slot = item_slots[item], start = item_qstart[item], count = item_qlen[item];
+    if (slot < 0) {                                    // a padding entry of a fixed-size batch
+        grid_dependency_wait();
+        return;
+    }
+    const int rg = tid & (SCAN_ROW_GROUPS - 1), cg = tid / SCAN_ROW_GROUPS, col0 = blockIdx.x * SCAN_COLS + cg * 4;
+    const bool mine = col0 < vdim;
+    float* at = state + (size_t)slot * state_stride + ((size_t)head * dim + rg * DR) * vdim + col0;
+    const float head_decay = decay ? decay[head] : 1.f;
+    if (!early) grid_dependency_wait();
+    float s[DR][4];
+#pragma unroll
+    for (int i = 0; i < DR; ++i) {
+        const float4 v = mine && rg * DR + i < dim ? *reinterpret_cast<const float4*>(at + (size_t)i * vdim)
+                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        s[i][0] = v.x; s[i][1] = v.y; s[i][2] = v.z; s[i][3] = v.w;
+    }
+    if (early) grid_dependency_wait();
+    grid_dependents_go();
+    for (int t = 0; t < count; ++t) {
+        const size_t token = start + t;
+        const T* row = proj + token * ld + (head / share) * dim + tid;
+        const int column = blockIdx.x * SCAN_COLS + tid;
+        float q = 0.f, k = 0.f, a = 0.f, v = 0.f;
+        if (tid < dim) {
+            q = to_float(row[q_off]);
+            k = to_float(row[k_off]);
+            if (ROWS) a = decay_row[(token * heads + head) * dim + tid];
+        }
+        if (tid < SCAN_COLS && column < vdim) v = to_float(proj[token * ld + v_off + head * vdim + column]);
+        const float lambda = ROWS ? 1.f : (decay_tok ? decay_tok[token * heads + head] : head_decay);
+        if (SILU) { q = silu_f(q); k = silu_f(k); v = silu_f(v); }
+        if (t) __syncthreads();
+        if (tid < DR * SCAN_ROW_GROUPS) {
+            qs[scan_row_at<DR>(tid)] = q;
+            ks[scan_row_at<DR>(tid)] = k;
+            if (ROWS) as[scan_row_at<DR>(tid)] = a;
+        }
+        if (tid < SCAN_COLS) vs[tid] = v;
+        __syncthreads();
+        const float4 v4 = *reinterpret_cast<const float4*>(vs + cg * 4);
+        const float vv[4] = {v4.x, v4.y, v4.z, v4.w};
+        float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i0 = 0; i0 < DR; i0 += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(ks + rg * PAD + i0), q4 = *reinterpret_cast<const float4*>(qs + rg * PAD + i0);
+            const float4 a4 = ROWS ? *reinterpret_cast<const float4*>(as + rg * PAD + i0) : make_float4(lambda, lambda, lambda, lambda);
+            const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w}, aa[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    s[i0 + i][x] = aa[i] * s[i0 + i][x] + kk[i] * vv[x];
+                    o[x] += s[i0 + i][x] * qq[i];
+                }
+        }
+        // the sum over the 16 row groups, as above
+        const bool upper = rg & 1, odd = rg & 2;
+        const float a0 = __shfl_xor_sync(0xffffffffu, upper ? o[0] : o[2], 1);
+        const float a1 = __shfl_xor_sync(0xffffffffu, upper ? o[1] : o[3], 1);
+        const float b0 = (upper ? o[2] : o[0]) + a0, b1 = (upper ? o[3] : o[1]) + a1;
+        float sum = (odd ? b1 : b0) + __shfl_xor_sync(0xffffffffu, odd ? b0 : b1, 2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        const int col = col0 + (upper ? 2 : 0) + (odd ? 1 : 0);
+        if (rg < 4 && col < vdim) out[(token * heads + head) * vdim + col] = sum * out_scale;
+    }
+#pragma unroll
+    for (int i = 0; i < DR; ++i)
+        if (mine && rg * DR + i < dim)
+            *reinterpret_cast<float4*>(at + (size_t)i * vdim) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+}
+
 // Chains the chunks' sums of every request: chunk_states[c] (on entry the sum of chunk c's own
 // tokens from a zero state) becomes the state at the start of chunk c, and the request's slot
 // receives the state after its last chunk.  S_after = decay^len * S_before + sum.  One thread per
@@ -498,7 +585,7 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
                         int dim, int vdim, const int* seg_item, const int* seg_row0, int num_segs,
                         int seg_tokens, float* chunk_states, int share, const float* decay_tok,
                         const float* decay_row, float out_scale, int dtype, long long state_stride, int silu,
-                        int early, cudaStream_t stream) {
+                        int early, int single, cudaStream_t stream) {
     if (items <= 0) return 0;
     if (heads <= 0 || dim <= 0 || vdim <= 0 || heads > 65535 || items > 65535 || share <= 0 ||
         heads % share || (!decay && !decay_tok && !decay_row) || (dtype != DTYPE_F32 && !decay_row && !silu) || (silu && decay_row) || state_stride < (long long)heads * dim * vdim)
@@ -535,6 +622,19 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
         else if (dtype == DTYPE_F32) FSIE_SCAN_SIZES(float, true, false);                        \
         else FSIE_SCAN_SIZES(bf16, true, false);                                                 \
     } while (0)
+    // (heads of up to 32 rows: one or two rows a thread, another order of the sums, and over soon)
+    if (!chunked && single && dim > SCAN_ROW_GROUPS * 2 && dim <= SCAN_ROW_GROUPS * 8 && vdim % 4 == 0 && state_stride % 4 == 0 && (((size_t)state) & 15) == 0) {
+#define FSIE_STEP(T, R, S, DPT)                                                                  \
+        launch_dependent(lightning_step_kernel<DPT, T, R, S>, grid, threads, 0, stream,          \
+            (const T*)proj, ld, q_off, k_off, v_off, item_qstart, item_qlen, item_slots, state,  \
+            decay, out, heads, dim, vdim, share, decay_tok, decay_row, out_scale, state_stride, early)
+#define FSIE_STEP_SIZES(T, R, S) (per_thread <= 4 ? FSIE_STEP(T, R, S, 4) : FSIE_STEP(T, R, S, 8))
+        if (silu) return dtype == DTYPE_F32 ? FSIE_STEP_SIZES(float, false, true) : FSIE_STEP_SIZES(bf16, false, true);
+        if (!decay_row) return FSIE_STEP_SIZES(float, false, false);
+        return dtype == DTYPE_F32 ? FSIE_STEP_SIZES(float, true, false) : FSIE_STEP_SIZES(bf16, true, false);
+#undef FSIE_STEP_SIZES
+#undef FSIE_STEP
+    }
     FSIE_SCAN_BY_SIZE();
     if (launch_code) return launch_code;
     if (chunked) {

@@ -1025,7 +1025,7 @@ def scan():
         lib = build.load_library("scan")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
         lib.fsie_lightning_scan.argtypes = [p, i, i, i, i, p, p, p, i, p, p, p, i, i, i, p, p, i, i, p,
-                                            i, p, p, f, i, ll, i, i, p]
+                                            i, p, p, f, i, ll, i, i, i, p]
         lib.fsie_row_decay.argtypes = [p, i, i, i, p, p, f, p, i, i, i, p]
         lib.fsie_head_norm_silu.argtypes = [p, p, i, i, p, p, i, i, i, f, i, p]
         lib.fsie_silu_rows.argtypes = [p, i, i, p, i, i, p]
@@ -1202,7 +1202,8 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                                       decay, out, heads, dim, vdim, seg_item,
                                       seg_row0, num_segs, seg_tokens, chunk_states,
                                       int(share), decay_tok, decay_row, float(out_scale),
-                                      _tag(proj.dtype), state_stride, int(silu), int(early), _stream()),
+                                      _tag(proj.dtype), state_stride, int(silu), int(early),
+                                      int(tokens == items), _stream()),
            "lightning_scan")
     return out
 
