@@ -336,6 +336,45 @@ struct MmaLayout {
     }
 };
 
+// A tile's query rows into shared memory as they are, zero beyond the tile: four rows and PIECES pieces of 16 bytes of each are a lane's
+// at once.  Asked for one after the other, each behind the store of the one before, a decoded token's rows of 576 values were
+// twelve trips to memory (QS_TIME).
+template <int ROWS, int WARPS, int PIECES>
+__device__ __forceinline__ void sa_stage_queries(const ScaledAttnParams& p, const bf16* q, bf16* Qs, int ldk, int kvh, int group,
+                                                 int qstart, int row0, int nrows, int dk, int warp, int lane) {
+    constexpr int TOGETHER = 4;
+    static_assert(ROWS % (WARPS * TOGETHER) == 0, "four rows of a warp at a time");
+    for (int r0 = warp; r0 < ROWS; r0 += WARPS * TOGETHER) {
+        int head[TOGETHER];
+        const bf16* src[TOGETHER];
+#pragma unroll
+        for (int i = 0; i < TOGETHER; ++i) {
+            const int r = r0 + i * WARPS, row = row0 + r, token = row / group;
+            head[i] = r < nrows ? kvh * group + (row - token * group) : -1;
+            src[i] = q + (size_t)(qstart + token) * p.q_ld + (size_t)head[i] * p.q_dim;
+        }
+        for (int c0 = lane; c0 < dk / 8; c0 += 32 * PIECES) {
+            uint4 v[PIECES][TOGETHER];
+#pragma unroll
+            for (int j = 0; j < PIECES; ++j)
+#pragma unroll
+                for (int i = 0; i < TOGETHER; ++i) {
+                    const int c = c0 + 32 * j;
+                    v[j][i] = make_uint4(0u, 0u, 0u, 0u);
+                    if (head[i] < 0 || c >= dk / 8) continue;
+                    const int at = sa_query_column(p, head[i], c * 8);
+                    if (at >= 0) v[j][i] = *reinterpret_cast<const uint4*>(src[i] + at);
+                }
+#pragma unroll
+            for (int j = 0; j < PIECES; ++j)
+#pragma unroll
+                for (int i = 0; i < TOGETHER; ++i)
+                    if (c0 + 32 * j < dk / 8)
+                        *reinterpret_cast<uint4*>(Qs + (r0 + i * WARPS) * ldk + (c0 + 32 * j) * 8) = v[j][i];
+        }
+    }
+}
+
 template <int NV, bool SHARED_V>
 __global__ void __launch_bounds__(SA_WARPS * 32) scaled_attention_mma_kernel(const ScaledAttnParams p) {
     extern __shared__ __align__(16) unsigned char tm_smem[];
@@ -422,17 +461,7 @@ __global__ void __launch_bounds__(SA_WARPS * 32) scaled_attention_mma_kernel(con
     if (!early && kbegin < kend) issue_tile(0, kbegin, first_page);
 
     // the tile's query rows as they are (the head's scale meets the scores), zero beyond the tile
-    for (int r = warp; r < SA_ROWS; r += SA_WARPS) {
-        const int row = row0 + r;
-        const int h = kvh * group + row % group;
-        const bf16* src = q + (size_t)(qstart + row / group) * p.q_ld + (size_t)h * p.q_dim;
-        for (int c = lane; c < dk / 8; c += 32) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            const int at = sa_query_column(p, h, c * 8);
-            if (r < nrows && at >= 0) v = *reinterpret_cast<const uint4*>(src + at);
-            *reinterpret_cast<uint4*>(Qs + r * L.ldk + c * 8) = v;
-        }
-    }
+    sa_stage_queries<SA_ROWS, SA_WARPS, 3>(p, q, Qs, L.ldk, kvh, group, qstart, row0, nrows, dk, warp, lane);
 
     // this thread's two rows: g and g + 8 of its group of 16
     int pos[2], first_key[2];
@@ -715,17 +744,7 @@ __global__ void __launch_bounds__(TR_WARPS * 32) scaled_attention_rows_kernel(co
     }
     int page_ahead = page_of(kbegin + (SLOTS - 1) * TM_KT);
 
-    for (int r = warp; r < ROWS; r += TR_WARPS) {
-        const int row = row0 + r;
-        const int h = kvh * group + row % group;
-        const bf16* src = q + (size_t)(qstart + row / group) * p.q_ld + (size_t)h * p.q_dim;
-        for (int c = lane; c < dk / 8; c += 32) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            const int at = sa_query_column(p, h, c * 8);
-            if (r < nrows && at >= 0) v = *reinterpret_cast<const uint4*>(src + at);
-            *reinterpret_cast<uint4*>(Qs + r * L.ldk + c * 8) = v;
-        }
-    }
+    sa_stage_queries<ROWS, TR_WARPS, 1>(p, q, Qs, L.ldk, kvh, group, qstart, row0, nrows, dk, warp, lane);
 
     int pos[2], first_key[2];
     float sc[2], m[2], l[2];
