@@ -969,7 +969,7 @@ __global__ void sa_combine_kernel(const float* __restrict__ part_o, const float*
     grid_dependency_wait();
     grid_dependents_go();
     // every thread of a warp takes every turn of the loops (the weights travel by shuffles)
-    for (int d0 = 0; d0 < dv; d0 += blockDim.x) {
+    for (int d0 = blockIdx.z * blockDim.x; d0 < dv; d0 += blockDim.x * gridDim.z) {
         const int d = d0 + threadIdx.x;
         const bool mine = d < dv;
         float mmax = -INFINITY, denom = 0.f, o = 0.f;
@@ -1527,9 +1527,11 @@ int fsie_scaled_attention(const void* q, int q_ld, const float* head_scale, cons
                                 : scaled_attention_dispatch<bf16>(p, tiles, values_in_keys != 0, stream);
     }
     if (rc != 0 || nsplit == 1 || partial) return rc;
-    const dim3 cgrid(combine_tokens ? num_combine : tokens, heads);
-    if (cgrid.x == 0) return 0;
     const int threads = value_dim >= 128 ? 128 : (value_dim >= 64 ? 64 : 32);
+    // a block for every 128 columns: one that went over 512 of them was four trips to memory, one after the other (6.6 us of a
+    // step's chain for 8 tokens of 16 heads, COMB_TIME now)
+    const dim3 cgrid(combine_tokens ? num_combine : tokens, heads, (value_dim + threads - 1) / threads);
+    if (cgrid.x == 0) return 0;
     if (dtype == DTYPE_F32)
         return launch_dependent(sa_combine_kernel<float>, cgrid, dim3(threads), 0, stream, part_o, part_ml, (float*)out,
                                 out_ld, tokens, heads, value_dim, nsplit, (const float*)gate, gate_ld,
