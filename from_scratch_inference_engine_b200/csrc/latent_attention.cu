@@ -225,7 +225,7 @@ __device__ __forceinline__ void hm_cp16(void* dst, const void* src, bool valid) 
 // ---- the same for few tokens of bfloat16 where rows start on 16 bytes and k is up to 1,024: a lane's weights of HQ_ROWS rows
 // are on their way before the kernel before has finished and x comes straight to the lanes that use it.  What bounds it is the
 // chain from that kernel to its result: staging x as floats in shared memory, a value at a time and behind a barrier, for 8
-// rows a block took 10.5 us (4 tokens, 16 heads of 512 x 128), HQ_TIME now.  A row has LANES lanes (16 where k <= 128 would leave
+// rows a block took 10.5 us (4 tokens, 16 heads of 512 x 128), 3.8 now.  A row has LANES lanes (16 where k <= 128 would leave
 // the others idle), which add up what they had above in the same order: the same bits.
 constexpr int HQ_WARPS = 4, HQ_ROWS = 4;
 template <int LANES, int CHUNKS, int TOK>

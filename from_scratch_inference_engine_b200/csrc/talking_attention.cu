@@ -139,7 +139,7 @@ __global__ void conv_norm_rotate_kernel(const T* __restrict__ proj, int ld, int 
 // everything a row needs on its way at once (weights, gains, angles and lists before the kernel that makes
 // the projection has finished).  A decode step's rows are few, so the chain of trips to memory is what it takes: with a
 // channel per thread and turn, and the tails in a launch behind it, 4 tokens of 3,072 channels took 22 + 10 us of
-// the step's chain, CV_TIME now.  The squares are added up from shared memory as the general kernel's threads and warps
+// the step's chain, 6.8 now.  The squares are added up from shared memory as the general kernel's threads and warps
 // do it, so that both leave the same bits.
 // FOLD (every request brings one token): the row's own channels move the request's tail on as well, which conv_tails
 // does otherwise (a longer portion's first tokens still read the old tail when its last one is done).
