@@ -39,9 +39,8 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o, const floa
     float2 ahead[AHEAD];
 #pragma unroll
     for (int j = 0; j < AHEAD; ++j) {
-        const int z = min(j, nsplit - 1);
-        ahead[j] = d_first < HD ? *reinterpret_cast<const float2*>(part_o + (z * stride + slot) * HD + d_first)
-                                : make_float2(0.f, 0.f);
+        ahead[j] = j < nsplit && d_first < HD ? *reinterpret_cast<const float2*>(part_o + (j * stride + slot) * HD + d_first)
+                                              : make_float2(0.f, 0.f);
     }
     const float mmax = warp_max(fmaxf(mz, mz_hi));
     const float wz = mz == -INFINITY ? 0.f : __expf(mz - mmax);
@@ -62,17 +61,18 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o, const floa
             float2 v[AHEAD];
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j) {
-                const int z = min(z0 + j, nsplit - 1);
+                const int z = z0 + j;
                 if (d0 == 0 && z0 == 0) v[j] = ahead[j];
-                else v[j] = mine ? *reinterpret_cast<const float2*>(part_o + (z * stride + slot) * HD + d)
-                                 : make_float2(0.f, 0.f);
+                else v[j] = mine && z < nsplit ? *reinterpret_cast<const float2*>(part_o + (z * stride + slot) * HD + d)
+                                               : make_float2(0.f, 0.f);
             }
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j) {
-                const int z = min(z0 + j, MAX_KEY_SPLITS - 1);
+                const int z = z0 + j;
+                if (z >= nsplit) break;                    // (a prompt's tokens have two or three splits, and are many)
                 const float lo = __shfl_sync(0xffffffffu, wz, z & 31), hi = __shfl_sync(0xffffffffu, wz_hi, z & 31);
                 const float w = z < 32 ? lo : hi;
-                if (z0 + j < nsplit && w != 0.f) { a0 += v[j].x * w; a1 += v[j].y * w; }   // a split without keys may hold anything
+                if (w != 0.f) { a0 += v[j].x * w; a1 += v[j].y * w; }   // a split without keys may hold anything
             }
         }
         if (mine) {

@@ -985,7 +985,7 @@ __global__ void sa_combine_kernel(const float* __restrict__ part_o, const float*
             float ahead[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j)
-                ahead[j] = mine ? part_o[((size_t)(z0 + min(j, n - 1)) * stride + slot) * dv + d] : 0.f;
+                ahead[j] = mine && j < n ? part_o[((size_t)(z0 + j) * stride + slot) * dv + d] : 0.f;
             const float m_new = fmaxf(mmax, warp_max(mz));
             const float corr = mmax == -INFINITY ? 0.f : expf(mmax - m_new);
             const float w = mz == -INFINITY ? 0.f : expf(mz - m_new);
@@ -996,12 +996,13 @@ __global__ void sa_combine_kernel(const float* __restrict__ part_o, const float*
                 if (j0) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        ahead[j] = mine ? part_o[((size_t)(z0 + min(j0 + j, n - 1)) * stride + slot) * dv + d] : 0.f;
+                        ahead[j] = mine && j0 + j < n ? part_o[((size_t)(z0 + j0 + j) * stride + slot) * dv + d] : 0.f;
                 }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const float wj = __shfl_sync(0xffffffffu, w, min(j0 + j, 31));
-                    if (j0 + j < n && wj != 0.f) o += ahead[j] * wj;        // a range without keys may hold anything
+                    if (j0 + j >= n) break;
+                    const float wj = __shfl_sync(0xffffffffu, w, j0 + j);
+                    if (wj != 0.f) o += ahead[j] * wj;        // a range without keys may hold anything
                 }
             }
         }
