@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(512) add_layernorm_regs_kernel(const S* __rest
         if (c >= width) break;
         float n = (v[i] - mean) * inv * g[i];
         if (xr) {
-            n = __fadd_rn(n, old[i]);                   // (a sum of its own above: not part of the product before it)
+            n = fmaf((v[i] - mean) * inv, g[i], old[i]);        // (written out: the general kernel's product is not rounded before)
             xr[c] = n;
         }
         if (yr) yr[c] = from_float<T>(n);
