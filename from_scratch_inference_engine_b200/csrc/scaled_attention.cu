@@ -338,7 +338,7 @@ struct MmaLayout {
 
 // A tile's query rows into shared memory as they are, zero beyond the tile: four rows and PIECES pieces of 16 bytes of each are a lane's
 // at once.  Asked for one after the other, each behind the store of the one before, a decoded token's rows of 576 values were
-// twelve trips to memory (QS_TIME).
+// twelve trips to memory (8 tokens of 16 heads, with prompts of 400: 21.3 -> 19.2 us a launch; rows of 128 values 12.6 -> 11.5).
 template <int ROWS, int WARPS, int PIECES>
 __device__ __forceinline__ void sa_stage_queries(const ScaledAttnParams& p, const bf16* q, bf16* Qs, int ldk, int kvh, int group,
                                                  int qstart, int row0, int nrows, int dk, int warp, int lane) {
