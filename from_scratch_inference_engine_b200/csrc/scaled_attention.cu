@@ -1530,7 +1530,7 @@ int fsie_scaled_attention(const void* q, int q_ld, const float* head_scale, cons
     if (rc != 0 || nsplit == 1 || partial) return rc;
     const int threads = value_dim >= 128 ? 128 : (value_dim >= 64 ? 64 : 32);
     // a block for every 128 columns: one that went over 512 of them was four trips to memory, one after the other (6.6 us of a
-    // step's chain for 8 tokens of 16 heads, COMB_TIME now)
+    // step's chain for 8 tokens of 16 heads, 2.6 now)
     const dim3 cgrid(combine_tokens ? num_combine : tokens, heads, (value_dim + threads - 1) / threads);
     if (cgrid.x == 0) return 0;
     if (dtype == DTYPE_F32)
