@@ -99,7 +99,9 @@ class StepContext:
         self.h_slots = np.asarray(slots, dtype=np.int32)
         self.max_context = max_context or (int((self.h_pos0 + self.h_qlen).max()) if I else 0)
         self.fixed_context = max_context
-        if T == I:                   # one token per request: a decode step
+        # every request brings exactly one token: a decode step (as many tokens as requests may also be two and none)
+        self.one_each = T == I and bool((self.h_qlen == 1).all())
+        if self.one_each:
             positions, token_item = self.h_pos0, np.arange(I, dtype=np.int32)
         else:
             positions = np.concatenate([np.arange(p, p + n, dtype=np.int32)

@@ -1217,7 +1217,7 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
              state: Optional[torch.Tensor], tail_off: int, conv_w: torch.Tensor,
              conv_b: Optional[torch.Tensor], dt_bias: torch.Tensor, a_log: torch.Tensor, heads: int,
              vdim: int, act: torch.Tensor, decay: torch.Tensor,
-             conv_wt: Optional[torch.Tensor] = None, move_tails: bool = False) -> None:
+             conv_wt: Optional[torch.Tensor] = None, move_tails: bool = False, one_each: bool = False) -> None:
     """What a state-space mixer's scan reads, per token of proj [tokens, ld] (the stored projection
     with the convolution's input columns at conv_off and the step sizes at dt_off):
     act [tokens, channels + heads * vdim] float32 = [silu(causal convolution + bias) | dt * x] with x
@@ -1226,8 +1226,8 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
     the inputs of the taps - 1 tokens before a step's first live in the request's slot of `state`
     [slots, n] (float32) from float tail_off on, oldest first (`ssd_tails` moves them on).  conv_wt:
     conv_w transposed ([taps, channels], contiguous), with which sizes in multiples of 8 take eight
-    channels per thread.  `move_tails`: the slots move on too, as by `ssd_tails`: in the same launch where every
-    request brings one token and the kernel for these sizes can, else by a call of it."""
+    channels per thread.  `move_tails`: the slots move on too, as by `ssd_tails`: in the same launch where the caller
+    knows that every request brings exactly one token (`one_each`) and the kernel for these sizes can, else by a call of it."""
     _need(proj, None, "proj")
     _need(conv_w, torch.float32, "conv_w")
     _need(dt_bias, torch.float32, "dt_bias")
@@ -1255,7 +1255,7 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
                                 item_slots, items, state, stride, tail_off, conv_w,
                                 conv_b, taps, channels, dt_bias, a_log, heads, vdim,
                                 act, act.stride(0), decay, conv_wt, tokens,
-                                _tag(proj.dtype), int(move_tails and taps > 1 and tokens == items),
+                                _tag(proj.dtype), int(move_tails and taps > 1 and one_each),
                                 ctypes.addressof(moved), _stream()), "ssd_prep")
     if move_tails and taps > 1 and not moved.value:
         ssd_tails(proj, conv_off, channels, taps, item_qstart, item_qlen, item_slots, items, state, tail_off)
@@ -1353,12 +1353,13 @@ def conv_norm_rotate(proj: torch.Tensor, items: int, item_qstart: torch.Tensor,
                      k_pages: Optional[torch.Tensor], v_pages: Optional[torch.Tensor],
                      page_stride: int, page_size: int, q_out: torch.Tensor, heads: int,
                      kv_heads: int, dim: int, vdim: int, has_kv: bool, eps: float,
-                     error: torch.Tensor, item_qlen: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     error: torch.Tensor, item_qlen: Optional[torch.Tensor] = None,
+                     one_each: bool = False) -> torch.Tensor:
     """Causal convolution over time of the projected q | k | v rows (earlier rows of the step, or
     the request's tail of taps - 1 rows), RMS norm of the whole q and the whole k with gains,
     rotation of interleaved pairs, per-head RMS of v; q -> q_out (float32), k and v -> pages.
-    With `item_qlen` the tails are moved on too, as `conv_tails` does: in the same launch where every request
-    brings one token and the kernel for these sizes can, else by a call of it."""
+    With `item_qlen` the tails are moved on too, as `conv_tails` does: in the same launch where the caller knows that
+    every request brings exactly one token (`one_each`) and the kernel for these sizes can, else by a call of it."""
     _need(proj, None, "proj")
     _need(conv_w, torch.float32, "conv_w")
     _need(q_gain, torch.float32, "q_gain")
@@ -1391,7 +1392,7 @@ def conv_norm_rotate(proj: torch.Tensor, items: int, item_qstart: torch.Tensor,
         cos_sin, cos_sin.shape[0], rot_dims, slot_of if has_kv else None,
         k_pages if has_kv else None, v_pages if has_kv else None, page_stride,
         page_size, q_out, heads, kv_heads, dim, vdim, int(has_kv), float(eps),
-        _tag(proj.dtype), error, int(move_tails and tokens == items), ctypes.addressof(moved), _stream()),
+        _tag(proj.dtype), error, int(move_tails and one_each), ctypes.addressof(moved), _stream()),
         "conv_norm_rotate")
     if move_tails and not moved.value:
         conv_tails(proj, item_qstart, item_qlen, item_slots, items, tails, taps)

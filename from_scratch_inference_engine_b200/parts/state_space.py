@@ -106,7 +106,7 @@ class StateSpaceDuality(Mixer):
         items = (ctx.item_qstart, ctx.item_qlen, ctx.item_slots, ctx.num_items)
         ops.ssd_prep(proj, inner, inner + self.channels, *items, cache.state, self.matrix_floats,
                      self.conv, self.conv_bias, self.dt_bias, self.a_log, self.heads, self.vdim, act, decay,
-                     conv_wt=self.conv_by_tap, move_tails=True)
+                     conv_wt=self.conv_by_tap, move_tails=True, one_each=ctx.one_each)
         chunks = {}
         if int(ctx.h_qlen.max()) > 2 * self.CHUNK_TOKENS:
             tiles = ctx.attention_tiles(1, self.CHUNK_TOKENS)

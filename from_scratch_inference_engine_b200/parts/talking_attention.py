@@ -133,7 +133,8 @@ class TalkingWindowAttention(Mixer):
                              cache.k_pages if self.own_keys else None,
                              cache.v_pages if self.own_keys else None,
                              cache.page_stride, group.page_size, q, self.heads, self.kv_heads,
-                             self.dim, self.vdim, self.own_keys, self.eps, ctx.error, ctx.item_qlen)
+                             self.dim, self.vdim, self.own_keys, self.eps, ctx.error, ctx.item_qlen,
+                             one_each=ctx.one_each)
         out = rt.buffer("talking.out", tokens, self.heads * self.vdim, proj.dtype)
         if self.tensor_cores and ctx.num_tokens != ctx.num_items:
             # a step with prompt portions, bfloat16, sizes the tensor-core form takes

@@ -32,7 +32,7 @@ def test_one_launch_is_the_two(heads, vdim, extra, taps, order, dtype):
         mine = state.clone()
         lists = (ints(list(order)), ints([1] * items), ints(slots), items)
         ops.ssd_prep(proj, inner, inner + channels, *lists, mine, matrix, conv, bias, dt_bias, a_log, heads, vdim, act, decay,
-                     conv_wt=conv.t().contiguous(), move_tails=move)
+                     conv_wt=conv.t().contiguous(), move_tails=move, one_each=move)
         if not move:
             ops.ssd_tails(proj, inner, channels, taps, *lists, mine, matrix)
         results.append((act, decay, mine))
@@ -40,6 +40,36 @@ def test_one_launch_is_the_two(heads, vdim, extra, taps, order, dtype):
         assert torch.equal(got.nan_to_num(7e7), want.nan_to_num(7e7))
     assert torch.isnan(results[0][0]).any(1).tolist() == [order.index(t) == 1 for t in range(items)]      # the padding entry's
     assert torch.equal(results[0][2][:, :matrix], state[:, :matrix])
+
+
+# as many tokens as requests, but not one each: a request's second token, and requests without any
+@pytest.mark.parametrize("counts", [(2, 0), (0, 2), (1, 0, 3, 0)])
+def test_as_many_tokens_as_requests(counts):
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(len(counts))
+    rand = lambda *shape: torch.randn(shape, generator=generator, device="cuda")
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    heads, vdim, taps, items = 3, 8, 4, len(counts)
+    inner = heads * vdim
+    channels = inner + 16
+    proj, conv = rand(items, 2 * inner + 24), rand(channels, taps)
+    bias, dt_bias, a_log, state = rand(channels), rand(heads), rand(heads), rand(items, (taps - 1) * channels)
+    lists = (ints([sum(counts[:i]) for i in range(items)]), ints(list(counts)), ints(list(range(items))), items)
+    act, decay, mine = torch.full((items, channels + inner), float("nan"), device="cuda"), torch.empty(items, heads, device="cuda"), state.clone()
+    call = lambda **given: ops.ssd_prep(proj, inner, inner + channels, *lists, mine, 0, conv, bias, dt_bias, a_log, heads, vdim, act,
+                                        decay, conv_wt=conv.t().contiguous(), move_tails=True, **given)
+    call()
+    t = 0
+    for i, n in enumerate(counts):
+        history = torch.cat([state[i].view(taps - 1, channels), proj[t:t + n, inner:inner + channels]]).double()
+        assert torch.equal(mine[i].double().view(taps - 1, channels), history[n:])
+        for r in range(n):
+            want = torch.nn.functional.silu((history[r:r + taps] * conv.t().double()).sum(0) + bias.double())
+            assert ((act[t + r, :channels].double() - want).abs() <= 1e-5 * (1 + want.abs())).all()
+        t += n
+    with pytest.raises(ops.KernelError):                      # said to be one each, and not as many
+        ops.ssd_prep(proj[:1], inner, inner + channels, *lists, mine, 0, conv, bias, dt_bias, a_log, heads, vdim, act, decay,
+                     conv_wt=conv.t().contiguous(), move_tails=True, one_each=True)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

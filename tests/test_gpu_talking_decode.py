@@ -79,11 +79,11 @@ def test_a_page_that_was_given_back():
     assert torch.allclose(*outs, rtol=1e-4, atol=1e-5)
 
 
-# tokens of one request each (tails move in the launch) and longer portions beside them; before the sequence's start; taps 2 to
+# tokens of one request each (tails move in the launch), as many tokens as requests but not one each, and longer portions; before the sequence's start; taps 2 to
 # 4 and a count the row form does not take; without keys of its own; a refused position; a padding entry
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps,rot,qlens", [
-    (16, 4, 128, 128, 4, 128, (1, 1, 1, 1)), (16, 4, 128, 128, 4, 64, (1, 5, 2, 30)), (2, 1, 16, 24, 2, 10, (1, 1, 1, 1)),
+    (16, 4, 128, 128, 4, 128, (1, 1, 1, 1)), (16, 4, 128, 128, 4, 64, (1, 5, 2, 30)), (2, 1, 16, 24, 4, 10, (2, 0, 1, 1)), (2, 1, 16, 24, 2, 10, (1, 1, 1, 1)),
     (3, 1, 40, 8, 3, 0, (1, 1, 3, 1)), (4, 2, 8, 8, 5, 4, (1, 1, 1, 1)), (4, 0, 24, 8, 4, 24, (1, 1, 1, 1))])
 def test_rows_in_one_go(heads, kv_heads, dim, vdim, taps, rot, qlens, dtype):
     from from_scratch_inference_engine_b200.kernels import ops
@@ -107,7 +107,8 @@ def test_rows_in_one_go(heads, kv_heads, dim, vdim, taps, rot, qlens, dtype):
         ops.conv_norm_rotate(proj, items, device(starts), device(pos0), device(slots), tails, conv_w, taps, q_gain,
                              k_gain if has_kv else None, table, rot, slot_of if has_kv else None,
                              pages[:, :kvh * page * dim] if has_kv else None, pages[:, kvh * page * dim:] if has_kv else None,
-                             pages.stride(0), page, q, heads, kv_heads, dim, vdim, has_kv, 1e-6, error, qlen)
+                             pages.stride(0), page, q, heads, kv_heads, dim, vdim, has_kv, 1e-6, error, qlen,
+                             one_each=qlen is not None and set(qlens) == {1})
         return q
     got_pages, got_tails = pages.clone(), tails.clone()
     got = run(proj, got_pages, got_tails, device(list(qlens)))
