@@ -165,7 +165,10 @@ attn_generic_kernel(const AttnParams p) {
 }
 
 // Merge the splits of one (token, head): o = sum_z acc_z e^(m_z - M) / sum_z l_z e^(m_z - M).
-template <typename T>
+// STAGED: maxima, sums and weights wait in shared memory, 12 bytes a split; beyond what a block gets without being asked
+// for more (48 KB), every thread reads them again where it needs them.
+constexpr int COMBINE_STAGED = 4096;
+template <typename T, bool STAGED>
 __global__ void attn_combine_kernel(const float* __restrict__ part_o,
                                     const float* __restrict__ part_ml, T* __restrict__ out,
                                     int out_ld, int tokens, int heads, int hd, int nsplit) {
@@ -176,10 +179,11 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o,
     grid_dependency_wait();
     grid_dependents_go();
     // maxima, sums and the first eight splits' values travel together: none of their addresses depends on another
-    for (int z = threadIdx.x; z < nsplit; z += blockDim.x) {
-        m[z] = part_ml[(z * stride + slot) * 2];
-        l[z] = part_ml[(z * stride + slot) * 2 + 1];
-    }
+    if (STAGED)
+        for (int z = threadIdx.x; z < nsplit; z += blockDim.x) {
+            m[z] = part_ml[(z * stride + slot) * 2];
+            l[z] = part_ml[(z * stride + slot) * 2 + 1];
+        }
     constexpr int AHEAD = 8;
     float ahead[AHEAD];
     auto ask = [&](int z0, int d) {
@@ -189,12 +193,16 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o,
     ask(0, threadIdx.x);
     __syncthreads();
     float mmax = -INFINITY;
-    for (int z = 0; z < nsplit; ++z) mmax = fmaxf(mmax, m[z]);
-    for (int z = threadIdx.x; z < nsplit; z += blockDim.x) w[z] = m[z] == -INFINITY ? 0.f : expf(m[z] - mmax);
+    auto max_of = [&](int z) { return STAGED ? m[z] : part_ml[(z * stride + slot) * 2]; };
+    auto sum_of = [&](int z) { return STAGED ? l[z] : part_ml[(z * stride + slot) * 2 + 1]; };
+    auto weight_of = [&](int z) { return STAGED ? w[z] : expf(max_of(z) - mmax); };      // (of a split with keys)
+    for (int z = 0; z < nsplit; ++z) mmax = fmaxf(mmax, max_of(z));
+    if (STAGED)
+        for (int z = threadIdx.x; z < nsplit; z += blockDim.x) w[z] = m[z] == -INFINITY ? 0.f : expf(m[z] - mmax);
     __syncthreads();
     float denom = 0.f;
     for (int z = 0; z < nsplit; ++z)
-        if (m[z] != -INFINITY) denom += l[z] * w[z];
+        if (max_of(z) != -INFINITY) denom += sum_of(z) * weight_of(z);
     const float inv = denom > 0.f ? 1.0f / denom : 0.f;
     for (int d = threadIdx.x; d < hd; d += blockDim.x) {
         float o = 0.f;
@@ -202,7 +210,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o,
             if (z0 > 0 || d != (int)threadIdx.x) ask(z0, d);
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j)
-                if (z0 + j < nsplit && m[z0 + j] != -INFINITY) o += ahead[j] * w[z0 + j];     // a split without keys may hold anything
+                if (z0 + j < nsplit && max_of(z0 + j) != -INFINITY) o += ahead[j] * weight_of(z0 + j);     // a split without keys may hold anything
         }
         out[(size_t)tok * out_ld + h * hd + d] = from_float<T>(o * inv);
     }
@@ -753,13 +761,13 @@ int fsie_attn_tiles(const void* q, int q_ld, const void* k_pages, const void* v_
     if (rc != 0 || nsplit == 1 || !merge) return rc;
     dim3 cgrid(tokens, heads);
     const int threads = head_dim >= 128 ? 128 : (head_dim >= 64 ? 64 : 32);
-    const size_t room = 3 * (size_t)nsplit * sizeof(float);
-    if (room > 48 * 1024) return ERR_UNSUPPORTED;        // (4,096 splits; the grid's z dimension takes 65,535)
+    const bool staged = nsplit <= COMBINE_STAGED;
+    const size_t room = staged ? 3 * (size_t)nsplit * sizeof(float) : 0;
     if (dtype == DTYPE_F32)
-        return launch_dependent(attn_combine_kernel<float>, cgrid, dim3(threads), room, stream, part_o, part_ml, (float*)out,
-                                out_ld, tokens, heads, head_dim, nsplit);
-    return launch_dependent(attn_combine_kernel<bf16>, cgrid, dim3(threads), room, stream, part_o, part_ml, (bf16*)out, out_ld,
-                            tokens, heads, head_dim, nsplit);
+        return launch_dependent(staged ? attn_combine_kernel<float, true> : attn_combine_kernel<float, false>, cgrid, dim3(threads),
+                                room, stream, part_o, part_ml, (float*)out, out_ld, tokens, heads, head_dim, nsplit);
+    return launch_dependent(staged ? attn_combine_kernel<bf16, true> : attn_combine_kernel<bf16, false>, cgrid, dim3(threads), room,
+                            stream, part_o, part_ml, (bf16*)out, out_ld, tokens, heads, head_dim, nsplit);
 }
 
 // The launch as callers outside the engine know it: tiles of up to 32 rows, merged at once.

@@ -29,3 +29,13 @@ def test_values_that_a_row_does_not_see(ops, hd, heads, kv_heads, window, nsplit
     got = case.run(ops, nsplit)
     assert torch.equal(got[:-1], want[:-1])
     assert not torch.isfinite(got[-1]).any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd,rows16", [(64, False), (128, True), (96, False)])
+def test_more_splits_than_the_merge_stages(ops, hd, rows16, dtype):  # noqa: F811
+    """4,096 splits' maxima and sums fit the merge's shared memory; it takes more, with the same bits (each split has a tile or none)."""
+    case = PagedCase(dtype, 4, 2, hd, 8, [(300, 1), (0, 3)], seed=hd)
+    most, more = (case.run(ops, nsplit, rows16 and dtype is torch.float32) for nsplit in (4096, 4097))
+    assert_rows_close(more, case.want, case, dtype)
+    assert torch.equal(most, more)
