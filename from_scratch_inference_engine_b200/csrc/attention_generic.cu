@@ -701,7 +701,7 @@ int fsie_attn_tiles(const void* q, int q_ld, const void* k_pages, const void* v_
                     const int* item_qstart, const int* item_qlen, const int* item_pos0,
                     void* out, int out_ld, float* part_o, float* part_ml, int tokens, int heads,
                     int kv_heads, int head_dim, int window, int nsplit, float scale, int dtype,
-                    int rows16, int merge, cudaStream_t stream) {
+                    int rows16, int merge, int early, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (tiles > 65535) return ERR_UNSUPPORTED;          // tiles are the grid's y dimension
     if (head_dim <= 0 || head_dim > 32 * MAX_DPL || kv_heads <= 0 || heads % kv_heads != 0 ||
@@ -729,7 +729,7 @@ int fsie_attn_tiles(const void* q, int q_ld, const void* k_pages, const void* v_
 #define FSIE_ROWS16(HDV)                                                                                        \
     case HDV:                                                                                                   \
         cudaFuncSetAttribute(attn_rows16_kernel<HDV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-        rc = launch_dependent(attn_rows16_kernel<HDV>, grid, dim3(FTHREADS), smem, stream, p);                  \
+        rc = launch_dependent_if(early, attn_rows16_kernel<HDV>, grid, dim3(FTHREADS), smem, stream, p);        \
         break;
             switch (head_dim) {
                 FSIE_ROWS16(32) FSIE_ROWS16(64) FSIE_ROWS16(96) FSIE_ROWS16(128) FSIE_ROWS16(256)
@@ -782,7 +782,7 @@ int fsie_attn_generic(const void* q, int q_ld, const void* k_pages, const void* 
     return fsie_attn_tiles(q, q_ld, k_pages, v_pages, page_stride, page_size, block_tables, bt_stride,
                            tile_item, tile_row0, tiles, item_qstart, item_qlen, item_pos0, out, out_ld,
                            part_o, part_ml, tokens, heads, kv_heads, head_dim, window, nsplit, scale,
-                           dtype, 0, 1, stream);
+                           dtype, 0, 1, 0, stream);
 }
 
 }  // extern "C"

@@ -92,12 +92,19 @@ enum { ERR_BAD_ARGUMENT = -1, ERR_UNSUPPORTED = -2 };
 // kernel wrote (and before it writes anything that kernel may read).  A kernel that calls
 // grid_dependents_go() lets the kernel after it be scheduled from that point on.  Both are
 // no-ops for kernels launched the ordinary way.
+//
+// A kernel may read in front of its wait what is older than the kernel before it: what that kernel did not write, and what was
+// complete when that kernel's own wait returned.  The second holds behind a kernel whose blocks all call grid_dependents_go()
+// after their wait and leave after it, as all here do but one: attn_tc_decode_kernel (attention_tcgen05.cu) lets the next kernel
+// go before it waits, so that one may still overlap the kernel in front of it.  Behind it only merges and products run, which
+// read nothing early but weights.
+// Whether its operands are that old a kernel's caller knows: launch_dependent_if() with `early` = 0 launches the ordinary way.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... Params, typename... Args>
-inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
-                            cudaStream_t stream, Args... args) {
+inline int launch_dependent_if(int early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -107,8 +114,14 @@ inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, si
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attr;
-    config.numAttrs = 1;
+    config.numAttrs = early ? 1 : 0;
     return (int)cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                            cudaStream_t stream, Args... args) {
+    return launch_dependent_if(1, kernel, grid, block, smem, stream, args...);
 }
 
 }  // namespace fsie

@@ -37,8 +37,8 @@ template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("c
 // w: one block per SM stays for all of the matrix that falls to it.
 // The step's rows of x come through shared memory in chunks of XC elements, the next chunk copied while the
 // current one is used: one barrier per chunk, none but the first where a row of x is one chunk.
-// Launched as a programmatic dependent: the first rows of w are asked for before the kernel that
-// produces x has finished.
+// Launched as a programmatic dependent (where the caller knows that kernel not to write w): the first rows of w are
+// asked for before the kernel that produces x has finished.
 constexpr int ROWS_MAX_WARPS = 16;
 template <int MT, int R> struct RowsShape {
     static constexpr int XC = MT >= 16 ? 512 : (MT >= 8 ? 1024 : 2048);
@@ -201,7 +201,7 @@ template <int MT, int R> static size_t rows_smem(int warps, int K) {
 
 template <int MT, int R>
 static int launch_rows_as(const float* x, const float* w, const float* bias, float* y, int M, int N,
-                          int K, int ldx, int ldy, int m_tiles, int sms, int warps, cudaStream_t stream) {
+                          int K, int ldx, int ldy, int m_tiles, int sms, int warps, int early, cudaStream_t stream) {
     static bool raised = false;          // per instantiation: the limit of dynamic shared memory
     if (!raised) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -210,7 +210,7 @@ static int launch_rows_as(const float* x, const float* w, const float* bias, flo
         raised = true;
     }
     const int blocks = (N + warps * R - 1) / (warps * R), most = sms / m_tiles > 0 ? sms / m_tiles : 1;
-    return launch_dependent(gemm_f32_rows_kernel<MT, R>, dim3(m_tiles, blocks < most ? blocks : most), dim3(warps * 32),
+    return launch_dependent_if(early, gemm_f32_rows_kernel<MT, R>, dim3(m_tiles, blocks < most ? blocks : most), dim3(warps * 32),
                             rows_smem<MT, R>(warps, K), stream, x, w, bias, y, M, N, K, ldx, ldy);
 }
 
@@ -237,16 +237,16 @@ static float rows_cost(int N, int sms, int m_tiles, int& warps) {
 
 template <int MT>
 static int launch_rows(const float* x, const float* w, const float* bias, float* y, int M, int N,
-                       int K, int ldx, int ldy, int sms, int rows_per_warp, cudaStream_t stream) {
+                       int K, int ldx, int ldy, int sms, int rows_per_warp, int early, cudaStream_t stream) {
     const int m_tiles = (M + MT - 1) / MT;
     int w1 = 1, w2 = 1, w4 = 1;
     const float c1 = rows_cost<MT, 1>(N, sms, m_tiles, w1), c2 = rows_cost<MT, 2>(N, sms, m_tiles, w2),
                 c4 = rows_cost<MT, 4>(N, sms, m_tiles, w4);
     int r = c4 <= c2 && c4 <= c1 ? 4 : (c2 <= c1 ? 2 : 1);
     if (rows_per_warp == 1 || rows_per_warp == 2 || rows_per_warp == 4) r = rows_per_warp;
-    if (r == 4) return launch_rows_as<MT, 4>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w4, stream);
-    if (r == 2) return launch_rows_as<MT, 2>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w2, stream);
-    return launch_rows_as<MT, 1>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w1, stream);
+    if (r == 4) return launch_rows_as<MT, 4>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w4, early, stream);
+    if (r == 2) return launch_rows_as<MT, 2>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w2, early, stream);
+    return launch_rows_as<MT, 1>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w1, early, stream);
 }
 
 // ---------------------------------------------------------------------------- tiles
@@ -322,7 +322,7 @@ extern "C" int fsie_gemm_f32_rows_limit() { return 48; }
 // rows_per_warp: 0 = chosen by size; 1, 2 or 4 fix it for the few-rows kernel (tests, measurements).
 extern "C" int fsie_gemm_f32(const float* x, const float* w, const float* bias, float* y, int M,
                              int N, int K, int ldx, int ldy, int kind, int rows_per_warp,
-                             cudaStream_t stream) {
+                             int early, cudaStream_t stream) {
     using namespace fsie;
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || kind < 0 || kind > 3) return ERR_BAD_ARGUMENT;
@@ -344,9 +344,9 @@ extern "C" int fsie_gemm_f32(const float* x, const float* w, const float* bias, 
     int device = 0, sms = 148;
     if (cudaGetDevice(&device) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (M == 1) return launch_rows<1>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, stream);
-    if (M == 2) return launch_rows<2>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, stream);
-    if (M <= 4) return launch_rows<4>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, stream);
-    if (M <= 8) return launch_rows<8>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, stream);
-    return launch_rows<16>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, stream);
+    if (M == 1) return launch_rows<1>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, early, stream);
+    if (M == 2) return launch_rows<2>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, early, stream);
+    if (M <= 4) return launch_rows<4>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, early, stream);
+    if (M <= 8) return launch_rows<8>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, early, stream);
+    return launch_rows<16>(x, w, bias, y, M, N, K, ldx, ldy, sms, rows_per_warp, early, stream);
 }

@@ -389,7 +389,7 @@ int fsie_latent_prep(const void* proj, int ld, const int* positions, const float
 // x: head h of token t at t * x_ld + h * x_head (k columns); w [heads, n, k]; out: head h of token t
 // at t * out_ld + h * out_head (n columns).
 int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, void* out, long long out_ld,
-                      int out_head, int tokens, int heads, int n, int k, int dtype, cudaStream_t stream) {
+                      int out_head, int tokens, int heads, int n, int k, int dtype, int early, cudaStream_t stream) {
     if (tokens <= 0 || n <= 0) return 0;
     if (heads <= 0 || k <= 0 || heads > 65535) return ERR_BAD_ARGUMENT;
     if (tokens <= HF_TOKENS && (size_t)tokens * k * sizeof(float) <= 96 * 1024) {
@@ -405,7 +405,7 @@ int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, 
         // all of a row's weights in registers: up to 1,024 of them
         if (k % 8 == 0 && k <= 1024 && x_ld % 8 == 0 && x_head % 8 == 0 && ((((size_t)x) | ((size_t)w)) & 15) == 0) {
 #define FSIE_HEAD_ROWS(L, C, T)                                                                                    \
-            launch_dependent(head_product_rows_kernel<L, C, T>,                                                    \
+            launch_dependent_if(early, head_product_rows_kernel<L, C, T>,                                          \
                              dim3((n + HQ_ROWS * HQ_WARPS * 32 / L - 1) / (HQ_ROWS * HQ_WARPS * 32 / L), heads),   \
                              dim3(HQ_WARPS * 32), 0, stream, (const bf16*)x, x_ld, x_head, (const bf16*)w, (bf16*)out, \
                              out_ld, out_head, tokens, n, k)

@@ -70,7 +70,7 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
                       int vdim, const int* __restrict__ seg_item, const int* __restrict__ seg_row0,
                       int seg_tokens, float* __restrict__ chunk_states, int phase, int share,
                       const float* __restrict__ decay_tok, const float* __restrict__ decay_row,
-                      float out_scale, long long state_stride, float* __restrict__ chunk_decay, int early) {
+                      float out_scale, long long state_stride, float* __restrict__ chunk_decay) {
     // tokens staged in shared memory at a time (fewer where q, k and the rows' decays of large heads are staged)
     constexpr int SCAN_TOKENS = ROWS && DR > 8 ? 8 : 16;
     constexpr int PAD = DR > 4 ? DR + 4 : DR;
@@ -80,8 +80,8 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
     __shared__ __align__(16) float vs[SCAN_TOKENS * SCAN_COLS];
     __shared__ float ls[SCAN_TOKENS];                  // the decay of each staged token
     __shared__ __align__(16) float as[ROWS ? SCAN_TOKENS * ROW_LEN : 4];     // ... or of each of its state rows
-    // The lists were staged before the step and are read while the kernel before still runs; so is a request's state (phase 0)
-    // where the caller knows that kernel not to write it (early).
+    // The lists, the decay of a head and a request's state (phase 0) are read while the kernel before still runs: launched
+    // as a dependent only where the caller knows that kernel not to write them.
     const int item = seg_item ? seg_item[blockIdx.z] : blockIdx.z, head = blockIdx.y;
     const int slot = item_slots[item];
     if (slot < 0) {                                    // a padding entry of a fixed-size batch
@@ -110,7 +110,7 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
     };
     const int qk_head = head / share;                  // `share` heads read the same q and k columns
     float through = 1.f;                               // the product of the chunk's decays (phase 1)
-    if (phase != 0 || !early) grid_dependency_wait();  // (chunk_states is the kernel before's)
+    if (phase != 0) grid_dependency_wait();            // (chunk_states is the kernel before's)
     float s[DR][4];
 #pragma unroll
     for (int i = 0; i < DR; ++i) {
@@ -126,7 +126,7 @@ lightning_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
             for (int x = 0; x < 4; ++x) if (col0 + x < vdim) s[i][x] = at[x];
         }
     }
-    if (phase == 0 && early) grid_dependency_wait();
+    if (phase == 0) grid_dependency_wait();
     grid_dependents_go();
     for (int t0 = 0; t0 < count; t0 += SCAN_TOKENS) {
         const int n = min(SCAN_TOKENS, count - t0);
@@ -267,7 +267,7 @@ lightning_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
                       const int* __restrict__ item_qstart, const int* __restrict__ item_qlen,
                       const int* __restrict__ item_slots, float* __restrict__ state, const float* __restrict__ decay,
                       float* __restrict__ out, int heads, int dim, int vdim, int share, const float* __restrict__ decay_tok,
-                      const float* __restrict__ decay_row, float out_scale, long long state_stride, int early) {
+                      const float* __restrict__ decay_row, float out_scale, long long state_stride) {
     constexpr int PAD = DR > 4 ? DR + 4 : DR, ROW_LEN = SCAN_ROW_GROUPS * PAD;
     static_assert(DR % 4 == 0 && DR * SCAN_ROW_GROUPS <= SCAN_COLS / 4 * SCAN_ROW_GROUPS, "a thread's one value of q and k");
     __shared__ __align__(16) float qs[ROW_LEN], ks[ROW_LEN], vs[SCAN_COLS], as[ROWS ? ROW_LEN : 4];
@@ -281,7 +281,6 @@ lightning_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
     const bool mine = col0 < vdim;
     float* at = state + (size_t)slot * state_stride + ((size_t)head * dim + rg * DR) * vdim + col0;
     const float head_decay = decay ? decay[head] : 1.f;
-    if (!early) grid_dependency_wait();
     float s[DR][4];
 #pragma unroll
     for (int i = 0; i < DR; ++i) {
@@ -289,7 +288,7 @@ lightning_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, 
                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
         s[i][0] = v.x; s[i][1] = v.y; s[i][2] = v.z; s[i][3] = v.w;
     }
-    if (early) grid_dependency_wait();
+    grid_dependency_wait();
     grid_dependents_go();
     for (int t = 0; t < count; ++t) {
         const size_t token = start + t;
@@ -603,10 +602,10 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
     const int per_thread = (dim + SCAN_ROW_GROUPS - 1) / SCAN_ROW_GROUPS;
     int launch_code = 0;
 #define FSIE_SCAN(T, R, S, DPT)                                                                  \
-    launch_code = launch_dependent(lightning_scan_kernel<DPT, T, R, S>, grid, threads, 0, stream,   \
+    launch_code = launch_dependent_if(early || phase == 2, lightning_scan_kernel<DPT, T, R, S>, grid, threads, 0, stream, \
         (const T*)proj, ld, q_off, k_off, v_off, item_qstart, item_qlen, item_slots, state,      \
         decay, out, heads, dim, vdim, seg_item, seg_row0, seg_tokens, chunk_states, phase, share, \
-        decay_tok, decay_row, out_scale, state_stride, chunk_decay, early)
+        decay_tok, decay_row, out_scale, state_stride, chunk_decay)
 #define FSIE_SCAN_SIZES(T, R, S)                                                                 \
     do {                                                                                         \
         if (per_thread <= 1) FSIE_SCAN(T, R, S, 1);                                              \
@@ -626,9 +625,9 @@ int fsie_lightning_scan(const void* proj, int ld, int q_off, int k_off, int v_of
     // (heads of up to 32 rows: one or two rows a thread, another order of the sums, and over soon)
     if (!chunked && single && dim > SCAN_ROW_GROUPS * 2 && dim <= SCAN_ROW_GROUPS * 8 && vdim % 4 == 0 && state_stride % 4 == 0 && (((size_t)state) & 15) == 0) {
 #define FSIE_STEP(T, R, S, DPT)                                                                  \
-        launch_dependent(lightning_step_kernel<DPT, T, R, S>, grid, threads, 0, stream,          \
+        launch_dependent_if(early, lightning_step_kernel<DPT, T, R, S>, grid, threads, 0, stream,      \
             (const T*)proj, ld, q_off, k_off, v_off, item_qstart, item_qlen, item_slots, state,  \
-            decay, out, heads, dim, vdim, share, decay_tok, decay_row, out_scale, state_stride, early)
+            decay, out, heads, dim, vdim, share, decay_tok, decay_row, out_scale, state_stride)
 #define FSIE_STEP_SIZES(T, R, S) (per_thread <= 4 ? FSIE_STEP(T, R, S, 4) : FSIE_STEP(T, R, S, 8))
         if (silu) return dtype == DTYPE_F32 ? FSIE_STEP_SIZES(float, false, true) : FSIE_STEP_SIZES(bf16, false, true);
         if (!decay_row) return FSIE_STEP_SIZES(float, false, false);
@@ -688,15 +687,15 @@ int fsie_head_norm_silu(const float* o, const void* proj, int ld, int g_off, con
 }
 
 int fsie_gated_rmsnorm(const float* o, const void* proj, int ld, int g_off, const float* gain,
-                       void* y, int tokens, int width, float eps, int dtype, cudaStream_t stream) {
+                       void* y, int tokens, int width, float eps, int dtype, int early, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
     if (width <= 8 * threads) {             // (longer rows would spill: they are read twice)
         const bool four = width <= 4 * threads;
         if (dtype == DTYPE_F32)
-            return launch_dependent(four ? gated_rmsnorm_regs_kernel<float, 4> : gated_rmsnorm_regs_kernel<float, 8>, tokens, threads,
+            return launch_dependent_if(early, four ? gated_rmsnorm_regs_kernel<float, 4> : gated_rmsnorm_regs_kernel<float, 8>, tokens, threads,
                                     0, stream, o, (const float*)proj, ld, g_off, gain, (float*)y, width, eps);
-        return launch_dependent(four ? gated_rmsnorm_regs_kernel<bf16, 4> : gated_rmsnorm_regs_kernel<bf16, 8>, tokens, threads, 0,
+        return launch_dependent_if(early, four ? gated_rmsnorm_regs_kernel<bf16, 4> : gated_rmsnorm_regs_kernel<bf16, 8>, tokens, threads, 0,
                                 stream, o, (const bf16*)proj, ld, g_off, gain, (bf16*)y, width, eps);
     }
     if (dtype == DTYPE_F32)

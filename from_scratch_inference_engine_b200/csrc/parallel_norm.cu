@@ -192,7 +192,7 @@ extern "C" {
 
 int fsie_sum_layernorm(float* x, const void* d1, const void* d2, const float* gain, const float* bias,
                        const int* rows, void* y, int num_rows, int width, float eps, int write_x,
-                       int dtype, cudaStream_t stream) {
+                       int dtype, int early, cudaStream_t stream) {
     if (num_rows <= 0) return 0;
     if (width <= 0 || !x || (y && !gain)) return ERR_BAD_ARGUMENT;
     const size_t smem = (size_t)width * sizeof(float);
@@ -204,7 +204,7 @@ int fsie_sum_layernorm(float* x, const void* d1, const void* d2, const float* ga
     (smem > 48 * 1024 ? (void)cudaFuncSetAttribute(sum_layernorm_kernel<T, V>,                                 \
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)     \
                       : (void)0,                                                                               \
-     launch_dependent(sum_layernorm_kernel<T, V>, num_rows, threads, smem, stream, x, (const T*)d1, (const T*)d2, \
+     launch_dependent_if(early, sum_layernorm_kernel<T, V>, num_rows, threads, smem, stream, x, (const T*)d1, (const T*)d2, \
                       gain, bias, rows, (T*)y, width, eps, write_x))
     if (dtype == DTYPE_F32) return vec ? FSIE_NORM(float, true) : FSIE_NORM(float, false);
     return vec ? FSIE_NORM(bf16, true) : FSIE_NORM(bf16, false);

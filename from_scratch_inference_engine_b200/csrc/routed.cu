@@ -650,13 +650,14 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
         const bf16* __restrict__ x, long long x_ld, const bf16* __restrict__ w, bf16* __restrict__ out,
         long long out_ld, const int* __restrict__ offsets, const int* __restrict__ sorted,
         const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ meta,
-        int top, int n, int k, int gate_kind, int early) {
+        int top, int n, int k, int gate_kind) {
     constexpr bool GATED = MODE == 1, FIRST = MODE != 0;
     constexpr int COLS = GATED ? 16 : 32;                    // outputs per row and item
     extern __shared__ __align__(128) unsigned char few_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // early: the lists are older than the kernel before, and the first slots of w are asked for while it still runs
-    if (MODE != 0 || !early) {
+    // the second product: the lists are older than the kernel before (else it is not launched as a dependent), and the
+    // first slots of w are asked for while that one still runs
+    if (MODE != 0) {
         grid_dependency_wait();
         grid_dependents_go();
     }
@@ -664,7 +665,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
     // neighbouring items are the tiles of the same columns: an expert's further tiles find its rows in L2
     const int items = tiles * ((n + COLS - 1) / COLS);
     if ((int)blockIdx.x >= items) {
-        if (MODE == 0 && early) grid_dependency_wait();
+        if (MODE == 0) grid_dependency_wait();
         return;
     }
     const int per = (k + FEW_K - 1) / FEW_K;                 // slots per item
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
     };
     static_assert(FEW_THREADS == MOE_FEW_TILE * FEW_PIECES && FEW_ROWS == 2 * MOE_FEW_TILE, "a thread's pieces");
     point();
-    if (MODE == 0 && early) {
+    if (MODE == 0) {
 #pragma unroll
         for (int j = 0; j < FEW_SLOTS - 1; ++j) ask(true, false);
         grid_dependency_wait();
@@ -721,7 +722,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 3) moe_product_few_kernel(
         point();
     }
 #pragma unroll
-    for (int j = 0; j < FEW_SLOTS - 1; ++j) ask(MODE != 0 || !early, true);
+    for (int j = 0; j < FEW_SLOTS - 1; ++j) ask(MODE != 0, true);
 
     // ---- multiplying: warp = (16 rows of w, 8 rows of x)
     const int half = warp & 1, eight = warp >> 1;
@@ -900,9 +901,9 @@ static int launch_few(const void* x, long long x_ld, const void* w, void* out, l
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int cols = MODE == 1 ? FEW_ROWS / 2 : FEW_ROWS;
     const long long most = (long long)tiles * ((n + cols - 1) / cols);
-    return launch_dependent(moe_product_few_kernel<MODE>, dim3((unsigned)(most < 3 * sms ? most : 3 * sms)),
+    return launch_dependent_if(MODE != 0 || early, moe_product_few_kernel<MODE>, dim3((unsigned)(most < 3 * sms ? most : 3 * sms)),
                             dim3(FEW_THREADS), FEW_SMEM, stream, (const bf16*)x, x_ld, (const bf16*)w, (bf16*)out,
-                            out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind, early);
+                            out_ld, offsets, sorted, tile_expert, tile_row0, meta, top, n, k, gate_kind);
 }
 
 // -------------------------------------------------------------------------------- combine

@@ -57,6 +57,7 @@ struct ScaledAttnParams {
     int partial;
     int page_shift;                           // log2(page_size), or -1 where it is no power of two
     int* error;
+    int early;                     // keys in front of the requests' new tokens and the lists are older than the kernel before
 };
 
 // The first key that the query at `pos` sees: the window's start, or the start of its chunk.
@@ -1387,10 +1388,10 @@ static int scaled_attention_mma_launch(const ScaledAttnParams& p, int tiles, boo
     const dim3 grid(p.kv_heads, tiles, p.nsplit);
     if (shared_v) {
         cudaFuncSetAttribute(scaled_attention_mma_kernel<NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return launch_dependent(scaled_attention_mma_kernel<NV, true>, grid, dim3(SA_WARPS * 32), smem, stream, p);
+        return launch_dependent_if(p.early, scaled_attention_mma_kernel<NV, true>, grid, dim3(SA_WARPS * 32), smem, stream, p);
     }
     cudaFuncSetAttribute(scaled_attention_mma_kernel<NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_dependent(scaled_attention_mma_kernel<NV, false>, grid, dim3(SA_WARPS * 32), smem, stream, p);
+    return launch_dependent_if(p.early, scaled_attention_mma_kernel<NV, false>, grid, dim3(SA_WARPS * 32), smem, stream, p);
 }
 
 template <int NVT, bool FEW>
@@ -1399,7 +1400,7 @@ static int scaled_attention_rows_launch(const ScaledAttnParams& p, int tiles, bo
     const dim3 grid(p.kv_heads, tiles, p.nsplit);
     auto* kernel = shared_v ? scaled_attention_rows_kernel<NVT, true, FEW> : scaled_attention_rows_kernel<NVT, false, FEW>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_dependent(kernel, grid, dim3(TR_WARPS * 32), smem, stream, p);
+    return launch_dependent_if(p.early, kernel, grid, dim3(TR_WARPS * 32), smem, stream, p);
 }
 
 template <bool FEW>
@@ -1479,7 +1480,7 @@ int fsie_scaled_attention(const void* q, int q_ld, const float* head_scale, cons
                           const void* head_gate, int head_gate_ld, const float* sink, const float* pos_scale,
                           int pos_len, int maps, int partial, int nsplit,
                           const int* combine_tokens, int num_combine, int dtype, int form, int* error,
-                          cudaStream_t stream) {
+                          int early, cudaStream_t stream) {
     if (tokens <= 0 || tiles <= 0) return 0;
     if (tiles > 65535 || nsplit > 65535) return ERR_UNSUPPORTED;
     if (key_dim <= 0 || value_dim <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || nsplit < 1 ||
@@ -1500,7 +1501,7 @@ int fsie_scaled_attention(const void* q, int q_ld, const float* head_scale, cons
     p.chunk = chunk; p.softcap = softcap; p.gate = gate; p.gate_ld = gate_ld;
     p.head_gate = head_gate; p.head_gate_ld = head_gate_ld; p.sink = sink;
     p.pos_scale = pos_scale; p.pos_len = pos_len; p.maps = maps; p.q_dim = key_dim / maps; p.partial = partial;
-    p.error = error;
+    p.error = error; p.early = early;
     p.page_shift = -1;
     for (int b = 0; b < 30; ++b)
         if (page_size == 1 << b) p.page_shift = b;

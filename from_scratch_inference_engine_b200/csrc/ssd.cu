@@ -281,7 +281,7 @@ int fsie_ssd_prep(const void* proj, int ld, int conv_off, int dt_off, const int*
                   long long state_stride, long long tail_off, const float* conv_w, const float* conv_b,
                   int taps, int channels, const float* dt_bias, const float* a_log, int heads, int vdim,
                   float* act, int act_ld, float* decay, const float* conv_wt, int tokens, int dtype,
-                  int fold_tails, int* folded, cudaStream_t stream) {
+                  int fold_tails, int* folded, int early, cudaStream_t stream) {
     if (folded) *folded = 0;
     if (tokens <= 0 || items <= 0) return 0;
     if (fold_tails && (tokens != items || !folded)) return ERR_BAD_ARGUMENT;
@@ -297,7 +297,7 @@ int fsie_ssd_prep(const void* proj, int ld, int conv_off, int dt_off, const int*
         *folded = 1;
         const dim3 grid(tokens, (channels / 8 + SSD_ROW_THREADS - 1) / SSD_ROW_THREADS);
 #define FSIE_SSD_ROWS(T, N)                                                                                               \
-        launch_dependent(ssd_prep_rows_kernel<T, N>, grid, SSD_ROW_THREADS, 0, stream, (const T*)proj, ld, conv_off, dt_off, \
+        launch_dependent_if(early, ssd_prep_rows_kernel<T, N>, grid, SSD_ROW_THREADS, 0, stream, (const T*)proj, ld, conv_off, dt_off, \
                          item_qstart, item_slots, items, state, state_stride, tail_off, conv_wt, conv_b, channels, dt_bias, \
                          a_log, heads, vdim, act, act_ld, decay)
         if (dtype == DTYPE_F32)
@@ -334,7 +334,7 @@ int fsie_ssd_tails(const void* proj, int ld, int conv_off, const int* item_qstar
 // storage type with z at z_off; skip [heads], gain [inner] float; y [tokens, inner] of the storage type.
 int fsie_ssd_gate_norm(const float* o, const float* act, int act_ld, const void* proj, int ld, int z_off,
                        const float* skip, const float* gain, void* y, int tokens, int inner, int vdim,
-                       int parts, float eps, int dtype, cudaStream_t stream) {
+                       int parts, float eps, int dtype, int early, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (inner <= 0 || vdim <= 0 || inner % vdim || parts <= 0 || inner % parts || parts > 65535)
         return ERR_BAD_ARGUMENT;
@@ -344,10 +344,10 @@ int fsie_ssd_gate_norm(const float* o, const float* act, int act_ld, const void*
     if (width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
         const bool four = width <= 4 * threads;
         if (dtype == DTYPE_F32)
-            return launch_dependent(four ? ssd_gate_norm_regs_kernel<float, 4> : ssd_gate_norm_regs_kernel<float, 8>, grid,
+            return launch_dependent_if(early, four ? ssd_gate_norm_regs_kernel<float, 4> : ssd_gate_norm_regs_kernel<float, 8>, grid,
                                     dim3(threads), 0, stream, o, act, act_ld, (const float*)proj, ld, z_off, skip, gain, (float*)y,
                                     inner, vdim, parts, eps);
-        return launch_dependent(four ? ssd_gate_norm_regs_kernel<bf16, 4> : ssd_gate_norm_regs_kernel<bf16, 8>, grid,
+        return launch_dependent_if(early, four ? ssd_gate_norm_regs_kernel<bf16, 4> : ssd_gate_norm_regs_kernel<bf16, 8>, grid,
                                 dim3(threads), 0, stream, o, act, act_ld, (const bf16*)proj, ld, z_off, skip, gain, (bf16*)y,
                                 inner, vdim, parts, eps);
     }

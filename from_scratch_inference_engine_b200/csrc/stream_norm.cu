@@ -194,14 +194,14 @@ __global__ void __launch_bounds__(512, !FEW && S > 0 && S <= 4 ? 2 : 1) stream_n
 }
 
 template <typename T, int S, int STEP, bool FEW>
-static int stream_norm_launch_as(const StreamNormParams& p, int num_rows, int threads, size_t smem, cudaStream_t stream) {
+static int stream_norm_launch_as(const StreamNormParams& p, int num_rows, int threads, size_t smem, int early, cudaStream_t stream) {
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(stream_norm_kernel<T, S, STEP, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_dependent(stream_norm_kernel<T, S, STEP, FEW>, num_rows, threads, smem, stream, p);
+    return launch_dependent_if(early, stream_norm_kernel<T, S, STEP, FEW>, num_rows, threads, smem, stream, p);
 }
 
 template <typename T, int S, int STEP>
-static int stream_norm_launch(const StreamNormParams& p, int num_rows, cudaStream_t stream) {
+static int stream_norm_launch(const StreamNormParams& p, int num_rows, int early, cudaStream_t stream) {
     const int columns = (p.width + STEP - 1) / STEP;
     // few rows: as many threads as there is work for, so that a row is one trip to memory; many rows:
     // smaller blocks, more of which fit beside one another
@@ -210,22 +210,22 @@ static int stream_norm_launch(const StreamNormParams& p, int num_rows, cudaStrea
                           (S == 0 ? (size_t)p.streams * threads : 0);
     const size_t smem = floats * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
-    return S > 0 && num_rows <= 64 ? stream_norm_launch_as<T, S, STEP, (S > 0)>(p, num_rows, threads, smem, stream)
-                                   : stream_norm_launch_as<T, S, STEP, false>(p, num_rows, threads, smem, stream);
+    return S > 0 && num_rows <= 64 ? stream_norm_launch_as<T, S, STEP, (S > 0)>(p, num_rows, threads, smem, early, stream)
+                                   : stream_norm_launch_as<T, S, STEP, false>(p, num_rows, threads, smem, early, stream);
 }
 
 template <typename T, int STEP>
-static int stream_norm_dispatch(const StreamNormParams& p, int num_rows, cudaStream_t stream) {
+static int stream_norm_dispatch(const StreamNormParams& p, int num_rows, int early, cudaStream_t stream) {
     switch (p.streams) {
-        case 1: return stream_norm_launch<T, 1, STEP>(p, num_rows, stream);
-        case 2: return stream_norm_launch<T, 2, STEP>(p, num_rows, stream);
-        case 3: return stream_norm_launch<T, 3, STEP>(p, num_rows, stream);
-        case 4: return stream_norm_launch<T, 4, STEP>(p, num_rows, stream);
-        case 5: return stream_norm_launch<T, 5, STEP>(p, num_rows, stream);
-        case 6: return stream_norm_launch<T, 6, STEP>(p, num_rows, stream);
-        case 7: return stream_norm_launch<T, 7, STEP>(p, num_rows, stream);
-        case 8: return stream_norm_launch<T, 8, STEP>(p, num_rows, stream);
-        default: return stream_norm_launch<T, 0, 1>(p, num_rows, stream);
+        case 1: return stream_norm_launch<T, 1, STEP>(p, num_rows, early, stream);
+        case 2: return stream_norm_launch<T, 2, STEP>(p, num_rows, early, stream);
+        case 3: return stream_norm_launch<T, 3, STEP>(p, num_rows, early, stream);
+        case 4: return stream_norm_launch<T, 4, STEP>(p, num_rows, early, stream);
+        case 5: return stream_norm_launch<T, 5, STEP>(p, num_rows, early, stream);
+        case 6: return stream_norm_launch<T, 6, STEP>(p, num_rows, early, stream);
+        case 7: return stream_norm_launch<T, 7, STEP>(p, num_rows, early, stream);
+        case 8: return stream_norm_launch<T, 8, STEP>(p, num_rows, early, stream);
+        default: return stream_norm_launch<T, 0, 1>(p, num_rows, early, stream);
     }
 }
 
@@ -238,7 +238,7 @@ extern "C" {
 int fsie_stream_norm(float* x, const float* start, const void* y, const float* y_scale, const float* mix, const float* out,
                      const float* in, const float* gain, const float* bias, const int* rows, void* z,
                      int num_rows, int streams, int width, float eps, int write_x, int centred, int dtype,
-                     cudaStream_t stream) {
+                     int early, cudaStream_t stream) {
     if (num_rows <= 0) return 0;
     if (streams <= 0 || width <= 0 || !x || (y && (!mix || !out)) || (z && !gain) || (!y && !z)) return ERR_BAD_ARGUMENT;
     StreamNormParams p;
@@ -249,8 +249,8 @@ int fsie_stream_norm(float* x, const float* start, const void* y, const float* y
     const size_t stored = (size_t)y | (size_t)z;
     const bool vec = width % 4 == 0 && (wide & 15) == 0 && (stored & (dtype == DTYPE_F32 ? 15 : 7)) == 0;
     if (dtype == DTYPE_F32)
-        return vec ? stream_norm_dispatch<float, 4>(p, num_rows, stream) : stream_norm_dispatch<float, 1>(p, num_rows, stream);
-    return vec ? stream_norm_dispatch<bf16, 4>(p, num_rows, stream) : stream_norm_dispatch<bf16, 1>(p, num_rows, stream);
+        return vec ? stream_norm_dispatch<float, 4>(p, num_rows, early, stream) : stream_norm_dispatch<float, 1>(p, num_rows, early, stream);
+    return vec ? stream_norm_dispatch<bf16, 4>(p, num_rows, early, stream) : stream_norm_dispatch<bf16, 1>(p, num_rows, early, stream);
 }
 
 }  // extern "C"

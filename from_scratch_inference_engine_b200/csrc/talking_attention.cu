@@ -311,7 +311,7 @@ int fsie_conv_norm_rotate(const void* proj, int ld, int tokens, int items, const
                           const float* cos_sin, int table_len, int rot_dims, const int* slot_of,
                           void* k_pages, void* v_pages, long long page_stride, int page_size,
                           float* q_out, int heads, int kv_heads, int dim, int vdim, int has_kv,
-                          float eps, int dtype, int* error, int fold_tails, int* folded, cudaStream_t stream) {
+                          float eps, int dtype, int* error, int fold_tails, int* folded, int early, cudaStream_t stream) {
     if (folded) *folded = 0;
     if (tokens <= 0) return 0;
     if (items <= 0 || taps <= 0 || (taps > 1 && !tails) || rot_dims < 0 || rot_dims > dim || (rot_dims & 1) ||
@@ -326,7 +326,7 @@ int fsie_conv_norm_rotate(const void* proj, int ld, int tokens, int items, const
         const int threads = ((width / 8 + 31) / 32) * 32;
         if (folded) *folded = fold_tails;
 #define FSIE_PREPARE_VEC(T, N, F)                                                                                       \
-        launch_dependent(conv_norm_rotate_vec_kernel<T, N, F>, tokens, threads, kv_heads * sizeof(float), stream, (const T*)proj, ld, items, \
+        launch_dependent_if(early, conv_norm_rotate_vec_kernel<T, N, F>, tokens, threads, kv_heads * sizeof(float), stream, (const T*)proj, ld, items, \
                          item_qstart, item_pos0, item_slots, tails, conv_w, q_gain, k_gain, cos_sin, table_len, rot_dims, \
                          slot_of, (T*)k_pages, (T*)v_pages, page_stride, page_size, q_out, heads, kv_heads, dim, vdim, \
                          has_kv, eps, error)

@@ -35,7 +35,7 @@ struct TalkingArgs {
     int nsplit, mode;              // mode 0: both walks, out; 1: first walk, part_stats; 2: second walk, part_out
     float* part_stats;             // [tiles][nsplit][TA_ROWS][2]
     float* part_out;               // [nsplit][tokens][heads * vdim]
-    int tokens;
+    int tokens, early;             // early: the mixing matrix and the lists are older than the kernel before the first walk
 };
 
 __device__ __forceinline__ void load2(const float* p, float& a, float& b) {
@@ -446,7 +446,7 @@ int talking_attention_launch_tile(const TalkingArgs& a, int num_tiles, int key_t
     const dim3 grid(num_tiles, a.nsplit);
     const auto go = [&](auto kernel) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return launch_dependent(kernel, grid, TA_WARPS * 32, smem, stream, a);
+        return launch_dependent_if(a.early || a.mode == 2, kernel, grid, TA_WARPS * 32, smem, stream, a);
     };
     if constexpr (TOK == 1) {
         if (a.heads <= 2 * TA_WARPS)

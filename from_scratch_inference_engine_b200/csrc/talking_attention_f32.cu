@@ -29,11 +29,11 @@ int fsie_talking_attention(const float* q, const void* k_pages, const void* v_pa
                            const int* item_slots, const float* talk, void* out, int tokens, int heads,
                            int kv_heads, int dim, int vdim, int window, int keep_first, int tile_tokens,
                            float scale, int nsplit, float* part_stats, float* part_out, int dtype,
-                           int* error, cudaStream_t stream) {
+                           int* error, int early, cudaStream_t stream) {
     TalkingArgs a = {q, k_pages, v_pages, page_stride, page_size, block_tables, table_stride,
                      tile_item, tile_row0, item_qstart, item_qlen, item_pos0, item_slots, talk, out,
                      heads, kv_heads, dim, vdim, window, keep_first, tile_tokens, scale, error,
-                     nsplit, 0, part_stats, part_out, tokens};
+                     nsplit, 0, part_stats, part_out, tokens, early};
     if (dtype == DTYPE_F32) return talking_attention_launch<float>(a, num_tiles, stream);
     return fsie_talking_attention_bf16(a, num_tiles, stream);
 }

@@ -235,7 +235,7 @@ class Runtime:
         rows, (n, k) = x.shape[0], weight.shape
         out = self.buffer(tag, rows, n, torch.float32)
         if not f32_split_pays(rows, n, k, self.sm_count) or not ops.gemm_f32_split_takes(x, weight):
-            return ops.gemm_f32(x, weight, bias, out)
+            return ops.gemm_f32(x, weight, bias, out, early=True)
         planes, notes = ops.gemm_f32_split_room(rows, n, k)
         return ops.gemm_f32_split(x, weight, bias, out,
                                   self.buffer("gemm_f32.planes", 1, planes, torch.bfloat16).view(-1),

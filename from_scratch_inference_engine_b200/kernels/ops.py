@@ -4,6 +4,14 @@ Each function checks what the kernel assumes (device, dtype, contiguity, sizes),
 passes the tensors' addresses and the current CUDA stream to the C entry point (`build.fast_calls`: without ctypes),
 and raises on any non-zero return.  There is no other implementation behind these functions: on a
 machine without the compiled library or without a GPU they raise.
+
+Most kernels are launched while the kernel before them on the stream still runs, wait for it, and read in front of that
+wait what a step does not change: weights, gains, biases, scales and tables, the request lists and block tables, a
+recurrence's state, the keys and values in front of the requests' new tokens.  Where the stream's last kernel may have
+made one of these, the function has an argument `early`: False, the default, and its kernel starts behind that one; True
+says that all of them are older than the stream's last kernel (and that this is not `attention_tc_decode`, which may still
+run beside the kernel in front of it).  The functions without the argument (`gemm_skinny` and its forms, `gemm_decode`,
+`add_rmsnorm`, `row_decay`, and those that read no more than positions and lists early) always need them that old.
 """
 
 from __future__ import annotations
@@ -88,13 +96,13 @@ def core():
         lib.fsie_rope_kv_write.argtypes = [p, i, p, p, i, p, p, p, ll, i, i, i, i, i, i, i, i, p, p]
         lib.fsie_swiglu.argtypes = [p, p, ll, i, i, p]
         lib.fsie_place_tokens.argtypes = [p, p, p, p, i, p]
-        lib.fsie_gemm_f32.argtypes = [p, p, p, p, i, i, i, i, i, i, i, p]
+        lib.fsie_gemm_f32.argtypes = [p, p, p, p, i, i, i, i, i, i, i, i, p]
         lib.fsie_gemm_f32_rows_limit.argtypes = []
         lib.fsie_gemm_f32_rows_limit.restype = i
         lib.fsie_attn_generic.argtypes = [p, i, p, p, ll, i, p, i, p, p, i, p, p, p, p, i, p, p,
                                           i, i, i, i, i, i, f, i, p]
         lib.fsie_attn_tiles.argtypes = [p, i, p, p, ll, i, p, i, p, p, i, p, p, p, p, i, p, p,
-                                        i, i, i, i, i, i, f, i, i, i, p]
+                                        i, i, i, i, i, i, f, i, i, i, i, p]
         lib.fsie_attn_tiles.restype = i
         lib.fsie_attn_generic_rows.argtypes = []
         lib.fsie_attn_rows16_rows.argtypes = []
@@ -230,7 +238,7 @@ def gemm_f32_rows_limit() -> int:
 
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor],
              out: Optional[torch.Tensor] = None, kind: str = "auto",
-             rows_per_warp: int = 0) -> torch.Tensor:
+             rows_per_warp: int = 0, early: bool = False) -> torch.Tensor:
     """out = x @ weight.T (+ bias), all float32, plain FFMA.  `kind`
     names one of the three kernels (few rows, tiles, plain) instead of the choice by size;
     `rows_per_warp` (1, 2, 4) fixes how many rows of the weight a warp of the few-rows kernel
@@ -252,7 +260,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]
         raise KernelError("gemm_f32: out must be [rows of x, rows of weight] with unit inner stride")
     _check(core().fsie_gemm_f32(x, weight, bias, out, m, n, k,
                                 x.stride(0), out.stride(0), GEMM_F32_KINDS[kind], int(rows_per_warp),
-                                _stream()),
+                                int(early), _stream()),
            "gemm_f32")
     return out
 
@@ -331,7 +339,7 @@ def attention_generic(q: torch.Tensor, q_ld: int, k_pages: torch.Tensor, v_pages
                       window: int, scale: float, nsplit: int = 1,
                       part_o: Optional[torch.Tensor] = None,
                       part_ml: Optional[torch.Tensor] = None, rows16: bool = False,
-                      merge: bool = True) -> torch.Tensor:
+                      merge: bool = True, early: bool = False) -> torch.Tensor:
     """The 32-bit attention over tiles of up to 32 query rows (any storage, any head size up to
     256), or with `rows16` over tiles of up to 16 rows by the kernel for few rows (float storage,
     head sizes in steps of 4).  `merge=False` leaves the partial results of split key ranges
@@ -356,7 +364,7 @@ def attention_generic(q: torch.Tensor, q_ld: int, k_pages: torch.Tensor, v_pages
                                   item_qstart, item_qlen, item_pos0,
                                   out, out.stride(0), part_o, part_ml, tokens,
                                   heads, kv_heads, head_dim, window, nsplit, float(scale),
-                                  _tag(q.dtype), int(rows16), int(merge), _stream()),
+                                  _tag(q.dtype), int(rows16), int(merge), int(early), _stream()),
            "attention_generic")
     return out
 
@@ -1029,12 +1037,12 @@ def scan():
         lib.fsie_row_decay.argtypes = [p, i, i, i, p, p, f, p, i, i, i, p]
         lib.fsie_head_norm_silu.argtypes = [p, p, i, i, p, p, i, i, i, f, i, p]
         lib.fsie_silu_rows.argtypes = [p, i, i, p, i, i, p]
-        lib.fsie_gated_rmsnorm.argtypes = [p, p, i, i, p, p, i, i, f, i, p]
+        lib.fsie_gated_rmsnorm.argtypes = [p, p, i, i, p, p, i, i, f, i, i, p]
         lib.fsie_ssd_max_taps.argtypes = []
         lib.fsie_ssd_prep.argtypes = [p, i, i, i, p, p, p, i, p, ll, ll, p, p, i, i, p, p, i, i, p, i, p,
-                                      p, i, i, i, p, p]
+                                      p, i, i, i, p, i, p]
         lib.fsie_ssd_tails.argtypes = [p, i, i, p, p, p, i, p, ll, ll, i, i, i, p]
-        lib.fsie_ssd_gate_norm.argtypes = [p, p, i, p, i, i, p, p, p, i, i, i, i, f, i, p]
+        lib.fsie_ssd_gate_norm.argtypes = [p, p, i, p, i, i, p, p, p, i, i, i, i, f, i, i, p]
         for name in ("fsie_lightning_scan", "fsie_row_decay", "fsie_head_norm_silu", "fsie_silu_rows", "fsie_gated_rmsnorm", "fsie_ssd_max_taps",
                      "fsie_ssd_prep", "fsie_ssd_tails", "fsie_ssd_gate_norm"):
             getattr(lib, name).restype = i
@@ -1049,15 +1057,15 @@ def hybrid():
     if _hybrid is None:
         lib = build.load_library("hybrid")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
-        lib.fsie_add_layernorm.argtypes = [p, p, p, p, p, i, i, f, i, i, p]
+        lib.fsie_add_layernorm.argtypes = [p, p, p, p, p, i, i, f, i, i, i, p]
         lib.fsie_cast_rows.argtypes = [p, p, ll, i, p]
         lib.fsie_conv_norm_rotate.argtypes = [p, i, i, i, p, p, p, p, p, i, p, p, p, i, i, p, p, p,
-                                              ll, i, p, i, i, i, i, i, f, i, p, i, p, p]
+                                              ll, i, p, i, i, i, i, i, f, i, p, i, p, i, p]
         lib.fsie_conv_tails.argtypes = [p, i, p, p, p, i, p, i, i, i, p]
         lib.fsie_talking_attention_tile_tokens.argtypes = [i]
         lib.fsie_talking_attention_key_tile.argtypes = [i, i, i, i, i]
         lib.fsie_talking_attention.argtypes = [p, p, p, ll, i, p, i, p, p, i, p, p, p, p, p, p,
-                                               i, i, i, i, i, i, i, i, f, i, p, p, i, p, p]
+                                               i, i, i, i, i, i, i, i, f, i, p, p, i, p, i, p]
         lib.fsie_talking_attention_mma_takes.argtypes = [i, i, i, i]
         lib.fsie_talking_attention_mma.argtypes = [p, p, p, ll, i, p, i, p, p, i, p, p, p, p, p, p, p,
                                                    i, i, i, i, i, i, i, f, p, p]
@@ -1072,7 +1080,7 @@ def hybrid():
 
 
 def layernorm_rows(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.Tensor,
-                   rows: Optional[torch.Tensor] = None) -> torch.Tensor:
+                   rows: Optional[torch.Tensor] = None, early: bool = False) -> torch.Tensor:
     """out[r] = LN(x[rows[r]]) * gain in out's dtype; x is the float32 residual stream.
     LN(v) = (v - mean) / sqrt(mean((v - mean)^2) + eps)."""
     _need(x, torch.float32, "x")
@@ -1089,13 +1097,13 @@ def layernorm_rows(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.T
     if out.numel() < count * width:
         raise KernelError("layernorm_rows: out is too small")
     _check(hybrid().fsie_add_layernorm(x, rows, gain, None, out, count,
-                                       width, float(eps), 0, _tag(out.dtype), _stream()),
+                                       width, float(eps), 0, _tag(out.dtype), int(early), _stream()),
            "layernorm_rows")
     return out
 
 
 def add_layernorm(x: torch.Tensor, delta: torch.Tensor, gain: torch.Tensor, eps: float,
-                  copy: Optional[torch.Tensor]) -> None:
+                  copy: Optional[torch.Tensor], early: bool = False) -> None:
     """x (float32 residual) += LN(delta) * gain; `copy`, when given, gets the new x in delta's
     dtype (what the next matrix product reads)."""
     _need(x, torch.float32, "x")
@@ -1110,7 +1118,7 @@ def add_layernorm(x: torch.Tensor, delta: torch.Tensor, gain: torch.Tensor, eps:
         if copy.numel() < x.numel():
             raise KernelError("add_layernorm: copy is too small")
     _check(hybrid().fsie_add_layernorm(delta, None, gain, x, copy, count,
-                                       width, float(eps), 1, _tag(delta.dtype), _stream()),
+                                       width, float(eps), 1, _tag(delta.dtype), int(early), _stream()),
            "add_layernorm")
 
 
@@ -1160,7 +1168,7 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     `decay_tok` num_segs * heads more, with `decay_row` num_segs * heads * dim more) the
     chunks of long prompts run side by side: each sums its own tokens, the sums are chained into
     the state at every chunk's start, and each chunk runs again from there for its outputs.
-    `early`: the stream's last kernel does not write the state, which may be read while it still runs."""
+    `early`: the stream's last kernel writes neither the state nor `decay` nor the lists, which are read while it still runs."""
     _need(proj, torch.float32 if decay_row is None and not silu else None, "proj")
     if silu and decay_row is not None:
         raise KernelError("lightning_scan: a decay per state row comes with activated projections")
@@ -1217,7 +1225,8 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
              state: Optional[torch.Tensor], tail_off: int, conv_w: torch.Tensor,
              conv_b: Optional[torch.Tensor], dt_bias: torch.Tensor, a_log: torch.Tensor, heads: int,
              vdim: int, act: torch.Tensor, decay: torch.Tensor,
-             conv_wt: Optional[torch.Tensor] = None, move_tails: bool = False, one_each: bool = False) -> None:
+             conv_wt: Optional[torch.Tensor] = None, move_tails: bool = False, one_each: bool = False,
+             early: bool = False) -> None:
     """What a state-space mixer's scan reads, per token of proj [tokens, ld] (the stored projection
     with the convolution's input columns at conv_off and the step sizes at dt_off):
     act [tokens, channels + heads * vdim] float32 = [silu(causal convolution + bias) | dt * x] with x
@@ -1256,7 +1265,7 @@ def ssd_prep(proj: torch.Tensor, conv_off: int, dt_off: int, item_qstart: torch.
                                 conv_b, taps, channels, dt_bias, a_log, heads, vdim,
                                 act, act.stride(0), decay, conv_wt, tokens,
                                 _tag(proj.dtype), int(move_tails and taps > 1 and one_each),
-                                ctypes.addressof(moved), _stream()), "ssd_prep")
+                                ctypes.addressof(moved), int(early), _stream()), "ssd_prep")
     if move_tails and taps > 1 and not moved.value:
         ssd_tails(proj, conv_off, channels, taps, item_qstart, item_qlen, item_slots, items, state, tail_off)
 
@@ -1276,7 +1285,8 @@ def ssd_tails(proj: torch.Tensor, conv_off: int, channels: int, taps: int, item_
 
 
 def ssd_gate_norm(o: torch.Tensor, act: torch.Tensor, proj: torch.Tensor, z_off: int, skip: torch.Tensor,
-                  gain: torch.Tensor, out: torch.Tensor, vdim: int, parts: int, eps: float) -> torch.Tensor:
+                  gain: torch.Tensor, out: torch.Tensor, vdim: int, parts: int, eps: float,
+                  early: bool = False) -> torch.Tensor:
     """out[t] = v / sqrt(mean over each of `parts` equal parts of v^2 + eps) * gain with
     v = (o[t] + skip[head] * x[t]) * silu(z[t]); o float32 [tokens, inner], x the first inner
     columns of act (float32), z = proj[t, z_off : z_off + inner] of the storage type."""
@@ -1292,7 +1302,7 @@ def ssd_gate_norm(o: torch.Tensor, act: torch.Tensor, proj: torch.Tensor, z_off:
         raise KernelError("ssd_gate_norm: shapes do not fit")
     _check(scan().fsie_ssd_gate_norm(o, act, act.stride(0), proj, proj.shape[1], z_off,
                                      skip, gain, out, tokens, inner, vdim, int(parts),
-                                     float(eps), _tag(proj.dtype), _stream()), "ssd_gate_norm")
+                                     float(eps), _tag(proj.dtype), int(early), _stream()), "ssd_gate_norm")
     return out
 
 
@@ -1330,7 +1340,7 @@ def head_norm_silu(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.
 
 
 def gated_rmsnorm(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.Tensor, eps: float,
-                  out: torch.Tensor) -> torch.Tensor:
+                  out: torch.Tensor, early: bool = False) -> torch.Tensor:
     """out[t] = o[t] * rsqrt(mean(o[t]^2) + eps) * gain * sigmoid(proj[t, g_off:g_off + width])."""
     _need(o, torch.float32, "o")
     _need(proj, None, "proj")
@@ -1341,7 +1351,7 @@ def gated_rmsnorm(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.T
         raise KernelError("gated_rmsnorm: shapes do not fit")
     _check(scan().fsie_gated_rmsnorm(o, proj, proj.shape[1], g_off, gain,
                                        out, tokens, width, float(eps), _tag(proj.dtype),
-                                       _stream()), "gated_rmsnorm")
+                                       int(early), _stream()), "gated_rmsnorm")
     return out
 
 
@@ -1354,7 +1364,7 @@ def conv_norm_rotate(proj: torch.Tensor, items: int, item_qstart: torch.Tensor,
                      page_stride: int, page_size: int, q_out: torch.Tensor, heads: int,
                      kv_heads: int, dim: int, vdim: int, has_kv: bool, eps: float,
                      error: torch.Tensor, item_qlen: Optional[torch.Tensor] = None,
-                     one_each: bool = False) -> torch.Tensor:
+                     one_each: bool = False, early: bool = False) -> torch.Tensor:
     """Causal convolution over time of the projected q | k | v rows (earlier rows of the step, or
     the request's tail of taps - 1 rows), RMS norm of the whole q and the whole k with gains,
     rotation of interleaved pairs, per-head RMS of v; q -> q_out (float32), k and v -> pages.
@@ -1392,7 +1402,7 @@ def conv_norm_rotate(proj: torch.Tensor, items: int, item_qstart: torch.Tensor,
         cos_sin, cos_sin.shape[0], rot_dims, slot_of if has_kv else None,
         k_pages if has_kv else None, v_pages if has_kv else None, page_stride,
         page_size, q_out, heads, kv_heads, dim, vdim, int(has_kv), float(eps),
-        _tag(proj.dtype), error, int(move_tails and one_each), ctypes.addressof(moved), _stream()),
+        _tag(proj.dtype), error, int(move_tails and one_each), ctypes.addressof(moved), int(early), _stream()),
         "conv_norm_rotate")
     if move_tails and not moved.value:
         conv_tails(proj, item_qstart, item_qlen, item_slots, items, tails, taps)
@@ -1432,7 +1442,7 @@ def talking_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
                       kv_heads: int, dim: int, vdim: int, window: int, keep_first: int,
                       tile_tokens: int, scale: float, error: torch.Tensor, nsplit: int = 1,
                       part_stats: Optional[torch.Tensor] = None,
-                      part_out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      part_out: Optional[torch.Tensor] = None, early: bool = False) -> torch.Tensor:
     """Softmax attention of q (float32 [tokens, heads * dim]) over the visible keys of the pages
     (j <= i and (window == 0 or i - j < window or j < keep_first)); the normalised weights of all
     heads are mixed by `talk` [heads, heads] before head h applies its own to the values of its
@@ -1463,7 +1473,7 @@ def talking_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         block_tables.stride(0), tile_item, tile_row0, num_tiles, item_qstart,
         item_qlen, item_pos0, item_slots, talk, out, tokens, heads,
         kv_heads, dim, vdim, window, keep_first, tile_tokens, float(scale), nsplit,
-        part_stats, part_out, _tag(k_pages.dtype), error, _stream()),
+        part_stats, part_out, _tag(k_pages.dtype), error, int(early), _stream()),
         "talking_attention")
     return out
 
@@ -1532,7 +1542,7 @@ def mixers():
         lib.fsie_scaled_attention_tile_rows.argtypes = [i, i, i, i, i]
         lib.fsie_scaled_attention_tile_rows.restype = i
         lib.fsie_scaled_attention.argtypes = [p, i, p, p, p, ll, i, i, i, i, p, i, p, p, i, p, p, p, p,
-                                              p, i, p, p, i, i, i, i, i, f, p, i, p, i, p, p, i, i, i, i, p, i, i, i, p, p]
+                                              p, i, p, p, i, i, i, i, i, f, p, i, p, i, p, p, i, i, i, i, p, i, i, i, p, i, p]
         lib.fsie_difference_merge.argtypes = [p, p, p, i, i, i, i, i, f, f, f, p, i, p, i, i, p]
         lib.fsie_norm_rotate_write.argtypes = [p, i, p, p, i, p, p, p, ll, i, i, i, i, i, i, i, p, p, f,
                                                i, i, i, i, p, p]
@@ -1541,7 +1551,7 @@ def mixers():
         lib.fsie_rotate_mix_write.argtypes = [p, i, p, p, i, p, p, p, ll, i, i, i, i, i, i, i, i, p, p,
                                               i, p, p]
         lib.fsie_latent_prep.argtypes = [p, i, p, p, i, p, p, ll, i, p, f, p, i, i, i, i, i, i, i, i, p, p]
-        lib.fsie_head_product.argtypes = [p, ll, i, p, p, ll, i, i, i, i, i, i, p]
+        lib.fsie_head_product.argtypes = [p, ll, i, p, p, ll, i, i, i, i, i, i, i, p]
         for name in ("fsie_norm_add_norm", "fsie_gated_act", "fsie_mingru_scan",
                      "fsie_scaled_attention_rows", "fsie_scaled_attention", "fsie_rotate_mix_write",
                      "fsie_latent_prep", "fsie_head_product", "fsie_norm_rotate_write",
@@ -1659,7 +1669,7 @@ def scaled_attention(q: torch.Tensor, q_ld: int, head_scale: torch.Tensor, k_pag
                      combine_tokens: Optional[torch.Tensor] = None, num_combine: int = 0,
                      head_gate: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None,
                      pos_scale: Optional[torch.Tensor] = None, maps: int = 1,
-                     partial: bool = False) -> Optional[torch.Tensor]:
+                     partial: bool = False, early: bool = False) -> Optional[torch.Tensor]:
     """Causal (optionally windowed; `chunk` > 0: only over the keys j with j // chunk == i // chunk)
     softmax attention of q [tokens, heads x key_dim] over paged keys
     [kv_head][slot][key_dim] and values [kv_head][slot][value_dim] (or, values_in_keys, the first
@@ -1696,7 +1706,7 @@ def scaled_attention(q: torch.Tensor, q_ld: int, head_scale: torch.Tensor, k_pag
         out, heads * value_dim, part_o, part_ml, tokens, heads, kv_heads, window,
         int(chunk), float(softcap), gate, gate_ld, head_gate, head_gate_ld, sink, pos_scale,
         pos_len, int(maps), int(partial), nsplit, combine_tokens, num_combine, _tag(q.dtype),
-        SCALED_ATTENTION_FORMS[form], error, _stream()), "scaled_attention")
+        SCALED_ATTENTION_FORMS[form], error, int(early), _stream()), "scaled_attention")
     return out
 
 
@@ -1852,7 +1862,7 @@ def latent_prep(proj: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tens
 
 
 def head_product(x: torch.Tensor, x_ld: int, x_head: int, weight: torch.Tensor, out: torch.Tensor,
-                 out_ld: int, out_head: int, tokens: int) -> torch.Tensor:
+                 out_ld: int, out_head: int, tokens: int, early: bool = False) -> torch.Tensor:
     """out[t, h, :] = weight[h] @ x[t, h, :] for weight [heads, n, k]; head h of token t of x at
     t * x_ld + h * x_head, of out at t * out_ld + h * out_head.  32-bit sums."""
     _need(x, None, "x", contiguous=False)
@@ -1860,7 +1870,7 @@ def head_product(x: torch.Tensor, x_ld: int, x_head: int, weight: torch.Tensor, 
     _need(out, x.dtype, "out", contiguous=False)
     heads, n, k = weight.shape
     _check(mixers().fsie_head_product(x, x_ld, x_head, weight, out, out_ld, out_head,
-                                      tokens, heads, n, k, _tag(x.dtype), _stream()), "head_product")
+                                      tokens, heads, n, k, _tag(x.dtype), int(early), _stream()), "head_product")
     return out
 
 
@@ -1877,7 +1887,7 @@ def parallel():
     if _parallel is None:
         lib = build.load_library("parallel")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
-        lib.fsie_sum_layernorm.argtypes = [p, p, p, p, p, p, p, i, i, f, i, i, p]
+        lib.fsie_sum_layernorm.argtypes = [p, p, p, p, p, p, p, i, i, f, i, i, i, p]
         lib.fsie_settle_concat.argtypes = [p, p, p, p, p, i, i, i, p]
         lib.fsie_logit_cap.argtypes = [p, ll, f, f, p]
         lib.fsie_sigmoid_gate.argtypes = [p, i, p, i, i, i, i, p]
@@ -1912,7 +1922,7 @@ def routed():
 
 def sum_layernorm(x: torch.Tensor, deltas, gain: Optional[torch.Tensor], bias: Optional[torch.Tensor],
                   eps: float, out: Optional[torch.Tensor], rows: Optional[torch.Tensor] = None,
-                  write_x: bool = True) -> Optional[torch.Tensor]:
+                  write_x: bool = True, early: bool = False) -> Optional[torch.Tensor]:
     """x (float32 residual) += d1 + d2 for the up to two pending sublayer outputs in `deltas`;
     out = (x - mean) / sqrt(mean((x - mean)^2) + eps) * gain + bias in out's dtype.  Without `out`
     the sum alone.  With `rows` (int32 indices) only those rows, into out[0..len(rows)), and x is
@@ -1947,7 +1957,7 @@ def sum_layernorm(x: torch.Tensor, deltas, gain: Optional[torch.Tensor], bias: O
     d2 = deltas[1] if len(deltas) > 1 else None
     _check(parallel().fsie_sum_layernorm(x, d1, d2, gain, bias, rows,
                                        out, count, width, float(eps), int(write_x), _tag(dtype),
-                                       _stream()), "sum_layernorm")
+                                         int(early), _stream()), "sum_layernorm")
     return out
 
 
@@ -2210,7 +2220,7 @@ def streams_lib():
     if _streams is None:
         lib = build.load_library("streams")
         i, f, p = ctypes.c_int, ctypes.c_float, ctypes.c_void_p
-        lib.fsie_stream_norm.argtypes = [p, p, p, p, p, p, p, p, p, p, p, i, i, i, f, i, i, i, p]
+        lib.fsie_stream_norm.argtypes = [p, p, p, p, p, p, p, p, p, p, p, i, i, i, f, i, i, i, i, p]
         lib.fsie_stream_norm.restype = i
         _streams = build.fast_calls(lib)
     return _streams
@@ -2220,7 +2230,8 @@ def stream_norm(x: torch.Tensor, start: Optional[torch.Tensor], delta: Optional[
                 mix: Optional[torch.Tensor], spread: Optional[torch.Tensor], gather: Optional[torch.Tensor],
                 gain: Optional[torch.Tensor], bias: Optional[torch.Tensor], eps: float,
                 out: Optional[torch.Tensor], rows: Optional[torch.Tensor] = None, write_x: bool = True,
-                centred: bool = True, delta_scale: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+                centred: bool = True, delta_scale: Optional[torch.Tensor] = None,
+                early: bool = False) -> Optional[torch.Tensor]:
     """x (float32 [tokens, streams, width]) holds a token's streams; with `start` (float32 [tokens,
     width]) they do not exist yet and every one equals the token's row of it.  A pending sublayer
     output `delta` [tokens, width] (times `delta_scale`, float32 [width], where given) settles first: x_t <- sum_r mix[r, t] x_r + spread[t] delta for all
@@ -2264,6 +2275,6 @@ def stream_norm(x: torch.Tensor, start: Optional[torch.Tensor], delta: Optional[
             raise KernelError("stream_norm: gain, bias or out does not fit")
     _check(streams_lib().fsie_stream_norm(x, start, delta, delta_scale, mix, spread, gather,
                                           gain, bias, rows, out, count, streams, width,
-                                          float(eps), int(write_x), int(centred), _tag(dtype), _stream()),
+                                          float(eps), int(write_x), int(centred), _tag(dtype), int(early), _stream()),
            "stream_norm")
     return out

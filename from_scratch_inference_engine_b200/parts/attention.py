@@ -218,4 +218,4 @@ class GqaAttention(Mixer):
                                   ctx.item_qstart, ctx.item_qlen, ctx.item_pos0, out, tokens,
                                   self.num_heads, self.num_kv_heads, self.head_dim, self.window,
                                   self.scale, nsplit, part_o, part_ml, rows16=rows16,
-                                  merge=index == len(launches) - 1)
+                                  merge=index == len(launches) - 1, early=True)

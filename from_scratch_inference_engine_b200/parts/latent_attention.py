@@ -102,13 +102,13 @@ class LatentAttention(Mixer):
                         self.dim, self.rope_dim, self.rank, self.position.rotary_dim, ctx.error,
                         half_pairs=self.half_pairs)
         ops.head_product(proj, proj.stride(0), self.q_head, self.w_uk_t, qa, self.heads * self.row,
-                         self.row, tokens)
+                         self.row, tokens, early=True)
         over_c = rt.buffer("latent.over_c", tokens, self.heads * self.rank, proj.dtype)
         attend(ctx, rt, qa, self.head_scale, group, cache, over_c, self.heads, 1, self.row, self.rank,
                True, self.window)
         out = rt.buffer("latent.out", tokens, self.heads * self.vdim, proj.dtype)
         ops.head_product(over_c, self.heads * self.rank, self.rank, self.w_uv, out,
-                         self.heads * self.vdim, self.vdim, tokens)
+                         self.heads * self.vdim, self.vdim, tokens, early=True)
         if self.gate:
             first = self.heads * self.q_head + self.row
             ops.sigmoid_gate(out, proj[:, first:first + self.heads * self.vdim])

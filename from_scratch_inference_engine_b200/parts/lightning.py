@@ -84,5 +84,5 @@ class LightningAttention(Mixer):
                            ctx.item_qlen, ctx.item_slots, ctx.num_items, cache.state, self.decay, o,
                            self.heads, self.dim, self.vdim, silu=not chunks, early=True, **chunks)
         gated = rt.buffer("lightning.gated", tokens, self.v_width, proj.dtype)
-        ops.gated_rmsnorm(o, proj, 2 * self.qk_width + self.v_width, self.gain, self.eps, gated)
+        ops.gated_rmsnorm(o, proj, 2 * self.qk_width + self.v_width, self.gain, self.eps, gated, early=True)
         return rt.linear(gated, self.w_o, None, "lightning.out")

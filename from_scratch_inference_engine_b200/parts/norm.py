@@ -72,7 +72,7 @@ class StreamNorm:
         out = self.runtime.buffer(tag, count, self.width, self.runtime.dtype)
         return ops.stream_norm(x, pending.start, pending.delta, pending.mix, pending.spread, gather, gain, bias,
                                self.eps, out, rows=rows, write_x=write_x, centred=self.centred,
-                               delta_scale=pending.scale)
+                               delta_scale=pending.scale, early=True)
 
 
 @register_part("norm", "rmsnorm")
@@ -187,14 +187,14 @@ class LayerNorm(StreamNorm, Part):
         count = x.shape[0] if rows is None else rows.numel()
         out = self.runtime.buffer(tag, count, self.width, self.runtime.dtype)
         if delta is None and self.bias is None:
-            return ops.layernorm_rows(x, self.gain, self.eps, out, rows=rows)
+            return ops.layernorm_rows(x, self.gain, self.eps, out, rows=rows, early=True)
         deltas = delta.deltas if isinstance(delta, PendingSum) else (delta,)
         return ops.sum_layernorm(x, deltas, self.gain, self.bias, self.eps, out, rows=rows,
-                                 write_x=write_x)
+                                 write_x=write_x, early=True)
 
     def accumulate(self, x: torch.Tensor, delta: torch.Tensor,
                    copy: Optional[torch.Tensor]) -> None:
         """x += LN(delta) * gain; `copy` (compute dtype) receives the new x when given."""
         if self.bias is not None:
             raise ValueError("LayerNorm.accumulate takes a norm without bias")
-        ops.add_layernorm(x, delta, self.gain, self.eps, copy)
+        ops.add_layernorm(x, delta, self.gain, self.eps, copy, early=True)

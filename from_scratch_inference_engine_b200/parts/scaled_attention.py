@@ -106,7 +106,7 @@ def attend(ctx, rt, q: torch.Tensor, head_scale: torch.Tensor, group, cache: Lay
                              tiles.count, ctx.item_qstart, ctx.item_qlen, ctx.item_pos0,
                              ctx.item_slots, out, tokens, heads, kv_heads, window, ctx.error,
                              nsplit, *parts, form=class_form, combine_tokens=class_tokens, num_combine=count,
-                             **extras)
+                             early=True, **extras)
         if merge is not None:
             merge(*parts, nsplit, class_tokens, count)
     return out

@@ -106,7 +106,8 @@ class StateSpaceDuality(Mixer):
         items = (ctx.item_qstart, ctx.item_qlen, ctx.item_slots, ctx.num_items)
         ops.ssd_prep(proj, inner, inner + self.channels, *items, cache.state, self.matrix_floats,
                      self.conv, self.conv_bias, self.dt_bias, self.a_log, self.heads, self.vdim, act, decay,
-                     conv_wt=self.conv_by_tap, move_tails=True, one_each=ctx.one_each)
+                     conv_wt=self.conv_by_tap, move_tails=True, one_each=ctx.one_each,
+                     early=True)
         chunks = {}
         if int(ctx.h_qlen.max()) > 2 * self.CHUNK_TOKENS:
             tiles = ctx.attention_tiles(1, self.CHUNK_TOKENS)
@@ -120,5 +121,5 @@ class StateSpaceDuality(Mixer):
                            ctx.item_slots, ctx.num_items, cache.state, None, o, self.heads, self.state,
                            self.vdim, share=self.heads // self.groups, decay_tok=decay, early=True, **chunks)
         gated = rt.buffer("state_space.gated", tokens, inner, proj.dtype)
-        ops.ssd_gate_norm(o, act, proj, 0, self.skip, self.gain, gated, self.vdim, self.norm_groups, self.eps)
+        ops.ssd_gate_norm(o, act, proj, 0, self.skip, self.gain, gated, self.vdim, self.norm_groups, self.eps, early=True)
         return rt.linear(gated, self.w_o, None, "state_space.out")

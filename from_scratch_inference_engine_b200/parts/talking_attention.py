@@ -134,7 +134,7 @@ class TalkingWindowAttention(Mixer):
                              cache.v_pages if self.own_keys else None,
                              cache.page_stride, group.page_size, q, self.heads, self.kv_heads,
                              self.dim, self.vdim, self.own_keys, self.eps, ctx.error, ctx.item_qlen,
-                             one_each=ctx.one_each)
+                             one_each=ctx.one_each, early=True)
         out = rt.buffer("talking.out", tokens, self.heads * self.vdim, proj.dtype)
         if self.tensor_cores and ctx.num_tokens != ctx.num_items:
             # a step with prompt portions, bfloat16, sizes the tensor-core form takes
@@ -164,5 +164,5 @@ class TalkingWindowAttention(Mixer):
                               ctx.item_qstart, ctx.item_qlen, ctx.item_pos0, ctx.item_slots,
                               self.talk, out, self.heads, self.kv_heads, self.dim, self.vdim,
                               self.window, self.keep_first, tile_tokens, self.scale, ctx.error,
-                              nsplit, part_stats, part_out)
+                              nsplit, part_stats, part_out, early=True)
         return rt.linear(out, self.w_o, None, "talking.o")
