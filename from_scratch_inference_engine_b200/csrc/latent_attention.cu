@@ -399,7 +399,7 @@ int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, 
         if (dtype == DTYPE_F32) {
             if (smem > 48 * 1024)
                 cudaFuncSetAttribute(head_product_few_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            return launch_dependent(head_product_few_kernel<float>, few, dim3(HF_WARPS * 32), smem, stream, (const float*)x,
+            return launch_dependent_if(early, head_product_few_kernel<float>, few, dim3(HF_WARPS * 32), smem, stream, (const float*)x,
                                     x_ld, x_head, (const float*)w, (float*)out, out_ld, out_head, tokens, n, k);
         }
         // all of a row's weights in registers: up to 1,024 of them
@@ -417,7 +417,7 @@ int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, 
         }
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(head_product_few_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return launch_dependent(head_product_few_kernel<bf16>, few, dim3(HF_WARPS * 32), smem, stream, (const bf16*)x,
+        return launch_dependent_if(early, head_product_few_kernel<bf16>, few, dim3(HF_WARPS * 32), smem, stream, (const bf16*)x,
                                 x_ld, x_head, (const bf16*)w, (bf16*)out, out_ld, out_head, tokens, n, k);
     }
     if (dtype == DTYPE_BF16 && k % 8 == 0 && x_ld % 8 == 0 && x_head % 8 == 0 && out_ld % 2 == 0 && out_head % 2 == 0 &&
