@@ -233,7 +233,7 @@ def test_attention(form, nsplit):
     ops.cast_rows(source, pages[-24 * STRIDE:])
     assert torch.equal(go(), want)
     # without `early` all keys may be that new: the older ones as well, by a launch over all pages
-    everything = pages.float()
+    everything = pages.float().clone()
     pages.fill_(float("nan"))
     go = call(q, False)
     ops.cast_rows(everything, pages)
