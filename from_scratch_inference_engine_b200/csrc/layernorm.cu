@@ -123,15 +123,16 @@ extern "C" {
 
 // accumulate = 0: src is float [*, width] (read at `rows` if given), y gets the normed rows.
 // accumulate = 1: src is of the storage type, x (float) += LN(src) * gain, y (optional) = T(x).
+// general != 0: the kernel for rows of any width, whatever the width.
 int fsie_add_layernorm(const void* src, const int* rows, const float* gain, float* x, void* y,
                        int num_rows, int width, float eps, int accumulate, int dtype,
-                       int early, cudaStream_t stream) {
+                       int general, int early, cudaStream_t stream) {
     if (num_rows <= 0) return 0;
     if (width <= 0 || (!accumulate && !y) || (accumulate && !x)) return ERR_BAD_ARGUMENT;
     const size_t smem = (size_t)width * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    if (width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
+    if (!general && width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
 #define FSIE_LN_REGS(S, T, PER)                                                                                     \
         launch_dependent_if(early, add_layernorm_regs_kernel<S, T, PER>, num_rows, threads, 0, stream, (const S*)src, rows, gain, \
                          accumulate ? x : nullptr, (T*)y, width, eps)

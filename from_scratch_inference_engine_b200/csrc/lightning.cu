@@ -687,10 +687,10 @@ int fsie_head_norm_silu(const float* o, const void* proj, int ld, int g_off, con
 }
 
 int fsie_gated_rmsnorm(const float* o, const void* proj, int ld, int g_off, const float* gain,
-                       void* y, int tokens, int width, float eps, int dtype, int early, cudaStream_t stream) {
+                       void* y, int tokens, int width, float eps, int dtype, int general, int early, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    if (width <= 8 * threads) {             // (longer rows would spill: they are read twice)
+    if (!general && width <= 8 * threads) { // (longer rows would spill: they are read twice)
         const bool four = width <= 4 * threads;
         if (dtype == DTYPE_F32)
             return launch_dependent_if(early, four ? gated_rmsnorm_regs_kernel<float, 4> : gated_rmsnorm_regs_kernel<float, 8>, tokens, threads,

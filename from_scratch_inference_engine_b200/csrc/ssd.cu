@@ -334,14 +334,14 @@ int fsie_ssd_tails(const void* proj, int ld, int conv_off, const int* item_qstar
 // storage type with z at z_off; skip [heads], gain [inner] float; y [tokens, inner] of the storage type.
 int fsie_ssd_gate_norm(const float* o, const float* act, int act_ld, const void* proj, int ld, int z_off,
                        const float* skip, const float* gain, void* y, int tokens, int inner, int vdim,
-                       int parts, float eps, int dtype, int early, cudaStream_t stream) {
+                       int parts, float eps, int dtype, int general, int early, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (inner <= 0 || vdim <= 0 || inner % vdim || parts <= 0 || inner % parts || parts > 65535)
         return ERR_BAD_ARGUMENT;
     const int width = inner / parts;
     const dim3 grid(tokens, parts);
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    if (width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
+    if (!general && width <= 8 * threads) { // (longer rows would spill: they stay in shared memory)
         const bool four = width <= 4 * threads;
         if (dtype == DTYPE_F32)
             return launch_dependent_if(early, four ? ssd_gate_norm_regs_kernel<float, 4> : ssd_gate_norm_regs_kernel<float, 8>, grid,

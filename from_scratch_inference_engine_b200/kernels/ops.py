@@ -1037,12 +1037,12 @@ def scan():
         lib.fsie_row_decay.argtypes = [p, i, i, i, p, p, f, p, i, i, i, p]
         lib.fsie_head_norm_silu.argtypes = [p, p, i, i, p, p, i, i, i, f, i, p]
         lib.fsie_silu_rows.argtypes = [p, i, i, p, i, i, p]
-        lib.fsie_gated_rmsnorm.argtypes = [p, p, i, i, p, p, i, i, f, i, i, p]
+        lib.fsie_gated_rmsnorm.argtypes = [p, p, i, i, p, p, i, i, f, i, i, i, p]
         lib.fsie_ssd_max_taps.argtypes = []
         lib.fsie_ssd_prep.argtypes = [p, i, i, i, p, p, p, i, p, ll, ll, p, p, i, i, p, p, i, i, p, i, p,
                                       p, i, i, i, p, i, p]
         lib.fsie_ssd_tails.argtypes = [p, i, i, p, p, p, i, p, ll, ll, i, i, i, p]
-        lib.fsie_ssd_gate_norm.argtypes = [p, p, i, p, i, i, p, p, p, i, i, i, i, f, i, i, p]
+        lib.fsie_ssd_gate_norm.argtypes = [p, p, i, p, i, i, p, p, p, i, i, i, i, f, i, i, i, p]
         for name in ("fsie_lightning_scan", "fsie_row_decay", "fsie_head_norm_silu", "fsie_silu_rows", "fsie_gated_rmsnorm", "fsie_ssd_max_taps",
                      "fsie_ssd_prep", "fsie_ssd_tails", "fsie_ssd_gate_norm"):
             getattr(lib, name).restype = i
@@ -1057,7 +1057,7 @@ def hybrid():
     if _hybrid is None:
         lib = build.load_library("hybrid")
         i, f, ll, p = ctypes.c_int, ctypes.c_float, ctypes.c_longlong, ctypes.c_void_p
-        lib.fsie_add_layernorm.argtypes = [p, p, p, p, p, i, i, f, i, i, i, p]
+        lib.fsie_add_layernorm.argtypes = [p, p, p, p, p, i, i, f, i, i, i, i, p]
         lib.fsie_cast_rows.argtypes = [p, p, ll, i, p]
         lib.fsie_conv_norm_rotate.argtypes = [p, i, i, i, p, p, p, p, p, i, p, p, p, i, i, p, p, p,
                                               ll, i, p, i, i, i, i, i, f, i, p, i, p, i, p]
@@ -1080,9 +1080,10 @@ def hybrid():
 
 
 def layernorm_rows(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.Tensor,
-                   rows: Optional[torch.Tensor] = None, early: bool = False) -> torch.Tensor:
+                   rows: Optional[torch.Tensor] = None, early: bool = False,
+                   general: bool = False) -> torch.Tensor:
     """out[r] = LN(x[rows[r]]) * gain in out's dtype; x is the float32 residual stream.
-    LN(v) = (v - mean) / sqrt(mean((v - mean)^2) + eps)."""
+    LN(v) = (v - mean) / sqrt(mean((v - mean)^2) + eps).  `general`: by the kernel for rows of any width (the same bits)."""
     _need(x, torch.float32, "x")
     _need(gain, torch.float32, "gain")
     _need(out, None, "out")
@@ -1097,15 +1098,15 @@ def layernorm_rows(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.T
     if out.numel() < count * width:
         raise KernelError("layernorm_rows: out is too small")
     _check(hybrid().fsie_add_layernorm(x, rows, gain, None, out, count,
-                                       width, float(eps), 0, _tag(out.dtype), int(early), _stream()),
+                                       width, float(eps), 0, _tag(out.dtype), int(general), int(early), _stream()),
            "layernorm_rows")
     return out
 
 
 def add_layernorm(x: torch.Tensor, delta: torch.Tensor, gain: torch.Tensor, eps: float,
-                  copy: Optional[torch.Tensor], early: bool = False) -> None:
+                  copy: Optional[torch.Tensor], early: bool = False, general: bool = False) -> None:
     """x (float32 residual) += LN(delta) * gain; `copy`, when given, gets the new x in delta's
-    dtype (what the next matrix product reads)."""
+    dtype (what the next matrix product reads).  `general` as in `layernorm_rows`."""
     _need(x, torch.float32, "x")
     _need(delta, None, "delta")
     _need(gain, torch.float32, "gain")
@@ -1118,7 +1119,7 @@ def add_layernorm(x: torch.Tensor, delta: torch.Tensor, gain: torch.Tensor, eps:
         if copy.numel() < x.numel():
             raise KernelError("add_layernorm: copy is too small")
     _check(hybrid().fsie_add_layernorm(delta, None, gain, x, copy, count,
-                                       width, float(eps), 1, _tag(delta.dtype), int(early), _stream()),
+                                       width, float(eps), 1, _tag(delta.dtype), int(general), int(early), _stream()),
            "add_layernorm")
 
 
@@ -1286,10 +1287,10 @@ def ssd_tails(proj: torch.Tensor, conv_off: int, channels: int, taps: int, item_
 
 def ssd_gate_norm(o: torch.Tensor, act: torch.Tensor, proj: torch.Tensor, z_off: int, skip: torch.Tensor,
                   gain: torch.Tensor, out: torch.Tensor, vdim: int, parts: int, eps: float,
-                  early: bool = False) -> torch.Tensor:
+                  early: bool = False, general: bool = False) -> torch.Tensor:
     """out[t] = v / sqrt(mean over each of `parts` equal parts of v^2 + eps) * gain with
     v = (o[t] + skip[head] * x[t]) * silu(z[t]); o float32 [tokens, inner], x the first inner
-    columns of act (float32), z = proj[t, z_off : z_off + inner] of the storage type."""
+    columns of act (float32), z = proj[t, z_off : z_off + inner] of the storage type.  `general` as in `layernorm_rows`."""
     _need(o, torch.float32, "o")
     _need(act, torch.float32, "act")
     _need(proj, None, "proj")
@@ -1302,7 +1303,7 @@ def ssd_gate_norm(o: torch.Tensor, act: torch.Tensor, proj: torch.Tensor, z_off:
         raise KernelError("ssd_gate_norm: shapes do not fit")
     _check(scan().fsie_ssd_gate_norm(o, act, act.stride(0), proj, proj.shape[1], z_off,
                                      skip, gain, out, tokens, inner, vdim, int(parts),
-                                     float(eps), _tag(proj.dtype), int(early), _stream()), "ssd_gate_norm")
+                                     float(eps), _tag(proj.dtype), int(general), int(early), _stream()), "ssd_gate_norm")
     return out
 
 
@@ -1340,8 +1341,9 @@ def head_norm_silu(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.
 
 
 def gated_rmsnorm(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.Tensor, eps: float,
-                  out: torch.Tensor, early: bool = False) -> torch.Tensor:
-    """out[t] = o[t] * rsqrt(mean(o[t]^2) + eps) * gain * sigmoid(proj[t, g_off:g_off + width])."""
+                  out: torch.Tensor, early: bool = False, general: bool = False) -> torch.Tensor:
+    """out[t] = o[t] * rsqrt(mean(o[t]^2) + eps) * gain * sigmoid(proj[t, g_off:g_off + width]).  `general` as in
+    `layernorm_rows`."""
     _need(o, torch.float32, "o")
     _need(proj, None, "proj")
     _need(gain, torch.float32, "gain")
@@ -1351,7 +1353,7 @@ def gated_rmsnorm(o: torch.Tensor, proj: torch.Tensor, g_off: int, gain: torch.T
         raise KernelError("gated_rmsnorm: shapes do not fit")
     _check(scan().fsie_gated_rmsnorm(o, proj, proj.shape[1], g_off, gain,
                                        out, tokens, width, float(eps), _tag(proj.dtype),
-                                       int(early), _stream()), "gated_rmsnorm")
+                                       int(general), int(early), _stream()), "gated_rmsnorm")
     return out
 
 

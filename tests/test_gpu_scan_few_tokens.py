@@ -63,3 +63,16 @@ def test_gated_norm_rows(width, dtype):
     got = ops.gated_rmsnorm(o, proj, 16, gain, 1e-6, torch.empty(3, width, device="cuda", dtype=dtype))
     want = o.double() / (o.double().square().mean(-1, keepdim=True) + 1e-6).sqrt() * gain * torch.sigmoid(proj[:, 16:].double())
     assert ((got.double() - want).abs() <= 1e-5 * (1 + want.abs()) + (2.0 ** -8 * want.abs() if dtype is torch.bfloat16 else 0)).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [8, 264, 500, 512, 700, 1024, 1025, 2048, 2049, 4096])
+def test_gated_norm_rows_are_the_general_kernels(width, dtype):
+    """The row in registers leaves the bits of the kernel for rows of any width."""
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(width)
+    rand = lambda *shape: torch.randn(shape, generator=generator, device="cuda")
+    o, proj, gain = rand(40, width), rand(40, width + 16).to(dtype), rand(width)
+    got, want = (ops.gated_rmsnorm(o, proj, 16, gain, 1e-6, torch.empty(40, width, device="cuda", dtype=dtype), general=general)
+                 for general in (False, True))
+    assert torch.equal(got, want)

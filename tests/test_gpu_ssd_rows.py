@@ -73,7 +73,8 @@ def test_as_many_tokens_as_requests(counts):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("heads,vdim,parts", [(64, 64, 1), (4, 8, 2), (3, 24, 1), (64, 128, 1), (65, 128, 1), (3, 12, 1)])
+@pytest.mark.parametrize("heads,vdim,parts", [(64, 64, 1), (4, 8, 2), (3, 24, 1), (64, 128, 1), (65, 128, 1), (3, 12, 1),
+                                              (25, 40, 1), (16, 64, 1), (16, 64, 2), (31, 64, 1), (40, 50, 1)])
 def test_gated_norm(heads, vdim, parts, dtype):
     from from_scratch_inference_engine_b200.kernels import ops
     generator = torch.Generator(device="cuda").manual_seed(heads + vdim)
@@ -86,5 +87,8 @@ def test_gated_norm(heads, vdim, parts, dtype):
     v = (o.double() + skip.double().repeat_interleave(vdim) * act[:, :inner].double()) * z * torch.sigmoid(z)
     norm = v.view(tokens, parts, -1)
     want = (norm / (norm.square().mean(-1, keepdim=True) + 1e-5).sqrt()).view(tokens, inner) * gain.double()
+    # the row in registers leaves the bits of the kernel for rows of any width
+    general = ops.ssd_gate_norm(o, act, proj, 8, skip, gain, torch.empty_like(y), vdim, parts, 1e-5, general=True)
+    assert torch.equal(y, general)
     # a few roundings of numbers of the order of one, times the gain, then one to the storage type
     assert ((y.double() - want).abs() <= 2e-5 * (1 + want.abs()) + (2.0 ** -8 * want.abs() if dtype is torch.bfloat16 else 0)).all()

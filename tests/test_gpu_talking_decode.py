@@ -145,3 +145,21 @@ def test_layer_norm_rows(width, dtype):
     want = x.double() + norm(delta)
     assert ((sum_.double() - want).abs() <= 1e-5 * (1 + want.abs())).all()      # the sum stays 32-bit
     assert torch.equal(copy, sum_.to(dtype))
+
+
+# widths at which a thread has at most four values and at most eight (with each number of threads), and rows that end inside
+@pytest.mark.parametrize("width", [3, 264, 500, 512, 700, 1024, 1025, 2000, 2048, 2049, 4096])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_layer_norm_rows_are_the_general_kernels(width, dtype):
+    """The row in registers leaves the bits of the kernel for rows of any width."""
+    from from_scratch_inference_engine_b200.kernels import ops
+    generator = torch.Generator(device="cuda").manual_seed(width)
+    src, gain, x = (torch.randn(shape, generator=generator, device="cuda") * 3 + 1.5 for shape in ((40, width), (width,), (40, width)))
+    results = []
+    for general in (False, True):
+        y, copy = (torch.full((40, width), float("nan"), device="cuda", dtype=dtype) for _ in range(2))
+        sum_ = x.clone()
+        ops.layernorm_rows(src, gain, 1e-6, y, general=general)
+        ops.add_layernorm(sum_, src.to(dtype), gain, 1e-6, copy, general=general)
+        results.append((y, sum_, copy))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
