@@ -32,15 +32,15 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o, const floa
         mz_hi = part_ml[((lane + 32) * stride + slot) * 2];
         lz_hi = part_ml[((lane + 32) * stride + slot) * 2 + 1];
     }
-    // the first sixteen splits' values are asked for at once, beside the maxima and sums above: their
-    // addresses do not depend on those (one trip to memory instead of two in a row, three beyond eight splits)
+    // the first eight splits' values are asked for at once, beside the maxima and sums above: their
+    // addresses do not depend on those (one trip to memory instead of two in a row)
     const int d_first = threadIdx.x * 2;
-    constexpr int AHEAD = 16;
-    float2 ahead[AHEAD];
+    float2 ahead[8];
 #pragma unroll
-    for (int j = 0; j < AHEAD; ++j) {
-        ahead[j] = j < nsplit && d_first < HD ? *reinterpret_cast<const float2*>(part_o + (j * stride + slot) * HD + d_first)
-                                              : make_float2(0.f, 0.f);
+    for (int j = 0; j < 8; ++j) {
+        const int z = min(j, nsplit - 1);
+        ahead[j] = d_first < HD ? *reinterpret_cast<const float2*>(part_o + (z * stride + slot) * HD + d_first)
+                                : make_float2(0.f, 0.f);
     }
     const float mmax = warp_max(fmaxf(mz, mz_hi));
     const float wz = mz == -INFINITY ? 0.f : __expf(mz - mmax);
@@ -55,24 +55,23 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o, const floa
         const int d = d0 + threadIdx.x * 2;
         const bool mine = d < HD;
         float a0 = 0.f, a1 = 0.f;
-        for (int z0 = 0; z0 < nsplit; z0 += AHEAD) {
-            // sixteen splits' values are asked for before the first is used: one trip to memory for
-            // all, not sixteen trips
-            float2 v[AHEAD];
+        for (int z0 = 0; z0 < nsplit; z0 += 8) {
+            // eight splits' values are asked for before the first is used: one trip to memory for
+            // eight, not eight trips
+            float2 v[8];
 #pragma unroll
-            for (int j = 0; j < AHEAD; ++j) {
-                const int z = z0 + j;
+            for (int j = 0; j < 8; ++j) {
+                const int z = min(z0 + j, nsplit - 1);
                 if (d0 == 0 && z0 == 0) v[j] = ahead[j];
-                else v[j] = mine && z < nsplit ? *reinterpret_cast<const float2*>(part_o + (z * stride + slot) * HD + d)
-                                               : make_float2(0.f, 0.f);
+                else v[j] = mine ? *reinterpret_cast<const float2*>(part_o + (z * stride + slot) * HD + d)
+                                 : make_float2(0.f, 0.f);
             }
 #pragma unroll
-            for (int j = 0; j < AHEAD; ++j) {
-                const int z = z0 + j;
-                if (z >= nsplit) break;                    // (a prompt's tokens have two or three splits, and are many: 7.5 -> 6.3 us)
+            for (int j = 0; j < 8; ++j) {
+                const int z = min(z0 + j, MAX_KEY_SPLITS - 1);
                 const float lo = __shfl_sync(0xffffffffu, wz, z & 31), hi = __shfl_sync(0xffffffffu, wz_hi, z & 31);
                 const float w = z < 32 ? lo : hi;
-                if (w != 0.f) { a0 += v[j].x * w; a1 += v[j].y * w; }   // a split without keys may hold anything
+                if (z0 + j < nsplit && w != 0.f) { a0 += v[j].x * w; a1 += v[j].y * w; }   // a split without keys may hold anything
             }
         }
         if (mine) {
