@@ -907,7 +907,11 @@ static int launch_few(const void* x, long long x_ld, const void* w, void* out, l
 }
 
 // -------------------------------------------------------------------------------- combine
-template <typename T, bool VEC>
+// VEC: eight columns per thread, 16-byte accesses; the sums run in the same order.  AHEAD > 0: so many choices' rows travel together,
+// where one after the other, each behind its id and place, they were the launch's time for few tokens (8 of 8 choices of 4,096
+// 5.6 -> 3.2 us).  Not more than there are choices: rows asked for twice and their registers cost 2,048 tokens of one
+// choice 4.3 -> 5.6.
+template <typename T, bool VEC, int AHEAD>
 __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float* __restrict__ weights,
                                    const T* __restrict__ shared, const int* __restrict__ place,
                                    T* __restrict__ out, int width, int top, const int* __restrict__ ids,
@@ -916,10 +920,7 @@ __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float
     grid_dependents_go();
     const size_t t = blockIdx.x;
     // a choice at or beyond `experts` is an identity expert: its output is the token's input row
-    // eight columns per thread, 16-byte accesses; the sums run in the same order.  Four choices' rows travel together: one after
-    // the other, each behind its id and place, they were the launch's time.
-    if (VEC) {
-        constexpr int AHEAD = 4;
+    if constexpr (VEC && AHEAD > 0) {
         for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
             float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, v[8];
             for (int j0 = 0; j0 < top; j0 += AHEAD) {
@@ -933,13 +934,37 @@ __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float
                     src[j] = own ? y + t * y_ld : expert_out + (place ? (own ? 0 : (size_t)place[at]) : at) * width;
                 }
 #pragma unroll
-                for (int j = 0; j < AHEAD; ++j) load8(src[j] + c, rows[j]);
+                for (int j = 0; j < AHEAD; ++j)
+                    if (j0 + j < top) load8(src[j] + c, rows[j]);
 #pragma unroll
                 for (int j = 0; j < AHEAD; ++j)
                     if (j0 + j < top) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) acc[i] = fmaf(w[j], rows[j][i], acc[i]);
                     }
+            }
+            if (shared) {
+                load8(shared + t * width + c, v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i] += v[i];
+            }
+            store8(out + t * width + c, acc);
+        }
+        return;
+    }
+    if constexpr (VEC) {
+        for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
+            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, v[8];
+            for (int j = 0; j < top; ++j) {
+                const float w = weights[t * top + j];
+                if (ids && ids[t * top + j] >= experts) {
+                    load8(y + t * y_ld + c, v);
+                } else {
+                    const size_t row = place ? (size_t)place[t * top + j] : t * top + j;
+                    load8(expert_out + row * width + c, v);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, v[i], acc[i]);
             }
             if (shared) {
                 load8(shared + t * width + c, v);
@@ -1106,11 +1131,18 @@ int fsie_moe_combine(const void* expert_out, const float* weights, const void* s
     const bool vec = width % 8 == 0 && (!ids || y_ld % 8 == 0) &&
         (((size_t)expert_out | (size_t)shared | (size_t)out | (size_t)y) & 15) == 0;
     const int threads = vec ? (width >= 2048 ? 256 : (width >= 1024 ? 128 : 64)) : (width >= 1024 ? 256 : 128);
-#define FSIE_COMBINE(T, V) launch_dependent(moe_combine_kernel<T, V>, tokens, threads, 0, stream, (const T*)expert_out, \
+    // Many tokens: one choice's row after the other, by more warps at a time, except four or eight choices in the order of their
+    // tokens.  us one after the other and together, 2,048 tokens of 2,048: 4 choices 7.2 and 6.1, 8 of 4,096 39 and 28, but 5 choices 8.3
+    // and 9.6, 6 with their places looked up 7.0 and 9.8; 512 tokens: 2 choices with places 2.4 and 2.5, 5 3.1 and 4.0.
+    const int ahead = tokens > 256 && (place || top % 4) ? 0 : (top < 3 ? top : 4);
+#define FSIE_COMBINE(T, V, A) launch_dependent(moe_combine_kernel<T, V, A>, tokens, threads, 0, stream, (const T*)expert_out, \
                                             weights, (const T*)shared, place, (T*)out, width, top, ids, experts, \
                                             (const T*)y, y_ld)
-    if (dtype == DTYPE_F32) return vec ? FSIE_COMBINE(float, true) : FSIE_COMBINE(float, false);
-    return vec ? FSIE_COMBINE(bf16, true) : FSIE_COMBINE(bf16, false);
+#define FSIE_COMBINE_AS(T)                                                                                          \
+    (!vec ? FSIE_COMBINE(T, false, 0) : ahead == 0 ? FSIE_COMBINE(T, true, 0) : ahead == 1 ? FSIE_COMBINE(T, true, 1) \
+     : ahead == 2 ? FSIE_COMBINE(T, true, 2) : FSIE_COMBINE(T, true, 4))
+    return dtype == DTYPE_F32 ? FSIE_COMBINE_AS(float) : FSIE_COMBINE_AS(bf16);
+#undef FSIE_COMBINE_AS
 #undef FSIE_COMBINE
 }
 
