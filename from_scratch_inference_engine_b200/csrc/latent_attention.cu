@@ -402,8 +402,14 @@ int fsie_head_product(const void* x, long long x_ld, int x_head, const void* w, 
             return launch_dependent_if(early, head_product_few_kernel<float>, few, dim3(HF_WARPS * 32), smem, stream, (const float*)x,
                                     x_ld, x_head, (const float*)w, (float*)out, out_ld, out_head, tokens, n, k);
         }
-        // all of a row's weights in registers: up to 1,024 of them
-        if (k % 8 == 0 && k <= 1024 && x_ld % 8 == 0 && x_head % 8 == 0 && ((((size_t)x) | ((size_t)w)) & 15) == 0) {
+        // All of a row's weights in registers: up to 1,024 of them.  A launch of that kernel takes 2.8 us for up to 8 tokens and 4.6 for
+        // 16, the one below 1.2 and 0.18 to 0.26 a token until its warps, one per output row, fill the SMs, so small products
+        // of short rows stay with it: (heads x outputs x k) 4 x 32 x 128 with 5 tokens 2.3 us, 2.6 by the other, with 9 3.5 and 4.6,
+        // with 8 3.1 and 2.7; 16 x 128 x 64 with 9 3.4 and 4.6, 16 x 256 x 128 with 9 5.0 and 4.6; one token of 8 x 64 x 128 1.5 and 1.6
+        const int last = tokens & 7;
+        const bool small = tokens == 1 ? heads * n < 1024 && k <= 256
+                                       : tokens > 4 && heads * n < 4096 && k <= 128 && !(k > 64 && (last == 0 || last == 7));
+        if (!small && k % 8 == 0 && k <= 1024 && x_ld % 8 == 0 && x_head % 8 == 0 && ((((size_t)x) | ((size_t)w)) & 15) == 0) {
 #define FSIE_HEAD_ROWS(L, C, T)                                                                                    \
             launch_dependent_if(early, head_product_rows_kernel<L, C, T>,                                          \
                              dim3((n + HQ_ROWS * HQ_WARPS * 32 / L - 1) / (HQ_ROWS * HQ_WARPS * 32 / L), heads),   \

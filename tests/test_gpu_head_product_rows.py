@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 # hold nothing; k that the kernel does not take, and rows that do not start on 16 bytes
 @pytest.mark.parametrize("tokens", [1, 4, 5, 8, 9, 16])
 @pytest.mark.parametrize("heads,n,k,gap", [(16, 512, 128, 8), (2, 40, 32, 0), (3, 129, 200, 16), (5, 128, 512, 8), (1, 17, 1024, 8),
-                                           (2, 19, 776, 8), (2, 24, 44, 4), (2, 32, 64, 4), (1, 8, 1032, 8)])
+                                           (2, 19, 776, 8), (2, 24, 44, 4), (2, 32, 64, 4), (1, 8, 1032, 8),
+                                           (130, 33, 40, 8), (64, 65, 128, 8), (32, 40, 256, 8)])
 def test_head_product(tokens, heads, n, k, gap):
     from from_scratch_inference_engine_b200.kernels import ops
     generator = torch.Generator(device="cuda").manual_seed(n + k)
