@@ -132,14 +132,22 @@ int fsie_add_layernorm(const void* src, const int* rows, const float* gain, floa
     const size_t smem = (size_t)width * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    if (!general && width <= 8 * threads) {             // (longer rows would spill: they stay in shared memory)
-#define FSIE_LN_REGS(S, T, PER)                                                                                     \
+    const int values = (width + threads - 1) / threads;
+    // (longer rows would spill: they stay in shared memory.  So do many plain ones of five to seven values a thread: us in
+    // shared memory and in registers, 2,048 rows of 2,304 14.6 and 15.9, of 3,072 16.4 and 17.6, of 1,536 8.2 and 8.4; of 2,048 values,
+    // four a thread, 10.3 and 9.4, of 4,096 24.2 and 23.7; with the sum, which reads a row more, of 2,304 17.8 and 16.6)
+    if (!general && values <= 8 && (accumulate || values < 5 || values == 8 || !many_rows(num_rows, threads))) {
+#define FSIE_LN_REGS(S, T, PER)                                                                                               \
         launch_dependent_if(early, add_layernorm_regs_kernel<S, T, PER>, num_rows, threads, 0, stream, (const S*)src, rows, gain, \
-                         accumulate ? x : nullptr, (T*)y, width, eps)
-        const bool four = width <= 4 * threads;
-        if (dtype == DTYPE_F32) return four ? FSIE_LN_REGS(float, float, 4) : FSIE_LN_REGS(float, float, 8);
-        if (accumulate) return four ? FSIE_LN_REGS(bf16, bf16, 4) : FSIE_LN_REGS(bf16, bf16, 8);
-        return four ? FSIE_LN_REGS(float, bf16, 4) : FSIE_LN_REGS(float, bf16, 8);
+                            accumulate ? x : nullptr, (T*)y, width, eps)
+#define FSIE_LN_F32(PER) FSIE_LN_REGS(float, float, PER)
+#define FSIE_LN_SUM(PER) FSIE_LN_REGS(bf16, bf16, PER)
+#define FSIE_LN_BF16(PER) FSIE_LN_REGS(float, bf16, PER)
+        if (dtype == DTYPE_F32) return FSIE_BY_VALUES(values, FSIE_LN_F32);
+        return accumulate ? FSIE_BY_VALUES(values, FSIE_LN_SUM) : FSIE_BY_VALUES(values, FSIE_LN_BF16);
+#undef FSIE_LN_F32
+#undef FSIE_LN_SUM
+#undef FSIE_LN_BF16
 #undef FSIE_LN_REGS
     }
     int code = 0;

@@ -690,13 +690,19 @@ int fsie_gated_rmsnorm(const float* o, const void* proj, int ld, int g_off, cons
                        void* y, int tokens, int width, float eps, int dtype, int general, int early, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    if (!general && width <= 8 * threads) { // (longer rows would spill: they are read twice)
-        const bool four = width <= 4 * threads;
-        if (dtype == DTYPE_F32)
-            return launch_dependent_if(early, four ? gated_rmsnorm_regs_kernel<float, 4> : gated_rmsnorm_regs_kernel<float, 8>, tokens, threads,
-                                    0, stream, o, (const float*)proj, ld, g_off, gain, (float*)y, width, eps);
-        return launch_dependent_if(early, four ? gated_rmsnorm_regs_kernel<bf16, 4> : gated_rmsnorm_regs_kernel<bf16, 8>, tokens, threads, 0,
-                                stream, o, (const bf16*)proj, ld, g_off, gain, (bf16*)y, width, eps);
+    const int values = (width + threads - 1) / threads;
+    // (longer rows would spill: they are read twice.  So are many of eight values a thread while L2 still has them from the first
+    // time: rows of 4,096, us read twice and in registers, 1,600 17.8 and 19.4, 2,048 23.2 and 24.1, but 3,000 45.4 and 40.4)
+    const bool again = values == 8 && many_rows(tokens, threads) && (long long)tokens * width < 10 << 20;
+    if (!general && values <= 8 && !again) {
+#define FSIE_GATED_REGS(T, PER) launch_dependent_if(early, gated_rmsnorm_regs_kernel<T, PER>, tokens, threads, 0, stream, o, \
+                                                    (const T*)proj, ld, g_off, gain, (T*)y, width, eps)
+#define FSIE_GATED_F32(PER) FSIE_GATED_REGS(float, PER)
+#define FSIE_GATED_BF16(PER) FSIE_GATED_REGS(bf16, PER)
+        return dtype == DTYPE_F32 ? FSIE_BY_VALUES(values, FSIE_GATED_F32) : FSIE_BY_VALUES(values, FSIE_GATED_BF16);
+#undef FSIE_GATED_F32
+#undef FSIE_GATED_BF16
+#undef FSIE_GATED_REGS
     }
     if (dtype == DTYPE_F32)
         return launch_dependent(gated_rmsnorm_kernel<float>, tokens, threads, 0, stream, o,

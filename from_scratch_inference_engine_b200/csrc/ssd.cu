@@ -341,15 +341,19 @@ int fsie_ssd_gate_norm(const float* o, const float* act, int act_ld, const void*
     const int width = inner / parts;
     const dim3 grid(tokens, parts);
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-    if (!general && width <= 8 * threads) { // (longer rows would spill: they stay in shared memory)
-        const bool four = width <= 4 * threads;
-        if (dtype == DTYPE_F32)
-            return launch_dependent_if(early, four ? ssd_gate_norm_regs_kernel<float, 4> : ssd_gate_norm_regs_kernel<float, 8>, grid,
-                                    dim3(threads), 0, stream, o, act, act_ld, (const float*)proj, ld, z_off, skip, gain, (float*)y,
-                                    inner, vdim, parts, eps);
-        return launch_dependent_if(early, four ? ssd_gate_norm_regs_kernel<bf16, 4> : ssd_gate_norm_regs_kernel<bf16, 8>, grid,
-                                dim3(threads), 0, stream, o, act, act_ld, (const bf16*)proj, ld, z_off, skip, gain, (bf16*)y,
-                                inner, vdim, parts, eps);
+    const int values = (width + threads - 1) / threads;
+    // (longer rows would spill: they stay in shared memory.  So do many of six values a thread and more: us in shared memory and
+    // in registers, 2,048 rows of 3,072 28.2 and 31.5, of 4,096 37.9 and 40.5, of 1,536 14.4 and 14.9; of 2,304, five a
+    // thread, 22.1 and 22.2, of 2,048 20.4 and 20.0)
+    if (!general && values <= 8 && (values < 6 || !many_rows((long long)tokens * parts, threads))) {
+#define FSIE_SSD_NORM(T, PER) launch_dependent_if(early, ssd_gate_norm_regs_kernel<T, PER>, grid, dim3(threads), 0, stream, o, act, act_ld, \
+                                                  (const T*)proj, ld, z_off, skip, gain, (T*)y, inner, vdim, parts, eps)
+#define FSIE_SSD_NORM_F32(PER) FSIE_SSD_NORM(float, PER)
+#define FSIE_SSD_NORM_BF16(PER) FSIE_SSD_NORM(bf16, PER)
+        return dtype == DTYPE_F32 ? FSIE_BY_VALUES(values, FSIE_SSD_NORM_F32) : FSIE_BY_VALUES(values, FSIE_SSD_NORM_BF16);
+#undef FSIE_SSD_NORM_F32
+#undef FSIE_SSD_NORM_BF16
+#undef FSIE_SSD_NORM
     }
     const size_t smem = (size_t)width * sizeof(float);
     if (smem > 200 * 1024) return ERR_UNSUPPORTED;

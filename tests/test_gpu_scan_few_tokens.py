@@ -66,7 +66,7 @@ def test_gated_norm_rows(width, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("width", [8, 264, 500, 512, 700, 1024, 1025, 2048, 2049, 4096])
+@pytest.mark.parametrize("width", [8, 130, 264, 500, 512, 700, 1024, 1025, 1300, 1700, 2000, 2048, 2049, 4096])
 def test_gated_norm_rows_are_the_general_kernels(width, dtype):
     """The row in registers leaves the bits of the kernel for rows of any width."""
     from from_scratch_inference_engine_b200.kernels import ops

@@ -74,7 +74,8 @@ def test_as_many_tokens_as_requests(counts):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,vdim,parts", [(64, 64, 1), (4, 8, 2), (3, 24, 1), (64, 128, 1), (65, 128, 1), (3, 12, 1),
-                                              (25, 40, 1), (16, 64, 1), (16, 64, 2), (31, 64, 1), (40, 50, 1)])
+                                              (25, 40, 1), (16, 64, 1), (16, 64, 2), (31, 64, 1), (40, 50, 1), (9, 40, 1),
+                                              (26, 50, 1), (34, 50, 1), (50, 64, 1)])
 def test_gated_norm(heads, vdim, parts, dtype):
     from from_scratch_inference_engine_b200.kernels import ops
     generator = torch.Generator(device="cuda").manual_seed(heads + vdim)

@@ -147,8 +147,8 @@ def test_layer_norm_rows(width, dtype):
     assert torch.equal(copy, sum_.to(dtype))
 
 
-# widths at which a thread has at most four values and at most eight (with each number of threads), and rows that end inside
-@pytest.mark.parametrize("width", [3, 264, 500, 512, 700, 1024, 1025, 2000, 2048, 2049, 4096])
+# every number of values a thread, one to eight, with each number of threads; rows that end inside
+@pytest.mark.parametrize("width", [3, 130, 264, 500, 512, 700, 1024, 1025, 1300, 1700, 2000, 2048, 2049, 4096])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_layer_norm_rows_are_the_general_kernels(width, dtype):
     """The row in registers leaves the bits of the kernel for rows of any width."""
