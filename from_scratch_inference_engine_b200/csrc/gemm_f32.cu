@@ -217,7 +217,9 @@ static int launch_rows_as(const float* x, const float* w, const float* bias, flo
 // How long the SM with most rows of w is busy, in clocks per pass: what is least decides the rows per warp and
 // the warps per block.  Of a pass of one row (512 bytes) an SM takes in 27 bytes a clock; shared memory moves 128
 // bytes a clock, the row in and out and MT rows of x for R rows of w; an instruction per clock and scheduler
-// gives 4 MT products for 32 lanes.  Fewer than 48 KB on their way leave the SM waiting.
+// gives 4 MT products for 32 lanes.  Fewer than 48 KB on their way leave the SM waiting.  A block that stays for many
+// rounds has 12 or 16 warps: the last round's idle warps are few against what an uneven share of the four schedulers and
+// fewer warps to switch between cost (8 rows, 151,936 x 1,536: 6 warps 223 us, 12 171; 2 rows: 13 warps 147 to 167, 12 135).
 template <int MT, int R>
 static float rows_cost(int N, int sms, int m_tiles, int& warps) {
     using S = RowsShape<MT, R>;
@@ -228,6 +230,7 @@ static float rows_cost(int N, int sms, int m_tiles, int& warps) {
     for (int count = ROWS_MAX_WARPS; count >= 4; --count) {
         const int blocks = (N + count * R - 1) / (count * R), grid = blocks < most ? blocks : most;
         const int rounds = (blocks + grid - 1) / grid;
+        if (rounds > 4 && count != 12 && count != 16) continue;       // (see above)
         const float wait = fmaxf(1.f, 48.f * 1024.f / ((float)count * S::WARP_BYTES));
         const float cost = (float)rounds * count * R * clocks * wait;
         if (cost < best) { best = cost; warps = count; }
@@ -243,6 +246,10 @@ static int launch_rows(const float* x, const float* w, const float* bias, float*
     const float c1 = rows_cost<MT, 1>(N, sms, m_tiles, w1), c2 = rows_cost<MT, 2>(N, sms, m_tiles, w2),
                 c4 = rows_cost<MT, 4>(N, sms, m_tiles, w4);
     int r = c4 <= c2 && c4 <= c1 ? 4 : (c2 <= c1 ? 2 : 1);
+    // where not even every SM has four rows of w, a warp's own chain from pass to pass is what takes the time, and it is
+    // shorter for one row than for two (8 rows of x, 256 x 1,536: 6.6 us with two, 5.8; 512 x 4,096 11.7 and 10.7; a row of one
+    // chunk is over before that shows: 256 x 256 2.6 and 3.5)
+    if (MT == 8 && N <= 4 * sms && K > RowsShape<MT, 1>::XC) { r = 1; w1 = 8; }
     if (rows_per_warp == 1 || rows_per_warp == 2 || rows_per_warp == 4) r = rows_per_warp;
     if (r == 4) return launch_rows_as<MT, 4>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w4, early, stream);
     if (r == 2) return launch_rows_as<MT, 2>(x, w, bias, y, M, N, K, ldx, ldy, m_tiles, sms, w2, early, stream);

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 # all SMs hold at once, with one chunk and with several
 @pytest.mark.parametrize("rows_per_warp", [0, 1, 2, 4])
 @pytest.mark.parametrize("m,n,k", [(1, 3, 4), (1, 9603, 2048), (2, 9603, 2052), (3, 20001, 2176), (4, 70, 8960), (5, 20001, 1028),
-                                   (8, 9603, 1536), (9, 20001, 516), (16, 300, 3588), (17, 9603, 640), (48, 77, 132)])
+                                   (8, 9603, 1536), (9, 20001, 516), (16, 300, 3588), (17, 9603, 640), (48, 77, 132),
+                                   (8, 592, 1028), (5, 593, 1028), (6, 100, 1024), (2, 150001, 132)])
 def test_few_rows(m, n, k, rows_per_warp):
     from from_scratch_inference_engine_b200.kernels import ops
     generator = torch.Generator(device="cuda").manual_seed(m + n + k)
