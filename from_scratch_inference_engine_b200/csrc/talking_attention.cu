@@ -143,7 +143,13 @@ __global__ void conv_norm_rotate_kernel(const T* __restrict__ proj, int ld, int 
 // do it, so that both leave the same bits.
 // FOLD (every request brings one token): the row's own channels move the request's tail on as well, which conv_tails
 // does otherwise (a longer portion's first tokens still read the old tail when its last one is done).
+// Rows of up to 6,144 channels fit a block of 768 threads with the registers that eight channels of four taps take.  A prompt's rows are
+// many, and there the chain counts less than how many rows an SM holds: two blocks of up to 384 threads, one of more.  With the
+// tails' launch, general kernel and this one, us: 2,048 tokens of 3,072 channels 69 and 58, of 3,584 77 and 88, of 5,120 102
+// and 108, of 6,144 121 and 122 to 130; 1,300 of 3,584 55 and 59, of 6,144 85 and 81; 700 of 3,584 37 and 37, of 6,144 58 and 51.
 constexpr int CONV_VEC_WIDTH = 6144;
+constexpr int CONV_VEC_SHARED = 3072;    // channels up to which two rows share an SM
+constexpr int CONV_VEC_TOKENS = 1024;    // tokens up to which longer rows take this kernel all the same
 __host__ __device__ constexpr int conv_threads(int width) { return width >= 1024 ? 512 : 256; }     // of the general kernel
 template <typename T, int TAPS, bool FOLD>
 __global__ void __launch_bounds__(CONV_VEC_WIDTH / 8)
@@ -322,7 +328,7 @@ int fsie_conv_norm_rotate(const void* proj, int ld, int tokens, int items, const
     const bool vec = taps >= 2 && taps <= 4 && dim % 8 == 0 && vdim % 8 == 0 && width <= CONV_VEC_WIDTH && ld % per == 0 &&
         (!has_kv || !k_pages || (page_stride % per == 0 && ((((size_t)k_pages) | ((size_t)v_pages)) & 15) == 0)) &&
         ((((size_t)proj) | ((size_t)tails) | ((size_t)conv_w) | ((size_t)q_gain) | ((size_t)k_gain) | ((size_t)q_out)) & 15) == 0;
-    if (vec) {
+    if (vec && (fold_tails || tokens <= CONV_VEC_TOKENS || width <= CONV_VEC_SHARED)) {
         const int threads = ((width / 8 + 31) / 32) * 32;
         if (folded) *folded = fold_tails;
 #define FSIE_PREPARE_VEC(T, N, F)                                                                                       \
