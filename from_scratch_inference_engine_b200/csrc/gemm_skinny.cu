@@ -24,7 +24,6 @@ constexpr int SK_WARPS = 16;
 constexpr int SK_CHUNK = 32;         // k elements per warp and step: 4 lanes x 16 bytes per row
 constexpr int SK_AHEAD = 4;          // chunks whose weights a warp has asked for (a ring of 4 KB per warp)
 constexpr int SK_DEEP = 8;           // the same where an SM has one block at most and a warp more chunks than SK_AHEAD
-constexpr int SK_SMS = 148;
 
 struct SkinnyParams {
     const bf16* w; const bf16* x; long long ldx;
@@ -64,16 +63,17 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // GATED: w holds N gate rows and then N up rows, the block's 16 rows are 8 gate rows and the 8 up rows of the
 // same outputs, and the epilogue is silu(gate) * up on the two as bfloat16 would store them: the bits of a
 // product and the SwiGLU kernel behind it, without that launch (1 token of 8,960 x 1,536 14.0 -> 11.4 us, 16 tokens of 2,816 x 2,048 11.4 -> 8.6).
-// A matrix of more tiles of 16 rows than the GPU holds blocks has the blocks stay and go on to their next tile: the ring runs on
+// STAYS: a matrix of more tiles of 16 rows than the GPU holds blocks has the blocks stay and go on to their next tile: the ring runs on
 // across tiles, where a block of its own for every tile of, say, 8,960 x 1,536 (three chunks per warp) was asked, waited and gone
 // (11.4 us of a token's step, 9.5 now).  With one block per SM or less the ring is twice as deep (1,536 x 8,960: 8.0 -> 6.8 us).
-// Neither changes which warp adds up what: the same bits.
-template <int TT, bool ROPE, bool GATED, int AHEAD>
+// Neither changes which warp adds up what: the same bits.  A block of one tile is compiled without the loop, whose registers
+// cost 9 to 16 tokens 5 to 23 % (2,048 x 1,536 with the rotation, 9 tokens: 3.3 us, 4.1 with the loop).
+template <int TT, bool ROPE, bool GATED, int AHEAD, bool STAYS>
 __global__ void __launch_bounds__(32 * SK_WARPS, AHEAD == SK_AHEAD ? 2 : 1)       // two blocks per SM: 64 registers at most
 gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     extern __shared__ __align__(16) unsigned char sk_ring[];
     constexpr int RED = SK_WARPS * SK_ROWS * 8 * TT;              // [warp][16 rows][8 * TT]
-    __shared__ float reds[ROPE ? 1 : 2][RED];                     // a tile's, while the tile before is still added up
+    __shared__ float reds[STAYS ? 2 : 1][RED];                    // a tile's, while the tile before is still added up
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int chunks = p.K / SK_CHUNK;
@@ -83,8 +83,8 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     int row0, row8;
     auto rows_of = [&](int tile) {
         if (ROPE) {
-            const int per_head = rope.head_dim / 16;              // blocks per head
-            const int head = tile / per_head, d0 = (tile - head * per_head) * 8;
+            const unsigned per_head = rope.head_dim / 16;         // blocks per head
+            const unsigned head = (unsigned)tile / per_head, d0 = ((unsigned)tile - head * per_head) * 8;
             row0 = head * rope.head_dim + d0;
             row8 = row0 + rope.head_dim / 2;
         } else {
@@ -94,30 +94,35 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     };
     unsigned char* mine = sk_ring + (size_t)warp * AHEAD * 1024 + lane * 16;        // slot s: + s * 1024; second row: + 512
 
-    // the next chunk to ask for: of which tile, which chunk, this lane's two rows there
-    int ask_tile = blockIdx.x, ask_c = warp;
-    const bf16 *w_lo, *w_hi;
-    auto ask_rows = [&]() {
-        rows_of(ask_tile);
+    const bf16 *w_lo, *w_hi;                                      // this lane's two rows of the tile asked for
+    auto ask_rows = [&](int tile) {
+        rows_of(tile);
         w_lo = p.w + (size_t)min(row0 + g, p.N - 1) * p.K + 8 * t;
         w_hi = p.w + (size_t)min(row8 + g, (GATED ? 2 : 1) * p.N - 1) * p.K + 8 * t;
     };
-    ask_rows();
-    auto ask = [&](int slot) {                                    // this lane's 32 bytes of it
-        if (ask_c < chunks) {
-            cp_async_16(mine + slot * 1024, w_lo + ask_c * SK_CHUNK);
-            cp_async_16(mine + slot * 1024 + 512, w_hi + ask_c * SK_CHUNK);
-            ask_c += SK_WARPS;
-            if (!ROPE && ask_c >= chunks && ask_tile + (int)gridDim.x < tiles) {
-                ask_tile += gridDim.x;
-                ask_c = warp;
-                ask_rows();
-            }
+    ask_rows(blockIdx.x);
+    auto ask = [&](int slot, int c) {                             // this lane's 32 bytes of chunk c
+        if (c < chunks) {
+            cp_async_16(mine + slot * 1024, w_lo + c * SK_CHUNK);
+            cp_async_16(mine + slot * 1024 + 512, w_hi + c * SK_CHUNK);
         }
         cp_async_commit();                                        // one group per slot, also when empty
     };
+    int ask_tile = blockIdx.x, ask_c = warp;                      // STAYS: the next chunk to ask for, on into the block's next tile
+    auto ask_next = [&](int slot) {
+        const int c = ask_c;
+        ask(slot, c);
+        if (c < chunks && (ask_c += SK_WARPS) >= chunks && ask_tile + (int)gridDim.x < tiles) {
+            ask_tile += gridDim.x;
+            ask_c = warp;
+            ask_rows(ask_tile);
+        }
+    };
 #pragma unroll
-    for (int j = 0; j < AHEAD; ++j) ask(j);                       // weights do not depend on the kernel before
+    for (int j = 0; j < AHEAD; ++j) {                             // weights do not depend on the kernel before
+        if (STAYS) ask_next(j);
+        else ask(j, warp + j * SK_WARPS);
+    }
     // Nor does what the epilogue's rotation needs: the token's position and slot were staged before
     // the step, the table and the bias are constants.  A thread of the epilogue owns one rotation
     // pair of one token (the block has more threads than such pairs) and fetches its angle now.
@@ -126,7 +131,6 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     int early_pos = 0, early_slot = -1;
     float early_cos = 1.f, early_sin = 0.f, early_bias_lo = 0.f, early_bias_hi = 0.f;
     if (ROPE) {
-        rows_of(blockIdx.x);
         const int token = threadIdx.x >> 3, r = threadIdx.x & 7;
         if (threadIdx.x < 8 * TP && token < p.T) {
             const int per_head = rope.head_dim / 16;
@@ -162,14 +166,14 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 b[j][n] = (c < chunks && x_of[n]) ? *reinterpret_cast<const uint4*>(x_of[n] + c * SK_CHUNK) : make_uint4(0, 0, 0, 0);
         }
     };
-    const bool x_stays = !ROPE && chunks <= X_AHEAD * SK_WARPS;
+    const bool x_stays = STAYS && chunks <= X_AHEAD * SK_WARPS;
     if (x_stays) ask_x(warp);
     int slot = 0, turn = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, turn ^= 1) {
+    for (int tile = blockIdx.x;; tile += gridDim.x, turn ^= 1) {
     float acc[TT][4];
 #pragma unroll
     for (int n = 0; n < TT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    if (GATED && p.bias && threadIdx.x < 8 * TP) {                // of the pair of outputs this thread finishes
+    if (STAYS && GATED && p.bias && threadIdx.x < 8 * TP) {       // of the pair of outputs this thread finishes
         const int n = min(tile * TILE_ROWS + (int)(threadIdx.x & 7), p.N - 1);
         early_bias_lo = __bfloat162float(p.bias[n]); early_bias_hi = __bfloat162float(p.bias[p.N + n]);
     }
@@ -177,7 +181,8 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
         if (!x_stays) ask_x(c0);
 #pragma unroll
         for (int j = 0; j < X_AHEAD; ++j) {
-            if (c0 + j * SK_WARPS >= chunks) break;
+            const int c = c0 + j * SK_WARPS;
+            if (c >= chunks) continue;
             cp_async_wait<AHEAD - 1>();                           // the oldest group - this slot - has landed
             const uint4 a_lo = *reinterpret_cast<const uint4*>(mine + slot * 1024);
             const uint4 a_hi = *reinterpret_cast<const uint4*>(mine + slot * 1024 + 512);
@@ -186,12 +191,14 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 mma_16x8x16(acc[n], a_lo.x, a_hi.x, a_lo.y, a_hi.y, b[j][n].x, b[j][n].y);
                 mma_16x8x16(acc[n], a_lo.z, a_hi.z, a_lo.w, a_hi.w, b[j][n].z, b[j][n].w);
             }
-            ask(slot);                                            // refill what has just been used
+            if (STAYS) ask_next(slot);                            // refill what has just been used
+            else ask(slot, c + SK_WARPS * AHEAD);
             slot = slot + 1 == AHEAD ? 0 : slot + 1;
         }
     }
+    if (!STAYS) cp_async_wait<0>();
     // acc[n]: rows g (0, 1) and g + 8 (2, 3), tokens 8 n + 2 t and 8 n + 2 t + 1
-    float* red = reds[ROPE ? 0 : turn];
+    float* red = reds[STAYS ? turn : 0];
 #pragma unroll
     for (int n = 0; n < TT; ++n) {
         float* part = red + ((size_t)warp * SK_ROWS) * TP + 8 * n + 2 * t;
@@ -256,7 +263,10 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 gate += red[((size_t)w * SK_ROWS + r) * TP + token];
                 up += red[((size_t)w * SK_ROWS + r + 8) * TP + token];
             }
-            if (p.bias) { gate += early_bias_lo; up += early_bias_hi; }     // (e is this thread's own pair: see above)
+            if (p.bias) {                                         // (e is this thread's own pair: see above)
+                gate += STAYS ? early_bias_lo : __bfloat162float(p.bias[n]);
+                up += STAYS ? early_bias_hi : __bfloat162float(p.bias[p.N + n]);
+            }
             gate = __bfloat162float(__float2bfloat16_rn(gate));
             up = __bfloat162float(__float2bfloat16_rn(up));
             reinterpret_cast<bf16*>(p.y)[(size_t)token * p.ldy + n] = __float2bfloat16_rn((gate / (1.0f + expf(-gate))) * up);
@@ -278,31 +288,40 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
         else reinterpret_cast<bf16*>(p.y)[(size_t)token * p.ldy + n] = __float2bfloat16_rn(sum);
     }
     }
+    if (!STAYS || tile + (int)gridDim.x >= tiles) break;
     }
-    cp_async_wait<0>();
+    if (STAYS) cp_async_wait<0>();
 }
 
-template <int TT, bool ROPE, bool GATED, int AHEAD>
+template <int TT, bool ROPE, bool GATED, int AHEAD, bool STAYS>
 static int launch_skinny_ring(const SkinnyParams& p, const SkinnyRope& rope, int blocks, cudaStream_t stream) {
     constexpr size_t smem = (size_t)SK_WARPS * AHEAD * 1024;
+    auto* kernel = gemm_skinny_kernel<TT, ROPE, GATED, AHEAD, STAYS>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TT, ROPE, GATED, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return launch_dependent(gemm_skinny_kernel<TT, ROPE, GATED, AHEAD>, dim3(blocks), dim3(32 * SK_WARPS), smem, stream, p, rope);
+    return launch_dependent(kernel, dim3(blocks), dim3(32 * SK_WARPS), smem, stream, p, rope);
 }
 
 template <int TT, bool ROPE, bool GATED = false>
 static int launch_skinny(const SkinnyParams& p, const SkinnyRope& rope, cudaStream_t stream) {
-    const int tiles = (p.N + (GATED ? SK_ROWS / 2 : SK_ROWS) - 1) / (GATED ? SK_ROWS / 2 : SK_ROWS);
+    constexpr int TILE_ROWS = GATED ? SK_ROWS / 2 : SK_ROWS;
+    const int tiles = (p.N + TILE_ROWS - 1) / TILE_ROWS;
+    int device = 0, sms = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if constexpr (!ROPE) {
-        if (tiles <= SK_SMS && p.K > SK_CHUNK * SK_WARPS * SK_AHEAD)
-            return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP>(p, rope, tiles, stream);
-        return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD>(p, rope, tiles < 2 * SK_SMS ? tiles : 2 * SK_SMS, stream);
+        if (tiles <= sms && p.K > SK_CHUNK * SK_WARPS * SK_AHEAD)
+            return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP, false>(p, rope, tiles, stream);
+        // From 12 tokens on, of rows of four to six chunks a warp, a second tile for less than half of the blocks takes longer
+        // behind the first than in a block of its own: us one each and staying, 16 tokens of 4,752 x 2,048 8.6 and 9.0, 6,400 x 2,048
+        // 9.0 and 10.0, but 5,600 x 1,088 6.8 and 6.6, 6,400 x 4,096 16.7 and 16.0, 7,104 x 2,048 11.0 and 10.3, 9 tokens of 4,752 x 2,048 7.4 and 6.6
+        const bool apart = p.T >= 12 && p.K > 1536 && p.K <= 3072 && 5 * tiles < 14 * sms;
+        if (tiles > 2 * sms && !apart) return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD, true>(p, rope, 2 * sms, stream);
     }
-    return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD>(p, rope, tiles, stream);
+    return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD, false>(p, rope, tiles, stream);
 }
 
 }  // namespace fsie
