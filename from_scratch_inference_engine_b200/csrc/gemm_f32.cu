@@ -43,8 +43,8 @@ constexpr int ROWS_MAX_WARPS = 16;
 template <int MT, int R> struct RowsShape {
     static constexpr int XC = MT >= 16 ? 512 : (MT >= 8 ? 1024 : 2048);
     static constexpr int PER_CHUNK = XC / 128;
-    // 6 to 8 KB per warp; not more passes than a chunk has, so that a chunk of x asked for at the start of
-    // the one before it has landed when its first pass has
+    // 6 to 8 KB per warp, and not more passes than a chunk has, so that a chunk of x asked for at the start of the one before
+    // it has landed when its first pass has: that leaves 4 KB of one row of w from 5 rows of x on, 2 from 9 on, and 4 of two rows from 9 on
     static constexpr int DEEP = R == 1 ? 12 : (R == 2 ? 8 : 4);
     static constexpr int DEPTH = DEEP < PER_CHUNK ? DEEP : PER_CHUNK;
     static constexpr int WARP_BYTES = DEPTH * R * 512;

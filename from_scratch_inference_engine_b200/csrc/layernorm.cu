@@ -49,7 +49,7 @@ __global__ void add_layernorm_kernel(const S* __restrict__ src, const int* __res
 
 // The same, to the bit, with the row in registers (at most PER values of a thread, all asked for at once): a step of few
 // tokens is a chain of such rows, each two sums over a block, and nothing but their trips to memory and barriers bounds it
-// (4 rows of 2,048 took 6.9 us of the step's chain, a turn through shared memory for each value, and 3.5 now); the gain, a
+// (4 rows of 2,048 took 6.9 us of the step's chain, a turn through shared memory for each value, and 3.7 now); the gain, a
 // constant, is asked for before the kernel before has finished.  A thread keeps the values that it has above, neighbours apart by
 // the block: eight neighbours of a thread would be one load, but another order of the sums.
 template <typename S, typename T, int PER>

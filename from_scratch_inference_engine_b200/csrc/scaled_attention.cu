@@ -339,7 +339,8 @@ struct MmaLayout {
 
 // A tile's query rows into shared memory as they are, zero beyond the tile: four rows and PIECES pieces of 16 bytes of each are a lane's
 // at once.  Asked for one after the other, each behind the store of the one before, a decoded token's rows of 576 values were
-// twelve trips to memory (8 tokens of 16 heads, with prompts of 400: 21.3 -> 19.2 us a launch; rows of 128 values 12.6 -> 11.5).
+// twelve trips to memory (with that and the older keys in front of the wait, 8 tokens of 16 heads with prompts of 400: 21.6 -> 18.0 us
+// of the step's chain; rows of 128 values 16 -> 12.6).
 template <int ROWS, int WARPS, int PIECES>
 __device__ __forceinline__ void sa_stage_queries(const ScaledAttnParams& p, const bf16* q, bf16* Qs, int ldk, int kvh, int group,
                                                  int qstart, int row0, int nrows, int dk, int warp, int lane) {
@@ -1530,7 +1531,7 @@ int fsie_scaled_attention(const void* q, int q_ld, const float* head_scale, cons
     }
     if (rc != 0 || nsplit == 1 || partial) return rc;
     const int threads = value_dim >= 128 ? 128 : (value_dim >= 64 ? 64 : 32);
-    // a block for every 128 columns: one that went over 512 of them was four trips to memory, one after the other (6.6 us of a
+    // a block for every 128 columns: one that went over 512 of them was four trips to memory, one after the other (7.5 us of a
     // step's chain for 8 tokens of 16 heads, 2.6 now)
     const dim3 cgrid(combine_tokens ? num_combine : tokens, heads, (value_dim + threads - 1) / threads);
     if (cgrid.x == 0) return 0;

@@ -113,7 +113,7 @@ __device__ __forceinline__ void talking_copies_done() { asm volatile("cp.async.w
 // and the mixing matrix are read before the kernel before has finished, and the second walk gets as far as its first tile's
 // scores and values then: the first walk only read the queries, keys and values.  Shared memory is laid out for the
 // tile's own rows, so that blocks of both walks fit an SM (4 requests of 1,024 keys, the three launches: 56 us, 20 now; code for
-// 64 heads where there are 16 alone cost 25 us, most of it the fetch of instructions).
+// 64 heads where there are 16 alone cost 20 us, 10 a walk, most of it the fetch of instructions).
 template <typename T, int TOK, int VC2, int KPL, int HS>
 __global__ void __launch_bounds__(TA_WARPS * 32) talking_attention_kernel(const TalkingArgs a) {
     constexpr int TK = 32 * KPL;

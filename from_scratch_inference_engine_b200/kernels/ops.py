@@ -835,7 +835,6 @@ def gemm_tiles_lib():
         pairs = lib.fsie_gemm_tiles_pairs()       # also sets the kernels up, outside any capture
         if pairs <= 0:
             raise KernelError(f"gemm_tiles: pairs of blocks cannot be launched here (code {pairs})")
-        lib.pairs = pairs
         _gemm_tiles = build.fast_calls(lib)
     return _gemm_tiles
 
