@@ -260,7 +260,7 @@ __global__ void silu_rows_kernel(const T* __restrict__ proj, int ld, int width, 
 // The same for steps of one token per request, heads of 33 to 128 rows and rows of the state on 16 bytes: every q, k and v value
 // is one thread's, asked for at once, and nothing of the segments is left in the code.  A launch is a chain that a few
 // warps per SM walk alone, so its instructions count: 4 requests of 16 heads of 128 x 128
-// took 19.9 us of a step with the activation in a launch before it, 9.3 without, 6.6 here.  Sums run in the order above: the same bits.
+// took 24.2 us of a step with the activation in a launch of its own (19.9 + 4.3), 9.3 with it in the walk above, 6.6 here.  Sums run in the order above: the same bits.
 template <int DR, typename T, bool ROWS, bool SILU>
 __global__ void __launch_bounds__(SCAN_COLS / 4 * SCAN_ROW_GROUPS)
 lightning_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off,
