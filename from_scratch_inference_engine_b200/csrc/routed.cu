@@ -907,10 +907,9 @@ static int launch_few(const void* x, long long x_ld, const void* w, void* out, l
 }
 
 // -------------------------------------------------------------------------------- combine
-// VEC: eight columns per thread, 16-byte accesses; the sums run in the same order.  AHEAD > 0: so many choices' rows travel together,
-// where one after the other, each behind its id and place, they were the launch's time for few tokens (8 of 8 choices of 4,096
-// 5.6 -> 3.2 us).  Not more than there are choices: rows asked for twice and their registers cost 2,048 tokens of one
-// choice 4.3 -> 5.6.
+// VEC: eight columns per thread, 16-byte accesses; the sums run in the same order.  AHEAD > 0: so many choices' rows travel together (a
+// last one again where there are fewer), where one after the other, each behind its id and place, they were the launch's time
+// (8 tokens of 8 choices of 4,096 5.6 -> 3.2 us).
 template <typename T, bool VEC, int AHEAD>
 __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float* __restrict__ weights,
                                    const T* __restrict__ shared, const int* __restrict__ place,
@@ -934,8 +933,7 @@ __global__ void moe_combine_kernel(const T* __restrict__ expert_out, const float
                     src[j] = own ? y + t * y_ld : expert_out + (place ? (own ? 0 : (size_t)place[at]) : at) * width;
                 }
 #pragma unroll
-                for (int j = 0; j < AHEAD; ++j)
-                    if (j0 + j < top) load8(src[j] + c, rows[j]);
+                for (int j = 0; j < AHEAD; ++j) load8(src[j] + c, rows[j]);
 #pragma unroll
                 for (int j = 0; j < AHEAD; ++j)
                     if (j0 + j < top) {
@@ -1131,10 +1129,12 @@ int fsie_moe_combine(const void* expert_out, const float* weights, const void* s
     const bool vec = width % 8 == 0 && (!ids || y_ld % 8 == 0) &&
         (((size_t)expert_out | (size_t)shared | (size_t)out | (size_t)y) & 15) == 0;
     const int threads = vec ? (width >= 2048 ? 256 : (width >= 1024 ? 128 : 64)) : (width >= 1024 ? 256 : 128);
-    // Many tokens: one choice's row after the other, by more warps at a time, except four or eight choices in the order of their
-    // tokens.  us one after the other and together, 2,048 tokens of 2,048: 4 choices 7.2 and 6.1, 8 of 4,096 39 and 28, but 5 choices 8.3
-    // and 9.6, 6 with their places looked up 7.0 and 9.8; 512 tokens: 2 choices with places 2.4 and 2.5, 5 3.1 and 4.0.
-    const int ahead = tokens > 256 && (place || top % 4) ? 0 : (top < 3 ? top : 4);
+    // Many tokens: one choice's row after the other where places are looked up, and for a medium number of them where a fourth row
+    // or more would be asked for twice.  us one after the other and together: 2,048 tokens of 2,048, 4 choices 7.3 and 6.1, 6 10.1
+    // and 9.0, with places 7.0 and 8.9; 512 tokens of 6 choices 3.9 and 4.1, of 4 3.3 and 3.0, of 2 2.7 and 2.8; 4,096 of 6 32 and 24.
+    // One choice or two have no more rows: 2,048 tokens of one choice 4.3 and 3.8, and 5.6 with four.
+    const bool in_turn = tokens > 256 && (place || (tokens <= 1024 && (top % 4 == 1 || top % 4 == 2)));
+    const int ahead = in_turn ? 0 : (top < 3 ? top : 4);
 #define FSIE_COMBINE(T, V, A) launch_dependent(moe_combine_kernel<T, V, A>, tokens, threads, 0, stream, (const T*)expert_out, \
                                             weights, (const T*)shared, place, (T*)out, width, top, ids, experts, \
                                             (const T*)y, y_ld)

@@ -6,10 +6,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# the edge of the tokens that take choices one after the other; every number of choices that travel together and remainders;
+# the edges of the tokens that take choices one after the other; every number of choices that travel together and remainders;
 # places looked up; identity experts; a shared expert
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("tokens", [1, 256, 257])
+@pytest.mark.parametrize("tokens", [1, 256, 257, 1025])
 @pytest.mark.parametrize("top", [1, 2, 3, 4, 5, 8, 9])
 def test_choices_together(tokens, top, dtype):
     from from_scratch_inference_engine_b200.kernels import ops
