@@ -135,8 +135,10 @@ int fsie_add_layernorm(const void* src, const int* rows, const float* gain, floa
     const int values = (width + threads - 1) / threads;
     // (longer rows would spill: they stay in shared memory.  So do many plain ones of five to seven values a thread: us in
     // shared memory and in registers, 2,048 rows of 2,304 14.6 and 15.9, of 3,072 16.4 and 17.6, of 1,536 8.2 and 8.4; of 2,048 values,
-    // four a thread, 10.3 and 9.4, of 4,096 24.2 and 23.7; with the sum, which reads a row more, of 2,304 17.8 and 16.6)
-    if (!general && values <= 8 && (accumulate || values < 5 || values == 8 || !many_rows(num_rows, threads))) {
+    // four a thread, 10.3 and 9.4, of 4,096 24.2 and 23.7; with the sum, which reads a row more, of 2,304 17.8 and 16.6; and of 8,192 rows
+    // of 3,072, more than L2 holds, 83 and 71)
+    const bool shared = !accumulate && values >= 5 && values <= 7 && many_rows(num_rows, threads) && (long long)num_rows * width < 16 << 20;
+    if (!general && values <= 8 && !shared) {
 #define FSIE_LN_REGS(S, T, PER)                                                                                               \
         launch_dependent_if(early, add_layernorm_regs_kernel<S, T, PER>, num_rows, threads, 0, stream, (const S*)src, rows, gain, \
                             accumulate ? x : nullptr, (T*)y, width, eps)
