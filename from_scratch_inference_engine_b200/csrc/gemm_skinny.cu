@@ -63,17 +63,18 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // GATED: w holds N gate rows and then N up rows, the block's 16 rows are 8 gate rows and the 8 up rows of the
 // same outputs, and the epilogue is silu(gate) * up on the two as bfloat16 would store them: the bits of a
 // product and the SwiGLU kernel behind it, without that launch (1 token of 8,960 x 1,536 14.0 -> 11.4 us, 16 tokens of 2,816 x 2,048 11.4 -> 8.6).
-// STAYS: a matrix of more tiles of 16 rows than the GPU holds blocks has the blocks stay and go on to their next tile: the ring runs on
+// LOOP: a matrix of more tiles of 16 rows than the GPU holds blocks has the blocks stay and go on to their next tile: the ring runs on
 // across tiles, where a block of its own for every tile of, say, 8,960 x 1,536 (three chunks per warp) was asked, waited and gone
 // (11.4 us of a token's step, 9.5 now).  With one block per SM or less the ring is twice as deep (1,536 x 8,960: 8.0 -> 6.8 us).
-// Neither changes which warp adds up what: the same bits.  A block of one tile is compiled without the loop, whose registers
-// cost 9 to 16 tokens 5 to 23 % (2,048 x 1,536 with the rotation, 9 tokens: 3.3 us, 4.1 with the loop).
-template <int TT, bool ROPE, bool GATED, int AHEAD, bool STAYS>
+// Neither changes which warp adds up what: the same bits.  The loop's registers cost blocks of one tile 5 to 23 % with 9 to 16 tokens
+// or the rotation (9 of 2,048 x 1,536 with the rotation 3.3 and 4.1 us), which are compiled without it; with up to 8 tokens the two are
+// ahead of one another by up to 10 % as the sizes go (launch_skinny).
+template <int TT, bool ROPE, bool GATED, int AHEAD, bool LOOP>
 __global__ void __launch_bounds__(32 * SK_WARPS, AHEAD == SK_AHEAD ? 2 : 1)       // two blocks per SM: 64 registers at most
 gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     extern __shared__ __align__(16) unsigned char sk_ring[];
     constexpr int RED = SK_WARPS * SK_ROWS * 8 * TT;              // [warp][16 rows][8 * TT]
-    __shared__ float reds[STAYS ? 2 : 1][RED];                    // a tile's, while the tile before is still added up
+    __shared__ float reds[LOOP ? 2 : 1][RED];                     // a tile's, while the tile before is still added up
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int chunks = p.K / SK_CHUNK;
@@ -94,34 +95,39 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
     };
     unsigned char* mine = sk_ring + (size_t)warp * AHEAD * 1024 + lane * 16;        // slot s: + s * 1024; second row: + 512
 
-    const bf16 *w_lo, *w_hi;                                      // this lane's two rows of the tile asked for
-    auto ask_rows = [&](int tile) {
-        rows_of(tile);
+    // the next chunk to ask for: of which tile, which chunk, this lane's two rows there
+    int ask_tile = blockIdx.x, ask_c = warp;
+    const bf16 *w_lo, *w_hi;
+    auto ask_rows = [&]() {
+        rows_of(ask_tile);
         w_lo = p.w + (size_t)min(row0 + g, p.N - 1) * p.K + 8 * t;
         w_hi = p.w + (size_t)min(row8 + g, (GATED ? 2 : 1) * p.N - 1) * p.K + 8 * t;
     };
-    ask_rows(blockIdx.x);
-    auto ask = [&](int slot, int c) {                             // this lane's 32 bytes of chunk c
+    ask_rows();
+    auto ask = [&](int slot) {                                    // LOOP: this lane's 32 bytes of it
+        if (ask_c < chunks) {
+            cp_async_16(mine + slot * 1024, w_lo + ask_c * SK_CHUNK);
+            cp_async_16(mine + slot * 1024 + 512, w_hi + ask_c * SK_CHUNK);
+            ask_c += SK_WARPS;
+            if (ask_c >= chunks && ask_tile + (int)gridDim.x < tiles) {
+                ask_tile += gridDim.x;
+                ask_c = warp;
+                ask_rows();
+            }
+        }
+        cp_async_commit();                                        // one group per slot, also when empty
+    };
+    auto ask_chunk = [&](int slot, int c) {                       // a tile alone: of chunk c
         if (c < chunks) {
             cp_async_16(mine + slot * 1024, w_lo + c * SK_CHUNK);
             cp_async_16(mine + slot * 1024 + 512, w_hi + c * SK_CHUNK);
         }
-        cp_async_commit();                                        // one group per slot, also when empty
-    };
-    int ask_tile = blockIdx.x, ask_c = warp;                      // STAYS: the next chunk to ask for, on into the block's next tile
-    auto ask_next = [&](int slot) {
-        const int c = ask_c;
-        ask(slot, c);
-        if (c < chunks && (ask_c += SK_WARPS) >= chunks && ask_tile + (int)gridDim.x < tiles) {
-            ask_tile += gridDim.x;
-            ask_c = warp;
-            ask_rows(ask_tile);
-        }
+        cp_async_commit();
     };
 #pragma unroll
     for (int j = 0; j < AHEAD; ++j) {                             // weights do not depend on the kernel before
-        if (STAYS) ask_next(j);
-        else ask(j, warp + j * SK_WARPS);
+        if (LOOP) ask(j);
+        else ask_chunk(j, warp + j * SK_WARPS);
     }
     // Nor does what the epilogue's rotation needs: the token's position and slot were staged before
     // the step, the table and the bias are constants.  A thread of the epilogue owns one rotation
@@ -166,14 +172,14 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 b[j][n] = (c < chunks && x_of[n]) ? *reinterpret_cast<const uint4*>(x_of[n] + c * SK_CHUNK) : make_uint4(0, 0, 0, 0);
         }
     };
-    const bool x_stays = STAYS && chunks <= X_AHEAD * SK_WARPS;
+    const bool x_stays = LOOP && chunks <= X_AHEAD * SK_WARPS;
     if (x_stays) ask_x(warp);
     int slot = 0, turn = 0;
-    for (int tile = blockIdx.x;; tile += gridDim.x, turn ^= 1) {
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, turn ^= 1) {
     float acc[TT][4];
 #pragma unroll
     for (int n = 0; n < TT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    if (STAYS && GATED && p.bias && threadIdx.x < 8 * TP) {       // of the pair of outputs this thread finishes
+    if (LOOP && GATED && p.bias && threadIdx.x < 8 * TP) {       // of the pair of outputs this thread finishes
         const int n = min(tile * TILE_ROWS + (int)(threadIdx.x & 7), p.N - 1);
         early_bias_lo = __bfloat162float(p.bias[n]); early_bias_hi = __bfloat162float(p.bias[p.N + n]);
     }
@@ -181,8 +187,8 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
         if (!x_stays) ask_x(c0);
 #pragma unroll
         for (int j = 0; j < X_AHEAD; ++j) {
-            const int c = c0 + j * SK_WARPS;
-            if (c >= chunks) continue;
+            if (LOOP && c0 + j * SK_WARPS >= chunks) break;
+            if (!LOOP && c0 + j * SK_WARPS >= chunks) continue;
             cp_async_wait<AHEAD - 1>();                           // the oldest group - this slot - has landed
             const uint4 a_lo = *reinterpret_cast<const uint4*>(mine + slot * 1024);
             const uint4 a_hi = *reinterpret_cast<const uint4*>(mine + slot * 1024 + 512);
@@ -191,14 +197,14 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 mma_16x8x16(acc[n], a_lo.x, a_hi.x, a_lo.y, a_hi.y, b[j][n].x, b[j][n].y);
                 mma_16x8x16(acc[n], a_lo.z, a_hi.z, a_lo.w, a_hi.w, b[j][n].z, b[j][n].w);
             }
-            if (STAYS) ask_next(slot);                            // refill what has just been used
-            else ask(slot, c + SK_WARPS * AHEAD);
+            if (LOOP) ask(slot);                                  // refill what has just been used
+            else ask_chunk(slot, c0 + (j + AHEAD) * SK_WARPS);
             slot = slot + 1 == AHEAD ? 0 : slot + 1;
         }
     }
-    if (!STAYS) cp_async_wait<0>();
+    if (!LOOP) cp_async_wait<0>();
     // acc[n]: rows g (0, 1) and g + 8 (2, 3), tokens 8 n + 2 t and 8 n + 2 t + 1
-    float* red = reds[STAYS ? turn : 0];
+    float* red = reds[LOOP ? turn : 0];
 #pragma unroll
     for (int n = 0; n < TT; ++n) {
         float* part = red + ((size_t)warp * SK_ROWS) * TP + 8 * n + 2 * t;
@@ -264,8 +270,8 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
                 up += red[((size_t)w * SK_ROWS + r + 8) * TP + token];
             }
             if (p.bias) {                                         // (e is this thread's own pair: see above)
-                gate += STAYS ? early_bias_lo : __bfloat162float(p.bias[n]);
-                up += STAYS ? early_bias_hi : __bfloat162float(p.bias[p.N + n]);
+                gate += LOOP ? early_bias_lo : __bfloat162float(p.bias[n]);
+                up += LOOP ? early_bias_hi : __bfloat162float(p.bias[p.N + n]);
             }
             gate = __bfloat162float(__float2bfloat16_rn(gate));
             up = __bfloat162float(__float2bfloat16_rn(up));
@@ -288,15 +294,15 @@ gemm_skinny_kernel(const SkinnyParams p, const SkinnyRope rope) {
         else reinterpret_cast<bf16*>(p.y)[(size_t)token * p.ldy + n] = __float2bfloat16_rn(sum);
     }
     }
-    if (!STAYS || tile + (int)gridDim.x >= tiles) break;
+    if (!LOOP) break;
     }
-    if (STAYS) cp_async_wait<0>();
+    if (LOOP) cp_async_wait<0>();
 }
 
-template <int TT, bool ROPE, bool GATED, int AHEAD, bool STAYS>
+template <int TT, bool ROPE, bool GATED, int AHEAD, bool LOOP>
 static int launch_skinny_ring(const SkinnyParams& p, const SkinnyRope& rope, int blocks, cudaStream_t stream) {
     constexpr size_t smem = (size_t)SK_WARPS * AHEAD * 1024;
-    auto* kernel = gemm_skinny_kernel<TT, ROPE, GATED, AHEAD, STAYS>;
+    auto* kernel = gemm_skinny_kernel<TT, ROPE, GATED, AHEAD, LOOP>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -313,13 +319,23 @@ static int launch_skinny(const SkinnyParams& p, const SkinnyRope& rope, cudaStre
     int device = 0, sms = 148;
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if constexpr (!ROPE) {
-        if (tiles <= sms && p.K > SK_CHUNK * SK_WARPS * SK_AHEAD)
-            return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP, false>(p, rope, tiles, stream);
-        // From 12 tokens on, of rows of four to six chunks a warp, a second tile for less than half of the blocks takes longer
-        // behind the first than in a block of its own: us one each and staying, 16 tokens of 4,752 x 2,048 8.6 and 9.0, 6,400 x 2,048
-        // 9.0 and 10.0, but 5,600 x 1,088 6.8 and 6.6, 6,400 x 4,096 16.7 and 16.0, 7,104 x 2,048 11.0 and 10.3, 9 tokens of 4,752 x 2,048 7.4 and 6.6
-        const bool apart = p.T >= 12 && p.K > 1536 && p.K <= 3072 && 5 * tiles < 14 * sms;
-        if (tiles > 2 * sms && !apart) return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD, true>(p, rope, 2 * sms, stream);
+        // Which of the forms is ahead turns with the chunks of k that a warp has (K / 512) and the blocks on an SM; us, a tile alone
+        // in its block and the loop.
+        //  - up to 8 tokens, one block on an SM: up to four chunks the loop (2,048 x 1,536 2.6 and 2.5), five or six a tile alone (2,048 x
+        //    2,816 3.2 and 3.6 with either ring), beyond that the loop with the deeper ring (2,048 x 4,096 4.6 and 4.4);
+        //  - up to 8 tokens, not every SM with two blocks: two to four chunks the loop (2,400 x 2,048 3.2 and 3.1), else a tile alone
+        //    (3,072 x 512 2.0 and 2.2, 2,400 x 3,072 4.1 and 4.3);
+        //  - 9 to 16 tokens: the loop where half of the SMs have two blocks, from two chunks on (16 of 4,384 x 2,048 6.4 and 6.2, but 3,072 x
+        //    2,048 5.4 and 5.6), a deeper ring for one block on an SM beyond four chunks (9 of 2,048 x 2,816 4.8 and 4.5);
+        //  - from 12 tokens on, rows of four or five chunks: a second tile for less than half of the blocks takes longer behind the
+        //    first than in a block of its own (16 of 4,752 x 2,048 8.6 and 9.0, 6,400 x 2,048 9.0 and 9.8, but 5,600 x 1,088 6.8 and 6.6,
+        //    6,400 x 3,072 13.8 and 13.0, 7,104 x 2,048 11.0 and 10.3, 9 tokens of 4,752 x 2,048 7.4 and 6.6).
+        const bool alone = tiles <= sms, crowded = 2 * tiles > 3 * sms;
+        const bool apart = p.T >= 12 && p.K > 1536 && p.K <= 2560 && tiles > 2 * sms && 5 * tiles < 14 * sms;
+        if (alone && p.K > (TT == 1 ? 3072 : 2048)) return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP, TT == 1>(p, rope, tiles, stream);
+        const bool loop = TT == 1 ? (alone ? p.K <= 2048 : crowded || (p.K >= 1024 && p.K <= 2048))
+                                  : !apart && (tiles > 2 * sms || (crowded && p.K >= 1024));
+        if (loop) return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD, true>(p, rope, tiles < 2 * sms ? tiles : 2 * sms, stream);
     }
     return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD, false>(p, rope, tiles, stream);
 }
