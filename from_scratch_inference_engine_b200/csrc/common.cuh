@@ -97,7 +97,7 @@ enum { ERR_BAD_ARGUMENT = -1, ERR_UNSUPPORTED = -2 };
 // complete when that kernel's own wait returned.  The second holds behind a kernel whose blocks all call grid_dependents_go()
 // after their wait and leave after it, as all here do but one: attn_tc_decode_kernel (attention_tcgen05.cu) lets the next kernel
 // go before it waits, so that one may still overlap the kernel in front of it.  Behind it only merges and products run, which
-// read nothing early but weights.
+// read nothing early but weights and lists.
 // Whether its operands are that old a kernel's caller knows: launch_dependent_if() with `early` = 0 launches the ordinary way.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
