@@ -327,12 +327,14 @@ static int launch_skinny(const SkinnyParams& p, const SkinnyRope& rope, cudaStre
         //    (3,072 x 512 2.0 and 2.2, 2,400 x 3,072 4.1 and 4.3);
         //  - 9 to 16 tokens: the loop where half of the SMs have two blocks, of two to five chunks (16 of 4,384 x 2,048 6.4 and 6.2, but 3,072 x
         //    2,048 5.4 and 5.6, 3,584 x 3,584 8.8 and 9.2), a deeper ring for one block on an SM beyond four chunks (9 of 2,048 x 2,816 4.8 and 4.5);
+        //    in the loop's code, alone in its block no slower, whose second buffer of sums keeps such a block off an SM that a gate / up
+        //    product still holds: beside that it took its bandwidth (12 steps of 12 tokens, 8 layers of width 2,048, 7.41 ms without, 7.31 with);
         //  - from 12 tokens on, rows of four or five chunks: a second tile for less than half of the blocks takes longer behind the
         //    first than in a block of its own (16 of 4,752 x 2,048 8.6 and 9.0, 6,400 x 2,048 9.0 and 9.8, but 5,600 x 1,088 6.8 and 6.6,
         //    6,400 x 3,072 13.8 and 13.0, 7,104 x 2,048 11.0 and 10.3, 9 tokens of 4,752 x 2,048 7.4 and 6.6).
         const bool alone = tiles <= sms, crowded = 2 * tiles > 3 * sms;
         const bool apart = p.T >= 12 && p.K > 1536 && p.K <= 2560 && tiles > 2 * sms && 5 * tiles < 14 * sms;
-        if (alone && p.K > (TT == 1 ? 3072 : 2048)) return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP, TT == 1>(p, rope, tiles, stream);
+        if (alone && p.K > (TT == 1 ? 3072 : 2048)) return launch_skinny_ring<TT, ROPE, GATED, SK_DEEP, true>(p, rope, tiles, stream);
         const bool loop = TT == 1 ? (alone ? p.K <= 2048 : crowded || (p.K >= 1024 && p.K <= 2048))
                                   : !apart && (tiles > 2 * sms || (crowded && p.K >= 1024 && p.K <= 2560));
         if (loop) return launch_skinny_ring<TT, ROPE, GATED, SK_AHEAD, true>(p, rope, tiles < 2 * sms ? tiles : 2 * sms, stream);
